@@ -21,7 +21,7 @@ cudaError_t launch_sigmoid_mul(const SigmoidParams& p, uint32_t n_cols, cudaStre
 cudaError_t launch_angles(const AnglesParams& p, cudaStream_t st);
 bool rope_vec_applies(const RopeParams& p, uint32_t n_cols);
 cudaError_t launch_epoch_bump(unsigned int* ctr, cudaStream_t st);
-cudaError_t launch_head_norm(const HeadNormParams& p, uint32_t n_cols, uint32_t n_heads, cudaStream_t st);
+cudaError_t launch_head_norm(const HeadNormParams& p, cudaStream_t st);
 int prefill_supported(const pa_ctx* ctx);
 cudaError_t launch_prefill(const pa_layer* L, const PrefillParams& p, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_q,
                            const CUtensorMap& tm_o, const CUtensorMap& tm_q2, cudaStream_t st);
@@ -952,7 +952,8 @@ extern "C" int pa_head_norm(pa_ctx* ctx, const void* x, uint64_t col_stride, uin
   HeadNormParams p{};
   p.x = x; p.x_col_stride = col_stride; p.x_head_stride = head_stride; p.y = y; p.y_col_stride = y_col_stride; p.y_head_stride = y_head_stride;
   p.w = w; p.eps = eps; p.hd = ctx->cfg.head_dim; p.f16 = ctx->cfg.act_dtype == PA_F16; p.n_first = n_heads_x;
-  CU_TRY(ctx, launch_head_norm(p, n_cols, n_heads_x, (cudaStream_t)stream));
+  p.n_cols = n_cols; p.n_heads = n_heads_x;
+  CU_TRY(ctx, launch_head_norm(p, (cudaStream_t)stream));
   ctx->stats.kernel_launches++;
   return PA_OK;
 }
@@ -1000,7 +1001,8 @@ static int layer_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, 
     hp.x2 = k; hp.x2_col_stride = kvcs; hp.x2_head_stride = ctx->cfg.head_dim; hp.y2 = ctx->norm_k; hp.y2_col_stride = ctx->kv_dim;
     hp.y2_head_stride = ctx->cfg.head_dim; hp.w2 = L->knorm_w;
     hp.eps = L->norm_eps; hp.hd = ctx->cfg.head_dim; hp.f16 = ctx->cfg.act_dtype == PA_F16;
-    CU_TRY(ctx, launch_head_norm(hp, n_cols, ctx->cfg.n_heads + ctx->cfg.n_kv_heads, st));
+    hp.n_cols = n_cols; hp.n_heads = ctx->cfg.n_heads + ctx->cfg.n_kv_heads;
+    CU_TRY(ctx, launch_head_norm(hp, st));
     ctx->stats.kernel_launches++;
     q = ctx->norm_q; qcs = ctx->q_dim; qhs = ctx->cfg.head_dim;
     k = ctx->norm_k; kcs = ctx->kv_dim;
@@ -1401,7 +1403,8 @@ extern "C" int pa_attn_items(pa_layer* L, const pa_item* items, uint32_t n_items
     hp.x2 = k; hp.x2_col_stride = kv_col_stride; hp.x2_head_stride = ctx->cfg.head_dim; hp.y2 = ctx->norm_k; hp.y2_col_stride = ctx->kv_dim;
     hp.y2_head_stride = ctx->cfg.head_dim; hp.w2 = L->knorm_w;
     hp.eps = L->norm_eps; hp.hd = ctx->cfg.head_dim; hp.f16 = ctx->cfg.act_dtype == PA_F16;
-    CU_TRY(ctx, launch_head_norm(hp, n_items, ctx->cfg.n_heads + ctx->cfg.n_kv_heads, st));
+    hp.n_cols = n_items; hp.n_heads = ctx->cfg.n_heads + ctx->cfg.n_kv_heads;
+    CU_TRY(ctx, launch_head_norm(hp, st));
     ctx->stats.kernel_launches++;
     q = ctx->norm_q; qcs = ctx->q_dim; qhs = ctx->cfg.head_dim;
     k = ctx->norm_k; kcs = ctx->kv_dim;

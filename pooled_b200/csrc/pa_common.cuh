@@ -169,6 +169,39 @@ __device__ __forceinline__ float rot_exact(float x, float y, const Angle& g, boo
   return (float)(minus ? __dsub_rn(a, b) : __dadd_rn(a, b));
 }
 
+__device__ __forceinline__ float ld_act(const void* p, uint64_t i, int f16) {
+  return f16 ? __half2float(reinterpret_cast<const __half*>(p)[i]) : reinterpret_cast<const float*>(p)[i];
+}
+
+// QK head-norm: out = f32((x * inv) * w), inv = 1 / sqrt(ss / hd + eps), with ss the float64 sum of the squares of a
+// head's values IN INDEX ORDER -- the order is part of the result.  The squares of f32 values are exact in float64, so
+// two orders differ by their additions' roundings only: at most hd * 2^-53 of ss each way for the in-order sum (hd at
+// most 512) and 2^-48 for a sum by lanes and shuffles, together below 2^-43.9.  The square root halves that, and the ten
+// roundings of the two evaluations add 2^-49: the two float64 results lie within 2^-44.8 of each other, and if f32
+// rounds everything within 2^-44 of one to the same number, the other order gives that number too.  head_norm_value
+// evaluates one output from a sum in any order and clears `ok` where that does not hold (one output in 2^19, and NaN);
+// the caller then repeats the sum in order.
+__device__ __forceinline__ double head_norm_inv(double ss, uint32_t hd, double eps) {
+  return __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__ddiv_rn(ss, (double)hd), eps)));
+}
+__device__ __forceinline__ float head_norm_value(float x, double inv, float w, bool& ok) {
+  const double r = __dmul_rn(__dmul_rn((double)x, inv), (double)w);
+  const float a = (float)__dmul_rn(r, 1.0 - 5.6843418860808015e-14), b = (float)__dmul_rn(r, 1.0 + 5.6843418860808015e-14);   // 2^-44
+  ok = ok && a == b;
+  return a;
+}
+static __device__ __noinline__ double head_norm_sum_in_order(const void* x, uint64_t off, uint32_t hd, int f16) {
+  double ss = 0.0;
+  for (uint32_t i = 0; i < hd; i += 16) {
+    float v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = ld_act(x, off + i + k, f16);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) ss = __dadd_rn(ss, __dmul_rn((double)v[k], (double)v[k]));
+  }
+  return ss;
+}
+
 // hi + lo f16 pair of an f32: x ~= hi + lo with about 22 significant bits
 __device__ __forceinline__ void split_h(float x, __half& hi, __half& lo) {
   hi = __float2half_rn(x);

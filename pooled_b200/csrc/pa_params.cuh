@@ -96,7 +96,8 @@ struct HeadNormParams {
   const void* x; uint64_t x_col_stride, x_head_stride;
   void* y; uint64_t y_col_stride, y_head_stride;
   const float* w;          // [hd]
-  // heads at or past n_first (blockIdx.y) belong to a second array with its own weight: q and k of a layer in one launch
+  uint32_t n_cols, n_heads;   // columns; heads of both arrays
+  // heads at or past n_first belong to a second array with its own weight: q and k of a layer in one launch
   uint32_t n_first;
   const void* x2; uint64_t x2_col_stride, x2_head_stride;
   void* y2; uint64_t y2_col_stride, y2_head_stride;

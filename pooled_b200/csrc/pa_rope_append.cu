@@ -16,10 +16,6 @@
 
 namespace pa {
 
-__device__ __forceinline__ float ld_act(const void* p, uint64_t i, int f16) {
-  return f16 ? __half2float(reinterpret_cast<const __half*>(p)[i]) : reinterpret_cast<const float*>(p)[i];
-}
-
 // f32 -> f16 round to nearest even with subnormals and overflow to inf (cvt.rn.f16.f32); NaN becomes the quiet
 // pattern sign | 0x7e00 that pooled's f16_rne produces (engine/wgsl/f16.js:22), not the hardware's 0x7fff
 __device__ __forceinline__ __half f16_rne(float x) {
@@ -315,36 +311,57 @@ __global__ void __launch_bounds__(128) pa_angles_kernel(const AnglesParams p) {
   p.out[i] = make_angle(c, s);
 }
 
-// QK head-norm (the step before RoPE in attn_glue, engine/wgsl/qwen35.js:1112-1122), with the arithmetic of the CPU
-// reference (tests/reference/ref_q38.mjs:50-57): the sum of squares is accumulated in float64 in index order by one
-// thread -- that order is part of the result -- then out = f32((x * inv) * w) with inv = 1 / sqrt(ss / hd + eps).
-// grid (columns, heads), 64 threads.
-__global__ void __launch_bounds__(64) pa_head_norm_kernel(const HeadNormParams p) {
-  __shared__ float s_x[512];
-  __shared__ double s_inv;
-  const uint32_t col = blockIdx.x, hd = p.hd;
-  const bool second = blockIdx.y >= p.n_first;
-  const uint32_t head = second ? blockIdx.y - p.n_first : blockIdx.y;
+// QK head-norm (the step before RoPE in attn_glue, engine/wgsl/qwen35.js:1112-1122), with the bits of the CPU reference
+// (tests/reference/ref_q38.mjs:50-57): out = f32((x * inv) * w), inv = 1 / sqrt(ss / hd + eps), ss the float64 sum of the
+// squares in index order.  A warp per (column, head), four warps per CTA; a lane holds hd / 32 values.  The squares are
+// summed in parallel and head_norm_value() says for each output whether the order of the sum could show in it; only
+// then (about one head in 2^12) the warp repeats the sum in index order.  What bounds it is latency: the in-order sum
+// alone is 256 dependent float64 additions, and one thread per head made them (eight layers of 203 columns of 24 + 4 heads, whole calls:
+// 1695 us so, 1640 us with the parallel sum).
+// grid (ceil(columns * heads / 4)).
+__global__ void __launch_bounds__(128) pa_head_norm_kernel(const HeadNormParams p) {
+  const uint32_t hd = p.hd, lane = threadIdx.x & 31, unit = blockIdx.x * 4 + (threadIdx.x >> 5);
+  pdl_wait();
+  pdl_trigger();
+  if (unit >= p.n_cols * p.n_heads) return;
+  const uint32_t col = unit / p.n_heads, slot = unit % p.n_heads;
+  const bool second = slot >= p.n_first;
+  const uint32_t head = second ? slot - p.n_first : slot;
   const void* x = second ? p.x2 : p.x;
   void* y = second ? p.y2 : p.y;
   const float* w = second ? p.w2 : p.w;
-  pdl_wait();
-  pdl_trigger();
   const uint64_t xo = (uint64_t)col * (second ? p.x2_col_stride : p.x_col_stride) + (uint64_t)head * (second ? p.x2_head_stride : p.x_head_stride);
-  for (uint32_t i = threadIdx.x; i < hd; i += blockDim.x) s_x[i] = ld_act(x, xo + i, p.f16);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double ss = 0.0;
-    for (uint32_t i = 0; i < hd; ++i) { const double v = (double)s_x[i]; ss = __dadd_rn(ss, __dmul_rn(v, v)); }
-    s_inv = __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__ddiv_rn(ss, (double)hd), p.eps)));
-  }
-  __syncthreads();
-  const double inv = s_inv;
   const uint64_t yo = (uint64_t)col * (second ? p.y2_col_stride : p.y_col_stride) + (uint64_t)head * (second ? p.y2_head_stride : p.y_head_stride);
-  for (uint32_t i = threadIdx.x; i < hd; i += blockDim.x) {
-    const float r = (float)__dmul_rn(__dmul_rn((double)s_x[i], inv), (double)w[i]);
-    if (p.f16) reinterpret_cast<__half*>(y)[yo + i] = __float2half_rn(r);
-    else reinterpret_cast<float*>(y)[yo + i] = r;
+  constexpr int MAXV = 16;   // head_dim up to 512
+  float xv[MAXV], wv[MAXV];
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) {
+    const uint32_t d = lane + 32 * i;
+    xv[i] = d < hd ? ld_act(x, xo + d, p.f16) : 0.f;
+    wv[i] = d < hd ? w[d] : 0.f;
+  }
+  double ss = 0.0;
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) if (32u * i < hd) ss = __fma_rn((double)xv[i], (double)xv[i], ss);   // a product of two f32 is exact in float64
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss = __dadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, o));
+  double inv = head_norm_inv(ss, hd, p.eps);
+  bool ok = true;
+  float r[MAXV];
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) if (lane + 32u * i < hd) r[i] = head_norm_value(xv[i], inv, wv[i], ok);
+  if (!__all_sync(0xffffffffu, ok)) {
+    inv = head_norm_inv(head_norm_sum_in_order(x, xo, hd, p.f16), hd, p.eps);
+#pragma unroll
+    for (int i = 0; i < MAXV; ++i) r[i] = (float)__dmul_rn(__dmul_rn((double)xv[i], inv), (double)wv[i]);
+  }
+  __syncwarp();   // in place: every lane of the warp has read its values, and the in-order sum its row
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) {
+    const uint32_t d = lane + 32 * i;
+    if (d >= hd) continue;
+    if (p.f16) reinterpret_cast<__half*>(y)[yo + d] = __float2half_rn(r[i]);
+    else reinterpret_cast<float*>(y)[yo + d] = r[i];
   }
 }
 
@@ -377,8 +394,8 @@ cudaError_t launch_rope_append(const RopeParams& p, uint32_t n_cols, cudaStream_
 cudaError_t launch_angles(const AnglesParams& p, cudaStream_t st) {
   return launch_pdl(pa_angles_kernel, dim3((p.n_cols * p.half + 127) / 128), dim3(128), 0, st, p);
 }
-cudaError_t launch_head_norm(const HeadNormParams& p, uint32_t n_cols, uint32_t n_heads, cudaStream_t st) {
-  return launch_pdl(pa_head_norm_kernel, dim3(n_cols, n_heads), dim3(64), 0, st, p);
+cudaError_t launch_head_norm(const HeadNormParams& p, cudaStream_t st) {
+  return launch_pdl(pa_head_norm_kernel, dim3((uint32_t)(((uint64_t)p.n_cols * p.n_heads + 3) / 4)), dim3(128), 0, st, p);
 }
 cudaError_t launch_sigmoid_mul(const SigmoidParams& p, uint32_t n_cols, cudaStream_t st) {
   pa_sigmoid_mul_kernel<<<n_cols, 256, 0, st>>>(p);

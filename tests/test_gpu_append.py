@@ -235,6 +235,25 @@ def test_head_norm_matches_the_reference_arithmetic_bit_for_bit(hd, heads, n_col
     assert torch.equal(dx[:, :heads * hs].view(n_cols, heads, hs)[:, :, :hd], out[:, :heads * hs].view(n_cols, heads, hs)[:, :, :hd])
 
 
+@pytest.mark.parametrize("hd,heads,n_cols,tie", [(64, 4, 700, False), (128, 6, 301, False), (256, 2, 2500, False), (64, 3, 1, True), (128, 2, 3, True), (256, 6, 5, True)])
+def test_head_norm_keeps_the_bits_of_the_in_order_sum(hd, heads, n_cols, tie):
+    # the kernel sums in parallel and repeats the sum in order where an output lies at a rounding boundary of f32: many
+    # random heads (a few of which do), and heads whose inv is exactly 1 and whose outputs 3 * w are exact ties
+    import torch
+    eng = _engine(n_heads=heads, n_kv_heads=1, head_dim=hd, n_rot=64, act_dtype=torch.float32)
+    rng = np.random.default_rng(17)
+    if tie:
+        x = np.tile(np.array([3.0] + [1.0] * 7 + [0.0] * 8, np.float32), (n_cols, heads * hd // 16))    # mean square 1 in every 16
+        x *= np.where(rng.random(x.shape) < 0.5, -1, 1).astype(np.float32)
+    else:
+        x = (rng.standard_normal((n_cols, heads * hd)) * 3).astype(np.float32)
+    w = (1 + 0.1 * rng.standard_normal(hd)).astype(np.float32)
+    eps = 0.0 if tie else 1e-6
+    got = eng.head_norm(util.torch_dev(x), heads, util.torch_dev(w), eps).cpu().numpy()
+    want = np.stack([po.head_norm_f64(x[c], heads, hd, w, eps) for c in range(n_cols)]).reshape(n_cols, -1)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
 def test_rope_append_items_equals_per_sequence_calls():
     # one token of each of 8 sequences at different positions in one launch == 8 pa_rope_append calls, bit for bit; with a
     # shard origin set, items outside the shard are rotated but not appended
