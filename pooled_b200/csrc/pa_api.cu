@@ -635,7 +635,10 @@ static int build_items(pa_layer* L, const pa_item* items, uint32_t n_items, Item
 
 // the tokens' unrotated k / v rows for the fused front of the decode kernel: one item at `pos` (cos / sin from the
 // host), or one token of each of several items (kv_stride elements between their rows; cos / sin on the device)
-struct FusedFront { const void* k; const void* v; uint32_t append_mask; uint32_t pos; uint64_t k_stride = 0, v_stride = 0; bool device_angles = false; };
+struct FusedFront {
+  const void* k; const void* v; uint32_t append_mask; uint32_t pos; uint64_t k_stride = 0, v_stride = 0; bool device_angles = false;
+  const pa_layer* norm = nullptr;   // the layer whose QK head-norm q and k still need (nullptr: none, or done already)
+};
 
 // a gathered call: the columns' row lists on the device, one list of `stride` words per column
 struct GatherLists { const uint32_t* lists; uint32_t stride; };
@@ -741,6 +744,7 @@ static int decode_impl(pa_layer* L, const pa_item* items, uint32_t n_items, cons
     p.fused = fz->device_angles ? 2u : 1u; p.append = fz->append_mask; p.k_new = fz->k; p.v_new = fz->v;
     p.k_new_stride = fz->k_stride; p.v_new_stride = fz->v_stride; p.inv_freq = ctx->inv_freq;
     p.k_cache = L->k; p.v_cache = L->v;
+    if (fz->norm) { p.qn_w = fz->norm->qnorm_w; p.kn_w = fz->norm->knorm_w; p.norm_eps = fz->norm->norm_eps; }
     if (!fz->device_angles) memcpy(p.rope_ang, host_angles(ctx, fz->pos, 1), (size_t)(ctx->cfg.n_rot / 2) * sizeof(Angle));
   }
   CUtensorMap tm_k, tm_v;
@@ -976,6 +980,8 @@ extern "C" int pa_sigmoid_mul(pa_ctx* ctx, void* a, uint64_t a_col_stride, const
 // One token of a model with head_dim 256 and 64 rotary dims, or head_dim 128 rotated in full (at most 8 heads per kv
 // head): the rotation of q and k and the append ride inside the decode kernel (attn_glue_kv folded into attn_dec, in
 // the reference's terms).
+// The head-norm of the layer rides along too (norm: its weights are read two floats at a time).
+static bool can_fuse_norm(const pa_layer* L) { return !((uintptr_t)L->qnorm_w & 7) && !((uintptr_t)L->knorm_w & 7); }
 static bool can_fuse_front(const pa_ctx* ctx, uint32_t n_cols, const void* q, uint64_t qcs, uint64_t qhs, const void* k, const void* v) {
   const uint32_t nr = ctx->cfg.n_rot, hd = ctx->cfg.head_dim;
   return !ctx->core_only && n_cols == 1 && ctx->cfg.rope_mode == PA_ROPE_F64 && ((hd == 256 && nr == 64) || (hd == 128 && nr == 128)) && ctx->G <= 8 &&
@@ -993,7 +999,10 @@ static int layer_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, 
   // call then reads (head_norm precedes RoPE in attn_glue, engine/wgsl/qwen35.js:1112-1131).  The gate keeps pointing
   // into the caller's q_full.
   uint64_t kcs = kvcs;   // k's column stride (v keeps the caller's)
-  if (L->qnorm_w && !ctx->core_only) {
+  // One token on the fused front normalises q and k in the decode kernel instead.
+  const bool norm_in_front = L->qnorm_w && L->kv_format == PA_KV_F16 && (sharded || mode != PA_MODE_PREFILL) && can_fuse_norm(L) &&
+                             can_fuse_front(ctx, n_cols, q, qcs, qhs, k, v);
+  if (L->qnorm_w && !ctx->core_only && !norm_in_front) {
     if (n_cols > ctx->cfg.max_cols) return fail(ctx, PA_EINVAL, "pa_attn_layer: %u columns exceed max_cols %u", n_cols, ctx->cfg.max_cols);
     HeadNormParams hp{};
     hp.x = q; hp.x_col_stride = qcs; hp.x_head_stride = qhs; hp.y = ctx->norm_q; hp.y_col_stride = ctx->q_dim; hp.y_head_stride = ctx->cfg.head_dim;
@@ -1026,6 +1035,7 @@ static int layer_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, 
     const bool owns = pos >= L->origin && (uint64_t)pos + n_cols <= (uint64_t)L->origin + L->max_seq;
     if (can_fuse_front(ctx, n_cols, q, qcs, qhs, k, v)) {
       FusedFront fz{k, v, owns ? 1u : 0u, pos};
+      if (norm_in_front) fz.norm = L;
       pa_item it{seq, pos, 1, 0};
       return decode_impl(L, &it, 1, q, (int)ctx->cfg.act_dtype, qcs, qhs, gate, gcs, ghs, out, ocs, nullptr, st, "pa_attn_layer_sharded", true, true, &fz);
     }
@@ -1059,6 +1069,7 @@ static int layer_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, 
   const bool prefill = mode == PA_MODE_PREFILL || (mode == PA_MODE_AUTO && n_cols * ctx->G > (uint32_t)kMaxRows);
   if (!prefill && can_fuse_front(ctx, n_cols, q, qcs, qhs, k, v)) {
     FusedFront fz{k, v, 1u, pos};
+    if (norm_in_front) fz.norm = L;
     pa_item it{seq, pos, 1, 0};
     return decode_impl(L, &it, 1, q, (int)ctx->cfg.act_dtype, qcs, qhs, gate, gcs, ghs, out, ocs, nullptr, st, "pa_attn_layer", true, false, &fz);
   }
@@ -1396,7 +1407,8 @@ extern "C" int pa_attn_items(pa_layer* L, const pa_item* items, uint32_t n_items
   }
   cudaSetDevice(ctx->device);
   uint64_t qcs = q_col_stride, qhs = q_head_stride, kcs = kv_col_stride;
-  if (L->qnorm_w && !ctx->core_only) {   // QK head-norm first, item i as column i (as pa_attn_layer does for its columns)
+  const bool norm_in_front = L->qnorm_w && !(kv_col_stride & 1) && can_fuse_norm(L) && can_fuse_front(ctx, 1, q, qcs, qhs, k, v);
+  if (L->qnorm_w && !ctx->core_only && !norm_in_front) {   // QK head-norm first, item i as column i (as pa_attn_layer does for its columns)
     HeadNormParams hp{};
     hp.x = q; hp.x_col_stride = qcs; hp.x_head_stride = qhs; hp.y = ctx->norm_q; hp.y_col_stride = ctx->q_dim; hp.y_head_stride = ctx->cfg.head_dim;
     hp.w = L->qnorm_w; hp.n_first = ctx->cfg.n_heads;
@@ -1412,6 +1424,7 @@ extern "C" int pa_attn_items(pa_layer* L, const pa_item* items, uint32_t n_items
   if (can_fuse_front(ctx, 1, q, qcs, qhs, k, v) && !(kcs & 1) && !(kv_col_stride & 1)) {
     // one item: cos / sin from the host's libm, as pa_attn_layer; several: each CTA evaluates its own item's
     FusedFront fz{k, v, mask, items[0].pos, kcs, kv_col_stride, n_items > 1};
+    if (norm_in_front) fz.norm = L;
     return decode_impl(L, items, n_items, q, (int)ctx->cfg.act_dtype, qcs, qhs, gate, gate_col_stride, gate_head_stride, out, out_col_stride, nullptr, st,
                        "pa_attn_items", true, exchange != 0, &fz);
   }

@@ -264,7 +264,9 @@ struct DecSmem {
 
 static_assert(sizeof(DecodeParams) + 4 * sizeof(CUtensorMap) <= 4096, "the decode kernel's launch parameters must fit 4 KB");
 
-template <int HD, int NT, bool PRECISE>
+// NORM: the fused front normalises q and k first (an instantiation of its own: as a run-time branch it cost the calls
+// without a head-norm 1 %)
+template <int HD, int NT, bool PRECISE, bool NORM = false>
 __global__ void __launch_bounds__(DecSmem<HD, NT, PRECISE>::THREADS, 1)
 pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_kn,
                  const __grid_constant__ CUtensorMap tm_vn, const DecodeParams p) {
@@ -390,6 +392,8 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
   constexpr int RHALF = NRD / 2, IPR = RHALF / 2;     // partner distance; items per row
   constexpr int RIT = CAN_FUSE ? ROWS * IPR / kConsumers : 1;   // rotated items per thread (1 or 2)
   constexpr int PPR = (HD - NRD) / 2;                 // unrotated pairs per row (96 or 0)
+  // the unrotated pairs of a row stay with the 16 threads that rotate it, so that a row's head-norm is theirs alone
+  auto plain_dim = [&](int it) { return NRD + 2 * (tid % IPR + IPR * (it - 2 * RIT)); };
   const bool fused = CAN_FUSE && p.fused;
   const bool own_new = fused && ((p.append >> item) & 1u) && tile1 == tiles;
   float2 kx = make_float2(0.f, 0.f), vx = make_float2(0.f, 0.f), kxb = make_float2(0.f, 0.f);
@@ -435,7 +439,7 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         for (int u = 0; u < RIT; ++u) { const int i = tid + u * kConsumers; q_pref_rd(i / IPR, 2 * (i % IPR)); }
         if (PPR > 0) {
 #pragma unroll
-          for (int it = 2 * RIT; it < (Q_IN_REGS ? QLD : 1); it += 2) { const int idx = tid + (it - 2 * RIT) * kConsumers; q_pref_rd(idx / (PPR ? PPR : 1), NRD + 2 * (idx % (PPR ? PPR : 1))); }
+          for (int it = 2 * RIT; it < (Q_IN_REGS ? QLD : 1); it += 2) q_pref_rd(tid / IPR, plain_dim(it));
         }
       } else {
 #pragma unroll
@@ -453,10 +457,7 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
           qreg[(2 * u + 1) % (Q_IN_REGS ? QLD : 1)] = q_load_rd(i / IPR, 2 * (i % IPR) + RHALF);
         }
 #pragma unroll
-        for (int it = 2 * RIT; it < (Q_IN_REGS ? QLD : 1); ++it) {
-          const int idx = tid + (it - 2 * RIT) * kConsumers;
-          qreg[it] = q_load_rd(idx / (PPR ? PPR : 1), NRD + 2 * (idx % (PPR ? PPR : 1)));
-        }
+        for (int it = 2 * RIT; it < (Q_IN_REGS ? QLD : 1); ++it) qreg[it] = q_load_rd(tid / IPR, plain_dim(it));
       } else {
 #pragma unroll
         for (int it = 0; it < (Q_IN_REGS ? QLD : 1); ++it) qreg[it] = q_load(tid + it * kConsumers);
@@ -621,6 +622,61 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
   if (Q_IN_REGS && grp == 0) {
     if (own_new) { kx = act_cvt(kx); vx = act_cvt(vx); kxb = act_cvt(kxb); }
     if (fused) {
+      // QK head-norm: a row's 16 (head_dim 128: 32) threads hold all of it, so its sum of squares is a few shuffles.  As
+      // a kernel of its own ahead of this one the norm cost a launch, its drain and a round trip through memory.
+      constexpr int QNP = CAN_FUSE && PPR > 0 ? QLD - 2 * RIT : 1;
+      constexpr bool normed = NORM;
+      float2 qa[RIT], qb[RIT], qn[QNP];
+      if constexpr (NORM) {
+        auto sq = [](double ss, float2 x) { return __fma_rn((double)x.y, (double)x.y, __fma_rn((double)x.x, (double)x.x, ss)); };
+        auto norm2 = [&](float2 x, const float* wp, double inv, const void* src, uint64_t off) {
+          const float2 w2 = *reinterpret_cast<const float2*>(wp);
+          bool ok = true;
+          float2 o;
+          o.x = head_norm_value(x.x, inv, w2.x, ok); o.y = head_norm_value(x.y, inv, w2.y, ok);
+          if (!ok) {   // the order of the sum could show in these two outputs
+            const double iv = head_norm_inv(head_norm_sum_in_order(src, off, HD, p.q_f16), HD, p.norm_eps);
+            o.x = (float)__dmul_rn(__dmul_rn((double)x.x, iv), (double)w2.x); o.y = (float)__dmul_rn(__dmul_rn((double)x.y, iv), (double)w2.y);
+          }
+          if (p.q_f16) { o.x = __half2float(__float2half_rn(o.x)); o.y = __half2float(__float2half_rn(o.y)); }   // the layer's activations are f16
+          return o;
+        };
+#pragma unroll
+        for (int u = 0; u < RIT; ++u) {
+          const int i = tid + u * kConsumers, row = i / IPR, b2 = 2 * (i % IPR);
+          const uint64_t off = (uint64_t)p.items.col0[item] * p.q_col_stride + (uint64_t)(g * G + row) * p.q_head_stride;
+          qa[u] = act_cvt(qreg[(2 * u) % (Q_IN_REGS ? QLD : 1)]); qb[u] = act_cvt(qreg[(2 * u + 1) % (Q_IN_REGS ? QLD : 1)]);
+          double ss = sq(sq(0.0, qa[u]), qb[u]);
+          if (PPR > 0) {
+#pragma unroll
+            for (int k = 0; k < QNP; ++k) { qn[k] = act_cvt(qreg[(2 * RIT + k) % (Q_IN_REGS ? QLD : 1)]); ss = sq(ss, qn[k]); }
+          }
+#pragma unroll
+          for (int o = IPR / 2; o > 0; o >>= 1) ss = __dadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, o));
+          if ((uint32_t)row >= live_rows) continue;
+          const double inv = head_norm_inv(ss, HD, p.norm_eps);
+          qa[u] = norm2(qa[u], p.qn_w + b2, inv, p.q, off); qb[u] = norm2(qb[u], p.qn_w + b2 + RHALF, inv, p.q, off);
+          if (PPR > 0) {
+#pragma unroll
+            for (int k = 0; k < QNP; ++k) qn[k] = norm2(qn[k], p.qn_w + plain_dim(2 * RIT + k), inv, p.q, off);
+          }
+        }
+        if (own_new) {
+          const uint64_t off = (uint64_t)p.items.col0[item] * p.k_new_stride + (uint64_t)g * HD;
+          double ss = HD == 256 ? sq(0.0, kx) : sq(sq(0.0, kx), kxb);
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) ss = __dadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, o));
+          if (HD == 256) {   // the row is spread over the four warps (the scratch is the maxima's, not yet in use)
+            double* s_ss = reinterpret_cast<double*>(s_max0);
+            if (lane == 0) s_ss[w] = ss;
+            named_bar_sync(gbar, kConsumers);
+            ss = __dadd_rn(__dadd_rn(s_ss[0], s_ss[1]), __dadd_rn(s_ss[2], s_ss[3]));
+          }
+          const double inv = head_norm_inv(ss, HD, p.norm_eps);
+          if (HD == 256) kx = norm2(kx, p.kn_w + 2 * tid, inv, p.k_new, off);
+          else if (tid < 32) { kx = norm2(kx, p.kn_w + 2 * tid, inv, p.k_new, off); kxb = norm2(kxb, p.kn_w + 2 * tid + RHALF, inv, p.k_new, off); }
+        }
+      }
 #pragma unroll
       for (int u = 0; u < RIT; ++u) {
         const int i = tid + u * kConsumers, row = i / IPR, b2 = 2 * (i % IPR);
@@ -628,7 +684,8 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
           q_store_rd(row, b2, make_float2(0.f, 0.f)); q_store_rd(row, b2 + RHALF, make_float2(0.f, 0.f));
           continue;
         }
-        const float2 a = act_cvt(qreg[(2 * u) % (Q_IN_REGS ? QLD : 1)]), b = act_cvt(qreg[(2 * u + 1) % (Q_IN_REGS ? QLD : 1)]);
+        float2 a = act_cvt(qreg[(2 * u) % (Q_IN_REGS ? QLD : 1)]), b = act_cvt(qreg[(2 * u + 1) % (Q_IN_REGS ? QLD : 1)]);
+        if (normed) { a = qa[u]; b = qb[u]; }
         float2 ra, rb;   // the bits of the float64 expression the stand-alone RoPE kernel evaluates
         ra.x = rot_exact(a.x, b.x, s_ang[b2], true);
         ra.y = rot_exact(a.y, b.y, s_ang[b2 + 1], true);
@@ -639,8 +696,10 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       }
 #pragma unroll
       for (int it = 2 * RIT; it < (Q_IN_REGS ? QLD : 1); ++it) {
-        const int idx = tid + (it - 2 * RIT) * kConsumers, rr = idx / (PPR ? PPR : 1), d = NRD + 2 * (idx % (PPR ? PPR : 1));
-        if (p.q_f16) {   // unrotated f16 values are their own high parts: the loaded bits go in as they are
+        const int rr = tid / IPR, d = plain_dim(it);
+        if (normed) {
+          q_store_rd(rr, d, qn[(it - 2 * RIT) % QNP]);
+        } else if (p.q_f16) {   // unrotated f16 values are their own high parts: the loaded bits go in as they are
           *reinterpret_cast<uint32_t*>(q_hi + rr * QP + d * 2) = __float_as_uint(qreg[it].x);
           if (PRECISE) *reinterpret_cast<uint32_t*>(q_lo + rr * QP + d * 2) = 0u;
         } else {
@@ -1232,7 +1291,7 @@ __global__ void __launch_bounds__(256) pa_combine_kernel(const CombineParams p) 
 
 // ------------------------------------------------------------------------------ launchers --
 
-template <int HD, int NT, bool PRECISE>
+template <int HD, int NT, bool PRECISE, bool NORM = false>
 static cudaError_t launch_decode_t(const pa_layer* L, const DecodeParams& p, dim3 grid, cudaStream_t st) {
   using S = DecSmem<HD, NT, PRECISE>;
   DecodeParams pp = p;
@@ -1242,7 +1301,7 @@ static cudaError_t launch_decode_t(const pa_layer* L, const DecodeParams& p, dim
   const int bytes = S::total_bytes(stages);
   static bool attr_set[64] = {};
   if (pp.gather && (!pp.k_cache || !pp.v_cache)) return cudaErrorInvalidValue;
-  auto kern = pa_decode_kernel<HD, NT, PRECISE>;
+  auto kern = pa_decode_kernel<HD, NT, PRECISE, NORM>;
   const int dev = L->ctx->device & 63;
   if (!attr_set[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -1258,7 +1317,7 @@ static cudaError_t launch_decode_t(const pa_layer* L, const DecodeParams& p, dim
 template <int HD, bool PRECISE>
 static cudaError_t launch_decode_nt(const pa_layer* L, const DecodeParams& p, dim3 grid, int nt, cudaStream_t st) {
   switch (nt) {
-    case 1: return launch_decode_t<HD, 1, PRECISE>(L, p, grid, st);
+    case 1: return HD >= 128 && p.qn_w ? launch_decode_t<HD, 1, PRECISE, HD >= 128>(L, p, grid, st) : launch_decode_t<HD, 1, PRECISE>(L, p, grid, st);
     case 2: return launch_decode_t<HD, 2, PRECISE>(L, p, grid, st);
     case 3: case 4: return launch_decode_t<HD, 4, PRECISE>(L, p, grid, st);
     default: return launch_decode_t<HD, 8, PRECISE>(L, p, grid, st);

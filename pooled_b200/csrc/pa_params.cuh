@@ -21,6 +21,8 @@ struct DecodeParams {
   const void* k_new; const void* v_new;               // the tokens' k / v rows, [items][n_kv * hd], dtype as q
   uint64_t k_new_stride, v_new_stride;                // elements between the rows of consecutive items
   const double* inv_freq;                             // theta^(-2i/n_rot), i < n_rot/2 (fused == 2)
+  // QK head-norm ahead of the rotation (fused front): weights [head_dim], nullptr: q and k come as they are
+  const float* qn_w; const float* kn_w; double norm_eps;
   __half* k_cache; __half* v_cache;                   // caches of the layer
   Angle rope_ang[64];       // cos / sin of pos * theta^(-2i/n_rot), i < n_rot/2, evaluated by the host in float64
   uint32_t prefetch_old_rows;  // 1: K/V tiles below the call's own new rows may be fetched before the predecessor kernel ends

@@ -502,3 +502,43 @@ def test_token_blocks_back_to_back_on_one_layer(n_cols, nH, nKV):
     q_rot = np.stack([po.rope_neox_f64(q[T - n_cols + c], nH, hd, 64, p0 + c, 1e7) for c in range(n_cols)])
     ref = po.attn_f64(q_rot, Kf, Vf, nH, nKV, hd, p0, n_cols, g[T - n_cols:])
     util.assert_close(o[T - n_cols:], ref, "token blocks, last block")
+
+
+@pytest.mark.parametrize("nH,nKV,hd,n_rot,act,tie", [(16, 2, 256, 64, "f16", False), (24, 4, 256, 64, "f32", True), (16, 8, 128, 128, "f16", True), (7, 1, 128, 128, "f32", False)])
+def test_head_norm_in_the_decode_front_keeps_the_bits_of_the_separate_kernel(nH, nKV, hd, n_rot, act, tie):
+    # one token of one and of three sequences: the layer's own head-norm (inside the decode kernel) against pa_head_norm
+    # and the same call on a layer without one.  tie: eps 0, inv exactly 1 and outputs 3 w on rounding boundaries of f32,
+    # which sends every thread of the front to the in-order sum
+    import torch
+    from pooled_b200 import AttnConfig, AttnEngine
+    td = torch.float16 if act == "f16" else torch.float32
+    ctx = [301, 64, 1500]
+    engs = [AttnEngine(AttnConfig(n_heads=nH, n_kv_heads=nKV, head_dim=hd, n_rot=n_rot, rope_theta=1e6, max_seq=1600, n_seqs=3, act_dtype=td, max_cols=8)) for _ in range(2)]
+    rng = np.random.default_rng(11)
+    for s, n in enumerate(ctx):
+        K, V = (po.np_f16_rne(rng.standard_normal((n, nKV * hd)).astype(np.float32)) for _ in range(2))
+        for e in engs:
+            util.load_cache(e, 0, s, K, V)
+    pat = np.array([3.0] + [1.0] * 7 + [0.0] * 8, np.float32)
+    vals = lambda n: (np.tile(pat, (3, n * hd // 16)) * np.where(rng.random((3, n * hd)) < 0.5, -1, 1)).astype(np.float32) if tie else rng.standard_normal((3, n * hd)).astype(np.float32)
+    qn = util.torch_dev(vals(nH), td); k = util.torch_dev(vals(nKV), td); v = util.torch_dev(rng.standard_normal((3, nKV * hd)).astype(np.float32), td)
+    q = torch.randn((3, nH, 2 * hd), device="cuda").to(td)
+    q[:, :, :hd] = qn.view(3, nH, hd)
+    q = q.view(3, -1)
+    w = [util.torch_dev((1 + 0.1 * rng.standard_normal(hd)).astype(np.float32)) for _ in range(2)]
+    eps = 0.0 if tie else 1e-6
+    engs[0].set_head_norm(0, w[0], w[1], eps)
+    nq, nk = torch.empty((3, nH * hd), dtype=td, device="cuda"), torch.empty_like(k)
+    engs[1].head_norm(qn, nH, w[0], eps, out=nq)
+    engs[1].head_norm(k, nKV, w[1], eps, out=nk)
+    gate, hs = q[:, hd:], 2 * hd
+    for e, a, b, qs in ((engs[0], q, k, hs), (engs[1], nq, nk, hd)):
+        e.outs = [e.encode_layer(0, ctx[0], a[:1], b[:1], v[:1], gate[:1], seq=0, q_head_stride=qs, gate_head_stride=hs),
+                  e.encode_items(0, [(0, ctx[0] + 1), (1, ctx[1]), (2, ctx[2])], a, b, v, gate, q_head_stride=qs, gate_head_stride=hs)]
+        e.sync()
+    it = torch.int16 if act == "f16" else torch.int32
+    for x, y in zip(engs[0].outs, engs[1].outs):
+        assert torch.equal(x.view(it), y.view(it)) and torch.isfinite(x).all()
+    for which in "kv":
+        for s, n in enumerate(ctx):
+            assert torch.equal(engs[0].cache(0, which)[s, :n + (2 if s == 0 else 1)], engs[1].cache(0, which)[s, :n + (2 if s == 0 else 1)])
