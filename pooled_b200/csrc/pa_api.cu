@@ -23,6 +23,8 @@ bool rope_vec_applies(const RopeParams& p, uint32_t n_cols);
 cudaError_t launch_epoch_bump(unsigned int* ctr, cudaStream_t st);
 cudaError_t launch_head_norm(const HeadNormParams& p, cudaStream_t st);
 int prefill_supported(const pa_ctx* ctx);
+cudaError_t launch_combine_few(int head_dim, const PrefillParams& p, cudaStream_t st);
+uint32_t prefill_splits(uint32_t pos, uint32_t n_cols, uint32_t n_heads, uint32_t head_dim, uint32_t sms, size_t slots);
 cudaError_t launch_prefill(const pa_layer* L, const PrefillParams& p, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_q,
                            const CUtensorMap& tm_o, const CUtensorMap& tm_q2, cudaStream_t st);
 cudaError_t launch_verify(const pa_layer* L, const PrefillParams& p, const CUtensorMap& tm_k, const CUtensorMap& tm_v, uint32_t n_kv, cudaStream_t st);
@@ -191,8 +193,10 @@ extern "C" int pa_create(int device, const pa_config* cfg, pa_ctx** out) {
   // split partials: one (o, m, l) record per (query row, split).  A call uses rows * splits of them, about
   // 64 rows x one CTA per SM; the split planner keeps every call inside this capacity.
   ctx->part_slots = 16384;
-  if ((e = cudaMalloc(&ctx->part_o, ctx->part_slots * cfg->head_dim * 4)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(part_o)", e);
-  if ((e = cudaMalloc(&ctx->part_ml, ctx->part_slots * 2 * 4)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(part_ml)", e);
+  // a prefill call of few columns splits its keys: 400 columns of 24 heads three ways are 28800 records
+  ctx->pf_slots = std::max<size_t>(ctx->part_slots, std::min<size_t>(32768, (size_t)cfg->max_cols * cfg->n_heads * kPrefillSplits));
+  if ((e = cudaMalloc(&ctx->part_o, ctx->pf_slots * cfg->head_dim * 4)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(part_o)", e);
+  if ((e = cudaMalloc(&ctx->part_ml, ctx->pf_slots * 2 * 4)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(part_ml)", e);
   ctx->merge_slots = 2u * kMaxItems * cfg->n_kv_heads;
   if ((e = cudaMalloc(&ctx->merge_ctr, ctx->merge_slots * 4)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(merge counters)", e);
   if ((e = cudaMemset(ctx->merge_ctr, 0, ctx->merge_slots * 4)) != cudaSuccess) return bail(PA_ECUDA, "cudaMemset(merge counters)", e);
@@ -920,6 +924,9 @@ static int prefill_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols
     if (int rc = make_cache_map(ctx, &tm_q, const_cast<void*>(q), n_cols, (uint32_t)qcs, ctx->cfg.head_dim, 128)) return rc;
     p.q_tma = 1;
   }
+  // few columns behind many keys: the keys are split and the records merged by a second kernel
+  p.n_splits = ctx->core_only ? 1u : prefill_splits(p.pos, n_cols, p.n_heads, ctx->cfg.head_dim, (uint32_t)ctx->sm_count, ctx->pf_slots);
+  p.part_o = ctx->part_o; p.part_ml = ctx->part_ml;
   // ... and f16 output tiles leave by TMA (any head_dim the kernel takes; gate, if any, f16 with 16-byte aligned rows)
   CUtensorMap tm_o = tm_k;
   if (ctx->cfg.act_dtype == PA_F16 && !(ocs & 63) && !ctx->tune.no_out_tma && (!gate || (!(gcs & 7) && !(ghs & 7) && !((uintptr_t)gate & 15)))) {
@@ -928,6 +935,7 @@ static int prefill_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols
   }
   timing_mark(ctx, st, 0);
   CU_TRY(ctx, launch_prefill(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, st));
+  if (p.n_splits > 1) { CU_TRY(ctx, launch_combine_few((int)ctx->cfg.head_dim, p, st)); ctx->stats.kernel_launches++; }
   timing_mark(ctx, st, 1);
   ctx->stats.kernel_launches++; ctx->stats.calls++;
   ctx->stats.kv_bytes_streamed += 2ull * (pos + n_cols) * ctx->kv_dim * 2;

@@ -230,6 +230,7 @@ __device__ __forceinline__ void named_bar_arrive(uint32_t id, uint32_t threads) 
 __host__ __device__ constexpr int decode_groups(int nt) { return nt >= 0 ? 1 : 2; }
 
 constexpr int kMaxItems = 32;     // items of one batched decode call
+constexpr int kPrefillSplits = 8; // most key splits of a prefill call
 constexpr int kMaxRows = 64;      // query rows (columns x heads of one kv head) one decode CTA carries
 
 template <typename... KArgs, typename... Args>
@@ -292,7 +293,8 @@ struct pa_ctx {
   float* part_o = nullptr;     // device: split partials, f32 [rows][splits][head_dim] of the current call
   float* part_ml = nullptr;    // device: f32 [rows][splits][2]
   uint32_t max_splits = 0;
-  size_t part_slots = 0;       // (query row, split) records the partial buffers hold
+  size_t part_slots = 0;       // (query row, split) records a decode / verify call may use
+  size_t pf_slots = 0;         // records the partial buffers hold, and a split prefill may use
   unsigned int* merge_ctr = nullptr;   // device: per (item, kv head) of a decode call, records left and CTAs done merging (zero between calls)
   uint32_t merge_slots = 0;
   uint32_t* dev_err = nullptr;   // device error word (bounded waits)

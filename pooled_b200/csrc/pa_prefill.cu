@@ -162,6 +162,8 @@ __device__ __forceinline__ void umma_commit_elected(uint32_t leader, uint32_t ba
 
 
 // MODE 0: causal prefill, one CTA per (128 query columns, q head).
+// MODE 3: the same with the keys split over blockIdx.z and a record per (row, split) instead of the output (an instantiation
+//   of its own: a run-time split cost the unsplit kernel 2.5 % at head_dim 128).
 // MODE 1 / 2: split-K form for a k-token verify block: one CTA per (split of the KV sequence, kv head); the rows of the
 //   tile are (column, head of the GQA group) pairs, at most 64 of them, and the CTA writes an unnormalised (o, m, l)
 //   partial per row for the LSE combine.  MODE 2 keeps about 22 bits of q and of the softmax weights at no extra
@@ -171,11 +173,12 @@ __device__ __forceinline__ void umma_commit_elected(uint32_t leader, uint32_t ba
 
 template <int HD, int MODE>
 struct PfSmem {
+  static constexpr bool PF = MODE == 0 || MODE == 3;
   // S / P tiles in tensor memory.  The loop S(j) -> softmax(j) -> P V(j) -> S(j + SBUF) is a cycle of fixed length
   // (about 2.9 us at head_dim 256): the tile rate is SBUF tiles per cycle.  The causal prefill at head_dim 256 takes
   // four (Q then comes from shared memory only: as an A operand in tensor memory it was no faster, and its 64 columns
   // are the fourth tile); the other forms keep three and the lower half of Q in tensor memory.
-  static constexpr int SBUF = (MODE == 0 && HD == 256) ? 4 : 3;
+  static constexpr int SBUF = (PF && HD == 256) ? 4 : 3;
   // K ring and V ring depth.  Split-K: three K slots (the scores run two tiles ahead) and two V slots, which leaves
   // 32 KB free so that its CTAs can join SMs that still run a small kernel.  Prefill: one K slot per scores issuer,
   // tile j in slot j % 2, so that the fills of a slot are consumed by ONE thread, in order.  (With three slots shared by
@@ -183,7 +186,7 @@ struct PfSmem {
   // before tile 0 has landed there -- TMA copies finish out of order under the burst of a kernel's start -- the barrier
   // is still in its first phase, and a wait for "parity 1" takes that for fill 1 done.  The second arrival on the
   // slot's empty barrier that follows ends in a trap, once in some hundred launches.)
-  static constexpr int NK = MODE == 0 ? 2 : 3, NV = MODE == 0 ? 3 : 2;
+  static constexpr int NK = PF ? 2 : 3, NV = PF ? 3 : 2;
   static constexpr int KV_BYTES = HD * 128;         // [HD/64][64 rows][128 B]
   // tensor memory columns: the first TQC 64-dim chunks of Q (32 columns of f16 pairs each) | S tiles (64 each; P
   // overwrites the first 32 of its S) | O (HD).  HD 256: 64 + 192 + 256, or 0 + 256 + 256 = 512.
@@ -200,7 +203,7 @@ struct PfSmem {
   // work apiece against about twice that to issue one, so a single issuing thread, not the tensor cores, set the
   // loop's pace; two threads take alternate tiles (a tile's instructions stay in one thread: the order of its sums is
   // fixed).
-  static constexpr int QK_ISSUERS = MODE == 0 ? 2 : 1;   // (the split-K form's 168 registers leave no room for a 13th warp)
+  static constexpr int QK_ISSUERS = PF ? 2 : 1;   // (the split-K form's 168 registers leave no room for a 13th warp)
   static_assert(QK_ISSUERS == 1 || (NK % QK_ISSUERS == 0 && SBUF >= 3), "a K slot belongs to one scores issuer");
   static constexpr int THREADS = 128 + 128 * NGRP + 32 * (QK_ISSUERS - 1);
   static constexpr int QK2_WARP = 4 + 4 * NGRP;      // the second scores issuer
@@ -219,7 +222,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
                   const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ CUtensorMap tm_q2, const PrefillParams p) {
   using L = PfSmem<HD, MODE>;
   constexpr int CH = HD / 64;
-  constexpr bool SK = MODE != 0, PREC = MODE == 2;
+  constexpr bool SK = MODE == 1 || MODE == 2, PREC = MODE == 2, SPLIT = MODE == 3;
   constexpr int NK = L::NK, NV = L::NV, NGRP = L::NGRP, kSBuf = L::SBUF;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -247,6 +250,13 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
   const uint32_t rows_valid = SK ? 0u : min((uint32_t)kBM, p.n_cols - c0);
   const uint32_t p0 = p.pos + c0;                       // cache row of column c0's own token
   uint32_t tile0 = 0, n_tiles = (p0 + rows_valid + kBN - 1) / kBN;
+  if constexpr (SPLIT) {
+    // a short prompt behind a long context: the keys of a q tile are split over blockIdx.z (see prefill_splits)
+    const uint32_t tps = (n_tiles + p.n_splits - 1) / p.n_splits;
+    tile0 = blockIdx.z * tps;
+    if (tile0 >= n_tiles) return;                       // uniform for the CTA; the merge derives the same count
+    n_tiles = min(n_tiles, tile0 + tps) - tile0;
+  }
   if (SK) {
     const uint32_t tiles = (p.n_rows + kBN - 1) / kBN, tps = (tiles + p.n_splits - 1) / p.n_splits;
     tile0 = blockIdx.x * tps;
@@ -256,7 +266,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
 
   // prefill at head_dim 256 with f16 q: the 128 query rows (64 KB) land in shared memory, in the layout the score
   // products read, by one TMA copy issued at once, instead of through the softmax threads' registers
-  const bool q_by_tma = MODE == 0 && L::TQC == 0 && p.q_tma;
+  const bool q_by_tma = !SK && L::TQC == 0 && p.q_tma;
   if (warp == 1 && lane == 0) {
     *s_err = 0;
     for (int i = 0; i < NK; ++i) { mbar_init(BAR(K_FULL, i), 1); mbar_init(BAR(K_EMPTY, i), 1); }
@@ -503,7 +513,9 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       tc_fence_before();
       mbar_arrive(BAR(Q_FULL, 0));
     }
-    float m_st = SK ? -1.0e30f : -INFINITY, l_sum = 0.f, m_l = m_st;
+    // (a split that does not begin at key 0 may hold no visible key of a row either)
+    const bool first0 = !SK && (!SPLIT || tile0 == 0);
+    float m_st = first0 ? -INFINITY : -1.0e30f, l_sum = 0.f, m_l = m_st;
     for (uint32_t j = wg; j < n_tiles; j += NGRP) {
       const uint32_t b = j % kSBuf, u = j / kSBuf, kv0 = (tile0 + j) * kBN;
       mbar_wait(BAR(S_FULL, b), u & 1, s_err, WAIT_MMA);
@@ -536,7 +548,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       }
       float alpha = 1.f;
       bool grow = false;
-      if (!SK && j == 0) m_st = mt;                 // key 0 is visible to every row, so mt is finite
+      if (first0 && j == 0) m_st = mt;                 // key 0 is visible to every row, so mt is finite
       else if (mt > m_st + 8.f) { alpha = ex2_approx(m_st - mt); m_st = mt; grow = true; }
       if (NGRP == 2) {
         // hand the reference on at once: the other group's next tile needs nothing else from this one
@@ -623,6 +635,30 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         if (sl != ~0ull) reinterpret_cast<float4*>(p.part_o + sl * HD)[c4] = xs[rr * RP + c4];
       }
       if (writer && wg == 0) { p.part_ml[slot * 2] = (NGRP == 2 ? s_rm[row] : m_st) * 0.6931471805599453f; p.part_ml[slot * 2 + 1] = l_sum; }
+    } else if constexpr (SPLIT) {
+      // this split's unnormalised (o, m, l) of every row, by way of shared memory (the rings are idle): a lane holds a row,
+      // and stored as they are the 32 lanes of an instruction would write into 32 records 1 KB and more apart
+      constexpr int RP = HD / 4 + 1;                                    // row pitch in float4: 16 bytes apart in their bank phase
+      static_assert(2048 + kBM * RP * 16 <= (L::NK + L::NV) * L::KV_BYTES, "the record tile fits the idle rings");
+      float4* xs = reinterpret_cast<float4*>(base + L::OFF_K + 2048);
+#pragma unroll 1
+      for (int c = 0; c < HD / 32; ++c) {
+        if (NGRP == 2 && (uint32_t)(c & 1) != wg) continue;
+        float o[32];
+        tmem_ld32(t_o + c * 32 + lane_addr, o);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) xs[row * RP + c * 8 + i] = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+      }
+      named_bar_sync(1, 128 * NGRP);
+      for (uint32_t idx = tid - 128; idx < rows_valid * (HD / 4); idx += 128 * NGRP) {
+        const uint32_t rr = idx / (HD / 4), c4 = idx % (HD / 4);
+        const uint64_t slot = ((uint64_t)(c0 + rr) * p.n_heads + h) * p.n_splits + blockIdx.z;
+        reinterpret_cast<float4*>(p.part_o + slot * HD)[c4] = xs[rr * RP + c4];
+      }
+      if (wg == 0 && row < rows_valid) {
+        const uint64_t slot = ((uint64_t)col * p.n_heads + h) * p.n_splits + blockIdx.z;
+        p.part_ml[slot * 2] = s_rm[row] * 0.6931471805599453f; p.part_ml[slot * 2 + 1] = l_sum;
+      }
     } else if (MODE == 0 && p.out_tma) {
       // The output tile leaves as the query tile came: through shared memory in the TMA layout ([64-dim chunk][row][128 B],
       // 16-byte pieces XOR-swizzled by the row), one bulk tensor store for the CTA.  The K ring is idle (every product
@@ -706,6 +742,108 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
   if (tid == 0 && *s_err) atomicMax(p.err, *s_err);
 }
 
+// LSE merge of the few (2..8) records a split prefill leaves per query row, gate and store: a warp per row, HD / 32 values
+// per lane, every record of the row requested at once.  (pa_combine_kernel, 256 threads per row and 64 dims, is made for
+// few rows of many records: at 4872 rows x 3 records it would be 19488 CTAs with 48 of 256 lanes at work.)  The
+// records were written just now and come from L2.  The same arithmetic: weights e^(m - M), sums in split order.
+template <int HD>
+__global__ void __launch_bounds__(256) pa_combine_few_kernel(const PrefillParams p) {
+  constexpr int NV = HD >= 128 ? HD / 128 : 1, W = HD >= 128 ? 4 : 2;   // vectors of W floats per lane
+  const uint32_t prow = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_trigger();
+  if (prow >= p.n_cols * p.n_heads) return;
+  const uint32_t col = prow / p.n_heads, h = prow % p.n_heads, c0 = col / kBM * kBM;
+  const uint32_t n_tiles = (p.pos + c0 + min((uint32_t)kBM, p.n_cols - c0) + kBN - 1) / kBN;
+  const uint32_t tps = (n_tiles + p.n_splits - 1) / p.n_splits, ns = (n_tiles + tps - 1) / tps;   // live splits of this q tile
+  const float* ml = p.part_ml + (uint64_t)prow * p.n_splits * 2;
+  const float* ob = p.part_o + (uint64_t)prow * p.n_splits * HD + lane * W;
+  float m[kPrefillSplits], l[kPrefillSplits], x[kPrefillSplits][NV * W];
+#pragma unroll
+  for (int s = 0; s < kPrefillSplits; ++s) {
+    m[s] = -3.0e38f; l[s] = 0.f;
+    if ((uint32_t)s >= ns) continue;
+    m[s] = ml[2 * s]; l[s] = ml[2 * s + 1];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      if (W == 4) *reinterpret_cast<float4*>(&x[s][4 * v]) = *reinterpret_cast<const float4*>(ob + s * HD + v * 128);
+      else *reinterpret_cast<float2*>(&x[s][0]) = *reinterpret_cast<const float2*>(ob + s * HD);
+    }
+  }
+  float gv[NV * W];
+  const uint64_t go = (uint64_t)col * p.gate_col_stride + (uint64_t)h * p.gate_head_stride;
+#pragma unroll
+  for (int i = 0; i < NV * W; ++i) {
+    const uint32_t d = (i / W) * 128 + lane * W + i % W;
+    gv[i] = p.gate ? ld_act(p.gate, go + d, p.act_f16) : 0.f;
+  }
+  float M = m[0];
+#pragma unroll
+  for (int s = 1; s < kPrefillSplits; ++s) M = fmaxf(M, m[s]);
+  float L = 0.f, acc[NV * W];
+#pragma unroll
+  for (int i = 0; i < NV * W; ++i) acc[i] = 0.f;
+#pragma unroll
+  for (int s = 0; s < kPrefillSplits; ++s) {
+    if ((uint32_t)s >= ns) continue;
+    const float w = __expf(m[s] - M);
+    L = __fmaf_rn(l[s], w, L);
+#pragma unroll
+    for (int i = 0; i < NV * W; ++i) acc[i] = __fmaf_rn(x[s][i], w, acc[i]);
+  }
+  const uint64_t oo = (uint64_t)col * p.out_col_stride + (uint64_t)h * HD;
+#pragma unroll
+  for (int i = 0; i < NV * W; ++i) {
+    acc[i] = __fdiv_rn(acc[i], L);
+    if (p.gate) acc[i] = __fmul_rn(acc[i], __fdiv_rn(1.0f, __fadd_rn(1.0f, __expf(-gv[i]))));
+  }
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const uint32_t d = v * 128 + lane * W;
+    if (p.act_f16) {
+      __half* dst = reinterpret_cast<__half*>(p.out) + oo + d;
+      if (W == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(pack_h2(acc[4 * v], acc[4 * v + 1]), pack_h2(acc[4 * v + 2], acc[4 * v + 3]));
+      else *reinterpret_cast<uint32_t*>(dst) = pack_h2(acc[0], acc[1]);
+    } else {
+      float* dst = reinterpret_cast<float*>(p.out) + oo + d;
+      if (W == 4) *reinterpret_cast<float4*>(dst) = make_float4(acc[4 * v], acc[4 * v + 1], acc[4 * v + 2], acc[4 * v + 3]);
+      else *reinterpret_cast<float2*>(dst) = make_float2(acc[0], acc[1]);
+    }
+  }
+}
+cudaError_t launch_combine_few(int head_dim, const PrefillParams& p, cudaStream_t st) {
+  const dim3 grid((p.n_cols * p.n_heads + 7) / 8);
+  switch (head_dim) {
+    case 256: return launch_pdl(pa_combine_few_kernel<256>, grid, dim3(256), 0, st, p);
+    case 128: return launch_pdl(pa_combine_few_kernel<128>, grid, dim3(256), 0, st, p);
+    default: return launch_pdl(pa_combine_few_kernel<64>, grid, dim3(256), 0, st, p);
+  }
+}
+
+// Key splits of a prefill call.  One CTA per (128 columns, head) leaves most of the chip idle when a short prompt follows
+// a long context (203 columns of 24 heads behind 9001: 48 CTAs of 145 tiles on 148 SMs, 205 us a layer; three ways
+// split 95 us).  The count is the one with the least estimated makespan, in units of a tile's time: a CTA costs its tiles and
+// about 8 more for its start and end, equal CTAs run in whole waves, CTAs of a causal triangle (heavy ones first) pack;
+// a split call adds the merge launch (6) and its records' way through L2 (1 KB each, about 3 TB/s both ways).
+uint32_t prefill_splits(uint32_t pos, uint32_t n_cols, uint32_t n_heads, uint32_t head_dim, uint32_t sms, size_t slots) {
+  const uint32_t q_tiles = (n_cols + kBM - 1) / kBM;
+  const double longest = (double)((pos + n_cols + kBN - 1) / kBN), avg = (double)((pos + n_cols / 2 + kBN - 1) / kBN);
+  const uint64_t rows = (uint64_t)n_cols * n_heads, ctas = (uint64_t)q_tiles * n_heads;
+  uint32_t best = 1;
+  double best_t = 0;
+  for (uint32_t ns = 1; ns <= (uint32_t)kPrefillSplits; ++ns) {
+    if (ns > 1 && (rows * ns > slots || longest / ns < 4.0)) break;
+    const double waves = (double)(ctas * ns) / sms;
+    double t;
+    if (waves <= 1.0) t = longest / ns + 8.0;
+    else if (avg >= 0.8 * longest) t = ceil(waves) * (longest / ns + 8.0);
+    else t = waves * (avg / ns + 8.0) + 0.5 * longest / ns;
+    if (ns > 1) t += 6.0 + (double)(rows * ns) * (head_dim * 8.0) / 3.0e6 / 0.8;
+    if (ns == 1 || t < 0.95 * best_t) { best = ns; best_t = t; }
+  }
+  return best;
+}
+
 int prefill_supported(const pa_ctx* ctx) { return ctx->cfg.head_dim == 256 || ctx->cfg.head_dim == 128 || ctx->cfg.head_dim == 64; }
 
 template <int HD, int MODE>
@@ -718,7 +856,7 @@ static cudaError_t launch_pf(const pa_layer* L, const PrefillParams& p, const CU
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  if (MODE == 0) {
+  if (MODE == 0 || MODE == 3) {
     pa_prefill_kernel<HD, MODE><<<grid, PfSmem<HD, MODE>::THREADS, PfSmem<HD, MODE>::TOTAL, st>>>(tm_k, tm_v, tm_q, tm_o, tm_q2, p);
     return cudaGetLastError();
   }
@@ -727,11 +865,11 @@ static cudaError_t launch_pf(const pa_layer* L, const PrefillParams& p, const CU
 
 cudaError_t launch_prefill(const pa_layer* L, const PrefillParams& p, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_q,
                            const CUtensorMap& tm_o, const CUtensorMap& tm_q2, cudaStream_t st) {
-  const dim3 grid((p.n_cols + kBM - 1) / kBM, p.n_heads);
+  const dim3 grid((p.n_cols + kBM - 1) / kBM, p.n_heads, p.n_splits);
   switch (L->ctx->cfg.head_dim) {
-    case 256: return launch_pf<256, 0>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st);
-    case 128: return launch_pf<128, 0>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st);
-    case 64: return launch_pf<64, 0>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st);
+    case 256: return p.n_splits > 1 ? launch_pf<256, 3>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st) : launch_pf<256, 0>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st);
+    case 128: return p.n_splits > 1 ? launch_pf<128, 3>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st) : launch_pf<128, 0>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st);
+    case 64: return p.n_splits > 1 ? launch_pf<64, 3>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st) : launch_pf<64, 0>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -151,6 +151,27 @@ def test_chunked_prefill_and_prefill_vs_decode():
     eng.sync()
 
 
+@pytest.mark.parametrize("nH,nKV,hd,n_cols,pos,act,gate", [
+    (24, 4, 256, 203, 3001, "f32", True),     # two q tiles, the second with 75 rows
+    (16, 2, 256, 48, 1500, "f16", True),      # less than one q tile
+    (8, 2, 256, 128, 1216, "f16", False),     # 21 tiles in fifths: the last split is one tile, out of sight of half of the rows
+    (16, 8, 128, 129, 1000, "f16", True), (8, 2, 64, 65, 700, "f32", False)])
+def test_few_columns_behind_a_long_context_split_their_keys(nH, nKV, hd, n_cols, pos, act, gate):
+    import torch
+    td = torch.float16 if act == "f16" else torch.float32
+    eng = _engine(nH, nKV, hd, pos + n_cols + 70, act=act, max_cols=n_cols, rope_mode="none")
+    T = pos + n_cols
+    q = util.normal_f16(21, (n_cols, nH * hd)); K = po.np_f16_rne(po.normal(22, T * nKV * hd)).reshape(T, -1); V = po.np_f16_rne(po.normal(23, T * nKV * hd)).reshape(T, -1)
+    g = util.normal_f16(24, (n_cols, nH * hd)) if gate else None
+    poison = np.full((70, nKV * hd), 0x7e00, np.uint16)      # rows past the last one hold NaN
+    util.load_cache(eng, 0, 0, np.concatenate([K, poison]), np.concatenate([V, poison]))
+    before = eng.stats()["kernel_launches"]
+    out = eng.prefill(0, 0, pos, util.torch_dev(q, td), util.torch_dev(g, td) if gate else None)
+    eng.sync()
+    assert eng.stats()["kernel_launches"] - before == 2      # the keys were split: prefill and merge
+    util.assert_close(out.float().cpu().numpy(), po.attn_f64(q, K, V, nH, nKV, hd, pos, n_cols, g), f"split prefill {n_cols} at {pos}")
+
+
 def test_config3_full_size_properties():
     # the whole 8192-token prompt (0.82 TFLOP): checked on sampled columns against the oracle (the float64 oracle over
     # all 8192 columns takes minutes) and through size-independent properties
