@@ -23,13 +23,16 @@ bool rope_vec_applies(const RopeParams& p, uint32_t n_cols);
 cudaError_t launch_epoch_bump(unsigned int* ctr, cudaStream_t st);
 cudaError_t launch_head_norm(const HeadNormParams& p, cudaStream_t st);
 int prefill_supported(const pa_ctx* ctx);
+cudaError_t launch_q8(const Q8Params& p, uint32_t hd, uint32_t n_kv, int dev, cudaStream_t st);
+bool front_supported(uint32_t hd, uint32_t n_rot, bool rotates);
+cudaError_t launch_front(const FrontParams& p, uint32_t hd, uint32_t n_rot, cudaStream_t st);
 cudaError_t launch_combine_few(int head_dim, const PrefillParams& p, cudaStream_t st);
 uint32_t prefill_splits(uint32_t pos, uint32_t n_cols, uint32_t n_heads, uint32_t head_dim, uint32_t sms, size_t slots);
 cudaError_t launch_prefill(const pa_layer* L, const PrefillParams& p, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_q,
                            const CUtensorMap& tm_o, const CUtensorMap& tm_q2, cudaStream_t st);
 cudaError_t launch_verify(const pa_layer* L, const PrefillParams& p, const CUtensorMap& tm_k, const CUtensorMap& tm_v, uint32_t n_kv, cudaStream_t st);
 cudaError_t launch_kv_store(const KvStoreParams& p, uint32_t n_cols, cudaStream_t st);
-cudaError_t launch_decode_any(const AnyDecodeParams& p, int format, dim3 grid, cudaStream_t st);
+cudaError_t launch_decode_f32(const AnyDecodeParams& p, dim3 grid, int dev, cudaStream_t st);
 }  // namespace pa
 
 using namespace pa;
@@ -465,14 +468,54 @@ static int ensure_angles(pa_ctx* ctx, uint32_t pos, uint32_t n_cols, cudaStream_
   return PA_OK;
 }
 
+// Head-norm (norm: the layer has one and it has not been applied yet), rotation and append in one launch, where the
+// shapes allow it (front_supports); the caller has checked the columns.
+static bool front_supports(const pa_ctx* ctx, int mode) {
+  return (mode == PA_ROPE_F64 || mode == PA_ROPE_NONE) && front_supported(ctx->cfg.head_dim, ctx->cfg.n_rot, mode == PA_ROPE_F64);
+}
+static int front_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, const void* q, uint64_t qcs, uint64_t qhs, void* q_out, uint64_t q_out_cs,
+                      const void* k, const void* v, uint64_t kcs, uint64_t vcs, int mode, int in_f16, bool norm, cudaStream_t st, int q_out_f16 = 0) {
+  pa_ctx* ctx = L->ctx;
+  FrontParams p{};
+  p.q = q; p.q_col_stride = qcs; p.q_head_stride = qhs; p.q_heads = ctx->cfg.n_heads;
+  p.q_out = q_out; p.q_out_col_stride = q_out_cs; p.q_out_f16 = q_out_f16;
+  if (q_out_f16 == 2) p.q_lo_offset = (uint64_t)ctx->cfg.max_cols * ctx->q_dim;
+  p.k = k; p.v = v; p.k_col_stride = kcs; p.v_col_stride = vcs; p.kv_heads = ctx->cfg.n_kv_heads;
+  p.format = L->kv_format;
+  p.k_cache = L->kv_format == PA_KV_F16 ? (void*)L->k : L->k_alt; p.v_cache = L->kv_format == PA_KV_F16 ? (void*)L->v : L->v_alt;
+  p.k_scale = L->k_scale; p.v_scale = L->v_scale;
+  p.cache_row0 = (uint64_t)seq * L->max_seq + (pos - L->origin);
+  p.n_cols = n_cols; p.in_f16 = in_f16;
+  if (norm) { p.qn_w = L->qnorm_w; p.kn_w = L->knorm_w; p.norm_eps = L->norm_eps; }
+  const uint32_t half = mode == PA_ROPE_F64 ? ctx->cfg.n_rot / 2 : 0;
+  if (half) {
+    if (n_cols * half <= 64) {
+      p.n_ang = n_cols * half;
+      memcpy(p.ang, host_angles(ctx, pos, n_cols), (size_t)p.n_ang * sizeof(Angle));
+    } else {
+      if (int rc = ensure_angles(ctx, pos, n_cols, st)) return rc;
+      p.angles = ctx->angles;
+    }
+  }
+  CU_TRY(ctx, launch_front(p, ctx->cfg.head_dim, half ? ctx->cfg.n_rot : 0, st));
+  ctx->stats.kernel_launches++;
+  return PA_OK;
+}
+
 static int rope_append_impl(pa_layer* L, pa_ctx* ctx, uint32_t seq, uint32_t pos, uint32_t n_cols, const void* q, uint64_t qcs, uint64_t qhs,
                             uint32_t q_heads, void* q_out, uint64_t q_out_cs, const void* k, const void* v, uint64_t kvcs, const float* cs_table,
                             uint32_t mode, int in_f16, cudaStream_t st, int q_out_f16 = 0, bool in_layer_call = false, uint64_t vcs = 0,
                             bool* q_rot_only = nullptr) {   // in: write only the rotated dims of q if the kernel can; out: whether it will
   if (L && L->kv_format != PA_KV_F16) {
-    // int8 / f32 caches: q rotated as usual; k rotated into the context's f32 scratch (the rotation kernel's q path,
-    // with the kv heads as its heads), then the format's own store kernel -- attn_glue followed by kv_store_q8
+    // int8 / f32 caches: one launch where the front kernel knows the shape; else q rotated as usual, k rotated into the
+    // context's f32 scratch (the rotation kernel's q path, with the kv heads as its heads), then the format's own store
+    // kernel -- attn_glue followed by kv_store_q8
     if (n_cols > ctx->cfg.max_cols) return fail(ctx, PA_EINVAL, "rope: %u columns exceed max_cols %u", n_cols, ctx->cfg.max_cols);
+    if (k && v && front_supports(ctx, mode)) {
+      if (int rc = front_impl(L, seq, pos, n_cols, q, qcs, qhs, q_out, q_out_cs, k, v, kvcs, vcs ? vcs : kvcs, mode, in_f16, false, st, q_out_f16)) return rc;
+      ctx->inflight_layer = nullptr;
+      return PA_OK;
+    }
     if (q)
       if (int rc = rope_append_impl(nullptr, ctx, seq, pos, n_cols, q, qcs, qhs, q_heads, q_out, q_out_cs, nullptr, nullptr, 0, cs_table, mode, in_f16, st, q_out_f16, in_layer_call))
         return rc;
@@ -647,10 +690,57 @@ struct FusedFront {
 // a gathered call: the columns' row lists on the device, one list of `stride` words per column
 struct GatherLists { const uint32_t* lists; uint32_t stride; };
 
+// Decode / blocks / prompts over an int8 cache, one launch per item.  Splits fill two CTAs per SM; a call whose rows alone
+// do that is not split, and then writes its outputs itself.  early: the kernel before this one is the call's own front.
+static int decode_q8_item(pa_layer* L, const pa_item& it, const void* q, int q_dtype, uint64_t qcs, uint64_t qhs, const void* gate, uint64_t gcs,
+                          uint64_t ghs, void* out, uint64_t ocs, bool early, cudaStream_t st) {
+  pa_ctx* ctx = L->ctx;
+  const uint32_t hd = ctx->cfg.head_dim, nH = ctx->cfg.n_heads, rows = it.n_cols * ctx->G, n_rows = it.pos + it.n_cols - L->origin;
+  Q8Params p{};
+  p.q = q; p.q_f16 = q_dtype == PA_F16; p.q_col_stride = qcs; p.q_head_stride = qhs;
+  p.q_vec = q_dtype == PA_F32 && !(qcs & 3) && !(qhs & 3) && !((uintptr_t)q & 15);
+  p.k = (const int8_t*)L->k_alt; p.v = (const int8_t*)L->v_alt; p.ks = L->k_scale; p.vs = L->v_scale;
+  p.kv_dim = ctx->kv_dim; p.G = ctx->G; p.n_heads = nH; p.max_seq = L->max_seq;
+  p.rgw = rows <= 8 ? 1 : rows <= 16 ? 2 : 4;
+  p.seq = it.seq; p.lim0 = (int32_t)(it.pos + 1 - L->origin); p.n_rows = n_rows; p.n_cols = it.n_cols;
+  p.early = early ? 1u : 0u;
+  p.scale_log2 = (float)(1.4426950408889634 / sqrt((double)hd));
+  p.part_o = ctx->part_o; p.part_ml = ctx->part_ml;
+  p.gate = gate; p.gate_col_stride = gcs; p.gate_head_stride = ghs; p.out = out; p.out_col_stride = ocs; p.act_f16 = ctx->cfg.act_dtype == PA_F16;
+  const uint32_t ctas = ceil_div(rows, 8 * p.rgw) * ctx->cfg.n_kv_heads, tiles = ceil_div(n_rows, 64);
+  uint32_t ns = ctx->cfg.splits ? ctx->cfg.splits : std::max(1u, 2u * (uint32_t)ctx->sm_count / ctas);
+  ns = std::min(std::min(ns, std::max(1u, tiles / 2)), ctx->max_splits);
+  ns = (uint32_t)std::max<size_t>(1, std::min<size_t>(ns, ctx->pf_slots / ((size_t)it.n_cols * nH)));
+  p.n_splits = ns;
+  const uint32_t live = ceil_div(tiles, ceil_div(tiles, ns));
+  timing_mark(ctx, st, 0);
+  CU_TRY(ctx, launch_q8(p, hd, ctx->cfg.n_kv_heads, ctx->device, st));
+  timing_mark(ctx, st, 1);
+  ctx->stats.kernel_launches++;
+  ctx->stats.kv_bytes_streamed += 2ull * n_rows * (row_bytes_of(ctx, L->kv_format) + scale_row_bytes_of(ctx, L->kv_format));
+  if (live == 1 || ctx->core_only) return PA_OK;
+  if (live <= (uint32_t)kPrefillSplits) {
+    PrefillParams c{};
+    c.gate = gate; c.gate_col_stride = gcs; c.gate_head_stride = ghs; c.out = out; c.out_col_stride = ocs; c.act_f16 = p.act_f16;
+    c.n_cols = it.n_cols; c.n_heads = nH; c.part_o = ctx->part_o; c.part_ml = ctx->part_ml; c.n_splits = ns; c.merge_ns = live;
+    CU_TRY(ctx, launch_combine_few((int)hd, c, st));
+  } else {
+    CombineParams c{};
+    c.o = ctx->part_o; c.ml = ctx->part_ml;
+    c.o_row_stride = (uint64_t)ns * hd; c.o_part_stride = hd; c.ml_row_stride = (uint64_t)ns * 2; c.ml_part_stride = 2;
+    c.n_heads = nH; c.fixed_parts = live; c.n_splits = ns; c.groups = 1;
+    c.gate = gate; c.gate_col_stride = gcs; c.gate_head_stride = ghs; c.out = out; c.out_col_stride = ocs; c.act_f16 = p.act_f16;
+    c.err = ctx->dev_err;
+    CU_TRY(ctx, launch_combine((int)hd, c, it.n_cols * nH, st));
+  }
+  ctx->stats.kernel_launches++;
+  return PA_OK;
+}
+
 // Decode / verify / prefill over an int8 or f32 cache: per item, blocks of columns small enough for the record buffers;
 // each block is one launch of the plain split-K kernel (a CTA per (split, kv head, column)) and one combine.
 static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, const void* q, int q_dtype, uint64_t qcs, uint64_t qhs, const void* gate,
-                           uint64_t gcs, uint64_t ghs, void* out, uint64_t ocs, cudaStream_t st, const char* who) {
+                           uint64_t gcs, uint64_t ghs, void* out, uint64_t ocs, cudaStream_t st, const char* who, bool after_front = false) {
   pa_ctx* ctx = L->ctx;
   if (!q || !out) return fail(ctx, PA_EINVAL, "%s: null q or output", who);
   if (!items || n_items < 1) return fail(ctx, PA_EINVAL, "%s: no items", who);
@@ -661,6 +751,14 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
   uint64_t col = 0;
   for (uint32_t i = 0; i < n_items; ++i) {
     if (int rc = check_cols(L, items[i].seq, items[i].pos, items[i].n_cols, who)) return rc;
+    if (L->kv_format == PA_KV_Q8) {
+      if (int rc = decode_q8_item(L, items[i], reinterpret_cast<const uint8_t*>(q) + col * qcs * qes, q_dtype, qcs, qhs,
+                                  gate ? reinterpret_cast<const uint8_t*>(gate) + col * gcs * aes : nullptr, gcs, ghs,
+                                  reinterpret_cast<uint8_t*>(out) + col * ocs * aes, ocs, after_front, st))
+        return rc;
+      col += items[i].n_cols;
+      continue;
+    }
     for (uint32_t c0 = 0; c0 < items[i].n_cols; c0 += block) {
       const uint32_t nc = std::min(block, items[i].n_cols - c0);
       const uint32_t pos0 = items[i].pos + c0;
@@ -668,12 +766,12 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
       const uint32_t ns = plan_splits(ctx, rows, 1, nc, 1);
       AnyDecodeParams a{};
       a.q = reinterpret_cast<const uint8_t*>(q) + (col + c0) * qcs * qes; a.q_f16 = q_dtype == PA_F16; a.q_col_stride = qcs; a.q_head_stride = qhs;
-      a.k = L->k_alt; a.v = L->v_alt; a.ks = L->k_scale; a.vs = L->v_scale;
+      a.k = (const float*)L->k_alt; a.v = (const float*)L->v_alt;
       a.kv_dim = ctx->kv_dim; a.hd = hd; a.G = ctx->G; a.n_heads = nH; a.max_seq = L->max_seq; a.n_splits = ns;
       a.seq = items[i].seq; a.lim0 = (int32_t)(pos0 + 1 - L->origin); a.n_rows = rows; a.col0 = 0;
       a.part_o = ctx->part_o; a.part_ml = ctx->part_ml;
       timing_mark(ctx, st, 0);
-      CU_TRY(ctx, launch_decode_any(a, L->kv_format, dim3(ns, ctx->cfg.n_kv_heads, nc), st));
+      CU_TRY(ctx, launch_decode_f32(a, dim3(ns, ctx->cfg.n_kv_heads, nc), ctx->device, st));
       timing_mark(ctx, st, 1);
       CombineParams c{};
       c.o = ctx->part_o; c.ml = ctx->part_ml;
@@ -1008,9 +1106,10 @@ static int layer_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, 
   // into the caller's q_full.
   uint64_t kcs = kvcs;   // k's column stride (v keeps the caller's)
   // One token on the fused front normalises q and k in the decode kernel instead.
+  const bool alt_front = L->kv_format != PA_KV_F16 && !sharded && front_supports(ctx, ctx->cfg.rope_mode);   // one launch does it all
   const bool norm_in_front = L->qnorm_w && L->kv_format == PA_KV_F16 && (sharded || mode != PA_MODE_PREFILL) && can_fuse_norm(L) &&
                              can_fuse_front(ctx, n_cols, q, qcs, qhs, k, v);
-  if (L->qnorm_w && !ctx->core_only && !norm_in_front) {
+  if (L->qnorm_w && !ctx->core_only && !norm_in_front && !alt_front) {
     if (n_cols > ctx->cfg.max_cols) return fail(ctx, PA_EINVAL, "pa_attn_layer: %u columns exceed max_cols %u", n_cols, ctx->cfg.max_cols);
     HeadNormParams hp{};
     hp.x = q; hp.x_col_stride = qcs; hp.x_head_stride = qhs; hp.y = ctx->norm_q; hp.y_col_stride = ctx->q_dim; hp.y_head_stride = ctx->cfg.head_dim;
@@ -1031,12 +1130,16 @@ static int layer_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, 
   if (L->kv_format != PA_KV_F16) {
     if (sharded) return fail(ctx, PA_EUNSUPPORTED, "pa_attn_layer_sharded: the peer exchange is for f16 caches");
     if (n_cols > ctx->cfg.max_cols) return fail(ctx, PA_EINVAL, "pa_attn_layer: %u columns exceed max_cols %u", n_cols, ctx->cfg.max_cols);
-    if (!ctx->core_only)
-      if (int rc = rope_append_impl(L, ctx, seq, pos, n_cols, q, qcs, qhs, ctx->cfg.n_heads, ctx->q_rot, ctx->q_dim, k, v, kcs, cs_table, ctx->cfg.rope_mode,
-                                    ctx->cfg.act_dtype == PA_F16, st, 0, true, kvcs))
-        return rc;
+    if (!ctx->core_only) {
+      const int rc = alt_front ? front_impl(L, seq, pos, n_cols, q, qcs, qhs, ctx->q_rot, ctx->q_dim, k, v, kvcs, kvcs, ctx->cfg.rope_mode,
+                                            ctx->cfg.act_dtype == PA_F16, L->qnorm_w != nullptr, st)
+                               : rope_append_impl(L, ctx, seq, pos, n_cols, q, qcs, qhs, ctx->cfg.n_heads, ctx->q_rot, ctx->q_dim, k, v, kcs, cs_table,
+                                                  ctx->cfg.rope_mode, ctx->cfg.act_dtype == PA_F16, st, 0, true, kvcs);
+      if (rc) return rc;
+    }
     pa_item it{seq, pos, n_cols, 0};
-    return decode_any_impl(L, &it, 1, ctx->q_rot, PA_F32, ctx->q_dim, ctx->cfg.head_dim, gate, gcs, ghs, out, ocs, st, "pa_attn_layer");
+    return decode_any_impl(L, &it, 1, ctx->q_rot, PA_F32, ctx->q_dim, ctx->cfg.head_dim, gate, gcs, ghs, out, ocs, st, "pa_attn_layer",
+                           alt_front && !ctx->core_only);
   }
   if (sharded) {
     // this rank appends only if the new rows fall into its shard; every rank rotates q and decodes what it holds

@@ -1,14 +1,13 @@
 // KV caches in the other two formats pooled's engines keep: int8 with one f32 scale per 32 values (kvQ8: kv_store_q8 +
 // attn_flash_q8, engine/wgsl/qwen35.js:97-139, :908-946) and f32 (the dense engine, engine/wgsl/dense.js:22-136).
 //
-// The f16 cache has the TMA / tensor-core kernels of pa_decode.cu and pa_prefill.cu.  These two formats share one
-// split-K kernel of the same outer shape (one CTA per (split, kv head, column), an unnormalised (o, m, l) record per
-// (row, split) for pa_combine_kernel) built from plain vector loads: per chunk of 64 positions
+// The f16 cache has the TMA / tensor-core kernels of pa_decode.cu and pa_prefill.cu, the int8 cache pa_q8.cu.  The f32
+// cache has a split-K kernel of the same outer shape (one CTA per (split, kv head, column), an unnormalised (o, m, l)
+// record per (row, split) for pa_combine_kernel) built from plain vector loads: per chunk of 64 positions
 //   scores   four threads per K row, a quarter of the head each, the G heads of the group per thread; q in shared memory
 //   softmax  32 threads per head, online rescale across chunks (m starts at -3.0e38, as in the reference)
 //   values   a thread per four dims and group of positions, the groups summed in a fixed order at the end
 // A row of kv_dim values costs kv_dim * 1.125 bytes (int8) or kv_dim * 4 bytes (f32) against kv_dim * 2 for f16.
-// int8 values are dequantised as f32(int8) * scale, the order of the reference (attn_flash_q8's dot and vread).
 #include "pa_params.cuh"
 
 namespace pa {
@@ -65,51 +64,15 @@ cudaError_t launch_kv_store(const KvStoreParams& p, uint32_t n_cols, cudaStream_
   return launch_pdl(pa_kv_store_f32_kernel, dim3((p.kv_dim + 255) / 256, n_cols), dim3(256), 0, st, p);
 }
 
-// ---- split-K decode / verify / prefill over an int8 or f32 cache -----------------------------------------------
+// ---- split-K decode / verify / prefill over an f32 cache -----------------------------------------------
 
 constexpr int kAnyChunk = 64;     // positions per chunk
 constexpr int kAnyThreads = 256;
 constexpr int kAnyMaxG = 16;      // query heads per kv head
 
-template <int FMT> struct KvRead;
-template <> struct KvRead<PA_KV_Q8> {
-  // n consecutive values (n % 16 == 0) of a row starting at element e0 (e0 % 16 == 0)
-  template <typename F> static __device__ __forceinline__ void span(const void* cache, const float* scales, uint64_t row, uint32_t kv_dim, uint32_t e0, uint32_t n, F&& f) {
-    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const int8_t*>(cache) + row * kv_dim + e0);
-    const float* sc = scales + row * (kv_dim / 32);
-    for (uint32_t c = 0; c < n / 16; ++c) {
-      const uint4 w4 = src[c];
-      const float s = sc[(e0 + 16 * c) / 32];
-      const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) f(16 * c + 4 * j + b, __fmul_rn((float)(int8_t)(w[j] >> (8 * b)), s));
-    }
-  }
-  static __device__ __forceinline__ float4 quad(const void* cache, const float* scales, uint64_t row, uint32_t kv_dim, uint32_t e0) {
-    const uint32_t w = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const int8_t*>(cache) + row * kv_dim + e0);
-    const float s = scales[row * (kv_dim / 32) + e0 / 32];
-    return make_float4(__fmul_rn((float)(int8_t)w, s), __fmul_rn((float)(int8_t)(w >> 8), s), __fmul_rn((float)(int8_t)(w >> 16), s), __fmul_rn((float)(int8_t)(w >> 24), s));
-  }
-};
-template <> struct KvRead<PA_KV_F32> {
-  template <typename F> static __device__ __forceinline__ void span(const void* cache, const float*, uint64_t row, uint32_t kv_dim, uint32_t e0, uint32_t n, F&& f) {
-    const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(cache) + row * kv_dim + e0);
-    for (uint32_t c = 0; c < n / 4; ++c) {
-      const float4 x = src[c];
-      f(4 * c, x.x); f(4 * c + 1, x.y); f(4 * c + 2, x.z); f(4 * c + 3, x.w);
-    }
-  }
-  static __device__ __forceinline__ float4 quad(const void* cache, const float*, uint64_t row, uint32_t kv_dim, uint32_t e0) {
-    return *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(cache) + row * kv_dim + e0);
-  }
-};
-
 // grid (splits, kv heads, columns of one item).  Dynamic shared memory: q [G][hd] f32, then the chunk's scores /
 // weights [G][64], then m, l, alpha [G] each, then the values phase's partial sums.
-template <int FMT>
-__global__ void __launch_bounds__(kAnyThreads) pa_decode_any_kernel(const AnyDecodeParams p) {
+__global__ void __launch_bounds__(kAnyThreads) pa_decode_f32_any_kernel(const AnyDecodeParams p) {
   extern __shared__ float sm[];
   const uint32_t hd = p.hd, G = p.G, split = blockIdx.x, g = blockIdx.y, c = blockIdx.z;
   float* q_s = sm;                               // [G][hd]
@@ -151,10 +114,16 @@ __global__ void __launch_bounds__(kAnyThreads) pa_decode_any_kernel(const AnyDec
 #pragma unroll
       for (int h = 0; h < kAnyMaxG; ++h) s[h] = 0.f;
       if (r < n) {
-        KvRead<FMT>::span(p.k, p.ks, row0 + c0 + r, p.kv_dim, g * hd + part * span, span, [&](uint32_t i, float kv) {
+        const float4* src = reinterpret_cast<const float4*>(p.k + (row0 + c0 + r) * p.kv_dim + g * hd + part * span);
+        for (uint32_t i = 0; i < span; i += 4) {
+          const float4 x = src[i / 4];
 #pragma unroll
-          for (int h = 0; h < kAnyMaxG; ++h) if ((uint32_t)h < G) s[h] = __fmaf_rn(q_s[h * hd + part * span + i], kv, s[h]);
-        });
+          for (int h = 0; h < kAnyMaxG; ++h) {
+            if ((uint32_t)h >= G) break;
+            const float* qp = q_s + h * hd + part * span + i;
+            s[h] = __fmaf_rn(qp[3], x.w, __fmaf_rn(qp[2], x.z, __fmaf_rn(qp[1], x.y, __fmaf_rn(qp[0], x.x, s[h]))));
+          }
+        }
       }
 #pragma unroll
       for (int h = 0; h < kAnyMaxG; ++h) {
@@ -192,7 +161,7 @@ __global__ void __launch_bounds__(kAnyThreads) pa_decode_any_kernel(const AnyDec
       acc[h][0] *= a; acc[h][1] *= a; acc[h][2] *= a; acc[h][3] *= a;
     }
     for (uint32_t t = pg; t < n; t += n_pg) {
-      const float4 v = KvRead<FMT>::quad(p.v, p.vs, row0 + c0 + t, p.kv_dim, g * hd + dq * 4);
+      const float4 v = *reinterpret_cast<const float4*>(p.v + (row0 + c0 + t) * p.kv_dim + g * hd + dq * 4);
 #pragma unroll
       for (int h = 0; h < kAnyMaxG; ++h) {
         if ((uint32_t)h >= G) break;
@@ -229,21 +198,15 @@ size_t any_decode_smem(uint32_t G, uint32_t hd) {
   return ((((size_t)G * hd + (size_t)G * kAnyChunk + 3 * G + 3) & ~(size_t)3) + n_pg * G * hd) * sizeof(float);
 }
 
-cudaError_t launch_decode_any(const AnyDecodeParams& p, int format, dim3 grid, cudaStream_t st) {
+cudaError_t launch_decode_f32(const AnyDecodeParams& p, dim3 grid, int dev, cudaStream_t st) {
   const size_t smem = any_decode_smem(p.G, p.hd);
-  static bool attr_set[2][64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  auto kq = pa_decode_any_kernel<PA_KV_Q8>;
-  auto kf = pa_decode_any_kernel<PA_KV_F32>;
-  const int fi = format == PA_KV_Q8 ? 0 : 1;
-  if (!attr_set[fi][dev & 63]) {
-    cudaError_t e = fi == 0 ? cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)
-                            : cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  static bool attr_set[64] = {};
+  if (!attr_set[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(pa_decode_f32_any_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return e;
-    attr_set[fi][dev & 63] = true;
+    attr_set[dev & 63] = true;
   }
-  return fi == 0 ? launch_pdl(kq, grid, dim3(kAnyThreads), smem, st, p) : launch_pdl(kf, grid, dim3(kAnyThreads), smem, st, p);
+  return launch_pdl(pa_decode_f32_any_kernel, grid, dim3(kAnyThreads), smem, st, p);
 }
 
 }  // namespace pa

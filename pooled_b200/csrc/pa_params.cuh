@@ -122,14 +122,38 @@ struct KvStoreParams {
   uint32_t kv_dim; uint64_t cache_row0;          // cache row of column 0
 };
 
-// split-K decode / verify / prefill of the columns of one item over an int8 or f32 cache
+// split-K decode / verify / prefill of the columns of one item over an f32 cache
 struct AnyDecodeParams {
   const void* q; int q_f16; uint64_t q_col_stride, q_head_stride;
-  const void* k; const void* v; const float* ks; const float* vs;
+  const float* k; const float* v;
   uint32_t kv_dim, hd, G, n_heads, max_seq, n_splits;
   uint32_t seq; int32_t lim0; uint32_t n_rows;   // rows column 0 sees (before clamping), rows the last column sees
   uint64_t col0;                                 // first column of the item in q and in the record buffers
   float* part_o; float* part_ml;
+};
+
+// the front of a layer call in one launch (pa_front_kernel): head-norm, rotation, append in the cache's format
+struct FrontParams {
+  const void* q; uint64_t q_col_stride, q_head_stride; uint32_t q_heads;    // q == nullptr: k and v only
+  void* q_out; uint64_t q_out_col_stride; int q_out_f16; uint64_t q_lo_offset;   // as in RopeParams
+  const void* k; const void* v; uint64_t k_col_stride, v_col_stride; uint32_t kv_heads;
+  int format; void* k_cache; void* v_cache; float* k_scale; float* v_scale; uint64_t cache_row0;   // row of column 0
+  uint32_t n_cols; int in_f16;
+  const float* qn_w; const float* kn_w; double norm_eps;                    // nullptr: no head-norm
+  const Angle* angles; uint32_t n_ang; Angle ang[64];                       // as in RopeParams
+};
+
+// tensor-core attention over an int8 cache: the columns of one item (pa_q8_kernel)
+struct Q8Params {
+  const void* q; int q_f16; int q_vec; uint64_t q_col_stride, q_head_stride;   // q_vec: f32, every head row 16-byte aligned
+  const int8_t* k; const int8_t* v; const float* ks; const float* vs;
+  uint32_t kv_dim, G, n_heads, max_seq, n_splits, rgw;                      // rgw: 8-row groups per CTA
+  uint32_t seq; int32_t lim0; uint32_t n_rows, n_cols;                      // rows column 0 sees (before clamping), rows the last column sees
+  uint32_t early;                                                           // 1: rows older than the call's own may be fetched before the predecessor ends
+  float scale_log2;
+  float* part_o; float* part_ml;
+  const void* gate; uint64_t gate_col_stride, gate_head_stride;
+  void* out; uint64_t out_col_stride; int act_f16;
 };
 
 struct PrefillParams {
@@ -141,7 +165,7 @@ struct PrefillParams {
   float scale_log2;
   uint32_t* err;
   // split-K form (k-token verify on the tensor cores): one CTA per (split, kv head), rows = columns x heads of the group
-  float* part_o; float* part_ml; uint32_t n_splits; int32_t lim0; uint32_t n_rows, col0;
+  float* part_o; float* part_ml; uint32_t n_splits; uint32_t merge_ns; int32_t lim0; uint32_t n_rows, col0;
   uint32_t prefetch_old_rows;   // split-K form: K/V tiles wholly below the call's new rows may be fetched before the predecessor ends
   uint32_t early_limit;         // ... and below this row (the call before may still be writing its own row)
   uint32_t pre_stages;          // ... and only this many K tiles (one fewer V tiles) before the q loads are in flight

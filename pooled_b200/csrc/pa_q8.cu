@@ -1,0 +1,361 @@
+// Attention over an int8 KV cache (one f32 scale per 32 values) on the tensor cores: decode, blocks and prompts.
+//
+// The int8 values are exact in f16, so they enter mma.sync m16n8k16 unscaled and the scales are applied in f32 around it:
+//   scores   S[row, pos] = sum over 32-dim blocks b of ks[pos][b] * (q . k8)_b : a fresh accumulator per block, scaled
+//            and added in f32.  A (16 rows) holds q of eight query rows twice, the f16 high parts in rows 0-7 and the low
+//            parts in rows 8-15, B the int8 rows: both halves of the product come from one instruction.
+//   values   O^T[dim, row] += v8^T[dim, pos] . (P * vs)^T[pos, row] : the weights take each block's scale before they are
+//            split into high and low f16 parts.
+// q is first scaled by a power of two per row so that its largest value lies in [2^12, 2^13), P * vs by a running power of
+// two per warp so that the largest lies below 2^14 : high + low then carry 2^-24 of every value that matters, the
+// precision an f32 holds (an unscaled P * vs of 1e-4 would sit among f16's subnormals).
+//
+// A warp owns eight query rows (heads of the GQA group, columns) and runs an online softmax over the positions it takes,
+// P in registers from one product to the next; no barrier but the ring's.  A CTA is four warps over a ring of 64-position
+// tiles (cp.async, three or four tiles deep): with few query rows the warps share the positions of a tile and merge their (o, m, l)
+// at the end, with many each has rows of its own and all positions.  Two CTAs fit an SM.
+// What bounds it: conversions (int8 -> f16 costs a byte permute and an f16 subtraction per two values, and a warp
+// converts for its eight rows alone), about 700 instructions per 16 positions and eight rows against 64 MMAs; at long
+// contexts of a single token HBM (1.125 bytes a value).
+// Measured with its front (pa_front.cu) against plain f32 loops, a CTA per column: ten layers of a token over 12345 rows (16 q / 2 kv
+// heads x 256, head-norm) 918 -> 180 us, two layers of a 777-token prompt (24 / 4 x 256) 4231 -> 308 us; distance from float64
+// unchanged (4e-7 of the result between the two).
+//
+// Stands in for attn_flash_q8 of pooled (engine/wgsl/qwen35.js:946-1010 and its column-wise use in prefill).
+#include "pa_params.cuh"
+
+namespace pa {
+
+constexpr int kQ8Tile = 64, kQ8Threads = 128;
+
+template <int HD>
+struct Q8Smem {
+  static constexpr int NB = HD / 32;                       // scale blocks per row of a kv head
+  static constexpr int KB = kQ8Tile * HD, SB = kQ8Tile * NB * 4;
+  static constexpr int STAGE = 2 * KB + 2 * SB;            // K values, V values, K scales, V scales
+  static constexpr int STAGES = HD == 256 ? 3 : 4;
+  static constexpr int RING = STAGE * STAGES;
+  static constexpr int MERGE = 4 * 8 * (HD + 2) * 4;       // the warps' (o, m, l), over the idle ring
+  static constexpr int TOTAL = RING > MERGE ? RING : MERGE;
+};
+
+// 16-byte chunk c of row r, permuted so that the reads below hit 32 different banks: the score reads take four rows r ..
+// r + 3 at a time (8 bytes per lane), the value reads rows r, r + 2, r + 4, r + 6 (4 bytes per lane)
+template <int HD> __device__ __forceinline__ uint32_t q8_k_off(uint32_t r, uint32_t c) {
+  if (HD == 64) return r * HD + ((c ^ ((r >> 1) & 3u)) << 4);
+  return r * HD + ((c ^ (((r & 3u) << 1) | ((r >> 2) & 1u))) << 4);
+}
+template <int HD> __device__ __forceinline__ uint32_t q8_v_off(uint32_t r, uint32_t c) {
+  if (HD == 64) return r * HD + ((c ^ ((r >> 1) & 3u)) << 4);
+  return r * HD + ((c ^ (r & 7u)) << 4);
+}
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
+}
+// bytes (as v + 128) two at a time to f16: 0x6400 | u is 1024 + u, minus 1152 is v
+__device__ __forceinline__ uint32_t u8_h2(uint32_t w, uint32_t sel) {
+  const uint32_t x = prmt(w, 0x64646464u, sel);
+  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&x), __half2half2(__ushort_as_half(0x6480)));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ void split_h2(float x, float y, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x, y);
+  const float2 b = __half22float2(h);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = pack_h2(x - b.x, y - b.y);
+}
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp8(uint32_t dst, const void* src, bool live) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(live ? 8 : 0) : "memory");
+}
+
+// grid (splits, kv heads, row tiles).  rgw row groups per CTA (1, 2 or 4): warp w has row group w % rgw and takes the
+// 16-position steps w / rgw, w / rgw + 4 / rgw, ... of a tile.
+template <int HD>
+__global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) {
+  using L = Q8Smem<HD>;
+  constexpr int NB = L::NB;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t sm0 = smem_u32(smem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, j = lane & 3;
+  const uint32_t split = blockIdx.x, g = blockIdx.y, G = p.G, RT = 8 * p.rgw;
+  const uint32_t row0 = (gridDim.z - 1 - blockIdx.z) * RT, rows = p.n_cols * G;    // the longest rows first
+  const uint32_t rg = warp % p.rgw, pw = warp / p.rgw, n_pw = 4 / p.rgw;
+  // the plan is the call's (its last column's rows); a row tile stops at what its own last row sees
+  const uint32_t tiles = (p.n_rows + kQ8Tile - 1) / kQ8Tile;
+  const uint32_t ns_eff = min(p.n_splits, max(1u, tiles / 2)), tps = (tiles + ns_eff - 1) / max(ns_eff, 1u);
+  const uint32_t t_lo = split * tps;
+  if (t_lo >= tiles) return;                                  // no record expected from this split
+  auto row_lim = [&](uint32_t row) { return (uint32_t)min(max(p.lim0 + (int32_t)(min(row, rows - 1) / G), 0), (int32_t)p.n_rows); };
+  const uint32_t t_hi = min(min(tiles, t_lo + tps), (row_lim(row0 + RT - 1) + kQ8Tile - 1) / kQ8Tile);
+  const uint32_t n_tiles = t_hi > t_lo ? t_hi - t_lo : 0;
+  const uint64_t seq_row0 = (uint64_t)p.seq * p.max_seq;
+  const uint32_t kv_dim = p.kv_dim, nbk = kv_dim / 32;
+
+  auto load_tile = [&](uint32_t t) {      // one commit group per call, empty past the range
+    if (t < n_tiles) {
+      const uint32_t s = t % L::STAGES, pos0 = (t_lo + t) * kQ8Tile, base = sm0 + s * L::STAGE;
+      constexpr int CPR = HD / 16;
+#pragma unroll
+      for (int it = 0; it < kQ8Tile * CPR / kQ8Threads; ++it) {
+        const uint32_t idx = tid + it * kQ8Threads, rr = idx / CPR, c = idx % CPR;
+        const bool live = pos0 + rr < p.n_rows;
+        const uint64_t off = (seq_row0 + (live ? pos0 + rr : 0)) * kv_dim + (uint64_t)g * HD + c * 16;
+        cp16(base + q8_k_off<HD>(rr, c), p.k + off, live);
+        cp16(base + L::KB + q8_v_off<HD>(rr, c), p.v + off, live);
+      }
+      if (HD >= 128) {
+        constexpr int SC = NB >= 4 ? NB / 4 : 1;
+        for (uint32_t idx = tid; idx < kQ8Tile * SC; idx += kQ8Threads) {
+          const uint32_t rr = idx / SC, c = idx % SC;
+          const bool live = pos0 + rr < p.n_rows;
+          const uint64_t off = (seq_row0 + (live ? pos0 + rr : 0)) * nbk + g * NB + c * 4;
+          cp16(base + 2 * L::KB + rr * (NB * 4) + c * 16, p.ks + off, live);
+          cp16(base + 2 * L::KB + L::SB + rr * (NB * 4) + c * 16, p.vs + off, live);
+        }
+      } else if (tid < kQ8Tile) {
+        const bool live = pos0 + tid < p.n_rows;
+        const uint64_t off = (seq_row0 + (live ? pos0 + tid : 0)) * nbk + g * NB;
+        cp8(base + 2 * L::KB + tid * 8, p.ks + off, live);
+        cp8(base + 2 * L::KB + L::SB + tid * 8, p.vs + off, live);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // tiles of rows that the kernel before this one does not write may be fetched while it runs
+  const uint32_t old_rows = p.early ? p.n_rows - min(p.n_rows, p.n_cols) : 0u;
+  bool waited = false;
+#pragma unroll
+  for (int t = 0; t < L::STAGES - 1; ++t) {
+    if (!waited && (t_lo + t + 1) * kQ8Tile > old_rows) { pdl_wait(); waited = true; }
+    load_tile(t);
+  }
+  if (!waited) pdl_wait();
+  pdl_trigger();
+
+  // ---- this warp's eight query rows: thread (r, j) holds dims 32 b + 8 j .. + 7 of row r, as high and low f16 pairs ----
+  const uint32_t my_row = row0 + 8 * rg + r;
+  const bool live_row = my_row < rows;
+  uint32_t qa[2 * NB][4];
+  float q_scale;      // scores come out in log2 units
+  {
+    float x[NB][8];
+    const uint32_t qc = live_row ? my_row / G : 0, qh = live_row ? my_row % G : 0;
+    const uint64_t off = (uint64_t)qc * p.q_col_stride + (uint64_t)(g * G + qh) * p.q_head_stride + 8 * j;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      if (!live_row) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[b][e] = 0.f;
+      } else if (p.q_vec) {
+        const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.q) + off + 32 * b);
+        *reinterpret_cast<float4*>(&x[b][0]) = src[0]; *reinterpret_cast<float4*>(&x[b][4]) = src[1];
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[b][e] = ld_act(p.q, off + 32 * b + e, p.q_f16);
+      }
+    }
+    float mx = 0.f;
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) mx = fmaxf(mx, fabsf(x[b][e]));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    // times 2^(139 - e) with e the largest value's exponent field (at least 20, so that the factor is finite)
+    const uint32_t e = max(__float_as_uint(mx) >> 23, 20u);
+    const float up = __uint_as_float((266u - min(e, 254u)) << 23), down = __uint_as_float((min(e, 254u) - 12u) << 23);
+    q_scale = down * p.scale_log2;
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        split_h2(x[b][4 * h] * up, x[b][4 * h + 1] * up, qa[2 * b + h][0], qa[2 * b + h][1]);
+        split_h2(x[b][4 * h + 2] * up, x[b][4 * h + 3] * up, qa[2 * b + h][2], qa[2 * b + h][3]);
+      }
+  }
+  const uint32_t lim = live_row ? row_lim(my_row) : 0u;
+  const uint32_t warp_lim = row_lim(row0 + 8 * rg + 7);       // no position at or past it concerns this warp
+  const bool warp_live = row0 + 8 * rg < rows;
+
+  float m = -1.0e30f, l = 0.f;
+  uint32_t v_exp = 14;                                        // exponent field of the largest V scale so far
+  float oacc[2 * NB][4];
+#pragma unroll
+  for (int i = 0; i < 2 * NB; ++i) oacc[i][0] = oacc[i][1] = oacc[i][2] = oacc[i][3] = 0.f;
+
+  for (uint32_t t = 0; t < n_tiles; ++t) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(L::STAGES - 2) : "memory");
+    __syncthreads();                                          // tile t has landed for every thread, tile t - 1 is consumed
+    load_tile(t + L::STAGES - 1);
+    if (!warp_live) continue;
+    const uint8_t* kt = smem + (t % L::STAGES) * L::STAGE;
+    const uint8_t* vt = kt + L::KB;
+    const float* kst = reinterpret_cast<const float*>(kt + 2 * L::KB);
+    const float* vst = reinterpret_cast<const float*>(kt + 2 * L::KB + L::SB);
+#pragma unroll 1
+    for (uint32_t st = pw; st < kQ8Tile / 16; st += n_pw) {
+      const uint32_t pos0 = (t_lo + t) * kQ8Tile + 16 * st;
+      if (pos0 >= warp_lim) break;
+      // ---- scores of 16 positions: two groups of eight ----
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const uint32_t pr = 16 * st + 8 * n;
+        float k0[NB], k1[NB];                                  // scales of positions 2 j, 2 j + 1 of the group
+#pragma unroll
+        for (int b = 0; b < NB; b += (NB >= 4 ? 4 : 2)) {
+          if (NB >= 4) {
+            *reinterpret_cast<float4*>(&k0[b]) = *reinterpret_cast<const float4*>(kst + (pr + 2 * j) * NB + b);
+            *reinterpret_cast<float4*>(&k1[b]) = *reinterpret_cast<const float4*>(kst + (pr + 2 * j + 1) * NB + b);
+          } else {
+            *reinterpret_cast<float2*>(&k0[b]) = *reinterpret_cast<const float2*>(kst + (pr + 2 * j) * NB + b);
+            *reinterpret_cast<float2*>(&k1[b]) = *reinterpret_cast<const float2*>(kst + (pr + 2 * j + 1) * NB + b);
+          }
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          uint2 w = *reinterpret_cast<const uint2*>(kt + q8_k_off<HD>(pr + r, 2 * b + (j >> 1)) + (j & 1) * 8);
+          w.x ^= 0x80808080u; w.y ^= 0x80808080u;
+          float c[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_16816(c, qa[2 * b][0], qa[2 * b][1], qa[2 * b][2], qa[2 * b][3], u8_h2(w.x, 0x4140u), u8_h2(w.x, 0x4342u));
+          mma_16816(c, qa[2 * b + 1][0], qa[2 * b + 1][1], qa[2 * b + 1][2], qa[2 * b + 1][3], u8_h2(w.y, 0x4140u), u8_h2(w.y, 0x4342u));
+          s[2 * n] = __fmaf_rn(k0[b], c[0] + c[2], s[2 * n]);
+          s[2 * n + 1] = __fmaf_rn(k1[b], c[1] + c[3], s[2 * n + 1]);
+        }
+      }
+      // ---- mask, running maximum, weights ----
+      float mx = m;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t pos = pos0 + 8 * (e >> 1) + 2 * j + (e & 1);
+        s[e] = pos < lim ? s[e] * q_scale : -INFINITY;
+        mx = fmaxf(mx, s[e]);
+      }
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+      // ---- V scales of positions 2 j, 2 j + 1, 2 j + 8, 2 j + 9 and their largest exponent ----
+      float vsc[4][NB];
+      uint32_t ve = 0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t pr = 16 * st + 8 * (e >> 1) + 2 * j + (e & 1);
+#pragma unroll
+        for (int b = 0; b < NB; b += (NB >= 4 ? 4 : 2)) {
+          if (NB >= 4) *reinterpret_cast<float4*>(&vsc[e][b]) = *reinterpret_cast<const float4*>(vst + pr * NB + b);
+          else *reinterpret_cast<float2*>(&vsc[e][b]) = *reinterpret_cast<const float2*>(vst + pr * NB + b);
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b) ve = max(ve, __float_as_uint(vsc[e][b]) & 0x7fffffffu);
+      }
+      ve = min(__reduce_max_sync(0xffffffffu, ve) >> 23, 254u);
+      if (__any_sync(0xffffffffu, mx > m) || ve > v_exp) {
+        float al = exp2f(m - mx);
+        l *= al;
+        m = mx;
+        if (ve > v_exp) { al *= __uint_as_float((uint32_t)max(0, 127 - (int)(ve - v_exp)) << 23); v_exp = ve; }
+        const float a0 = __shfl_sync(0xffffffffu, al, 8 * j), a1 = __shfl_sync(0xffffffffu, al, 8 * j + 4);   // rows 2 j, 2 j + 1
+#pragma unroll
+        for (int i = 0; i < 2 * NB; ++i) { oacc[i][0] *= a0; oacc[i][1] *= a1; oacc[i][2] *= a0; oacc[i][3] *= a1; }
+      }
+      const float v_up = __uint_as_float((267u - v_exp) << 23);   // 2^(140 - field): the largest scale becomes 2^13 .. 2^14
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { s[e] = exp2f(s[e] - m); l += s[e]; s[e] *= v_up; }
+      // ---- values ----
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        uint32_t ph0, pl0, ph1, pl1;
+        split_h2(s[0] * vsc[0][b], s[1] * vsc[1][b], ph0, pl0);
+        split_h2(s[2] * vsc[2][b], s[3] * vsc[3][b], ph1, pl1);
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t pr = 16 * st + 8 * (e >> 1) + 2 * j + (e & 1);
+          w[e] = *reinterpret_cast<const uint32_t*>(vt + q8_v_off<HD>(pr, 2 * b + (r >> 2)) + (r & 3) * 4) ^ 0x80808080u;
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const uint32_t ta = prmt(w[0], w[1], e ? 0x7362u : 0x5140u), tb = prmt(w[2], w[3], e ? 0x7362u : 0x5140u);
+          const uint32_t a0 = u8_h2(ta, 0x4140u), a1 = u8_h2(ta, 0x4342u), a2 = u8_h2(tb, 0x4140u), a3 = u8_h2(tb, 0x4342u);
+          mma_16816(oacc[2 * b + e], a0, a1, a2, a3, ph0, ph1);
+          mma_16816(oacc[2 * b + e], a0, a1, a2, a3, pl0, pl1);
+        }
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();                                            // the ring is idle
+
+  // ---- the warps' (o, m, l) to shared memory, then one record (or the output) per query row ----
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  float* so = reinterpret_cast<float*>(smem) + warp * 8 * (HD + 2);   // [8][HD], then m[8], l[8]
+  const float v_down = __uint_as_float((v_exp - 13u) << 23);
+#pragma unroll
+  for (int i = 0; i < 2 * NB; ++i) {
+    const uint32_t d = 32 * (i >> 1) + 4 * r + 2 * (i & 1);
+    *reinterpret_cast<float2*>(so + (2 * j) * HD + d) = make_float2(oacc[i][0] * v_down, oacc[i][2] * v_down);
+    *reinterpret_cast<float2*>(so + (2 * j + 1) * HD + d) = make_float2(oacc[i][1] * v_down, oacc[i][3] * v_down);
+  }
+  if (j == 0) { so[8 * HD + r] = m; so[8 * HD + 8 + r] = l; }
+  __syncthreads();
+  const uint32_t n_rows_here = min(RT, rows - row0);
+  const uint32_t ns_live = (tiles + tps - 1) / tps;
+  for (uint32_t idx = tid; idx < n_rows_here * (HD / 4); idx += kQ8Threads) {
+    const uint32_t lr = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
+    const float* wb = reinterpret_cast<const float*>(smem) + (lr >> 3) * 8 * (HD + 2);      // the row group's first warp
+    const uint32_t step = p.rgw * 8 * (HD + 2), rr = lr & 7;
+    float M = -1.0e30f, Ls = 0.f;
+    for (uint32_t k = 0; k < n_pw; ++k) M = fmaxf(M, wb[k * step + 8 * HD + rr]);
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t k = 0; k < n_pw; ++k) {
+      const float w = exp2f(wb[k * step + 8 * HD + rr] - M);
+      const float4 x = *reinterpret_cast<const float4*>(wb + k * step + rr * HD + d);
+      Ls = __fmaf_rn(wb[k * step + 8 * HD + 8 + rr], w, Ls);
+      o.x = __fmaf_rn(x.x, w, o.x); o.y = __fmaf_rn(x.y, w, o.y); o.z = __fmaf_rn(x.z, w, o.z); o.w = __fmaf_rn(x.w, w, o.w);
+    }
+    const uint32_t row = row0 + lr, c = row / G, h = g * G + row % G;
+    if (ns_live > 1) {
+      const uint64_t slot = ((uint64_t)c * p.n_heads + h) * p.n_splits + split;
+      *reinterpret_cast<float4*>(p.part_o + slot * HD + d) = o;
+      if (d == 0) { p.part_ml[slot * 2] = M * 0.6931471805599453f; p.part_ml[slot * 2 + 1] = Ls; }
+      continue;
+    }
+    // a call of one split needs no merge: gate and store here
+    float ov[4] = {o.x, o.y, o.z, o.w};
+    const uint64_t go = (uint64_t)c * p.gate_col_stride + (uint64_t)h * p.gate_head_stride + d, oo = (uint64_t)c * p.out_col_stride + (uint64_t)h * HD + d;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      ov[e] = __fdiv_rn(ov[e], Ls);
+      if (p.gate) ov[e] = __fmul_rn(ov[e], __fdiv_rn(1.0f, __fadd_rn(1.0f, __expf(-ld_act(p.gate, go + e, p.act_f16)))));
+      if (p.act_f16) reinterpret_cast<__half*>(p.out)[oo + e] = __float2half_rn(ov[e]);
+      else reinterpret_cast<float*>(p.out)[oo + e] = ov[e];
+    }
+  }
+}
+
+template <int HD>
+static cudaError_t launch_q8_t(const Q8Params& p, dim3 grid, int dev, cudaStream_t st) {
+  static bool attr_set[64] = {};
+  if (!attr_set[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(pa_q8_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q8Smem<HD>::TOTAL);
+    if (e != cudaSuccess) return e;
+    attr_set[dev & 63] = true;
+  }
+  return launch_pdl(pa_q8_kernel<HD>, grid, dim3(kQ8Threads), (size_t)Q8Smem<HD>::TOTAL, st, p);
+}
+cudaError_t launch_q8(const Q8Params& p, uint32_t hd, uint32_t n_kv, int dev, cudaStream_t st) {
+  const dim3 grid(p.n_splits, n_kv, (p.n_cols * p.G + 8 * p.rgw - 1) / (8 * p.rgw));
+  switch (hd) {
+    case 256: return launch_q8_t<256>(p, grid, dev, st);
+    case 128: return launch_q8_t<128>(p, grid, dev, st);
+    case 64: return launch_q8_t<64>(p, grid, dev, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace pa

@@ -93,6 +93,65 @@ def test_layer_call_and_prefill_on_other_formats(fmt):
     util.assert_close(out, ref, f"{fmt} layer calls")
 
 
+@pytest.mark.parametrize("fmt,nH,nKV,hd", [("q8", 16, 1, 256), ("q8", 6, 2, 128), ("q8", 3, 1, 64), ("f32", 4, 4, 256), ("f32", 8, 4, 128), ("f32", 8, 2, 64), ("f32", 12, 4, 64)])
+def test_row_groups_splits_and_magnitudes(fmt, nH, nKV, hd):
+    # query rows of one, two and four 8-row groups and of several row tiles, contexts from one row to many splits, few
+    # and many records per row; scales from 1e-9 to 1e4 and q from 1e-6 to 30, which f16 operands cannot hold unscaled
+    import torch
+    rows = 2900
+    eng = _engine(fmt, nH, nKV, hd, rows + 4, max_cols=600)
+    rng = np.random.default_rng(5)
+    K = rng.standard_normal((rows, nKV * hd)).astype(np.float32); V = rng.standard_normal((rows, nKV * hd)).astype(np.float32)
+    mag = np.repeat(10.0 ** rng.uniform(-9, 0, (rows, nKV * hd // 32)), 32, axis=1).astype(np.float32)      # a scale per block
+    for k0 in range(0, rows, 580):
+        eng.kv_append(0, 0, k0, torch.from_numpy(K[k0:k0 + 580] * np.sqrt(mag[k0:k0 + 580])).cuda(), torch.from_numpy(V[k0:k0 + 580] * mag[k0:k0 + 580] * 1e4).cuda())
+    eng.sync()
+    Kh, Vh, _ = _held(eng, fmt, 0, rows)
+    for seq_len, nc in ((1, 1), (17, 1), (127, 2), (129, 3), (1500, 5), (rows, 1), (rows, 7), (500, 300), (2900, 70)):
+        pos = seq_len - nc
+        q = po.normal(10 + seq_len, nc * nH * hd).astype(np.float32).reshape(nc, nH, hd)
+        q *= (10.0 ** rng.uniform(-6, 1, (nc, nH, 1))).astype(np.float32)
+        if nc == 1:
+            q[0, 0] *= np.float32(30.0 / np.abs(q[0, 0]).max())     # logits stay below 50: f32 scores err by 50 * 2^-24 at most
+        q = q.reshape(nc, nH * hd)
+        out = eng.decode(0, [(0, pos, nc)], util.torch_dev(q)).cpu().numpy() if nc <= 8 else eng.prefill(0, 0, pos, util.torch_dev(q)).cpu().numpy()
+        eng.sync()
+        ref = po.attn_f64_kv32(q, Kh, Vh, nH, nKV, hd, pos, nc, None)
+        assert np.all(np.isfinite(out)) and util.errs(out, ref)[1] < util.REF_REL, f"{fmt} seq_len {seq_len} x {nc}: {util.errs(out, ref)}"
+
+
+@pytest.mark.parametrize("fmt,hd,n_rot,act,n_cols", [("q8", 256, 64, "f16", 1), ("q8", 128, 128, "f32", 3), ("q8", 128, 64, "f32", 70), ("f32", 64, 64, "f16", 2), ("f32", 256, 32, "f32", 5)])
+def test_front_of_a_layer_call_with_head_norm_keeps_the_bits(fmt, hd, n_rot, act, n_cols):
+    # head-norm, rotation and the format's append (in one launch where n_rot is 64, or 128 of 128): cache bytes as the CPU twins give them
+    import torch
+    from pooled_b200 import AttnConfig, AttnEngine
+    nH, nKV, theta, pos, eps = 4, 2, 1e6, 37, 1e-6
+    td = torch.float16 if act == "f16" else torch.float32
+    eng = AttnEngine(AttnConfig(n_heads=nH, n_kv_heads=nKV, head_dim=hd, n_rot=n_rot, rope_theta=theta, max_seq=256, act_dtype=td, max_cols=128, kv_format=fmt))
+    rng = np.random.default_rng(3)
+    mk = (lambda *s: util.normal_f16(int(rng.integers(1 << 20)), s)) if act == "f16" else (lambda *s: rng.standard_normal(s).astype(np.float32))
+    k0, v0 = mk(pos, nKV * hd), mk(pos, nKV * hd)
+    eng.kv_append(0, 0, 0, util.torch_dev(k0), util.torch_dev(v0))
+    q, k, v = mk(n_cols, 2 * nH * hd), mk(n_cols, nKV * hd), mk(n_cols, nKV * hd)       # q and gate interleaved
+    qw, kw = (1 + 0.1 * rng.standard_normal(hd)).astype(np.float32), (1 + 0.1 * rng.standard_normal(hd)).astype(np.float32)
+    eng.set_head_norm(0, util.torch_dev(qw), util.torch_dev(kw), eps)
+    dq = util.torch_dev(q, td)
+    out = eng.encode_layer(0, pos, dq, util.torch_dev(k, td), util.torch_dev(v, td), dq[:, hd:], q_head_stride=2 * hd, gate_head_stride=2 * hd).float().cpu().numpy()
+    eng.sync()
+    act_of = (lambda x: po.h2f(po.f16_rne(x))) if act == "f16" else (lambda x: x)
+    qh = np.ascontiguousarray(q.reshape(n_cols, nH, 2, hd)[:, :, 0]).reshape(n_cols, -1); g = np.ascontiguousarray(q.reshape(n_cols, nH, 2, hd)[:, :, 1]).reshape(n_cols, -1)
+    rot = lambda x, n, w: np.stack([po.rope_neox_f64(act_of(po.head_norm_f64(x[c], n, hd, w, eps)), n, hd, n_rot, pos + c, theta) for c in range(n_cols)])
+    kr, qr = rot(k, nKV, kw), rot(qh, nH, qw)
+    Kh, Vh, held = _held(eng, fmt, 0, pos + n_cols)
+    if fmt == "q8":
+        wk, wks = po.kv_store_q8(kr); wv, wvs = po.kv_store_q8(v)
+        assert np.array_equal(held[0][pos:], wk) and np.array_equal(held[2][pos:], wv)
+        assert np.array_equal(held[1][pos:].view(np.uint32), wks.view(np.uint32)) and np.array_equal(held[3][pos:].view(np.uint32), wvs.view(np.uint32))
+    else:
+        assert np.array_equal(Kh[pos:].view(np.uint32), kr.view(np.uint32)) and np.array_equal(Vh[pos:], v)
+    util.assert_close(out, po.attn_f64_kv32(qr, Kh, Vh, nH, nKV, hd, pos, n_cols, g), f"{fmt} layer call")
+
+
 def test_q8_state_round_trip_and_refusals():
     import torch
     from pooled_b200.lib import PaError
