@@ -23,6 +23,8 @@ bool rope_vec_applies(const RopeParams& p, uint32_t n_cols);
 cudaError_t launch_epoch_bump(unsigned int* ctr, cudaStream_t st);
 cudaError_t launch_head_norm(const HeadNormParams& p, cudaStream_t st);
 int prefill_supported(const pa_ctx* ctx);
+bool decode_f32_direct(uint32_t G);
+cudaError_t launch_decode_f32_direct(const F32DecodeParams& p, uint32_t hd, uint32_t G, uint32_t n_kv, cudaStream_t st);
 cudaError_t launch_q8(const Q8Params& p, uint32_t hd, uint32_t n_kv, int dev, cudaStream_t st);
 bool front_supported(uint32_t hd, uint32_t n_rot, bool rotates);
 cudaError_t launch_front(const FrontParams& p, uint32_t hd, uint32_t n_rot, cudaStream_t st);
@@ -763,20 +765,41 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
       const uint32_t nc = std::min(block, items[i].n_cols - c0);
       const uint32_t pos0 = items[i].pos + c0;
       const uint32_t rows = pos0 + nc - L->origin;                 // rows the block's last column sees
-      const uint32_t ns = plan_splits(ctx, rows, 1, nc, 1);
+      uint32_t ns = plan_splits(ctx, rows, 1, nc, 1), live = 0;
+      if (decode_f32_direct(ctx->G)) {
+        // rows in whole 16s over one CTA per SM; a short context gives every warp of a CTA its 16 rows before it takes more CTAs
+        ns = ctx->cfg.splits ? ctx->cfg.splits : std::max(1u, (uint32_t)ctx->sm_count / (ctx->cfg.n_kv_heads * nc));
+        ns = std::min(std::min(ns, ctx->max_splits), (uint32_t)(ctx->part_slots / ((size_t)nc * nH)));
+        F32DecodeParams f{};
+        f.rows_per_split = ceil_div(ceil_div(rows, std::max(1u, ns)), 16) * 16;
+        ns = live = ceil_div(rows, f.rows_per_split);
+        f.q = reinterpret_cast<const uint8_t*>(q) + (col + c0) * qcs * qes; f.q_f16 = q_dtype == PA_F16; f.q_col_stride = qcs; f.q_head_stride = qhs;
+        f.q_vec = q_dtype == PA_F32 && !(qcs & 3) && !(qhs & 3) && !((uintptr_t)f.q & 15);
+        f.k = (const float*)L->k_alt; f.v = (const float*)L->v_alt;
+        f.kv_dim = ctx->kv_dim; f.n_heads = nH; f.max_seq = L->max_seq; f.n_splits = ns;
+        f.seq = items[i].seq; f.lim0 = (int32_t)(pos0 + 1 - L->origin); f.n_rows = rows; f.n_cols = nc;
+        f.early = after_front && c0 == 0 ? 1u : 0u;   // (a later block of a wide call follows a merge, not the front)
+        f.scale_log2 = (float)(1.4426950408889634 / sqrt((double)hd));
+        f.part_o = ctx->part_o; f.part_ml = ctx->part_ml;
+        timing_mark(ctx, st, 0);
+        CU_TRY(ctx, launch_decode_f32_direct(f, hd, ctx->G, ctx->cfg.n_kv_heads, st));
+        timing_mark(ctx, st, 1);
+      }
       AnyDecodeParams a{};
       a.q = reinterpret_cast<const uint8_t*>(q) + (col + c0) * qcs * qes; a.q_f16 = q_dtype == PA_F16; a.q_col_stride = qcs; a.q_head_stride = qhs;
       a.k = (const float*)L->k_alt; a.v = (const float*)L->v_alt;
       a.kv_dim = ctx->kv_dim; a.hd = hd; a.G = ctx->G; a.n_heads = nH; a.max_seq = L->max_seq; a.n_splits = ns;
       a.seq = items[i].seq; a.lim0 = (int32_t)(pos0 + 1 - L->origin); a.n_rows = rows; a.col0 = 0;
       a.part_o = ctx->part_o; a.part_ml = ctx->part_ml;
-      timing_mark(ctx, st, 0);
-      CU_TRY(ctx, launch_decode_f32(a, dim3(ns, ctx->cfg.n_kv_heads, nc), ctx->device, st));
-      timing_mark(ctx, st, 1);
+      if (!live) {
+        timing_mark(ctx, st, 0);
+        CU_TRY(ctx, launch_decode_f32(a, dim3(ns, ctx->cfg.n_kv_heads, nc), ctx->device, st));
+        timing_mark(ctx, st, 1);
+      }
       CombineParams c{};
       c.o = ctx->part_o; c.ml = ctx->part_ml;
       c.o_row_stride = (uint64_t)ns * hd; c.o_part_stride = hd; c.ml_row_stride = (uint64_t)ns * 2; c.ml_part_stride = 2;
-      c.n_heads = nH; c.fixed_parts = 0; c.n_splits = ns; c.groups = 1;
+      c.n_heads = nH; c.fixed_parts = live; c.n_splits = ns; c.groups = 1;
       c.gate = gate ? reinterpret_cast<const uint8_t*>(gate) + (col + c0) * gcs * aes : nullptr; c.gate_col_stride = gcs; c.gate_head_stride = ghs;
       c.out = reinterpret_cast<uint8_t*>(out) + (col + c0) * ocs * aes; c.out_col_stride = ocs; c.act_f16 = ctx->cfg.act_dtype == PA_F16;
       c.items.seq[0] = items[i].seq; c.items.lim0[0] = a.lim0; c.items.n_rows[0] = rows; c.items.n_cols[0] = nc; c.items.col0[0] = 0; c.n_items = 1;

@@ -198,6 +198,147 @@ size_t any_decode_smem(uint32_t G, uint32_t hd) {
   return ((((size_t)G * hd + (size_t)G * kAnyChunk + 3 * G + 3) & ~(size_t)3) + n_pg * G * hd) * sizeof(float);
 }
 
+// The same for 1, 2 or 4 heads per kv head (the dense engine's models have 2), straight from memory to registers: HD / 16
+// lanes share a row, 16 dims each, so a warp instruction reads whole rows, and a warp requests the K and the V of 16 (head_dim
+// 64: 32, 256: 8; with four heads half of that) rows together, 128 registers a thread, before it uses the first: 128 KB
+// in flight per SM, which is what HBM's latency takes at full rate.  No barrier and no shared memory until the warps' (o, m, l) are merged at the end.  A CTA's
+// rows are one or two such batches per warp at the contexts these caches serve.  28 layers of a token over 2000 rows (16 q / 8 kv
+// heads x 128), whole calls: 644 us with the chunked kernel above, 360 us with this one (floor 69: 459 MB).
+template <int HD, int G>
+__global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodeParams p) {
+  constexpr int LPR = HD / 16, RPI = 32 / LPR, U = G == 4 ? 2 : 4, BATCH = RPI * U;   // lanes per row, rows per instruction and per batch
+  extern __shared__ float sm[];                                             // [8 warps][G][HD], then m[8][G], l[8][G]
+  const uint32_t split = blockIdx.x, g = blockIdx.y, c = blockIdx.z;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = lane / LPR, lr = lane % LPR;
+  const uint32_t lim = (uint32_t)min(max(p.lim0 + (int32_t)c, 0), (int32_t)p.n_rows);
+  const uint32_t r_lo = split * p.rows_per_split, r_hi = min(r_lo + p.rows_per_split, lim);
+  const uint64_t base = ((uint64_t)p.seq * p.max_seq) * p.kv_dim + (uint64_t)g * HD + lr * 4;
+  float4 k[U][4], v[U][4];
+  auto load = [&](uint32_t b0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t row = b0 + u * RPI + sub;
+      const float* kp = p.k + base + (uint64_t)row * p.kv_dim;
+      const float* vp = p.v + base + (uint64_t)row * p.kv_dim;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) k[u][i] = row < r_hi ? __ldcg(reinterpret_cast<const float4*>(kp + i * LPR * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[u][i] = row < r_hi ? __ldcg(reinterpret_cast<const float4*>(vp + i * LPR * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  uint32_t b0 = r_lo + warp * BATCH;
+  // rows the kernel before this one does not write may be fetched while it runs
+  const bool ahead = p.early && b0 + BATCH <= p.n_rows - min(p.n_rows, p.n_cols);
+  if (ahead && b0 < r_hi) load(b0);
+  pdl_wait();
+  pdl_trigger();
+  if (!ahead && b0 < r_hi) load(b0);
+  const uint64_t col = c;
+  float4 q[G][4];
+#pragma unroll
+  for (int h = 0; h < G; ++h)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint64_t off = col * p.q_col_stride + (uint64_t)(g * G + h) * p.q_head_stride + i * LPR * 4 + lr * 4;
+      if (p.q_vec) q[h][i] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.q) + off);
+      else q[h][i] = make_float4(ld_act(p.q, off, p.q_f16), ld_act(p.q, off + 1, p.q_f16), ld_act(p.q, off + 2, p.q_f16), ld_act(p.q, off + 3, p.q_f16));
+    }
+  float m[G], l[G];
+  float4 o[G][4];
+#pragma unroll
+  for (int h = 0; h < G; ++h) {
+    m[h] = -1.0e30f; l[h] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[h][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  while (b0 < r_hi) {
+#pragma unroll
+    for (int h = 0; h < G; ++h) {
+      float s[U], mx = m[h];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float a = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          a = __fmaf_rn(q[h][i].w, k[u][i].w, __fmaf_rn(q[h][i].z, k[u][i].z, __fmaf_rn(q[h][i].y, k[u][i].y, __fmaf_rn(q[h][i].x, k[u][i].x, a))));
+#pragma unroll
+        for (int x = LPR / 2; x > 0; x >>= 1) a += __shfl_xor_sync(0xffffffffu, a, x);
+        s[u] = b0 + u * RPI + sub < r_hi ? a * p.scale_log2 : -INFINITY;
+        mx = fmaxf(mx, s[u]);
+      }
+#pragma unroll
+      for (int x = LPR; x < 32; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+      const float al = exp2f(m[h] - mx);
+      m[h] = mx; l[h] *= al;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { o[h][i].x *= al; o[h][i].y *= al; o[h][i].z *= al; o[h][i].w *= al; }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float w = exp2f(s[u] - mx);
+        l[h] += w;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          o[h][i].x = __fmaf_rn(w, v[u][i].x, o[h][i].x); o[h][i].y = __fmaf_rn(w, v[u][i].y, o[h][i].y);
+          o[h][i].z = __fmaf_rn(w, v[u][i].z, o[h][i].z); o[h][i].w = __fmaf_rn(w, v[u][i].w, o[h][i].w);
+        }
+      }
+    }
+    b0 += 8 * BATCH;
+    if (b0 < r_hi) load(b0);
+  }
+  // ---- the row groups of a warp, then the warps ----
+  float* so = sm + warp * G * HD;
+  float* sml = sm + 8 * G * HD;
+#pragma unroll
+  for (int h = 0; h < G; ++h) {
+#pragma unroll
+    for (int x = LPR; x < 32; x <<= 1) {
+      l[h] += __shfl_xor_sync(0xffffffffu, l[h], x);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        o[h][i].x += __shfl_xor_sync(0xffffffffu, o[h][i].x, x); o[h][i].y += __shfl_xor_sync(0xffffffffu, o[h][i].y, x);
+        o[h][i].z += __shfl_xor_sync(0xffffffffu, o[h][i].z, x); o[h][i].w += __shfl_xor_sync(0xffffffffu, o[h][i].w, x);
+      }
+    }
+    if (sub == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(so + h * HD + i * LPR * 4 + lr * 4) = o[h][i];
+    }
+    if (lane == 0) { sml[warp * G + h] = m[h]; sml[8 * G + warp * G + h] = l[h]; }
+  }
+  __syncthreads();
+  for (uint32_t idx = tid; idx < G * HD; idx += 256) {
+    const uint32_t h = idx / HD, d = idx % HD;
+    float M = sml[h], L = 0.f, a = 0.f;
+#pragma unroll
+    for (int w = 1; w < 8; ++w) M = fmaxf(M, sml[w * G + h]);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const float e = exp2f(sml[w * G + h] - M);
+      L = __fmaf_rn(sml[8 * G + w * G + h], e, L);
+      a = __fmaf_rn(sm[w * G * HD + idx], e, a);
+    }
+    const uint64_t slot = (col * p.n_heads + g * G + h) * p.n_splits + split;
+    p.part_o[slot * HD + d] = a;
+    if (d == 0) { p.part_ml[slot * 2] = M * 0.6931471805599453f; p.part_ml[slot * 2 + 1] = L; }
+  }
+}
+
+template <int HD, int G>
+static cudaError_t launch_f32_t(const F32DecodeParams& p, dim3 grid, cudaStream_t st) {
+  return launch_pdl(pa_decode_f32_kernel<HD, G>, grid, dim3(256), (size_t)(8 * G * (HD + 2)) * 4, st, p);
+}
+bool decode_f32_direct(uint32_t G) { return G == 1 || G == 2 || G == 4; }
+cudaError_t launch_decode_f32_direct(const F32DecodeParams& p, uint32_t hd, uint32_t G, uint32_t n_kv, cudaStream_t st) {
+  const dim3 grid(p.n_splits, n_kv, p.n_cols);
+#define PA_F32_CASE(H) case H: return G == 1 ? launch_f32_t<H, 1>(p, grid, st) : G == 2 ? launch_f32_t<H, 2>(p, grid, st) : launch_f32_t<H, 4>(p, grid, st);
+  switch (hd) {
+    PA_F32_CASE(256) PA_F32_CASE(128) PA_F32_CASE(64)
+    default: return cudaErrorInvalidValue;
+  }
+#undef PA_F32_CASE
+}
+
 cudaError_t launch_decode_f32(const AnyDecodeParams& p, dim3 grid, int dev, cudaStream_t st) {
   const size_t smem = any_decode_smem(p.G, p.hd);
   static bool attr_set[64] = {};

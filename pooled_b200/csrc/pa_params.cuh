@@ -132,6 +132,16 @@ struct AnyDecodeParams {
   float* part_o; float* part_ml;
 };
 
+// the same for 1, 2 or 4 heads per kv head (pa_decode_f32_kernel): columns 0 .. n_cols - 1 of one item
+struct F32DecodeParams {
+  const void* q; int q_f16; int q_vec; uint64_t q_col_stride, q_head_stride;   // q_vec: f32, every head row 16-byte aligned
+  const float* k; const float* v;
+  uint32_t kv_dim, n_heads, max_seq, n_splits, rows_per_split;
+  uint32_t seq; int32_t lim0; uint32_t n_rows, n_cols, early;                  // as in Q8Params
+  float scale_log2;
+  float* part_o; float* part_ml;
+};
+
 // the front of a layer call in one launch (pa_front_kernel): head-norm, rotation, append in the cache's format
 struct FrontParams {
   const void* q; uint64_t q_col_stride, q_head_stride; uint32_t q_heads;    // q == nullptr: k and v only
