@@ -114,6 +114,7 @@ class AttnEngine:
     def __init__(self, cfg: AttnConfig, device: int = 0):
         self.cfg, self.device = cfg, device
         self.L = _l.load()
+        self._call = self.L.call
         pc = _l.PaConfig(n_heads=cfg.n_heads, n_kv_heads=cfg.n_kv_heads, head_dim=cfg.head_dim, n_rot=cfg.n_rot, rope_theta=cfg.rope_theta,
                          rope_mode=_ROPE[cfg.rope_mode], act_dtype=_dt(cfg.act_dtype), max_cols=cfg.max_cols, splits=cfg.splits,
                          flags=_l.PA_FLAG_FAST if cfg.fast else 0)
@@ -143,6 +144,9 @@ class AttnEngine:
     # ---- plumbing ----
     def _st(self):
         return C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+
+    def _raw_st(self) -> int:
+        return torch._C._cuda_getCurrentRawStream(self.device)
 
     def _ck(self, rc: int):
         self.L.check(rc, self.ctx)
@@ -230,8 +234,9 @@ class AttnEngine:
                     cs_table: torch.Tensor | None = None) -> torch.Tensor:
         n_cols = q.shape[0]
         q_rot = torch.empty((n_cols, self.cfg.q_dim), dtype=torch.float32, device=q.device)
-        self._ck(self.L.pa_rope_append(self.layers[li], seq, pos, n_cols, self._p(q), q.stride(0), q_head_stride or self.cfg.head_dim, self._p(k),
-                                       self._p(v), k.stride(0), self._p(cs_table), self._p(q_rot), self._st()))
+        rc = self._call.rope_append(self.layers[li].value, seq, pos, q, q_head_stride or self.cfg.head_dim, k, v, cs_table, q_rot, self._raw_st())
+        if rc:
+            self._ck(rc)
         return q_rot
 
     def rope_append_items(self, li: int, seqs_pos, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, q_head_stride: int | None = None) -> torch.Tensor:
@@ -248,13 +253,13 @@ class AttnEngine:
                      gate_head_stride: int | None = None) -> torch.Tensor:
         """One decode token of each of several sequences through the layer in one C-ABI call: seqs_pos = [(seq, pos)],
         row i of q / k / v / gate / out belongs to item i.  sharded: KV-sequence shards with the peer exchange."""
-        n = len(seqs_pos)
+        hd = self.cfg.head_dim
         if out is None:
-            out = torch.empty((n, self.cfg.q_dim), dtype=self.cfg.act_dtype, device=q.device)
-        gp, gcs, ghs = self._gate(gate, gate_head_stride)
-        self._ck(self.L.pa_attn_items(self.layers[li], self._items([(s, p, 1) for s, p in seqs_pos]), n, self._p(q), q.stride(0),
-                                      q_head_stride or self.cfg.head_dim, self._p(k), self._p(v), k.stride(0), gp, gcs, ghs, self._p(out),
-                                      out.stride(0), 1 if sharded else 0, self._st()))
+            out = torch.empty((len(seqs_pos), self.cfg.q_dim), dtype=self.cfg.act_dtype, device=q.device)
+        rc = self._call.attn_items(self.layers[li].value, seqs_pos, q, q_head_stride or hd, k, v, gate, gate_head_stride or hd, out, 1 if sharded else 0,
+                                   self._raw_st())
+        if rc:
+            self._ck(rc)
         return out
 
     def _items(self, items):
@@ -287,9 +292,11 @@ class AttnEngine:
         assert row_lists.dtype == torch.int32 and row_lists.is_cuda and row_lists.shape[0] == n_cols and row_lists.is_contiguous()
         if out is None:
             out = torch.empty((n_cols, self.cfg.q_dim), dtype=self.cfg.act_dtype, device=q.device)
-        gp, gcs, ghs = self._gate(gate, gate_head_stride)
-        self._ck(self.L.pa_decode_gather(self.layers[li], seq, n_cols, self._p(row_lists), row_lists.shape[1], self._p(q), _dt(q.dtype), q.stride(0),
-                                         q_head_stride or self.cfg.head_dim, gp, gcs, ghs, self._p(out), out.stride(0), self._st()))
+        hd = self.cfg.head_dim
+        rc = self._call.decode_gather(self.layers[li].value, seq, row_lists, row_lists.shape[1], q, _dt(q.dtype), q_head_stride or hd, gate, gate_head_stride or hd, out,
+                                      self._raw_st())
+        if rc:
+            self._ck(rc)
         return out
 
     def decode_partial(self, li: int, items, q: torch.Tensor, q_head_stride: int | None = None) -> torch.Tensor:
@@ -353,12 +360,13 @@ class AttnEngine:
 
         One token is the attention block of _encodeLayerR (engine/qwen35.js:1598-1640); several are _encAttnGlue +
         _encAttnCore (engine/qwen35.js:2473-2517): all columns' K/V are appended before any column attends."""
-        n_cols = q.shape[0]
+        hd = self.cfg.head_dim
         if out is None:
-            out = torch.empty((n_cols, self.cfg.q_dim), dtype=self.cfg.act_dtype, device=q.device)
-        gp, gcs, ghs = self._gate(gate, gate_head_stride)
-        self._ck(self.L.pa_attn_layer(self.layers[li], seq, pos, n_cols, _MODE[mode], self._p(q), q.stride(0), q_head_stride or self.cfg.head_dim,
-                                      self._p(k), self._p(v), k.stride(0), gp, gcs, ghs, self._p(cs_table), self._p(out), out.stride(0), self._st()))
+            out = torch.empty((q.shape[0], self.cfg.q_dim), dtype=self.cfg.act_dtype, device=q.device)
+        rc = self._call.attn_layer(self.layers[li].value, seq, pos, _MODE[mode], q, q_head_stride or hd, k, v, gate, gate_head_stride or hd, cs_table, out,
+                                   self._raw_st())
+        if rc:
+            self._ck(rc)
         return out
 
     def encode_layer_host(self, li: int, pos: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: torch.Tensor | None, out: torch.Tensor,

@@ -5,10 +5,12 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libpooled_attn.so")
+CALL_OUT = os.path.join(HERE, "_pa_call.so")      # CPython module: the per-layer calls without ctypes
 SOURCES = ["pa_api.cu", "pa_rope_append.cu", "pa_decode.cu", "pa_prefill.cu", "pa_kvfmt.cu", "pa_q8.cu", "pa_front.cu", "pa_noalloc.cu"]
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo", "--use_fast_math=false",
          "-Xcompiler", "-fPIC,-fvisibility=hidden", "--expt-relaxed-constexpr"]
@@ -26,9 +28,9 @@ def _deps() -> list[str]:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(OUT):
+    if not os.path.exists(OUT) or not os.path.exists(CALL_OUT):
         return True
-    t = os.path.getmtime(OUT)
+    t = min(os.path.getmtime(OUT), os.path.getmtime(CALL_OUT))
     return any(os.path.getmtime(d) > t for d in _deps())
 
 
@@ -54,6 +56,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
         failed |= p.returncode != 0
     if failed:
         raise RuntimeError("nvcc failed")
+    cc = shutil.which("gcc") or shutil.which("cc")
+    if not cc:
+        raise RuntimeError("a C compiler is needed for the call module")
+    subprocess.check_call([cc, "-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], os.path.join(CSRC, "pa_call.c"), "-o", CALL_OUT])
     subprocess.check_call([nvcc(), "-shared", "-o", OUT, *objs, "-lcudart_static", "-lpthread", "-ldl", "-lrt"])
     return OUT
 

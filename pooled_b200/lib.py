@@ -2,10 +2,13 @@
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SO_PATH = os.path.join(HERE, "libpooled_attn.so")
+CALL_PATH = os.path.join(HERE, "_pa_call.so")
 
 PA_F32, PA_F16 = 0, 1
 PA_ROPE_NONE, PA_ROPE_F64, PA_ROPE_TABLE = 0, 1, 2
@@ -114,6 +117,17 @@ class Lib:
             fn = getattr(self.dll, name)   # AttributeError when the library lacks a declared symbol
             fn.restype, fn.argtypes = res, args
             setattr(self, name, fn)
+        self.call = self._load_call()
+
+    def _load_call(self):
+        """The CPython module with the per-layer calls (csrc/pa_call.c), bound to this library's entry points."""
+        if not os.path.exists(CALL_PATH):
+            raise PaError(-4, f"{CALL_PATH} is missing: build it with `python -m pooled_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_pa_call", CALL_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_pa_call", CALL_PATH, loader=loader))
+        loader.exec_module(mod)
+        mod.bind(*(C.cast(getattr(self.dll, n), C.c_void_p).value for n in ("pa_attn_layer", "pa_attn_items", "pa_rope_append", "pa_decode_gather")))
+        return mod
 
     def check(self, rc: int, ctx=None):
         if rc != 0:
