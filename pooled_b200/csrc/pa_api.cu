@@ -501,6 +501,11 @@ static int front_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, 
   }
   CU_TRY(ctx, launch_front(p, ctx->cfg.head_dim, half ? ctx->cfg.n_rot : 0, st));
   ctx->stats.kernel_launches++;
+  if (L->kv_format == PA_KV_F16) {   // as rope_append_impl: the rows that may still be in flight
+    uint32_t r0 = pos - L->origin;
+    if (ctx->inflight_layer == L && ctx->inflight_row0 < r0) r0 = ctx->inflight_row0;
+    ctx->inflight_layer = L; ctx->inflight_row0 = r0;
+  }
   return PA_OK;
 }
 
@@ -1132,7 +1137,12 @@ static int layer_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, 
   const bool alt_front = L->kv_format != PA_KV_F16 && !sharded && front_supports(ctx, ctx->cfg.rope_mode);   // one launch does it all
   const bool norm_in_front = L->qnorm_w && L->kv_format == PA_KV_F16 && (sharded || mode != PA_MODE_PREFILL) && can_fuse_norm(L) &&
                              can_fuse_front(ctx, n_cols, q, qcs, qhs, k, v);
-  if (L->qnorm_w && !ctx->core_only && !norm_in_front && !alt_front) {
+  // Blocks and chunks over an f16 cache: the front kernel takes a head-norm along (two launches and a round trip of q and
+  // k through memory otherwise), and chunks of f32 activations, whose RoPE kernel is a CTA per column (eight layers of
+  // 203 columns of 24 + 4 heads with a norm, whole calls: 765 us with the separate kernels, 598 us with this one); f16 chunks without a norm keep the vectorised kernel, which copies less.
+  const bool f16_front = L->kv_format == PA_KV_F16 && !sharded && !norm_in_front && !ctx->core_only && ctx->cfg.rope_mode == PA_ROPE_F64 &&
+                         front_supports(ctx, PA_ROPE_F64) && (L->qnorm_w || (n_cols >= 16 && ctx->cfg.act_dtype == PA_F32));
+  if (L->qnorm_w && !ctx->core_only && !norm_in_front && !alt_front && !f16_front) {
     if (n_cols > ctx->cfg.max_cols) return fail(ctx, PA_EINVAL, "pa_attn_layer: %u columns exceed max_cols %u", n_cols, ctx->cfg.max_cols);
     HeadNormParams hp{};
     hp.x = q; hp.x_col_stride = qcs; hp.x_head_stride = qhs; hp.y = ctx->norm_q; hp.y_col_stride = ctx->q_dim; hp.y_head_stride = ctx->cfg.head_dim;
@@ -1211,9 +1221,13 @@ static int layer_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, 
   // where that kernel fetches its query rows by TMA, the dims no rotation touches (192 of 256 in the hybrid models)
   // are not copied at all: the kernel takes those chunks from the caller's q and only the rotated chunk from q_rot
   const uint32_t rot = ctx->cfg.n_rot;
-  bool rot_only = prefill && !ctx->core_only && ctx->cfg.act_dtype == PA_F16 && ctx->cfg.rope_mode == PA_ROPE_F64 && rot >= 64 && rot % 64 == 0 &&
+  bool rot_only = prefill && !f16_front && !ctx->core_only && ctx->cfg.act_dtype == PA_F16 && ctx->cfg.rope_mode == PA_ROPE_F64 && rot >= 64 && rot % 64 == 0 &&
                   rot < ctx->cfg.head_dim && q_tma_ok(ctx, PA_F16, qcs, qhs, q) && q_tma_ok(ctx, PA_F16, ctx->q_dim, ctx->cfg.head_dim, ctx->q_rot);
-  if (!ctx->core_only)
+  if (f16_front) {
+    if (int rc = front_impl(L, seq, pos, n_cols, q, qcs, qhs, ctx->q_rot, ctx->q_dim, k, v, kvcs, kvcs, ctx->cfg.rope_mode, ctx->cfg.act_dtype == PA_F16,
+                            L->qnorm_w != nullptr, st, prefill ? 1 : (planes ? 2 : 0)))
+      return rc;
+  } else if (!ctx->core_only)
     if (int rc = rope_append_impl(L, ctx, seq, pos, n_cols, q, qcs, qhs, ctx->cfg.n_heads, ctx->q_rot, ctx->q_dim, k, v, kcs, cs_table, ctx->cfg.rope_mode,
                                   ctx->cfg.act_dtype == PA_F16, st, prefill ? 1 : (planes ? 2 : 0), true, kvcs, &rot_only))
       return rc;
