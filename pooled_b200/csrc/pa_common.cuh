@@ -251,6 +251,9 @@ struct ItemList {
   uint32_t n_cols[kMaxItems];
   uint32_t col0[kMaxItems];    // first column of the item in q / gate / out
   uint32_t pos[kMaxItems];     // position of the item's first column
+  // balanced plan of a batch of unequal lengths (tps[0] != 0): tiles per split of each item, and its first CTA in
+  // blockIdx.x; otherwise blockIdx.z is the item and the split plan follows from n_splits and the item's rows
+  uint16_t tps[kMaxItems], cta0[kMaxItems];
 };
 
 // Peer exchange of merged (o, m, l) records between the GPUs of one box.  Every rank owns one buffer that all ranks

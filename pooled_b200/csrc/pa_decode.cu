@@ -276,7 +276,13 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
   constexpr int MT = HD / 64;        // 16-dim output tiles per consumer warp
   constexpr int CH = HD / 64;        // 128-byte chunks per cache row of one kv head
 
-  const uint32_t split = blockIdx.x, g = blockIdx.y, item = blockIdx.z;
+  const uint32_t g = blockIdx.y;
+  uint32_t split = blockIdx.x, item = blockIdx.z;
+  const bool balanced = p.items.tps[0] != 0;
+  if (balanced) {   // the CTAs of the items follow one another (an item without rows has none)
+    for (uint32_t i = 1; i < p.n_items; ++i) if (blockIdx.x >= p.items.cta0[i]) item = i;
+    split = blockIdx.x - p.items.cta0[item];
+  }
   if (p.xch_ctr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) {
     pdl_wait();                    // the exchanging call before this one has read the counter
     atomicAdd(p.xch_ctr, 1u);      // this call's number: its combine kernel starts after this kernel's end
@@ -291,7 +297,7 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
   // every item plans for its own length: at least two tiles per CTA, at most the launch's split count (the longest
   // item's plan, or in gather mode the most any list could need)
   const uint32_t ns_eff = min(p.n_splits, max(1u, tiles / 2));
-  const uint32_t tps = (tiles + ns_eff - 1) / max(ns_eff, 1u);  // tiles per split
+  const uint32_t tps = balanced ? p.items.tps[item] : (tiles + ns_eff - 1) / max(ns_eff, 1u);  // tiles per split
   const uint32_t tile0 = split * tps;
   if (tile0 >= tiles) {
     if constexpr (NT <= 2) {
@@ -1196,7 +1202,7 @@ __global__ void __launch_bounds__(256) pa_combine_kernel(const CombineParams p) 
     const uint32_t n_rows = p.gather ? min(p.gather[(size_t)col * p.gather_stride], p.gather_stride - 1u) : p.items.n_rows[it];
     const uint32_t tiles = (n_rows + kT - 1) / kT;
     const uint32_t n_sp = min(p.n_splits, max(1u, tiles / 2));
-    const uint32_t tps = (tiles + n_sp - 1) / max(n_sp, 1u);
+    const uint32_t tps = p.items.tps[0] ? p.items.tps[it] : (tiles + n_sp - 1) / max(n_sp, 1u);
     ns = tiles ? ((tiles + tps - 1) / tps) * p.groups : 0;   // a shard that holds no row of the item: an empty record
   }
   // Everything the CTA reads is requested before the first use: the (m, l) pairs, the o records of the first 128

@@ -44,7 +44,7 @@ struct DecodeParams {
   const void* gate; uint64_t gate_col_stride, gate_head_stride;
   void* out; uint64_t out_col_stride; int act_f16;
   uint32_t* err;
-  ItemList items;
+  ItemList items; uint32_t n_items;
 };
 
 struct CombineParams {

@@ -542,3 +542,31 @@ def test_head_norm_in_the_decode_front_keeps_the_bits_of_the_separate_kernel(nH,
     for which in "kv":
         for s, n in enumerate(ctx):
             assert torch.equal(engs[0].cache(0, which)[s, :n + (2 if s == 0 else 1)], engs[1].cache(0, which)[s, :n + (2 if s == 0 else 1)])
+
+
+@pytest.mark.parametrize("nH,nKV,hd,lens", [(16, 2, 256, [14000, 3, 64, 900, 7000]), (16, 8, 128, [2900 - 120 * i for i in range(24)]), (8, 4, 64, [1, 40000])])
+def test_batches_of_unequal_lengths_share_the_tiles_out(nH, nKV, hd, lens):
+    # long and short conversations in one call: every sequence as it comes out of a call of its own
+    import torch
+    from pooled_b200 import AttnConfig, AttnEngine
+    n = len(lens)
+    mk = lambda: AttnEngine(AttnConfig(n_heads=nH, n_kv_heads=nKV, head_dim=hd, n_rot=64 if hd != 128 else 128, rope_theta=1e6, max_seq=max(lens) + 2, n_seqs=n,
+                                       act_dtype=torch.float32, max_cols=32))
+    a, b = mk(), mk()
+    g = torch.Generator(device="cuda"); g.manual_seed(3)
+    for s, ctx in enumerate(lens):
+        for which in "kv":
+            x = torch.randn((ctx, nKV * hd), generator=g, device="cuda").half().view(torch.int16)
+            for e in (a, b):
+                e.cache(0, which)[s, :ctx] = x
+    q, k, v = (torch.randn((n, d), generator=g, device="cuda") for d in (nH * hd, nKV * hd, nKV * hd))
+    out = a.encode_items(0, list(enumerate(lens)), q, k, v)
+    a.sync()
+    for s, ctx in enumerate(lens):
+        one = b.encode_layer(0, ctx, q[s:s + 1], k[s:s + 1], v[s:s + 1], seq=s)
+        b.sync()
+        assert util.errs(out[s:s + 1].cpu().numpy(), one.cpu().numpy())[1] < util.REF_REL, f"sequence {s} of {ctx} rows"
+        for which in "kv":   # (one angle evaluation on the device, the other by the host's libm: the last place of a rotated k)
+            x, y = (e.cache(0, which)[s, ctx].view(torch.float16).float() for e in (a, b))
+            assert torch.allclose(x, y, rtol=2 ** -10, atol=1e-7)
+            assert torch.equal(a.cache(0, which)[s, :ctx], b.cache(0, which)[s, :ctx])
