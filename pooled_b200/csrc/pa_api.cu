@@ -121,8 +121,7 @@ static uint32_t plan_splits(const pa_ctx* ctx, uint32_t n_rows, uint32_t n_items
   if (!total_cols) total_cols = n_items;
   uint32_t want = ctx->cfg.splits ? ctx->cfg.splits : (uint32_t)ctx->sm_count / (ctx->cfg.n_kv_heads * n_items);
   if (want < 1) want = 1;
-  uint32_t cap = tiles / 2;
-  if (cap < 1) cap = 1;
+  const uint32_t cap = plan_cap(tiles);
   if (want > cap) want = cap;
   if (want > ctx->max_splits) want = ctx->max_splits;
   const uint32_t fit = (uint32_t)(ctx->part_slots / ((size_t)total_cols * ctx->cfg.n_heads * groups));   // records: one per (row, split, consumer group)
@@ -716,7 +715,7 @@ static int decode_q8_item(pa_layer* L, const pa_item& it, const void* q, int q_d
   p.gate = gate; p.gate_col_stride = gcs; p.gate_head_stride = ghs; p.out = out; p.out_col_stride = ocs; p.act_f16 = ctx->cfg.act_dtype == PA_F16;
   const uint32_t ctas = ceil_div(rows, 8 * p.rgw) * ctx->cfg.n_kv_heads, tiles = ceil_div(n_rows, 64);
   uint32_t ns = ctx->cfg.splits ? ctx->cfg.splits : std::max(1u, 2u * (uint32_t)ctx->sm_count / ctas);
-  ns = std::min(std::min(ns, std::max(1u, tiles / 2)), ctx->max_splits);
+  ns = std::min(std::min(ns, plan_cap(tiles)), ctx->max_splits);
   ns = (uint32_t)std::max<size_t>(1, std::min<size_t>(ns, ctx->pf_slots / ((size_t)it.n_cols * nH)));
   p.n_splits = ns;
   const uint32_t live = ceil_div(tiles, ceil_div(tiles, ns));
@@ -833,7 +832,7 @@ static uint32_t balance_items(const pa_ctx* ctx, ItemList* il, uint32_t n_items,
   for (uint32_t i = 0; i < n_items; ++i) {
     tiles[i] = ceil_div(il->n_rows[i], 64);
     longest = std::max(longest, tiles[i]);
-    if (tiles[i]) t_old = std::max(t_old, ceil_div(tiles[i], std::min(ns_common, std::max(1u, tiles[i] / 2))));
+    if (tiles[i]) t_old = std::max(t_old, ceil_div(tiles[i], std::min(ns_common, plan_cap(tiles[i]))));
   }
   if (t_old < 12 || longest > 0xffffu) return 0;
   uint32_t limit = C * ceil_div(n_items, C);
@@ -887,7 +886,7 @@ static int decode_impl(pa_layer* L, const pa_item* items, uint32_t n_items, cons
     // the lists' lengths live on the device: the grid is sized for the longest list possible and each CTA derives its
     // own column's plan (plan_splits' rule without the cap by the row count, which the kernel applies)
     ns = plan_splits(ctx, 0x40000000u, n_items, total_cols, groups);
-    const uint32_t most = std::max(1u, ceil_div(gl->stride - 1, 64) / 2);
+    const uint32_t most = plan_cap(ceil_div(gl->stride - 1, 64));
     if (ns > most) ns = most;
     p.gather = gl->lists; p.gather_stride = gl->stride; p.k_cache = L->k; p.v_cache = L->v;
   }
@@ -945,8 +944,13 @@ static int decode_impl(pa_layer* L, const pa_item* items, uint32_t n_items, cons
   for (uint32_t i = 0; i < n_items; ++i) all_rows = all_rows && p.items.n_rows[i] > 0;
   const bool merge = !flat && !partial && !exchange && !verify_tc && nt <= 2 && all_rows && !ctx->core_only && !ctx->tune.no_merge && max_rows > 0 &&
                      (uint64_t)ns * ctx->cfg.n_kv_heads * n_items <= (uint64_t)ctx->sm_count && 2 * ns >= units;
-  if (merge) {
-    p.merge = ctx->tune.old_tail ? 1u : 2u; p.merge_ctr = ctx->merge_ctr;
+  // ... and with at most eight splits the CTAs of an (item, kv head) are launched as a cluster and merge through its shared
+  // memory, however many items there are: clusters do not wait for one another
+  const bool cluster = !flat && !partial && !exchange && !verify_tc && nt <= 2 && all_rows && !ctx->core_only && !ctx->tune.no_merge && max_rows > 0 &&
+                       ns <= (uint32_t)kMaxCluster;
+  if (cluster) while (ns & (ns - 1)) ++ns;      // 1, 2, 4 or 8 CTAs (those without a tile leave at once); the plan is p.n_splits'
+  if (merge || cluster) {
+    p.merge = cluster ? 3u : ctx->tune.old_tail ? 1u : 2u; p.merge_ctr = ctx->merge_ctr;
     p.gate = gate; p.gate_col_stride = gcs; p.gate_head_stride = ghs; p.out = out; p.out_col_stride = ocs; p.act_f16 = ctx->cfg.act_dtype == PA_F16;
   }
   // an exchanging call numbers itself ahead of its combine kernel: in the decode kernel where that runs
@@ -972,8 +976,8 @@ static int decode_impl(pa_layer* L, const pa_item* items, uint32_t n_items, cons
   c.exchange = exchange ? 1 : 0; c.xc = ctx->xc; c.err = ctx->dev_err;
   c.xch_sweeps = ctx->tune.wait_polls ? ctx->tune.wait_polls : (1u << 20);
   c.items = p.items; c.n_items = n_items;
-  if (!ctx->core_only && !merge) CU_TRY(ctx, launch_combine((int)ctx->cfg.head_dim, c, total_cols * ctx->cfg.n_heads, st));
-  ctx->stats.kernel_launches += (ctx->core_only || merge) ? 1 : 2; ctx->stats.kv_bytes_streamed += kv_bytes; ctx->stats.calls++;
+  if (!ctx->core_only && !merge && !cluster) CU_TRY(ctx, launch_combine((int)ctx->cfg.head_dim, c, total_cols * ctx->cfg.n_heads, st));
+  ctx->stats.kernel_launches += (ctx->core_only || merge || cluster) ? 1 : 2; ctx->stats.kv_bytes_streamed += kv_bytes; ctx->stats.calls++;
   // this call's kernel waited for everything before it; what it appends itself is what may still be in flight
   if (fz && fz->append_mask) {
     uint32_t r0 = 0xffffffffu;

@@ -125,6 +125,26 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
 __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
+// all threads of the cluster that have not exited; what was written before is visible after, in shared memory of peers too
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address of this CTA's shared variable in the CTA of rank `cta` of the cluster
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t cta) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));
+  return r;
+}
+__device__ __forceinline__ float4 cluster_ld4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 cluster_ld2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
   __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&h);
@@ -230,6 +250,12 @@ __device__ __forceinline__ void named_bar_arrive(uint32_t id, uint32_t threads) 
 __host__ __device__ constexpr int decode_groups(int nt) { return nt >= 0 ? 1 : 2; }
 
 constexpr int kMaxItems = 32;     // items of one batched decode call
+// Most splits of a decode call over `tiles` 64-row tiles.  Up to eight tiles one each: their records are merged through
+// cluster shared memory (see the end of pa_decode_kernel), so another split costs little and a tile is 0.7 to 1.2 us of a chain
+// of latencies.  Beyond 16 tiles two tiles at least, so that a CTA's start and end are shared.
+__host__ __device__ constexpr uint32_t plan_cap(uint32_t tiles) { return tiles <= 1 ? 1u : tiles <= 8 ? tiles : tiles < 16 ? 8u : tiles / 2; }
+constexpr int kMaxCluster = 8;    // the portable cluster size
+
 constexpr int kPrefillSplits = 8; // most key splits of a prefill call
 constexpr int kMaxRows = 64;      // query rows (columns x heads of one kv head) one decode CTA carries
 

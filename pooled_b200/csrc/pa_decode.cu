@@ -264,9 +264,9 @@ struct DecSmem {
 
 static_assert(sizeof(DecodeParams) + 4 * sizeof(CUtensorMap) <= 4096, "the decode kernel's launch parameters must fit 4 KB");
 
-// NORM: the fused front normalises q and k first (an instantiation of its own: as a run-time branch it cost the calls
-// without a head-norm 1 %)
-template <int HD, int NT, bool PRECISE, bool NORM = false>
+// NORM: the fused front normalises q and k first.  CL: at most eight splits, merged through the shared memory of a
+// cluster.  (Instantiations of their own: as run-time branches they cost the calls that need neither 1 to 3 %.)
+template <int HD, int NT, bool PRECISE, bool NORM = false, bool CL = false>
 __global__ void __launch_bounds__(DecSmem<HD, NT, PRECISE>::THREADS, 1)
 pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_kn,
                  const __grid_constant__ CUtensorMap tm_vn, const DecodeParams p) {
@@ -294,9 +294,9 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
   const uint32_t* g_list = p.gather ? p.gather + (size_t)p.items.col0[item] * p.gather_stride : nullptr;
   const uint32_t n_rows = g_list ? min(g_list[0], p.gather_stride - 1u) : p.items.n_rows[item];   // cache rows the last column sees
   const uint32_t tiles = (n_rows + kT - 1) / kT;
-  // every item plans for its own length: at least two tiles per CTA, at most the launch's split count (the longest
+  // every item plans for its own length: plan_cap(tiles) splits, at most the launch's split count (the longest
   // item's plan, or in gather mode the most any list could need)
-  const uint32_t ns_eff = min(p.n_splits, max(1u, tiles / 2));
+  const uint32_t ns_eff = min(p.n_splits, plan_cap(tiles));
   const uint32_t tps = balanced ? p.items.tps[item] : (tiles + ns_eff - 1) / max(ns_eff, 1u);  // tiles per split
   const uint32_t tile0 = split * tps;
   if (tile0 >= tiles) {
@@ -1097,6 +1097,71 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     put_rows(false, xml_out);
   }
   named_bar_sync(gbar, kConsumers);
+  if constexpr (CL) {
+    // ---- at most eight splits: a cluster.  Every CTA's rows lie in its shared memory (xo, xml_out); after one cluster
+    //      barrier the CTAs share out the output, four dims per thread, and read one another's rows.  Through global
+    //      memory the same merge is a record written, a fence, a counter, a wait and a round trip: 4.3 us of a 9.6 us call over
+    //      301 rows.  The arithmetic is pa_combine_kernel's for up to eight records, operation for operation and in
+    //      its order, so the bits are the same whichever merges. ----
+    const uint32_t ns_live = (tiles + tps - 1) / tps, n_it = live_rows * (HD / 4);
+    uint32_t idx = split * kConsumers + ltid;
+    auto where = [&](uint32_t ix, uint64_t& go, uint64_t& oo) {
+      const uint32_t row = ix / (HD / 4), c = row / G, h = g * G + row % G, col = p.items.col0[item] + c, d = (ix % (HD / 4)) * 4;
+      go = (uint64_t)col * p.gate_col_stride + (uint64_t)h * p.gate_head_stride + d;
+      oo = (uint64_t)col * p.out_col_stride + (uint64_t)h * HD + d;
+    };
+    auto gate4 = [&](uint32_t ix, float (&gv)[4]) {
+      uint64_t go, oo;
+      where(ix, go, oo);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) gv[k] = ld_act(p.gate, go + k, p.act_f16);
+    };
+    float gv[4] = {0.f, 0.f, 0.f, 0.f};
+    if (p.gate && idx < n_it) gate4(idx, gv);      // lands while the cluster meets
+    cluster_sync();
+    const uint32_t xo_s = smem_u32(xo), xml_s = smem_u32(xml_out);
+    for (bool first = true; idx < n_it; idx += ns_live * kConsumers, first = false) {
+      if (p.gate && !first) gate4(idx, gv);
+      const uint32_t row = idx / (HD / 4), c4 = idx % (HD / 4);
+      float2 ml[kMaxCluster];
+      float4 x[kMaxCluster];
+#pragma unroll
+      for (uint32_t s = 0; s < kMaxCluster; ++s) {
+        ml[s] = make_float2(-3.0e38f, 0.f); x[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s >= ns_live) continue;
+        ml[s] = cluster_ld2(cluster_map(xml_s, s) + row * 8);
+        x[s] = cluster_ld4(cluster_map(xo_s, s) + (row * HD + c4 * 4) * 4);
+        ml[s].x *= 0.6931471805599453f;
+      }
+      float M = ml[0].x;
+#pragma unroll
+      for (int s = 1; s < kMaxCluster; ++s) M = fmaxf(M, ml[s].x);
+      float w[kMaxCluster], a[kMaxCluster];
+#pragma unroll
+      for (uint32_t s = 0; s < kMaxCluster; ++s) { w[s] = s < ns_live ? __expf(ml[s].x - M) : 0.f; a[s] = __fmul_rn(ml[s].y, w[s]); }
+      // the order of the shuffle sum: lanes 4, 2, 1 apart
+      const float Lsum = __fadd_rn(__fadd_rn(__fadd_rn(a[0], a[4]), __fadd_rn(a[2], a[6])), __fadd_rn(__fadd_rn(a[1], a[5]), __fadd_rn(a[3], a[7])));
+      float t[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int s = 0; s < kMaxCluster; ++s) {
+        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+        fma4(y, x[s], w[s]);
+        t[0] = s ? __fadd_rn(t[0], y.x) : y.x; t[1] = s ? __fadd_rn(t[1], y.y) : y.y;
+        t[2] = s ? __fadd_rn(t[2], y.z) : y.z; t[3] = s ? __fadd_rn(t[3], y.w) : y.w;
+      }
+      uint64_t go, oo;
+      where(idx, go, oo);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float rv = (p.gather && Lsum == 0.f) ? 0.f : __fdiv_rn(t[k], Lsum);
+        if (p.gate) rv = __fmul_rn(rv, __fdiv_rn(1.0f, __fadd_rn(1.0f, __expf(-gv[k]))));
+        if (p.act_f16) reinterpret_cast<__half*>(p.out)[oo + k] = __float2half_rn(rv);
+        else reinterpret_cast<float*>(p.out)[oo + k] = rv;
+      }
+    }
+    cluster_sync();                                // no CTA leaves while another reads its rows
+    if (*s_err && tid == 0) atomicMax(p.err, *s_err);
+  } else {
   for (uint32_t idx = ltid; idx < live_rows * (HD / 4); idx += kConsumers) {
     const uint32_t row = idx / (HD / 4), c4 = idx % (HD / 4);
     const uint32_t c = row / G, hh = row % G;
@@ -1166,6 +1231,7 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     if (ltid == 0 && atomicAdd(ctr + 1, 1u) == ns_live - 1) { ctr[0] = 0; ctr[1] = 0; }
   }
   if (*s_err && tid == 0) atomicMax(p.err, *s_err);
+  }
 }
 
 // the exchange's call counter for a call whose decode kernel does not run (a shard that holds no row of the call) or
@@ -1201,7 +1267,7 @@ __global__ void __launch_bounds__(256) pa_combine_kernel(const CombineParams p) 
     // gather: one column per item, its length on the device; the plan is the one the decode kernel derived from it
     const uint32_t n_rows = p.gather ? min(p.gather[(size_t)col * p.gather_stride], p.gather_stride - 1u) : p.items.n_rows[it];
     const uint32_t tiles = (n_rows + kT - 1) / kT;
-    const uint32_t n_sp = min(p.n_splits, max(1u, tiles / 2));
+    const uint32_t n_sp = min(p.n_splits, plan_cap(tiles));
     const uint32_t tps = p.items.tps[0] ? p.items.tps[it] : (tiles + n_sp - 1) / max(n_sp, 1u);
     ns = tiles ? ((tiles + tps - 1) / tps) * p.groups : 0;   // a shard that holds no row of the item: an empty record
   }
@@ -1297,7 +1363,7 @@ __global__ void __launch_bounds__(256) pa_combine_kernel(const CombineParams p) 
 
 // ------------------------------------------------------------------------------ launchers --
 
-template <int HD, int NT, bool PRECISE, bool NORM = false>
+template <int HD, int NT, bool PRECISE, bool NORM = false, bool CL = false>
 static cudaError_t launch_decode_t(const pa_layer* L, const DecodeParams& p, dim3 grid, cudaStream_t st) {
   using S = DecSmem<HD, NT, PRECISE>;
   DecodeParams pp = p;
@@ -1307,12 +1373,24 @@ static cudaError_t launch_decode_t(const pa_layer* L, const DecodeParams& p, dim
   const int bytes = S::total_bytes(stages);
   static bool attr_set[64] = {};
   if (pp.gather && (!pp.k_cache || !pp.v_cache)) return cudaErrorInvalidValue;
-  auto kern = pa_decode_kernel<HD, NT, PRECISE, NORM>;
+  auto kern = pa_decode_kernel<HD, NT, PRECISE, NORM, CL>;
   const int dev = L->ctx->device & 63;
   if (!attr_set[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
+  }
+  if constexpr (CL) {   // one cluster per (item, kv head)
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = dim3(S::THREADS); cfg.dynamicSmemBytes = (size_t)bytes; cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = grid.x; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 2;
+    pp.next_tiles = 0; pp.next_max_seq = L->max_seq;
+    return cudaLaunchKernelEx(&cfg, kern, L->tm_k64, L->tm_v64, L->tm_k64, L->tm_v64, pp);
   }
   const pa_layer* N = L->next;
   if (!N || !pp.next_tiles || N->n_seqs != L->n_seqs) { N = L; pp.next_tiles = 0; }
@@ -1323,8 +1401,12 @@ static cudaError_t launch_decode_t(const pa_layer* L, const DecodeParams& p, dim
 template <int HD, bool PRECISE>
 static cudaError_t launch_decode_nt(const pa_layer* L, const DecodeParams& p, dim3 grid, int nt, cudaStream_t st) {
   switch (nt) {
-    case 1: return HD >= 128 && p.qn_w ? launch_decode_t<HD, 1, PRECISE, HD >= 128>(L, p, grid, st) : launch_decode_t<HD, 1, PRECISE>(L, p, grid, st);
-    case 2: return launch_decode_t<HD, 2, PRECISE>(L, p, grid, st);
+    case 1: {
+      constexpr bool NM = HD >= 128;     // the shapes of the fused front
+      if (p.merge == 3) return NM && p.qn_w ? launch_decode_t<HD, 1, PRECISE, NM, true>(L, p, grid, st) : launch_decode_t<HD, 1, PRECISE, false, true>(L, p, grid, st);
+      return NM && p.qn_w ? launch_decode_t<HD, 1, PRECISE, NM>(L, p, grid, st) : launch_decode_t<HD, 1, PRECISE>(L, p, grid, st);
+    }
+    case 2: return p.merge == 3 ? launch_decode_t<HD, 2, PRECISE, false, true>(L, p, grid, st) : launch_decode_t<HD, 2, PRECISE>(L, p, grid, st);
     case 3: case 4: return launch_decode_t<HD, 4, PRECISE>(L, p, grid, st);
     default: return launch_decode_t<HD, 8, PRECISE>(L, p, grid, st);
   }

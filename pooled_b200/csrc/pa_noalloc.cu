@@ -128,7 +128,7 @@ extern "C" PA_API int pa_decode_static(int device, const void* k_cache, const vo
   const uint32_t n_rows = pos + n_cols, tiles = (n_rows + 63) / 64;
   uint32_t ns = (uint32_t)ctx.sm_count / n_kv_heads;
   if (ns < 1) ns = 1;
-  if (ns > (tiles / 2 > 1 ? tiles / 2 : 1)) ns = tiles / 2 > 1 ? tiles / 2 : 1;
+  if (ns > plan_cap(tiles)) ns = plan_cap(tiles);
   if (ns > PA_STATIC_RECORDS / (rows * groups)) ns = PA_STATIC_RECORDS / (rows * groups);   // fit the records into the fixed array
   if (ns > 256) ns = 256;
 

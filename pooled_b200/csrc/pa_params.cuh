@@ -39,6 +39,7 @@ struct DecodeParams {
   const uint32_t* gather; uint32_t gather_stride;
   // merge != 0: no combine kernel follows; the CTAs of each (item, kv head) merge their own records, gate and store
   // (2: CTAs without a merge unit leave as soon as their record is counted; 1: they wait like the others)
+  // (3: the CTAs of an (item, kv head) are one thread-block cluster and merge through its shared memory, no record leaves the SMs)
   uint32_t merge; unsigned int* merge_ctr;
   unsigned int* xch_ctr;   // != nullptr: the call ends in a cross-GPU exchange; the kernel's first thread advances its call counter
   const void* gate; uint64_t gate_col_stride, gate_head_stride;

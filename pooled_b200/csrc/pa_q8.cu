@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   const uint32_t rg = warp % p.rgw, pw = warp / p.rgw, n_pw = 4 / p.rgw;
   // the plan is the call's (its last column's rows); a row tile stops at what its own last row sees
   const uint32_t tiles = (p.n_rows + kQ8Tile - 1) / kQ8Tile;
-  const uint32_t ns_eff = min(p.n_splits, max(1u, tiles / 2)), tps = (tiles + ns_eff - 1) / max(ns_eff, 1u);
+  const uint32_t ns_eff = min(p.n_splits, plan_cap(tiles)), tps = (tiles + ns_eff - 1) / max(ns_eff, 1u);
   const uint32_t t_lo = split * tps;
   if (t_lo >= tiles) return;                                  // no record expected from this split
   auto row_lim = [&](uint32_t row) { return (uint32_t)min(max(p.lim0 + (int32_t)(min(row, rows - 1) / G), 0), (int32_t)p.n_rows); };

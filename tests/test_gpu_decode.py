@@ -570,3 +570,31 @@ def test_batches_of_unequal_lengths_share_the_tiles_out(nH, nKV, hd, lens):
             x, y = (e.cache(0, which)[s, ctx].view(torch.float16).float() for e in (a, b))
             assert torch.allclose(x, y, rtol=2 ** -10, atol=1e-7)
             assert torch.equal(a.cache(0, which)[s, :ctx], b.cache(0, which)[s, :ctx])
+
+
+@pytest.mark.parametrize("nH,nKV,hd,act", [(16, 2, 256, "f16"), (16, 8, 128, "f32"), (16, 1, 64, "f32"), (24, 4, 256, "f32")])
+def test_cluster_merge_gives_the_combine_kernels_bits(nH, nKV, hd, act, monkeypatch):
+    # one to eight splits (contexts of one to sixteen tiles and a few rows around the steps), one item and three, gate and
+    # none, against the same calls with every merge in the combine kernel, and against float64
+    import torch
+    from pooled_b200 import AttnConfig, AttnEngine
+    td = torch.float16 if act == "f16" else torch.float32
+    rows = 1100
+    mk = lambda: AttnEngine(AttnConfig(n_heads=nH, n_kv_heads=nKV, head_dim=hd, n_rot=64, rope_theta=1e6, max_seq=rows, n_seqs=1, rope_mode="none", act_dtype=td, max_cols=8))
+    a = mk()
+    monkeypatch.setenv("POOLED_ATTN_NO_MERGE", "1")
+    b = mk()
+    K, V = po.np_f16_rne(po.normal(1, rows * nKV * hd)).reshape(rows, -1), po.np_f16_rne(po.normal(2, rows * nKV * hd)).reshape(rows, -1)
+    for e in (a, b):
+        util.load_cache(e, 0, 0, K, V)
+    it = torch.int16 if act == "f16" else torch.int32
+    for lens in ([1], [64], [65], [128], [129], [320], [449], [512], [513], [640], [1023], [1024], [1025], [1, 200, 700], [64, 64, 512]):
+        n = len(lens)
+        q, g = util.normal_f16(3 + lens[0], (n, nH * hd)), util.normal_f16(4 + lens[0], (n, nH * hd))
+        dq, dg = util.torch_dev(q, td), util.torch_dev(g, td)
+        for gate in (dg, None):
+            x, y = (e.decode(0, [(0, m - 1, 1) for m in lens], dq, gate) for e in (a, b))
+            a.sync(); b.sync()
+            assert torch.equal(x.view(it), y.view(it)), f"{lens}"
+        ref = np.concatenate([po.attn_f64(q[i:i + 1], K, V, nH, nKV, hd, m - 1, 1) for i, m in enumerate(lens)])
+        util.assert_close(x.float().cpu().numpy(), ref, f"{lens}")
