@@ -719,26 +719,21 @@ static int decode_q8_item(pa_layer* L, const pa_item& it, const void* q, int q_d
   ns = (uint32_t)std::max<size_t>(1, std::min<size_t>(ns, ctx->pf_slots / ((size_t)it.n_cols * nH)));
   p.n_splits = ns;
   const uint32_t live = ceil_div(tiles, ceil_div(tiles, ns));
+  // two to eight splits: a cluster merges them itself (with core_only too: there is no second kernel to leave out)
+  if (live > 1 && ns <= (uint32_t)kMaxCluster) for (p.cluster = ns; p.cluster & (p.cluster - 1); ++p.cluster) {}
   timing_mark(ctx, st, 0);
   CU_TRY(ctx, launch_q8(p, hd, ctx->cfg.n_kv_heads, ctx->device, st));
   timing_mark(ctx, st, 1);
   ctx->stats.kernel_launches++;
   ctx->stats.kv_bytes_streamed += 2ull * n_rows * (row_bytes_of(ctx, L->kv_format) + scale_row_bytes_of(ctx, L->kv_format));
-  if (live == 1 || ctx->core_only) return PA_OK;
-  if (live <= (uint32_t)kPrefillSplits) {
-    PrefillParams c{};
-    c.gate = gate; c.gate_col_stride = gcs; c.gate_head_stride = ghs; c.out = out; c.out_col_stride = ocs; c.act_f16 = p.act_f16;
-    c.n_cols = it.n_cols; c.n_heads = nH; c.part_o = ctx->part_o; c.part_ml = ctx->part_ml; c.n_splits = ns; c.merge_ns = live;
-    CU_TRY(ctx, launch_combine_few((int)hd, c, st));
-  } else {
-    CombineParams c{};
-    c.o = ctx->part_o; c.ml = ctx->part_ml;
-    c.o_row_stride = (uint64_t)ns * hd; c.o_part_stride = hd; c.ml_row_stride = (uint64_t)ns * 2; c.ml_part_stride = 2;
-    c.n_heads = nH; c.fixed_parts = live; c.n_splits = ns; c.groups = 1;
-    c.gate = gate; c.gate_col_stride = gcs; c.gate_head_stride = ghs; c.out = out; c.out_col_stride = ocs; c.act_f16 = p.act_f16;
-    c.err = ctx->dev_err;
-    CU_TRY(ctx, launch_combine((int)hd, c, it.n_cols * nH, st));
-  }
+  if (live == 1 || p.cluster || ctx->core_only) return PA_OK;
+  CombineParams c{};
+  c.o = ctx->part_o; c.ml = ctx->part_ml;
+  c.o_row_stride = (uint64_t)ns * hd; c.o_part_stride = hd; c.ml_row_stride = (uint64_t)ns * 2; c.ml_part_stride = 2;
+  c.n_heads = nH; c.fixed_parts = live; c.n_splits = ns; c.groups = 1;
+  c.gate = gate; c.gate_col_stride = gcs; c.gate_head_stride = ghs; c.out = out; c.out_col_stride = ocs; c.act_f16 = p.act_f16;
+  c.err = ctx->dev_err;
+  CU_TRY(ctx, launch_combine((int)hd, c, it.n_cols * nH, st));
   ctx->stats.kernel_launches++;
   return PA_OK;
 }
@@ -770,13 +765,20 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
       const uint32_t pos0 = items[i].pos + c0;
       const uint32_t rows = pos0 + nc - L->origin;                 // rows the block's last column sees
       uint32_t ns = plan_splits(ctx, rows, 1, nc, 1), live = 0;
+      bool merged = false;
       if (decode_f32_direct(ctx->G)) {
         // rows in whole 16s over one CTA per SM; a short context gives every warp of a CTA its 16 rows before it takes more CTAs
         ns = ctx->cfg.splits ? ctx->cfg.splits : std::max(1u, (uint32_t)ctx->sm_count / (ctx->cfg.n_kv_heads * nc));
         ns = std::min(std::min(ns, ctx->max_splits), (uint32_t)(ctx->part_slots / ((size_t)nc * nH)));
+        // up to 2048 rows eight splits do (two batches a warp): a cluster merges them, which saves the merge kernel
         F32DecodeParams f{};
+        if (rows <= 2048 && !ctx->cfg.splits) ns = std::min(ns, (uint32_t)kMaxCluster);
         f.rows_per_split = ceil_div(ceil_div(rows, std::max(1u, ns)), 16) * 16;
         ns = live = ceil_div(rows, f.rows_per_split);
+        if (ns <= (uint32_t)kMaxCluster) for (f.cluster = ns; f.cluster & (f.cluster - 1); ++f.cluster) {}
+        f.gate = gate ? reinterpret_cast<const uint8_t*>(gate) + (col + c0) * gcs * aes : nullptr; f.gate_col_stride = gcs; f.gate_head_stride = ghs;
+        f.out = reinterpret_cast<uint8_t*>(out) + (col + c0) * ocs * aes; f.out_col_stride = ocs; f.act_f16 = ctx->cfg.act_dtype == PA_F16;
+        merged = f.cluster != 0;
         f.q = reinterpret_cast<const uint8_t*>(q) + (col + c0) * qcs * qes; f.q_f16 = q_dtype == PA_F16; f.q_col_stride = qcs; f.q_head_stride = qhs;
         f.q_vec = q_dtype == PA_F32 && !(qcs & 3) && !(qhs & 3) && !((uintptr_t)f.q & 15);
         f.k = (const float*)L->k_alt; f.v = (const float*)L->v_alt;
@@ -808,8 +810,8 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
       c.out = reinterpret_cast<uint8_t*>(out) + (col + c0) * ocs * aes; c.out_col_stride = ocs; c.act_f16 = ctx->cfg.act_dtype == PA_F16;
       c.items.seq[0] = items[i].seq; c.items.lim0[0] = a.lim0; c.items.n_rows[0] = rows; c.items.n_cols[0] = nc; c.items.col0[0] = 0; c.n_items = 1;
       c.err = ctx->dev_err;
-      if (!ctx->core_only) CU_TRY(ctx, launch_combine((int)hd, c, nc * nH, st));
-      ctx->stats.kernel_launches += ctx->core_only ? 1 : 2;
+      if (!ctx->core_only && !merged) CU_TRY(ctx, launch_combine((int)hd, c, nc * nH, st));
+      ctx->stats.kernel_launches += ctx->core_only || merged ? 1 : 2;
       ctx->stats.kv_bytes_streamed += 2ull * rows * (row_bytes_of(ctx, L->kv_format) + scale_row_bytes_of(ctx, L->kv_format));
     }
     col += items[i].n_cols;

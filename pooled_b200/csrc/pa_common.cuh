@@ -22,6 +22,12 @@ constexpr uint32_t kWaitPolls = 1u << 24;  // with 32..64 ns back-off: well unde
 
 enum : uint32_t { WAIT_KFULL = 1, WAIT_VFULL = 2, WAIT_EMPTY = 3, WAIT_MMA = 4, WAIT_TMEM = 5, WAIT_QFULL = 6, WAIT_PEER = 7, WAIT_MERGE = 8 };
 
+// Most splits of a decode call over `tiles` 64-row tiles.  Up to eight tiles one each: their records are merged through
+// cluster shared memory (see the end of pa_decode_kernel), so another split costs little and a tile is 0.7 to 1.2 us of a chain
+// of latencies.  Beyond 16 tiles two tiles at least, so that a CTA's start and end are shared.
+__host__ __device__ constexpr uint32_t plan_cap(uint32_t tiles) { return tiles <= 1 ? 1u : tiles <= 8 ? tiles : tiles < 16 ? 8u : tiles / 2; }
+constexpr int kMaxCluster = 8;    // the portable cluster size
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -145,6 +151,43 @@ __device__ __forceinline__ float2 cluster_ld2(uint32_t addr) {
   asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
   return v;
 }
+__device__ __forceinline__ float ld_act(const void* p, uint64_t i, int f16) {
+  return f16 ? __half2float(reinterpret_cast<const __half*>(p)[i]) : reinterpret_cast<const float*>(p)[i];
+}
+
+// merge of one row's four dims over the CTAs of a cluster: o4 and ml are this CTA's shared addresses of its own unnormalised
+// o and of its (m in log2 units, l); every CTA keeps its rows at the same addresses.  Sums in CTA order.
+__device__ __forceinline__ float4 cluster_merge4(uint32_t o4, uint32_t ml, uint32_t n, float& L) {
+  float2 v[kMaxCluster];
+  float4 x[kMaxCluster], o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (uint32_t s = 0; s < kMaxCluster; ++s) {
+    v[s] = make_float2(-3.0e38f, 0.f); x[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (s < n) { v[s] = cluster_ld2(cluster_map(ml, s)); x[s] = cluster_ld4(cluster_map(o4, s)); }
+  }
+  float M = v[0].x;
+#pragma unroll
+  for (int s = 1; s < kMaxCluster; ++s) M = fmaxf(M, v[s].x);
+  L = 0.f;
+#pragma unroll
+  for (uint32_t s = 0; s < kMaxCluster; ++s) {
+    const float w = s < n ? exp2f(v[s].x - M) : 0.f;
+    L = __fmaf_rn(v[s].y, w, L);
+    o.x = __fmaf_rn(x[s].x, w, o.x); o.y = __fmaf_rn(x[s].y, w, o.y); o.z = __fmaf_rn(x[s].z, w, o.z); o.w = __fmaf_rn(x[s].w, w, o.w);
+  }
+  return o;
+}
+// o / L, sigmoid gate, store in the activation type: four dims of one head
+__device__ __forceinline__ void gate_store4(float4 o, float L, const void* gate, uint64_t go, void* out, uint64_t oo, int f16) {
+  const float v[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float r = __fdiv_rn(v[e], L);
+    if (gate) r = __fmul_rn(r, __fdiv_rn(1.0f, __fadd_rn(1.0f, __expf(-ld_act(gate, go + e, f16)))));
+    if (f16) reinterpret_cast<__half*>(out)[oo + e] = __float2half_rn(r);
+    else reinterpret_cast<float*>(out)[oo + e] = r;
+  }
+}
 __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
   __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&h);
@@ -187,10 +230,6 @@ __device__ __forceinline__ float rot_exact(float x, float y, const Angle& g, boo
   if (safe) return hi;
   const double a = __dmul_rn((double)x, g.c), b = __dmul_rn((double)y, g.s);
   return (float)(minus ? __dsub_rn(a, b) : __dadd_rn(a, b));
-}
-
-__device__ __forceinline__ float ld_act(const void* p, uint64_t i, int f16) {
-  return f16 ? __half2float(reinterpret_cast<const __half*>(p)[i]) : reinterpret_cast<const float*>(p)[i];
 }
 
 // QK head-norm: out = f32((x * inv) * w), inv = 1 / sqrt(ss / hd + eps), with ss the float64 sum of the squares of a
@@ -250,12 +289,6 @@ __device__ __forceinline__ void named_bar_arrive(uint32_t id, uint32_t threads) 
 __host__ __device__ constexpr int decode_groups(int nt) { return nt >= 0 ? 1 : 2; }
 
 constexpr int kMaxItems = 32;     // items of one batched decode call
-// Most splits of a decode call over `tiles` 64-row tiles.  Up to eight tiles one each: their records are merged through
-// cluster shared memory (see the end of pa_decode_kernel), so another split costs little and a tile is 0.7 to 1.2 us of a chain
-// of latencies.  Beyond 16 tiles two tiles at least, so that a CTA's start and end are shared.
-__host__ __device__ constexpr uint32_t plan_cap(uint32_t tiles) { return tiles <= 1 ? 1u : tiles <= 8 ? tiles : tiles < 16 ? 8u : tiles / 2; }
-constexpr int kMaxCluster = 8;    // the portable cluster size
-
 constexpr int kPrefillSplits = 8; // most key splits of a prefill call
 constexpr int kMaxRows = 64;      // query rows (columns x heads of one kv head) one decode CTA carries
 
@@ -267,6 +300,20 @@ static inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 blo
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+// the same with `cluster` neighbouring CTAs along x as one thread-block cluster
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_pdl_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, uint32_t cluster, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 

@@ -1381,16 +1381,8 @@ static cudaError_t launch_decode_t(const pa_layer* L, const DecodeParams& p, dim
     attr_set[dev] = true;
   }
   if constexpr (CL) {   // one cluster per (item, kv head)
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid; cfg.blockDim = dim3(S::THREADS); cfg.dynamicSmemBytes = (size_t)bytes; cfg.stream = st;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = grid.x; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
-    cfg.attrs = at; cfg.numAttrs = 2;
     pp.next_tiles = 0; pp.next_max_seq = L->max_seq;
-    return cudaLaunchKernelEx(&cfg, kern, L->tm_k64, L->tm_v64, L->tm_k64, L->tm_v64, pp);
+    return launch_pdl_cluster(kern, grid, dim3(S::THREADS), (size_t)bytes, st, grid.x, L->tm_k64, L->tm_v64, L->tm_k64, L->tm_v64, pp);
   }
   const pa_layer* N = L->next;
   if (!N || !pp.next_tiles || N->n_seqs != L->n_seqs) { N = L; pp.next_tiles = 0; }

@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = lane / LPR, lr = lane % LPR;
   const uint32_t lim = (uint32_t)min(max(p.lim0 + (int32_t)c, 0), (int32_t)p.n_rows);
   const uint32_t r_lo = split * p.rows_per_split, r_hi = min(r_lo + p.rows_per_split, lim);
+  if (split >= p.n_splits) return;                                          // (a cluster's size is a power of two)
   const uint64_t base = ((uint64_t)p.seq * p.max_seq) * p.kv_dim + (uint64_t)g * HD + lr * 4;
   float4 k[U][4], v[U][4];
   auto load = [&](uint32_t b0) {
@@ -318,19 +319,39 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
       L = __fmaf_rn(sml[8 * G + w * G + h], e, L);
       a = __fmaf_rn(sm[w * G * HD + idx], e, a);
     }
+    if (p.cluster) {         // behind the warps' shares
+      float* mine = sm + 8 * G * (HD + 2);
+      mine[idx] = a;
+      if (d == 0) { mine[G * HD + 2 * h] = M; mine[G * HD + 2 * h + 1] = L; }
+      continue;
+    }
     const uint64_t slot = (col * p.n_heads + g * G + h) * p.n_splits + split;
     p.part_o[slot * HD + d] = a;
     if (d == 0) { p.part_ml[slot * 2] = M * 0.6931471805599453f; p.part_ml[slot * 2 + 1] = L; }
   }
+  if (!p.cluster) return;
+  // at most eight splits: the CTAs of a (kv head, column) are a cluster and merge without another launch
+  cluster_sync();
+  const uint32_t mine_s = smem_u32(sm + 8 * G * (HD + 2));
+  for (uint32_t idx = split * 256 + tid; idx < G * (HD / 4); idx += p.n_splits * 256) {
+    const uint32_t h = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
+    float L;
+    const float4 o4 = cluster_merge4(mine_s + (h * HD + d) * 4, mine_s + (G * HD + 2 * h) * 4, p.n_splits, L);
+    gate_store4(o4, L, p.gate, col * p.gate_col_stride + (uint64_t)(g * G + h) * p.gate_head_stride + d, p.out,
+                col * p.out_col_stride + (uint64_t)(g * G + h) * HD + d, p.act_f16);
+  }
+  cluster_sync();            // no CTA leaves while another reads its rows
 }
 
 template <int HD, int G>
 static cudaError_t launch_f32_t(const F32DecodeParams& p, dim3 grid, cudaStream_t st) {
-  return launch_pdl(pa_decode_f32_kernel<HD, G>, grid, dim3(256), (size_t)(8 * G * (HD + 2)) * 4, st, p);
+  const size_t smem = (size_t)(9 * G * (HD + 2)) * 4;       // (at most 37 KB)
+  if (p.cluster) return launch_pdl_cluster(pa_decode_f32_kernel<HD, G>, grid, dim3(256), smem, st, p.cluster, p);
+  return launch_pdl(pa_decode_f32_kernel<HD, G>, grid, dim3(256), smem, st, p);
 }
 bool decode_f32_direct(uint32_t G) { return G == 1 || G == 2 || G == 4; }
 cudaError_t launch_decode_f32_direct(const F32DecodeParams& p, uint32_t hd, uint32_t G, uint32_t n_kv, cudaStream_t st) {
-  const dim3 grid(p.n_splits, n_kv, p.n_cols);
+  const dim3 grid(p.cluster ? p.cluster : p.n_splits, n_kv, p.n_cols);
 #define PA_F32_CASE(H) case H: return G == 1 ? launch_f32_t<H, 1>(p, grid, st) : G == 2 ? launch_f32_t<H, 2>(p, grid, st) : launch_f32_t<H, 4>(p, grid, st);
   switch (hd) {
     PA_F32_CASE(256) PA_F32_CASE(128) PA_F32_CASE(64)

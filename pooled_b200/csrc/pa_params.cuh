@@ -138,9 +138,11 @@ struct F32DecodeParams {
   const void* q; int q_f16; int q_vec; uint64_t q_col_stride, q_head_stride;   // q_vec: f32, every head row 16-byte aligned
   const float* k; const float* v;
   uint32_t kv_dim, n_heads, max_seq, n_splits, rows_per_split;
-  uint32_t seq; int32_t lim0; uint32_t n_rows, n_cols, early;                  // as in Q8Params
+  uint32_t seq; int32_t lim0; uint32_t n_rows, n_cols, early, cluster;         // as in Q8Params
   float scale_log2;
   float* part_o; float* part_ml;
+  const void* gate; uint64_t gate_col_stride, gate_head_stride;                // cluster: gate and output
+  void* out; uint64_t out_col_stride; int act_f16;
 };
 
 // the front of a layer call in one launch (pa_front_kernel): head-norm, rotation, append in the cache's format
@@ -159,6 +161,7 @@ struct Q8Params {
   const void* q; int q_f16; int q_vec; uint64_t q_col_stride, q_head_stride;   // q_vec: f32, every head row 16-byte aligned
   const int8_t* k; const int8_t* v; const float* ks; const float* vs;
   uint32_t kv_dim, G, n_heads, max_seq, n_splits, rgw;                      // rgw: 8-row groups per CTA
+  uint32_t cluster;                                                         // CTAs of a cluster that merges a row tile's splits (0: records)
   uint32_t seq; int32_t lim0; uint32_t n_rows, n_cols;                      // rows column 0 sees (before clamping), rows the last column sees
   uint32_t early;                                                           // 1: rows older than the call's own may be fetched before the predecessor ends
   float scale_log2;
@@ -176,7 +179,7 @@ struct PrefillParams {
   float scale_log2;
   uint32_t* err;
   // split-K form (k-token verify on the tensor cores): one CTA per (split, kv head), rows = columns x heads of the group
-  float* part_o; float* part_ml; uint32_t n_splits; uint32_t merge_ns; int32_t lim0; uint32_t n_rows, col0;
+  float* part_o; float* part_ml; uint32_t n_splits; int32_t lim0; uint32_t n_rows, col0;
   uint32_t prefetch_old_rows;   // split-K form: K/V tiles wholly below the call's new rows may be fetched before the predecessor ends
   uint32_t early_limit;         // ... and below this row (the call before may still be writing its own row)
   uint32_t pre_stages;          // ... and only this many K tiles (one fewer V tiles) before the q loads are in flight

@@ -756,7 +756,7 @@ __global__ void __launch_bounds__(256) pa_combine_few_kernel(const PrefillParams
   const uint32_t col = prow / p.n_heads, h = prow % p.n_heads, c0 = col / kBM * kBM;
   const uint32_t n_tiles = (p.pos + c0 + min((uint32_t)kBM, p.n_cols - c0) + kBN - 1) / kBN;
   const uint32_t tps = (n_tiles + p.n_splits - 1) / p.n_splits;
-  const uint32_t ns = p.merge_ns ? p.merge_ns : (n_tiles + tps - 1) / tps;   // live splits of this q tile (or of every row)
+  const uint32_t ns = (n_tiles + tps - 1) / tps;   // live splits of this q tile
   const float* ml = p.part_ml + (uint64_t)prow * p.n_splits * 2;
   const float* ob = p.part_o + (uint64_t)prow * p.n_splits * HD + lane * W;
   float m[kPrefillSplits], l[kPrefillSplits], x[kPrefillSplits][NV * W];

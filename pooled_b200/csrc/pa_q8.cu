@@ -36,7 +36,8 @@ struct Q8Smem {
   static constexpr int STAGES = HD == 256 ? 3 : 4;
   static constexpr int RING = STAGE * STAGES;
   static constexpr int MERGE = 4 * 8 * (HD + 2) * 4;       // the warps' (o, m, l), over the idle ring
-  static constexpr int TOTAL = RING > MERGE ? RING : MERGE;
+  static constexpr int MINE = 32 * (HD + 2) * 4;           // the CTA's merged rows behind them, for the cluster's merge
+  static constexpr int TOTAL = RING > MERGE + MINE ? RING : MERGE + MINE;
 };
 
 // 16-byte chunk c of row r, permuted so that the reads below hit 32 different banks: the score reads take four rows r ..
@@ -319,6 +320,12 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
       o.x = __fmaf_rn(x.x, w, o.x); o.y = __fmaf_rn(x.y, w, o.y); o.z = __fmaf_rn(x.z, w, o.z); o.w = __fmaf_rn(x.w, w, o.w);
     }
     const uint32_t row = row0 + lr, c = row / G, h = g * G + row % G;
+    if (p.cluster) {       // this CTA's share of the row, for the cluster's merge below
+      float* mine = reinterpret_cast<float*>(smem + L::MERGE);
+      *reinterpret_cast<float4*>(mine + lr * HD + d) = o;
+      if (d == 0) { mine[32 * HD + 2 * lr] = M; mine[32 * HD + 2 * lr + 1] = Ls; }
+      continue;
+    }
     if (ns_live > 1) {
       const uint64_t slot = ((uint64_t)c * p.n_heads + h) * p.n_splits + split;
       *reinterpret_cast<float4*>(p.part_o + slot * HD + d) = o;
@@ -326,16 +333,22 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
       continue;
     }
     // a call of one split needs no merge: gate and store here
-    float ov[4] = {o.x, o.y, o.z, o.w};
-    const uint64_t go = (uint64_t)c * p.gate_col_stride + (uint64_t)h * p.gate_head_stride + d, oo = (uint64_t)c * p.out_col_stride + (uint64_t)h * HD + d;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      ov[e] = __fdiv_rn(ov[e], Ls);
-      if (p.gate) ov[e] = __fmul_rn(ov[e], __fdiv_rn(1.0f, __fadd_rn(1.0f, __expf(-ld_act(p.gate, go + e, p.act_f16)))));
-      if (p.act_f16) reinterpret_cast<__half*>(p.out)[oo + e] = __float2half_rn(ov[e]);
-      else reinterpret_cast<float*>(p.out)[oo + e] = ov[e];
-    }
+    gate_store4(o, Ls, p.gate, (uint64_t)c * p.gate_col_stride + (uint64_t)h * p.gate_head_stride + d, p.out, (uint64_t)c * p.out_col_stride + (uint64_t)h * HD + d,
+                p.act_f16);
   }
+  if (!p.cluster) return;
+  // at most eight splits: the CTAs of a row tile are a cluster, share out its outputs and read one another's rows (a second
+  // kernel for the merge was a third of a short call's time)
+  cluster_sync();
+  const uint32_t mine_s = sm0 + L::MERGE;
+  for (uint32_t idx = split * kQ8Threads + tid; idx < n_rows_here * (HD / 4); idx += ns_live * kQ8Threads) {
+    const uint32_t lr = idx / (HD / 4), d = (idx % (HD / 4)) * 4, row = row0 + lr, c = row / G, h = g * G + row % G;
+    float Ls;
+    const float4 o = cluster_merge4(mine_s + (lr * HD + d) * 4, mine_s + (32 * HD + 2 * lr) * 4, ns_live, Ls);
+    gate_store4(o, Ls, p.gate, (uint64_t)c * p.gate_col_stride + (uint64_t)h * p.gate_head_stride + d, p.out, (uint64_t)c * p.out_col_stride + (uint64_t)h * HD + d,
+                p.act_f16);
+  }
+  cluster_sync();          // no CTA leaves while another reads its rows
 }
 
 template <int HD>
@@ -346,10 +359,11 @@ static cudaError_t launch_q8_t(const Q8Params& p, dim3 grid, int dev, cudaStream
     if (e != cudaSuccess) return e;
     attr_set[dev & 63] = true;
   }
+  if (p.cluster) return launch_pdl_cluster(pa_q8_kernel<HD>, grid, dim3(kQ8Threads), (size_t)Q8Smem<HD>::TOTAL, st, p.cluster, p);
   return launch_pdl(pa_q8_kernel<HD>, grid, dim3(kQ8Threads), (size_t)Q8Smem<HD>::TOTAL, st, p);
 }
 cudaError_t launch_q8(const Q8Params& p, uint32_t hd, uint32_t n_kv, int dev, cudaStream_t st) {
-  const dim3 grid(p.n_splits, n_kv, (p.n_cols * p.G + 8 * p.rgw - 1) / (8 * p.rgw));
+  const dim3 grid(p.cluster ? p.cluster : p.n_splits, n_kv, (p.n_cols * p.G + 8 * p.rgw - 1) / (8 * p.rgw));
   switch (hd) {
     case 256: return launch_q8_t<256>(p, grid, dev, st);
     case 128: return launch_q8_t<128>(p, grid, dev, st);
