@@ -232,6 +232,20 @@ __device__ __forceinline__ float rot_exact(float x, float y, const Angle& g, boo
   return (float)(minus ? __dsub_rn(a, b) : __dadd_rn(a, b));
 }
 
+// fl16(fl32( fl64( fl64(x * cos) -/+ fl64(y * sin) ) )), the rotation of rot_exact() rounded on to f16, for a third of
+// its instructions: the f32 expression with the high parts of cos and sin lies within 2^-22 (|x cos| + |y sin|) of the
+// f32 result (two roundings of cos / sin, two products, one sum, the result's own rounding: 2^-24 each), so where f16
+// rounds everything within 1.5 * 2^-22 of it to one number, that is the number.  `ok` is cleared where it does not, and for NaN
+// and values near f16's overflow (one output in some 500): the caller then takes rot_exact().
+__device__ __forceinline__ uint32_t rot_h(float x, float y, float c, float s, bool minus, bool& ok) {
+  const float t1 = __fmul_rn(x, c), t2 = __fmul_rn(y, s), v = minus ? __fsub_rn(t1, t2) : __fadd_rn(t1, t2);
+  const float M = __fadd_rn(fabsf(t1), fabsf(t2));
+  const __half2 h = __floats2half2_rn(__fmaf_rn(M, -3.5762787e-7f, v), __fmaf_rn(M, 3.5762787e-7f, v));
+  const uint32_t u = *reinterpret_cast<const uint32_t*>(&h);
+  ok = (u >> 16) == (u & 0xffffu) && M < 60000.f;
+  return u & 0xffffu;
+}
+
 // QK head-norm: out = f32((x * inv) * w), inv = 1 / sqrt(ss / hd + eps), with ss the float64 sum of the squares of a
 // head's values IN INDEX ORDER -- the order is part of the result.  The squares of f32 values are exact in float64, so
 // two orders differ by their additions' roundings only: at most hd * 2^-53 of ss each way for the in-order sum (hd at

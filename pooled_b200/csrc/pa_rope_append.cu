@@ -187,9 +187,8 @@ __global__ void __launch_bounds__(256) pa_rope_append_cols_kernel(const RopePara
 
 
 // Prefill chunks of f16 activations with the rotated q stored as f16 (what the prefill kernel consumes): the same
-// arithmetic as the kernels above.  One CTA per column, two passes: the rotated dims two at a time (every lane of
-// a warp does the same four rotations: mixed with copies, the few rotating lanes would hold their warps up), then
-// 16-byte vectors of everything that is only copied (NaNs take the pattern the scalar path produces).
+// results as the kernels above.  The rotated dims first, then 16-byte vectors of everything that is only copied (NaNs
+// take the pattern the scalar path produces).
 __device__ __forceinline__ uint32_t fix_nan2(uint32_t w, bool cache) {
   // per half: NaN -> 0x7fff (q, cvt.rn.f16.f32 of a NaN) or sign | 0x7e00 (cache, f16_rne)
   uint32_t out = w;
@@ -203,18 +202,26 @@ __device__ __forceinline__ uint32_t fix_nan2(uint32_t w, bool cache) {
   }
   return out;
 }
-__global__ void __launch_bounds__(256) pa_rope_append_vec_kernel(const RopeParams p) {
-  __shared__ Angle s_g[128];
-  const uint32_t col = blockIdx.x, half = p.n_rot / 2, hd = p.hd;
+// one output the way of the other kernels, in the few cases rot_h() leaves open: the cache takes f16_rne's NaN pattern
+static __device__ __noinline__ uint32_t rot_h_slow(uint32_t xw, uint32_t yw, int shift, const Angle* g, bool minus, bool cache) {
+  const float x = __half2float(__ushort_as_half((unsigned short)(xw >> shift))), y = __half2float(__ushort_as_half((unsigned short)(yw >> shift)));
+  const float r = rot_exact(x, y, *g, minus);
+  return cache ? __half_as_ushort(f16_rne(r)) : __half_as_ushort(__float2half_rn(r));
+}
+// 64 threads per column, four columns per CTA.  Thread t of a column holds the cos / sin of eight neighbouring dims and
+// walks the heads t / (half / 8), + 64 / (half / 8), ...: 16-byte loads and stores on both sides, the angles loaded once,
+// rot_h() for the arithmetic.  (Before: a CTA per column, two dims per thread, rot_exact().  Eight layers of 2999 columns of 16 + 8
+// heads x 128, whole calls, together with the order of the prefill kernel's CTAs: 834 us then, 677 now, 96 of the difference
+// in that kernel.)  n_rot / 16 is a power of two up to 16.
+__global__ void __launch_bounds__(256) pa_rope_append_vec_kernel(const RopeParams p, const uint32_t n_cols) {
+  __shared__ float2 s_cs[4][128];
+  const uint32_t cl = threadIdx.x >> 6, t = threadIdx.x & 63, col = blockIdx.x * 4 + cl, half = p.n_rot / 2, hd = p.hd;
+  const bool live = col < n_cols;
   if (p.trigger_early) pdl_trigger();
   pdl_wait();
   if (!p.trigger_early) pdl_trigger();
-  // the column's angles are requested now and go to shared memory after the first items' loads have been requested
-  // too: one memory round trip for both (half <= 128 <= blockDim.x)
-  Angle my_g;
-  const bool has_g = threadIdx.x < half;
-  if (has_g) my_g = p.n_ang ? p.ang[col * half + threadIdx.x] : p.angles[(uint64_t)col * half + threadIdx.x];
-  bool g_staged = false;
+  const Angle* ang = p.angles + (uint64_t)col * half;
+  if (live) for (uint32_t i = t; i < half; i += 64) s_cs[cl][i] = make_float2(ang[i].c_hi, ang[i].s_hi);
   const uint32_t kvd = p.kv_heads * hd;
   const __half* qs = reinterpret_cast<const __half*>(p.q) + (uint64_t)col * p.q_col_stride;
   const __half* ks = reinterpret_cast<const __half*>(p.k) + (uint64_t)col * p.kv_col_stride;
@@ -222,56 +229,61 @@ __global__ void __launch_bounds__(256) pa_rope_append_vec_kernel(const RopeParam
   __half* qd = reinterpret_cast<__half*>(p.q_out) + (uint64_t)col * p.q_out_col_stride;
   __half* kd = p.k_cache + (p.cache_row0 + col) * (uint64_t)kvd;
   __half* vd = p.v_cache + (p.cache_row0 + col) * (uint64_t)kvd;
-  const uint32_t nqh = p.q ? p.q_heads : 0, nkh = p.k ? p.kv_heads : 0;
-
-  // ---- rotated dims: an item is two adjacent dims (d, d + 1) with their partners (d + half, d + half + 1) of one
-  //      head, so every lane of a warp carries the same four rotations ----
-  {
-    const uint32_t per = half / 2, total = (nqh + nkh) * per;
-    for (uint32_t base = 0; base < total; base += 2 * blockDim.x) {   // (the same trips for every thread: a barrier sits inside)
-      const uint32_t w0 = base + threadIdx.x;
-      uint32_t A[2], B[2]; const __half* src[2]; __half* dst[2]; uint32_t dd[2]; int kind[2];
+  const uint32_t nqh = p.q ? p.q_heads : 0, nh = nqh + (p.k ? p.kv_heads : 0);
+  const uint32_t groups = half / 8, step = 64 / groups, d = (t % groups) * 8;
+  __syncthreads();
+  if (!live) return;
+  float2 cs[8];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const uint32_t w = w0 + u * blockDim.x;
-        kind[u] = -1;
-        if (w >= total) continue;
-        const uint32_t head = w / per, d = 2 * (w % per);
-        const bool is_q = head < nqh;
-        kind[u] = is_q ? 0 : 1; dd[u] = d;
-        src[u] = (is_q ? qs + (uint64_t)head * p.q_head_stride : ks + (uint64_t)(head - nqh) * hd) + d;
-        dst[u] = (is_q ? qd + (uint64_t)head * hd : kd + (uint64_t)(head - nqh) * hd) + d;
-        A[u] = *reinterpret_cast<const uint32_t*>(src[u]);
-        B[u] = *reinterpret_cast<const uint32_t*>(src[u] + half);
-      }
-      if (!g_staged) {
-        if (has_g) s_g[threadIdx.x] = my_g;
-        __syncthreads();
-        g_staged = true;
-      }
+  for (int e = 0; e < 8; ++e) cs[e] = s_cs[cl][d + e];
+  // ---- rotated dims: d .. d + 7 with their partners half further on, two heads in flight ----
+  for (uint32_t h0 = t / groups; h0 < nh; h0 += 2 * step) {
+    uint4 A[2], B[2];
+    __half* dst[2];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (kind[u] < 0) continue;
-        const bool cache = kind[u] != 0;
-        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&A[u])), b = __half22float2(*reinterpret_cast<const __half2*>(&B[u]));
-        const Angle g0 = s_g[dd[u]], g1 = s_g[dd[u] + 1];
-        const float ra0 = rot_exact(a.x, b.x, g0, true), ra1 = rot_exact(a.y, b.y, g1, true);
-        const float rb0 = rot_exact(b.x, a.x, g0, false), rb1 = rot_exact(b.y, a.y, g1, false);
-        auto h = [&](float x) -> uint32_t { return cache ? __half_as_ushort(f16_rne(x)) : __half_as_ushort(__float2half_rn(x)); };
-        *reinterpret_cast<uint32_t*>(dst[u]) = h(ra0) | (h(ra1) << 16);
-        *reinterpret_cast<uint32_t*>(dst[u] + half) = h(rb0) | (h(rb1) << 16);
+    for (int u = 0; u < 2; ++u) {
+      const uint32_t h = h0 + u * step;
+      if (h >= nh) continue;
+      const __half* src = (h < nqh ? qs + (uint64_t)h * p.q_head_stride : ks + (uint64_t)(h - nqh) * hd) + d;
+      dst[u] = (h < nqh ? qd + (uint64_t)h * hd : kd + (uint64_t)(h - nqh) * hd) + d;
+      A[u] = *reinterpret_cast<const uint4*>(src);
+      B[u] = *reinterpret_cast<const uint4*>(src + half);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (h0 + u * step >= nh) continue;
+      const uint32_t aw[4] = {A[u].x, A[u].y, A[u].z, A[u].w}, bw[4] = {B[u].x, B[u].y, B[u].z, B[u].w};
+      uint32_t ra[8], rb[8], bad = 0;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float2 a2 = __half22float2(*reinterpret_cast<const __half2*>(&aw[e >> 1])), b2 = __half22float2(*reinterpret_cast<const __half2*>(&bw[e >> 1]));
+        const float x = e & 1 ? a2.y : a2.x, y = e & 1 ? b2.y : b2.x;
+        bool ok1, ok2;
+        ra[e] = rot_h(x, y, cs[e].x, cs[e].y, true, ok1);
+        rb[e] = rot_h(y, x, cs[e].x, cs[e].y, false, ok2);
+        bad |= (ok1 ? 0u : 1u << e) | (ok2 ? 0u : 256u << e);
       }
+      if (bad) {
+        const bool cache = h0 + u * step >= nqh;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          if (bad & (1u << e)) ra[e] = rot_h_slow(aw[e >> 1], bw[e >> 1], 16 * (e & 1), ang + d + e, true, cache);
+          if (bad & (256u << e)) rb[e] = rot_h_slow(bw[e >> 1], aw[e >> 1], 16 * (e & 1), ang + d + e, false, cache);
+        }
+      }
+      *reinterpret_cast<uint4*>(dst[u]) = make_uint4(ra[0] | (ra[1] << 16), ra[2] | (ra[3] << 16), ra[4] | (ra[5] << 16), ra[6] | (ra[7] << 16));
+      *reinterpret_cast<uint4*>(dst[u] + half) = make_uint4(rb[0] | (rb[1] << 16), rb[2] | (rb[3] << 16), rb[4] | (rb[5] << 16), rb[6] | (rb[7] << 16));
     }
   }
   // ---- everything else: 16-byte vectors of the unrotated dims of q and k, and all of v ----
   {
     const uint32_t cv = (hd - p.n_rot) / 8, vv = hd / 8;
-    const uint32_t nq = p.q_rot_only ? 0u : nqh * cv, nk = nkh * cv, nv = p.v ? p.kv_heads * vv : 0, total = nq + nk + nv;
-    for (uint32_t w0 = threadIdx.x; w0 < total; w0 += 4 * blockDim.x) {
+    const uint32_t nq = p.q_rot_only ? 0u : nqh * cv, nk = (nh - nqh) * cv, nv = p.v ? p.kv_heads * vv : 0, total = nq + nk + nv;
+    for (uint32_t w0 = t; w0 < total; w0 += 4 * 64) {
       uint4 A[4]; __half* dst[4]; int kind[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const uint32_t w = w0 + u * blockDim.x;
+        const uint32_t w = w0 + u * 64;
         kind[u] = -1;
         if (w >= total) continue;
         const __half* src;
@@ -280,10 +292,10 @@ __global__ void __launch_bounds__(256) pa_rope_append_vec_kernel(const RopeParam
           kind[u] = 1; src = vs + 8 * x; dst[u] = vd + 8 * x;
         } else {
           const bool is_q = w < nq;
-          const uint32_t ww = is_q ? w : w - nq, head = ww / cv, d = p.n_rot + 8 * (ww % cv);
+          const uint32_t ww = is_q ? w : w - nq, head = ww / cv, dd = p.n_rot + 8 * (ww % cv);
           kind[u] = is_q ? 0 : 1;
-          src = (is_q ? qs + (uint64_t)head * p.q_head_stride : ks + (uint64_t)head * hd) + d;
-          dst[u] = (is_q ? qd + (uint64_t)head * hd : kd + (uint64_t)head * hd) + d;
+          src = (is_q ? qs + (uint64_t)head * p.q_head_stride : ks + (uint64_t)head * hd) + dd;
+          dst[u] = (is_q ? qd + (uint64_t)head * hd : kd + (uint64_t)head * hd) + dd;
         }
         A[u] = *reinterpret_cast<const uint4*>(src);
       }
@@ -380,13 +392,14 @@ __global__ void __launch_bounds__(256) pa_sigmoid_mul_kernel(const SigmoidParams
 // whether a call goes to the vectorised kernel (the only one that knows q_rot_only)
 bool rope_vec_applies(const RopeParams& p, uint32_t n_cols) {
   auto al16 = [](const void* x) { return ((uintptr_t)x & 15) == 0; };
-  return !p.n_items && n_cols >= 16 && p.mode == PA_ROPE_F64 && (p.angles || p.n_ang) && p.in_f16 && p.n_rot % 16 == 0 && p.n_rot <= 256 && p.hd % 8 == 0 &&
+  return !p.n_items && n_cols >= 16 && p.mode == PA_ROPE_F64 && p.angles && p.in_f16 && p.n_rot % 16 == 0 && p.n_rot <= 256 && !((p.n_rot / 16) & (p.n_rot / 16 - 1)) &&
+         p.hd % 8 == 0 &&
          (!p.q || (p.q_out_f16 == 1 && al16(p.q) && al16(p.q_out) && p.q_col_stride % 8 == 0 && p.q_head_stride % 8 == 0 && p.q_out_col_stride % 8 == 0)) &&
          (!p.k || (p.v && al16(p.k) && al16(p.v) && p.kv_col_stride % 8 == 0 && p.v_col_stride % 8 == 0));
 }
 
 cudaError_t launch_rope_append(const RopeParams& p, uint32_t n_cols, cudaStream_t st) {
-  if (rope_vec_applies(p, n_cols)) return launch_pdl(pa_rope_append_vec_kernel, dim3(n_cols), dim3(256), 0, st, p);
+  if (rope_vec_applies(p, n_cols)) return launch_pdl(pa_rope_append_vec_kernel, dim3((n_cols + 3) / 4), dim3(256), 0, st, p, n_cols);
   if (n_cols >= 16 && !p.n_items) return launch_pdl(pa_rope_append_cols_kernel, dim3(n_cols), dim3(256), 0, st, p);
   const uint32_t slots = (p.q ? p.q_heads : 0) + (p.k ? p.kv_heads : 0) + (p.v ? p.kv_heads : 0);
   return launch_pdl(pa_rope_append_kernel, dim3(n_cols, slots), dim3(128), 0, st, p);

@@ -254,6 +254,31 @@ def test_head_norm_keeps_the_bits_of_the_in_order_sum(hd, heads, n_cols, tie):
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
 
 
+@pytest.mark.parametrize("hd,n_rot,n_cols,heads", [(256, 64, 16, 2), (128, 128, 67, 8), (256, 256, 17, 1), (64, 32, 130, 3), (128, 16, 21, 2), (256, 96, 18, 2)])
+def test_prompt_rotation_of_f16_rows_keeps_the_bits(hd, n_rot, n_cols, heads):
+    # chunks of f16 activations: the short f16 rotation with its exact path behind it (n_rot 96 takes the kernel of other
+    # widths), over ordinary values, zeros of both signs, subnormals, values whose rotation overflows f16, infinities and NaN.
+    # The angles of wide calls come from the device's sincos, whose last place may differ from libm's: a few halves in
+    # ten thousand of them by one, as an f32 result does then (probability about 1e-8 each; two are allowed)
+    import torch
+    pos, theta = 1000, 1e6
+    eng = _engine(n_heads=heads, n_kv_heads=heads, head_dim=hd, n_rot=n_rot, rope_theta=theta, max_seq=pos + n_cols, act_dtype=torch.float16, max_cols=256)
+    rng = np.random.default_rng(29)
+    k = po.h2f(po.f16_rne((rng.standard_normal((n_cols, heads * hd)) * 3).astype(np.float32)))
+    odd = np.array([0.0, -0.0, 6e-8, -6e-8, 3e-5, 60000.0, -65504.0, np.inf, -np.inf, np.nan], np.float32)
+    mask = rng.random(k.shape) < 0.2
+    k = po.h2f(po.f16_rne(np.where(mask, rng.choice(odd, k.shape), k).astype(np.float32)))
+    q, v = torch.zeros((n_cols, heads * hd), dtype=torch.float16, device="cuda"), torch.zeros((n_cols, heads * hd), dtype=torch.float16, device="cuda")
+    eng.encode_layer(0, pos, q, util.torch_dev(k, torch.float16), v, mode="prefill")
+    eng.sync()
+    got = eng.cache(0, "k")[0, pos:pos + n_cols].cpu().numpy().view(np.uint16)
+    with np.errstate(all="ignore"):
+        want = np.stack([po.f16_rne(po.rope_neox_f64(k[c], heads, hd, n_rot, pos + c, theta)) for c in range(n_cols)])
+    nan = (want & 0x7fff) > 0x7c00
+    assert np.array_equal(nan, (got & 0x7fff) > 0x7c00) and np.all((got[nan] & 0x7fff) == 0x7e00)
+    assert int(np.count_nonzero(got[~nan] != want[~nan])) <= 2
+
+
 def test_rope_append_items_equals_per_sequence_calls():
     # one token of each of 8 sequences at different positions in one launch == 8 pa_rope_append calls, bit for bit; with a
     # shard origin set, items outside the shard are rotated but not appended
