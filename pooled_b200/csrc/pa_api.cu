@@ -900,6 +900,14 @@ static int decode_impl(pa_layer* L, const pa_item* items, uint32_t n_items, cons
     if (flat) ns = max_ns;
   }
   p.n_items = n_items;
+  // one item: the device need not derive the plan (in the merge kernel that was a chain of parameter loads ahead of the
+  // first record's)
+  uint32_t live = 0;
+  if (n_items == 1 && !gl && max_rows > 0) {
+    const uint32_t tiles = ceil_div(max_rows, 64), n = verify_tc ? ns : std::min(ns, plan_cap(tiles));
+    p.tps = ceil_div(tiles, n);
+    live = ceil_div(tiles, p.tps);
+  }
   p.q = q; p.q_f16 = q_dtype == PA_F16; p.q_col_stride = qcs; p.q_head_stride = qhs;
   p.part_o = ctx->part_o; p.part_ml = ctx->part_ml; p.n_splits = ns;
   p.n_heads = ctx->cfg.n_heads; p.G = ctx->G; p.max_seq = L->max_seq;
@@ -970,7 +978,7 @@ static int decode_impl(pa_layer* L, const pa_item* items, uint32_t n_items, cons
   const uint32_t rs = ns * groups;
   c.o_row_stride = (uint64_t)rs * ctx->cfg.head_dim; c.o_part_stride = ctx->cfg.head_dim;
   c.ml_row_stride = (uint64_t)rs * 2; c.ml_part_stride = 2;
-  c.n_heads = ctx->cfg.n_heads; c.fixed_parts = 0; c.n_splits = ns; c.groups = groups;
+  c.n_heads = ctx->cfg.n_heads; c.fixed_parts = live; c.n_splits = ns; c.groups = groups;
   c.gather = p.gather; c.gather_stride = p.gather_stride;
   c.gate = gate; c.gate_col_stride = gcs; c.gate_head_stride = ghs; c.out = out; c.out_col_stride = ocs;
   c.act_f16 = ctx->cfg.act_dtype == PA_F16;

@@ -278,7 +278,7 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
 
   const uint32_t g = blockIdx.y;
   uint32_t split = blockIdx.x, item = blockIdx.z;
-  const bool balanced = p.items.tps[0] != 0;
+  const bool balanced = !p.tps && p.items.tps[0] != 0;     // (a single item touches none of the batch's plan)
   if (balanced) {   // the CTAs of the items follow one another (an item without rows has none)
     for (uint32_t i = 1; i < p.n_items; ++i) if (blockIdx.x >= p.items.cta0[i]) item = i;
     split = blockIdx.x - p.items.cta0[item];
@@ -297,7 +297,7 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
   // every item plans for its own length: plan_cap(tiles) splits, at most the launch's split count (the longest
   // item's plan, or in gather mode the most any list could need)
   const uint32_t ns_eff = min(p.n_splits, plan_cap(tiles));
-  const uint32_t tps = balanced ? p.items.tps[item] : (tiles + ns_eff - 1) / max(ns_eff, 1u);  // tiles per split
+  const uint32_t tps = p.tps ? p.tps : balanced ? p.items.tps[item] : (tiles + ns_eff - 1) / max(ns_eff, 1u);  // tiles per split
   const uint32_t tile0 = split * tps;
   if (tile0 >= tiles) {
     if constexpr (NT <= 2) {

@@ -11,6 +11,7 @@ struct DecodeParams {
   float* part_o;            // [rows][n_splits][HD]
   float* part_ml;           // [rows][n_splits][2]   (m in natural-log units, l)
   uint32_t n_splits;
+  uint32_t tps;             // one item: its tiles per split, as the host planned it (0: derived on the device)
   uint32_t n_heads, G, max_seq, n_stages;
   // fused front (one token; head_dim 256 with 64 rotary dims, or head_dim 128 rotated in full): q arrives unrotated and the consumers rotate
   // it; the CTA that walks the sequence's last tile also rotates k, converts v and appends the token's row

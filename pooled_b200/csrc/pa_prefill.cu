@@ -244,8 +244,10 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // prefill: q tile (longest rows first) x q head.  split-K: split x kv head.
-  const uint32_t q_tile = gridDim.x - 1 - blockIdx.x;
-  const uint32_t h = blockIdx.y, g = SK ? blockIdx.y : h / p.G;
+  // Every head's longest q tile first, then every head's next one: with the q tiles of a head following one another the
+  // last heads' longest tiles began when the other SMs had run out of work (2048 columns of 24 heads: SMs busy 71 %).
+  const uint32_t q_tile = gridDim.y - 1 - blockIdx.y;
+  const uint32_t h = SK ? blockIdx.y : blockIdx.x, g = SK ? blockIdx.y : h / p.G;
   const uint32_t c0 = q_tile * kBM;
   const uint32_t rows_valid = SK ? 0u : min((uint32_t)kBM, p.n_cols - c0);
   const uint32_t p0 = p.pos + c0;                       // cache row of column c0's own token
@@ -857,16 +859,12 @@ static cudaError_t launch_pf(const pa_layer* L, const PrefillParams& p, const CU
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  if (MODE == 0 || MODE == 3) {
-    pa_prefill_kernel<HD, MODE><<<grid, PfSmem<HD, MODE>::THREADS, PfSmem<HD, MODE>::TOTAL, st>>>(tm_k, tm_v, tm_q, tm_o, tm_q2, p);
-    return cudaGetLastError();
-  }
   return launch_pdl(pa_prefill_kernel<HD, MODE>, grid, dim3(PfSmem<HD, MODE>::THREADS), (size_t)PfSmem<HD, MODE>::TOTAL, st, tm_k, tm_v, tm_q, tm_o, tm_q2, p);
 }
 
 cudaError_t launch_prefill(const pa_layer* L, const PrefillParams& p, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_q,
                            const CUtensorMap& tm_o, const CUtensorMap& tm_q2, cudaStream_t st) {
-  const dim3 grid((p.n_cols + kBM - 1) / kBM, p.n_heads, p.n_splits);
+  const dim3 grid(p.n_heads, (p.n_cols + kBM - 1) / kBM, p.n_splits);
   switch (L->ctx->cfg.head_dim) {
     case 256: return p.n_splits > 1 ? launch_pf<256, 3>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st) : launch_pf<256, 0>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st);
     case 128: return p.n_splits > 1 ? launch_pf<128, 3>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st) : launch_pf<128, 0>(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, grid, st);
