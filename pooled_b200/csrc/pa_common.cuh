@@ -24,8 +24,8 @@ enum : uint32_t { WAIT_KFULL = 1, WAIT_VFULL = 2, WAIT_EMPTY = 3, WAIT_MMA = 4, 
 
 // Most splits of a decode call over `tiles` 64-row tiles.  Up to eight tiles one each: their records are merged through
 // cluster shared memory (see the end of pa_decode_kernel), so another split costs little and a tile is 0.7 to 1.2 us of a chain
-// of latencies.  Beyond 16 tiles two tiles at least, so that a CTA's start and end are shared.
-__host__ __device__ constexpr uint32_t plan_cap(uint32_t tiles) { return tiles <= 1 ? 1u : tiles <= 8 ? tiles : tiles < 16 ? 8u : tiles / 2; }
+// of latencies.  Beyond 16 tiles two tiles each (the last one perhaps one), so that a CTA's start and end are shared.
+__host__ __device__ constexpr uint32_t plan_cap(uint32_t tiles) { return tiles <= 1 ? 1u : tiles <= 8 ? tiles : tiles < 16 ? 8u : (tiles + 1) / 2; }
 constexpr int kMaxCluster = 8;    // the portable cluster size
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
