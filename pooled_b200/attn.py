@@ -114,7 +114,8 @@ class AttnEngine:
     def __init__(self, cfg: AttnConfig, device: int = 0):
         self.cfg, self.device = cfg, device
         self.L = _l.load()
-        self._call = self.L.call
+        self._call, e = self.L.call, self.L.entry
+        self._f_layer, self._f_items, self._f_rope, self._f_gather = e["pa_attn_layer"], e["pa_attn_items"], e["pa_rope_append"], e["pa_decode_gather"]
         pc = _l.PaConfig(n_heads=cfg.n_heads, n_kv_heads=cfg.n_kv_heads, head_dim=cfg.head_dim, n_rot=cfg.n_rot, rope_theta=cfg.rope_theta,
                          rope_mode=_ROPE[cfg.rope_mode], act_dtype=_dt(cfg.act_dtype), max_cols=cfg.max_cols, splits=cfg.splits,
                          flags=_l.PA_FLAG_FAST if cfg.fast else 0)
@@ -234,7 +235,7 @@ class AttnEngine:
                     cs_table: torch.Tensor | None = None) -> torch.Tensor:
         n_cols = q.shape[0]
         q_rot = torch.empty((n_cols, self.cfg.q_dim), dtype=torch.float32, device=q.device)
-        rc = self._call.rope_append(self.layers[li].value, seq, pos, q, q_head_stride or self.cfg.head_dim, k, v, cs_table, q_rot, self._raw_st())
+        rc = self._call.rope_append(self._f_rope, self.layers[li].value, seq, pos, q, q_head_stride or self.cfg.head_dim, k, v, cs_table, q_rot, self._raw_st())
         if rc:
             self._ck(rc)
         return q_rot
@@ -256,7 +257,7 @@ class AttnEngine:
         hd = self.cfg.head_dim
         if out is None:
             out = torch.empty((len(seqs_pos), self.cfg.q_dim), dtype=self.cfg.act_dtype, device=q.device)
-        rc = self._call.attn_items(self.layers[li].value, seqs_pos, q, q_head_stride or hd, k, v, gate, gate_head_stride or hd, out, 1 if sharded else 0,
+        rc = self._call.attn_items(self._f_items, self.layers[li].value, seqs_pos, q, q_head_stride or hd, k, v, gate, gate_head_stride or hd, out, 1 if sharded else 0,
                                    self._raw_st())
         if rc:
             self._ck(rc)
@@ -293,7 +294,7 @@ class AttnEngine:
         if out is None:
             out = torch.empty((n_cols, self.cfg.q_dim), dtype=self.cfg.act_dtype, device=q.device)
         hd = self.cfg.head_dim
-        rc = self._call.decode_gather(self.layers[li].value, seq, row_lists, row_lists.shape[1], q, _dt(q.dtype), q_head_stride or hd, gate, gate_head_stride or hd, out,
+        rc = self._call.decode_gather(self._f_gather, self.layers[li].value, seq, row_lists, row_lists.shape[1], q, _dt(q.dtype), q_head_stride or hd, gate, gate_head_stride or hd, out,
                                       self._raw_st())
         if rc:
             self._ck(rc)
@@ -363,7 +364,7 @@ class AttnEngine:
         hd = self.cfg.head_dim
         if out is None:
             out = torch.empty((q.shape[0], self.cfg.q_dim), dtype=self.cfg.act_dtype, device=q.device)
-        rc = self._call.attn_layer(self.layers[li].value, seq, pos, _MODE[mode], q, q_head_stride or hd, k, v, gate, gate_head_stride or hd, cs_table, out,
+        rc = self._call.attn_layer(self._f_layer, self.layers[li].value, seq, pos, _MODE[mode], q, q_head_stride or hd, k, v, gate, gate_head_stride or hd, cs_table, out,
                                    self._raw_st())
         if rc:
             self._ck(rc)

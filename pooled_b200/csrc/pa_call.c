@@ -19,10 +19,8 @@ typedef int (*fn_rope_append)(pa_layer*, uint32_t, uint32_t, uint32_t, const voi
                               void*);
 typedef int (*fn_decode_gather)(pa_layer*, uint32_t, uint32_t, const uint32_t*, uint32_t, const void*, int, uint64_t, uint64_t, const void*, uint64_t,
                                 uint64_t, void*, uint64_t, void*);
-static fn_attn_layer f_attn_layer;
-static fn_attn_items f_attn_items;
-static fn_rope_append f_rope_append;
-static fn_decode_gather f_decode_gather;
+/* Every call names the entry point (its address in the library the engine loaded) as its first argument: the module keeps
+ * nothing of its own. */
 static PyObject *s_data_ptr, *s_stride, *s_size, *i_zero;
 
 static int ptr_of(PyObject* t, void** p) {
@@ -57,36 +55,36 @@ static int args_are(Py_ssize_t n, Py_ssize_t want, const char* who) {
   return -1;
 }
 
-/* attn_layer(layer, seq, pos, mode, q, q_head_stride, k, v, gate, gate_head_stride, cs_table, out, stream) -> status */
+/* attn_layer(entry, layer, seq, pos, mode, q, q_head_stride, k, v, gate, gate_head_stride, cs_table, out, stream) -> status */
 static PyObject* attn_layer(PyObject* self, PyObject* const* a, Py_ssize_t n) {
-  uint64_t layer, qcs, qhs, kcs, gcs = 0, ghs = 0, ocs, stream;
+  uint64_t fn, layer, qcs, qhs, kcs, gcs = 0, ghs = 0, ocs, stream;
   uint32_t seq, pos, mode, cols;
   void *q, *k, *v, *g, *cs, *out;
   (void)self;
-  if (args_are(n, 13, "attn_layer") || u64_of(a[0], &layer) || u32_of(a[1], &seq) || u32_of(a[2], &pos) || u32_of(a[3], &mode) || rows_of(a[4], &cols) ||
-      ptr_of(a[4], &q) || stride0(a[4], &qcs) || u64_of(a[5], &qhs) || ptr_of(a[6], &k) || stride0(a[6], &kcs) || ptr_of(a[7], &v) || ptr_of(a[8], &g) ||
-      (a[8] != Py_None && (stride0(a[8], &gcs) || u64_of(a[9], &ghs))) || ptr_of(a[10], &cs) || ptr_of(a[11], &out) || stride0(a[11], &ocs) ||
-      u64_of(a[12], &stream))
+  if (args_are(n, 14, "attn_layer") || u64_of(a[0], &fn) || u64_of(a[1], &layer) || u32_of(a[2], &seq) || u32_of(a[3], &pos) || u32_of(a[4], &mode) || rows_of(a[5], &cols) ||
+      ptr_of(a[5], &q) || stride0(a[5], &qcs) || u64_of(a[6], &qhs) || ptr_of(a[7], &k) || stride0(a[7], &kcs) || ptr_of(a[8], &v) || ptr_of(a[9], &g) ||
+      (a[9] != Py_None && (stride0(a[9], &gcs) || u64_of(a[10], &ghs))) || ptr_of(a[11], &cs) || ptr_of(a[12], &out) || stride0(a[12], &ocs) ||
+      u64_of(a[13], &stream))
     return NULL;
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = f_attn_layer((pa_layer*)(uintptr_t)layer, seq, pos, cols, (int)mode, q, qcs, qhs, k, v, kcs, g, gcs, ghs, (const float*)cs, out, ocs,
+  rc = ((fn_attn_layer)(uintptr_t)fn)((pa_layer*)(uintptr_t)layer, seq, pos, cols, (int)mode, q, qcs, qhs, k, v, kcs, g, gcs, ghs, (const float*)cs, out, ocs,
                     (void*)(uintptr_t)stream);
   Py_END_ALLOW_THREADS
   return PyLong_FromLong(rc);
 }
 
-/* attn_items(layer, [(seq, pos)], q, q_head_stride, k, v, gate, gate_head_stride, out, exchange, stream) -> status */
+/* attn_items(entry, layer, [(seq, pos)], q, q_head_stride, k, v, gate, gate_head_stride, out, exchange, stream) -> status */
 static PyObject* attn_items(PyObject* self, PyObject* const* a, Py_ssize_t n) {
-  uint64_t layer, qcs, qhs, kcs, gcs = 0, ghs = 0, ocs, stream;
+  uint64_t fn, layer, qcs, qhs, kcs, gcs = 0, ghs = 0, ocs, stream;
   uint32_t exch;
   void *q, *k, *v, *g, *out;
   (void)self;
-  if (args_are(n, 11, "attn_items") || u64_of(a[0], &layer) || ptr_of(a[2], &q) || stride0(a[2], &qcs) || u64_of(a[3], &qhs) || ptr_of(a[4], &k) ||
-      stride0(a[4], &kcs) || ptr_of(a[5], &v) || ptr_of(a[6], &g) || (a[6] != Py_None && (stride0(a[6], &gcs) || u64_of(a[7], &ghs))) || ptr_of(a[8], &out) ||
-      stride0(a[8], &ocs) || u32_of(a[9], &exch) || u64_of(a[10], &stream))
+  if (args_are(n, 12, "attn_items") || u64_of(a[0], &fn) || u64_of(a[1], &layer) || ptr_of(a[3], &q) || stride0(a[3], &qcs) || u64_of(a[4], &qhs) || ptr_of(a[5], &k) ||
+      stride0(a[5], &kcs) || ptr_of(a[6], &v) || ptr_of(a[7], &g) || (a[7] != Py_None && (stride0(a[7], &gcs) || u64_of(a[8], &ghs))) || ptr_of(a[9], &out) ||
+      stride0(a[9], &ocs) || u32_of(a[10], &exch) || u64_of(a[11], &stream))
     return NULL;
-  PyObject* list = PySequence_Fast(a[1], "the items are a sequence of (seq, pos) pairs");
+  PyObject* list = PySequence_Fast(a[2], "the items are a sequence of (seq, pos) pairs");
   if (!list) return NULL;
   const Py_ssize_t cnt = PySequence_Fast_GET_SIZE(list);
   pa_item* items = (pa_item*)calloc((size_t)(cnt ? cnt : 1), sizeof(pa_item));
@@ -103,60 +101,48 @@ static PyObject* attn_items(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   Py_DECREF(list);
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = f_attn_items((pa_layer*)(uintptr_t)layer, items, (uint32_t)cnt, q, qcs, qhs, k, v, kcs, g, gcs, ghs, out, ocs, (int)exch, (void*)(uintptr_t)stream);
+  rc = ((fn_attn_items)(uintptr_t)fn)((pa_layer*)(uintptr_t)layer, items, (uint32_t)cnt, q, qcs, qhs, k, v, kcs, g, gcs, ghs, out, ocs, (int)exch, (void*)(uintptr_t)stream);
   Py_END_ALLOW_THREADS
   free(items);
   return PyLong_FromLong(rc);
 }
 
-/* rope_append(layer, seq, pos, q, q_head_stride, k, v, cs_table, q_rot, stream) -> status */
+/* rope_append(entry, layer, seq, pos, q, q_head_stride, k, v, cs_table, q_rot, stream) -> status */
 static PyObject* rope_append(PyObject* self, PyObject* const* a, Py_ssize_t n) {
-  uint64_t layer, qcs, qhs, kcs, stream;
+  uint64_t fn, layer, qcs, qhs, kcs, stream;
   uint32_t seq, pos, cols;
   void *q, *k, *v, *cs, *qr;
   (void)self;
-  if (args_are(n, 10, "rope_append") || u64_of(a[0], &layer) || u32_of(a[1], &seq) || u32_of(a[2], &pos) || rows_of(a[3], &cols) || ptr_of(a[3], &q) ||
-      stride0(a[3], &qcs) || u64_of(a[4], &qhs) || ptr_of(a[5], &k) || stride0(a[5], &kcs) || ptr_of(a[6], &v) || ptr_of(a[7], &cs) || ptr_of(a[8], &qr) ||
-      u64_of(a[9], &stream))
+  if (args_are(n, 11, "rope_append") || u64_of(a[0], &fn) || u64_of(a[1], &layer) || u32_of(a[2], &seq) || u32_of(a[3], &pos) || rows_of(a[4], &cols) || ptr_of(a[4], &q) ||
+      stride0(a[4], &qcs) || u64_of(a[5], &qhs) || ptr_of(a[6], &k) || stride0(a[6], &kcs) || ptr_of(a[7], &v) || ptr_of(a[8], &cs) || ptr_of(a[9], &qr) ||
+      u64_of(a[10], &stream))
     return NULL;
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = f_rope_append((pa_layer*)(uintptr_t)layer, seq, pos, cols, q, qcs, qhs, k, v, kcs, (const float*)cs, (float*)qr, (void*)(uintptr_t)stream);
+  rc = ((fn_rope_append)(uintptr_t)fn)((pa_layer*)(uintptr_t)layer, seq, pos, cols, q, qcs, qhs, k, v, kcs, (const float*)cs, (float*)qr, (void*)(uintptr_t)stream);
   Py_END_ALLOW_THREADS
   return PyLong_FromLong(rc);
 }
 
-/* decode_gather(layer, seq, lists, list_stride, q, q_dtype, q_head_stride, gate, gate_head_stride, out, stream) -> status */
+/* decode_gather(entry, layer, seq, lists, list_stride, q, q_dtype, q_head_stride, gate, gate_head_stride, out, stream) -> status */
 static PyObject* decode_gather(PyObject* self, PyObject* const* a, Py_ssize_t n) {
-  uint64_t layer, qcs, qhs, gcs = 0, ghs = 0, ocs, stream;
+  uint64_t fn, layer, qcs, qhs, gcs = 0, ghs = 0, ocs, stream;
   uint32_t seq, list_stride, cols, qdt;
   void *lists, *q, *g, *out;
   (void)self;
-  if (args_are(n, 11, "decode_gather") || u64_of(a[0], &layer) || u32_of(a[1], &seq) || ptr_of(a[2], &lists) || u32_of(a[3], &list_stride) ||
-      rows_of(a[4], &cols) || ptr_of(a[4], &q) || u32_of(a[5], &qdt) || stride0(a[4], &qcs) || u64_of(a[6], &qhs) || ptr_of(a[7], &g) ||
-      (a[7] != Py_None && (stride0(a[7], &gcs) || u64_of(a[8], &ghs))) || ptr_of(a[9], &out) || stride0(a[9], &ocs) || u64_of(a[10], &stream))
+  if (args_are(n, 12, "decode_gather") || u64_of(a[0], &fn) || u64_of(a[1], &layer) || u32_of(a[2], &seq) || ptr_of(a[3], &lists) || u32_of(a[4], &list_stride) ||
+      rows_of(a[5], &cols) || ptr_of(a[5], &q) || u32_of(a[6], &qdt) || stride0(a[5], &qcs) || u64_of(a[7], &qhs) || ptr_of(a[8], &g) ||
+      (a[8] != Py_None && (stride0(a[8], &gcs) || u64_of(a[9], &ghs))) || ptr_of(a[10], &out) || stride0(a[10], &ocs) || u64_of(a[11], &stream))
     return NULL;
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = f_decode_gather((pa_layer*)(uintptr_t)layer, seq, cols, (const uint32_t*)lists, list_stride, q, (int)qdt, qcs, qhs, g, gcs, ghs, out, ocs,
+  rc = ((fn_decode_gather)(uintptr_t)fn)((pa_layer*)(uintptr_t)layer, seq, cols, (const uint32_t*)lists, list_stride, q, (int)qdt, qcs, qhs, g, gcs, ghs, out, ocs,
                        (void*)(uintptr_t)stream);
   Py_END_ALLOW_THREADS
   return PyLong_FromLong(rc);
 }
 
-/* bind(addresses of pa_attn_layer, pa_attn_items, pa_rope_append, pa_decode_gather) */
-static PyObject* bind(PyObject* self, PyObject* const* a, Py_ssize_t n) {
-  uint64_t f[4];
-  (void)self;
-  if (args_are(n, 4, "bind")) return NULL;
-  for (int i = 0; i < 4; ++i) if (u64_of(a[i], &f[i])) return NULL;
-  f_attn_layer = (fn_attn_layer)(uintptr_t)f[0]; f_attn_items = (fn_attn_items)(uintptr_t)f[1];
-  f_rope_append = (fn_rope_append)(uintptr_t)f[2]; f_decode_gather = (fn_decode_gather)(uintptr_t)f[3];
-  Py_RETURN_NONE;
-}
-
 static PyMethodDef methods[] = {
-    {"bind", (PyCFunction)(void (*)(void))bind, METH_FASTCALL, "take the library's entry points"},
     {"attn_layer", (PyCFunction)(void (*)(void))attn_layer, METH_FASTCALL, "pa_attn_layer on tensors"},
     {"attn_items", (PyCFunction)(void (*)(void))attn_items, METH_FASTCALL, "pa_attn_items on tensors"},
     {"rope_append", (PyCFunction)(void (*)(void))rope_append, METH_FASTCALL, "pa_rope_append on tensors"},

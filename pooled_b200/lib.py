@@ -120,13 +120,13 @@ class Lib:
         self.call = self._load_call()
 
     def _load_call(self):
-        """The CPython module with the per-layer calls (csrc/pa_call.c), bound to this library's entry points."""
+        """The CPython module with the per-layer calls (csrc/pa_call.c); `entry` holds this library's addresses for them."""
         if not os.path.exists(CALL_PATH):
             raise PaError(-4, f"{CALL_PATH} is missing: build it with `python -m pooled_b200.build`")
         loader = importlib.machinery.ExtensionFileLoader("_pa_call", CALL_PATH)
         mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_pa_call", CALL_PATH, loader=loader))
         loader.exec_module(mod)
-        mod.bind(*(C.cast(getattr(self.dll, n), C.c_void_p).value for n in ("pa_attn_layer", "pa_attn_items", "pa_rope_append", "pa_decode_gather")))
+        self.entry = {n: C.cast(getattr(self.dll, n), C.c_void_p).value for n in ("pa_attn_layer", "pa_attn_items", "pa_rope_append", "pa_decode_gather")}
         return mod
 
     def check(self, rc: int, ctx=None):
