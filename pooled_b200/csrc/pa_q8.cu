@@ -337,8 +337,8 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
                 p.act_f16);
   }
   if (!p.cluster) return;
-  // at most eight splits: the CTAs of a row tile are a cluster, share out its outputs and read one another's rows (a second
-  // kernel for the merge was a third of a short call's time)
+  // at most eight splits: the CTAs of a row tile are a cluster, share out its outputs and read one another's rows (71
+  // columns of 16 q / 8 kv heads x 128 into an empty cache: 15.1 us a layer call with a merge kernel, 14.5 so)
   cluster_sync();
   const uint32_t mine_s = sm0 + L::MERGE;
   for (uint32_t idx = split * kQ8Threads + tid; idx < n_rows_here * (HD / 4); idx += ns_live * kQ8Threads) {

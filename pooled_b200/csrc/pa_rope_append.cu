@@ -1,6 +1,6 @@
 // RoPE (full or partial, NeoX pairing), the f16 KV-cache append and the standalone sigmoid gate.
 //
-// One small CTA per (column, head), or one CTA per column for prefill chunks.
+// One small CTA per (column, head); for prefill chunks 64 threads per column (f16) or one CTA per column.
 //   PA_ROPE_F64    angle = pos * inv_freq[i] in float64 (inv_freq = theta^(-2i/n_rot) comes from the host's
 //                  libm), cos / sin in float64, the two products and their difference / sum rounded one by
 //                  one in float64, the result rounded to f32 — the arithmetic of pooled's CPU reference
