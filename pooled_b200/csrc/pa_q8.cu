@@ -6,9 +6,13 @@
 //            parts in rows 8-15, B the int8 rows: both halves of the product come from one instruction.
 //   values   O^T[dim, row] += v8^T[dim, pos] . (P * vs)^T[pos, row] : the weights take each block's scale before they are
 //            split into high and low f16 parts.
-// q is first scaled by a power of two per row so that its largest value lies in [2^12, 2^13), P * vs by a running power of
-// two per warp so that the largest lies below 2^14 : high + low then carry 2^-24 of every value that matters, the
-// precision an f32 holds (an unscaled P * vs of 1e-4 would sit among f16's subnormals).
+// q is first scaled by a power of two per row so that its largest value lies in [2^12, 2^13), P * vs by one per row, 32-dim
+// block and step of 16 positions so that its largest lies in [2^13, 2^14) : high + low are then within 2^-23 of that value and
+// within 2^-38 of it of every smaller one (an unscaled P * vs of 1e-4 would sit among f16's subnormals).  The power is a row's
+// and a block's own, and positions a row does not see are not in it: with one for all rows and dims of a warp, a large V scale
+// anywhere took bits from everything else (a block at 2^-20 of its neighbours was off by 9e-6 of itself, now 3e-7 as with f32
+// operands), and an infinite one of a later column made NaN of earlier ones.  It takes 4 shuffles and some 30
+// instructions per pair of blocks and step: 179 us where one power took 173 (the token below), 341 where 319 (the prompt).
 //
 // A warp owns eight query rows (heads of the GQA group, columns) and runs an online softmax over the positions it takes,
 // P in registers from one product to the next; no barrier but the ring's.  A CTA is four warps over a ring of 64-position
@@ -18,7 +22,7 @@
 // converts for its eight rows alone), about 700 instructions per 16 positions and eight rows against 64 MMAs; at long
 // contexts of a single token HBM (1.125 bytes a value).
 // Measured with its front (pa_front.cu) against plain f32 loops, a CTA per column: ten layers of a token over 12345 rows (16 q / 2 kv
-// heads x 256, head-norm) 918 -> 180 us, two layers of a 777-token prompt (24 / 4 x 256) 4231 -> 320 us; distance from float64
+// heads x 256, head-norm) 918 -> 179 us, two layers of a 777-token prompt (24 / 4 x 256) 4231 -> 341 us; distance from float64
 // no larger: 2.3e-7 against 2.9e-7 (that token), 1.7e-7 against 2.1e-7 (that prompt), relative.
 //
 // Stands in for attn_flash_q8 of pooled (engine/wgsl/qwen35.js:946-1010 and its column-wise use in prefill).
@@ -66,6 +70,11 @@ __device__ __forceinline__ void split_h2(float x, float y, uint32_t& hi, uint32_
   const float2 b = __half22float2(h);
   hi = *reinterpret_cast<const uint32_t*>(&h);
   lo = pack_h2(x - b.x, y - b.y);
+}
+// a low part is at most 4 here; that of an infinity would be inf - inf (min takes the number)
+__device__ __forceinline__ uint32_t h2_min8(uint32_t x) {
+  const __half2 r = __hmin2(*reinterpret_cast<const __half2*>(&x), __half2half2(__ushort_as_half(0x4800)));
+  return *reinterpret_cast<const uint32_t*>(&r);
 }
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool live) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
@@ -181,10 +190,10 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   }
   const uint32_t lim = live_row ? row_lim(my_row) : 0u;
   const uint32_t warp_lim = row_lim(row0 + 8 * rg + 7);       // no position at or past it concerns this warp
+  const uint32_t first_lim = row_lim(row0 + 8 * rg);          // every row of the warp sees the positions below it
   const bool warp_live = row0 + 8 * rg < rows;
 
   float m = -1.0e30f, l = 0.f;
-  uint32_t v_exp = 14;                                        // exponent field of the largest V scale so far
   float oacc[2 * NB][4];
 #pragma unroll
   for (int i = 0; i < 2 * NB; ++i) oacc[i][0] = oacc[i][1] = oacc[i][2] = oacc[i][3] = 0.f;
@@ -239,56 +248,78 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
       }
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-      // ---- V scales of positions 2 j, 2 j + 1, 2 j + 8, 2 j + 9 and their largest exponent ----
-      float vsc[4][NB];
-      uint32_t ve = 0;
+      if (__any_sync(0xffffffffu, mx > m)) {
+        const float al = exp2f(m - mx);
+        l *= al;
+        m = mx;
+        const float a0 = __shfl_sync(0xffffffffu, al, 8 * j), a1 = __shfl_sync(0xffffffffu, al, 8 * j + 4);   // rows 2 j, 2 j + 1
+#pragma unroll
+        for (int i = 0; i < 2 * NB; ++i) { oacc[i][0] *= a0; oacc[i][1] *= a1; oacc[i][2] *= a0; oacc[i][3] *= a1; }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { s[e] = exp2f(s[e] - m); l += s[e]; }
+      // ---- weights times the V scales of positions 2 j, 2 j + 1, 2 j + 8, 2 j + 9 ----
+      float pv[4][NB];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const uint32_t pr = 16 * st + 8 * (e >> 1) + 2 * j + (e & 1);
 #pragma unroll
         for (int b = 0; b < NB; b += (NB >= 4 ? 4 : 2)) {
-          if (NB >= 4) *reinterpret_cast<float4*>(&vsc[e][b]) = *reinterpret_cast<const float4*>(vst + pr * NB + b);
-          else *reinterpret_cast<float2*>(&vsc[e][b]) = *reinterpret_cast<const float2*>(vst + pr * NB + b);
+          if (NB >= 4) *reinterpret_cast<float4*>(&pv[e][b]) = *reinterpret_cast<const float4*>(vst + pr * NB + b);
+          else *reinterpret_cast<float2*>(&pv[e][b]) = *reinterpret_cast<const float2*>(vst + pr * NB + b);
         }
-#pragma unroll
-        for (int b = 0; b < NB; ++b) ve = max(ve, __float_as_uint(vsc[e][b]) & 0x7fffffffu);
       }
-      ve = min(__reduce_max_sync(0xffffffffu, ve) >> 23, 254u);
-      if (__any_sync(0xffffffffu, mx > m) || ve > v_exp) {
-        float al = exp2f(m - mx);
-        l *= al;
-        m = mx;
-        if (ve > v_exp) { al *= __uint_as_float((uint32_t)max(0, 127 - (int)(ve - v_exp)) << 23); v_exp = ve; }
-        const float a0 = __shfl_sync(0xffffffffu, al, 8 * j), a1 = __shfl_sync(0xffffffffu, al, 8 * j + 4);   // rows 2 j, 2 j + 1
+      if (pos0 + 16 > first_lim) {      // a position the row does not see counts as nothing, whatever its scale (0 * inf is NaN)
 #pragma unroll
-        for (int i = 0; i < 2 * NB; ++i) { oacc[i][0] *= a0; oacc[i][1] *= a1; oacc[i][2] *= a0; oacc[i][3] *= a1; }
+        for (int e = 0; e < 4; ++e)
+          if (pos0 + 8 * (e >> 1) + 2 * j + (e & 1) >= lim) {
+#pragma unroll
+            for (int b = 0; b < NB; ++b) pv[e][b] = 0.f;
+          }
       }
-      const float v_up = __uint_as_float((267u - v_exp) << 23);   // 2^(140 - field): the largest scale becomes 2^13 .. 2^14
+      // ---- values, two blocks at a time ----
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { s[e] = exp2f(s[e] - m); l += s[e]; s[e] *= v_up; }
-      // ---- values ----
+      for (int b2 = 0; b2 < NB; b2 += 2) {
+        // a power of two per (row, block): the largest product of the step, over the row's four threads, to 2^13 .. 2^14.
+        // dn: 2^(E - 140) of the two blocks as the upper halves of their f32s, E the largest's exponent field
+        float mb[2];
 #pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        uint32_t ph0, pl0, ph1, pl1;
-        split_h2(s[0] * vsc[0][b], s[1] * vsc[1][b], ph0, pl0);
-        split_h2(s[2] * vsc[2][b], s[3] * vsc[3][b], ph1, pl1);
-        uint32_t w[4];
+        for (int u = 0; u < 2; ++u) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint32_t pr = 16 * st + 8 * (e >> 1) + 2 * j + (e & 1);
-          w[e] = *reinterpret_cast<const uint32_t*>(vt + q8_v_off<HD>(pr, 2 * b + (r >> 2)) + (r & 3) * 4) ^ 0x80808080u;
+          for (int e = 0; e < 4; ++e) pv[e][b2 + u] *= s[e];
+          mb[u] = fmaxf(fmaxf(fabsf(pv[0][b2 + u]), fabsf(pv[1][b2 + u])), fmaxf(fabsf(pv[2][b2 + u]), fabsf(pv[3][b2 + u])));
         }
+        uint32_t dn = prmt(__float_as_uint(mb[0]), __float_as_uint(mb[1]), 0x7632u);
+        dn = __vmaxu2(dn, __shfl_xor_sync(0xffffffffu, dn, 1));
+        dn = __vmaxu2(dn, __shfl_xor_sync(0xffffffffu, dn, 2));
+        dn = (__vmaxu2(dn, 0x07000700u) & 0x7f807f80u) - 0x06800680u;           // E at least 14, so that both factors are normal
+        const uint32_t dn0 = __shfl_sync(0xffffffffu, dn, 8 * j), dn1 = __shfl_sync(0xffffffffu, dn, 8 * j + 4);   // rows 2 j, 2 j + 1
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const uint32_t ta = prmt(w[0], w[1], e ? 0x7362u : 0x5140u), tb = prmt(w[2], w[3], e ? 0x7362u : 0x5140u);
-          const uint32_t a0 = u8_h2(ta, 0x4140u), a1 = u8_h2(ta, 0x4342u), a2 = u8_h2(tb, 0x4140u), a3 = u8_h2(tb, 0x4342u);
-          // into a fresh accumulator, added in f32: the tensor cores' own accumulation rounds towards zero, and over the
-          // 250 steps of 4000 rows the result lost 4.4e-6 of itself (2.9e-7 so, as f32 loops do; a 777-token prompt takes 3 % longer)
-          float c[4] = {0.f, 0.f, 0.f, 0.f};
-          mma_16816(c, a0, a1, a2, a3, ph0, ph1);
-          mma_16816(c, a0, a1, a2, a3, pl0, pl1);
+        for (int b = b2; b < b2 + 2; ++b) {
+          auto factor = [&](uint32_t x) { return b & 1 ? x & 0xffff0000u : x << 16; };
+          const float up = __uint_as_float(0x7f000000u - factor(dn)), d0 = __uint_as_float(factor(dn0)), d1 = __uint_as_float(factor(dn1));
+          uint32_t ph0, pl0, ph1, pl1;
+          split_h2(pv[0][b] * up, pv[1][b] * up, ph0, pl0);
+          split_h2(pv[2][b] * up, pv[3][b] * up, ph1, pl1);
+          pl0 = h2_min8(pl0); pl1 = h2_min8(pl1);
+          uint32_t w[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) oacc[2 * b + e][k] += c[k];
+          for (int e = 0; e < 4; ++e) {
+            const uint32_t pr = 16 * st + 8 * (e >> 1) + 2 * j + (e & 1);
+            w[e] = *reinterpret_cast<const uint32_t*>(vt + q8_v_off<HD>(pr, 2 * b + (r >> 2)) + (r & 3) * 4) ^ 0x80808080u;
+          }
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const uint32_t ta = prmt(w[0], w[1], e ? 0x7362u : 0x5140u), tb = prmt(w[2], w[3], e ? 0x7362u : 0x5140u);
+            const uint32_t a0 = u8_h2(ta, 0x4140u), a1 = u8_h2(ta, 0x4342u), a2 = u8_h2(tb, 0x4140u), a3 = u8_h2(tb, 0x4342u);
+            // into a fresh accumulator, added in f32: the tensor cores' own accumulation rounds towards zero, and over the
+            // 250 steps of 4000 rows the result lost 4.4e-6 of itself (2.9e-7 so, as f32 loops do; a 777-token prompt takes 3 % longer)
+            float c[4] = {0.f, 0.f, 0.f, 0.f};
+            mma_16816(c, a0, a1, a2, a3, ph0, ph1);
+            mma_16816(c, a0, a1, a2, a3, pl0, pl1);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) oacc[2 * b + e][k] = __fmaf_rn(c[k], k & 1 ? d1 : d0, oacc[2 * b + e][k]);
+          }
         }
       }
     }
@@ -300,12 +331,11 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
   float* so = reinterpret_cast<float*>(smem) + warp * 8 * (HD + 2);   // [8][HD], then m[8], l[8]
-  const float v_down = __uint_as_float((v_exp - 13u) << 23);
 #pragma unroll
   for (int i = 0; i < 2 * NB; ++i) {
     const uint32_t d = 32 * (i >> 1) + 4 * r + 2 * (i & 1);
-    *reinterpret_cast<float2*>(so + (2 * j) * HD + d) = make_float2(oacc[i][0] * v_down, oacc[i][2] * v_down);
-    *reinterpret_cast<float2*>(so + (2 * j + 1) * HD + d) = make_float2(oacc[i][1] * v_down, oacc[i][3] * v_down);
+    *reinterpret_cast<float2*>(so + (2 * j) * HD + d) = make_float2(oacc[i][0], oacc[i][2]);
+    *reinterpret_cast<float2*>(so + (2 * j + 1) * HD + d) = make_float2(oacc[i][1], oacc[i][3]);
   }
   if (j == 0) { so[8 * HD + r] = m; so[8 * HD + 8 + r] = l; }
   __syncthreads();

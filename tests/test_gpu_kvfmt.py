@@ -120,6 +120,63 @@ def test_row_groups_splits_and_magnitudes(fmt, nH, nKV, hd):
         assert np.all(np.isfinite(out)) and util.errs(out, ref)[1] < util.REF_REL, f"{fmt} seq_len {seq_len} x {nc}: {util.errs(out, ref)}"
 
 
+@pytest.mark.parametrize("fmt,nH,nKV,hd", [("q8", 16, 2, 256), ("q8", 6, 2, 128), ("q8", 3, 1, 64), ("f32", 4, 2, 128), ("f32", 6, 1, 256)])
+@pytest.mark.parametrize("pos,n_cols", [(0, 70), (37, 21), (1000, 5), (59, 8)])
+@pytest.mark.parametrize("bad", [np.inf, np.nan, 1e30])
+def test_rows_a_column_does_not_see_leave_no_trace(fmt, nH, nKV, hd, pos, n_cols, bad):
+    # columns of one call, the last few of whose K or V rows hold an infinity, a NaN or values that dwarf all others: the bits
+    # of the columns before them are those of the same call over ordinary rows
+    import torch
+    eng = _engine(fmt, nH, nKV, hd, 1100, max_cols=1024)
+    T, cut = pos + n_cols, n_cols // 2
+    K, V = (torch.from_numpy(po.normal(40 + i, T * nKV * hd).astype(np.float32).reshape(T, -1)).cuda() for i in range(2))
+    q = util.torch_dev(po.normal(50, n_cols * nH * hd).astype(np.float32).reshape(n_cols, -1))
+    run = lambda: eng.decode(0, [(0, pos, n_cols)], q) if n_cols <= 8 else eng.prefill(0, 0, pos, q)
+    eng.kv_append(0, 0, 0, K, V)
+    clean = run()
+    Kb, Vb = K[pos + cut:].clone(), V[pos + cut:].clone()
+    Kb[1::2, 3::40] = bad
+    Vb[:, ::33] = bad
+    eng.kv_append(0, 0, pos + cut, Kb, Vb)
+    dirty = run()
+    eng.sync()
+    assert torch.isfinite(clean).all() and not torch.equal(clean[cut:], dirty[cut:])
+    assert torch.equal(clean[:cut].view(torch.int32), dirty[:cut].view(torch.int32))
+
+
+def _block_errs(got, ref, nH, hd):
+    """Largest error of each 32-dim block of each head, relative to the block's own largest output."""
+    d, r = (np.abs(x.astype(np.float64)).reshape(-1, nH, hd // 32, 32).max(axis=3) for x in (got - ref, ref))
+    return d / r
+
+
+@pytest.mark.parametrize("fmt", ["q8", "f32"])
+@pytest.mark.parametrize("nH,nKV,hd,rows,n_cols", [(16, 2, 256, 3000, 1), (16, 8, 128, 700, 5), (4, 2, 64, 2000, 33), (8, 2, 128, 64, 20)])
+@pytest.mark.parametrize("log2_v", [-30, -16, 24])
+def test_value_blocks_of_any_magnitude_keep_f32_precision(fmt, nH, nKV, hd, rows, n_cols, log2_v):
+    # the V of every other 32-dim block 2^-30 or 2^-16 of its neighbours', or one row's V 2^24 times all others where the row has next
+    # to no weight.  Judged per block of the output, relative to its own largest value: scores below 8 in 32 bits leave 8 * 2^-24
+    # in a weight, and the sums as much again (their terms add up without their signs to some 8 times the largest output): 1e-6,
+    # doubled for the largest of several thousand blocks
+    import torch
+    eng = _engine(fmt, nH, nKV, hd, rows, max_cols=rows)
+    g = np.random.default_rng(9)
+    K, V, q = (g.standard_normal(s).astype(np.float32) for s in ((rows, nKV * hd), (rows, nKV * hd), (n_cols, nH * hd)))
+    if log2_v < 0:
+        V.reshape(rows, -1, 2, 32)[:, :, 1] *= np.float32(2.0 ** log2_v)
+    else:
+        V[7] *= np.float32(2.0 ** log2_v)
+        K[7] = -np.abs(K[7]) * 4
+        q = np.abs(q)                                             # row 7 scores about -2.5 sqrt(hd)
+    eng.kv_append(0, 0, 0, util.torch_dev(K), util.torch_dev(V))
+    dq, pos = util.torch_dev(q), rows - n_cols
+    out = (eng.decode(0, [(0, pos, n_cols)], dq) if n_cols <= 8 else eng.prefill(0, 0, pos, dq)).cpu().numpy()
+    eng.sync()
+    Kh, Vh, _ = _held(eng, fmt, 0, rows)
+    e = _block_errs(out, po.attn_f64_kv32(q, Kh, Vh, nH, nKV, hd, pos, n_cols, None), nH, hd)
+    assert e.max() < 2e-6, f"{e.max(axis=(0, 1))}"
+
+
 @pytest.mark.parametrize("fmt,hd,n_rot,act,n_cols", [("q8", 256, 64, "f16", 1), ("q8", 128, 128, "f32", 3), ("q8", 128, 64, "f32", 70), ("f32", 64, 64, "f16", 2), ("f32", 256, 32, "f32", 5)])
 def test_front_of_a_layer_call_with_head_norm_keeps_the_bits(fmt, hd, n_rot, act, n_cols):
     # head-norm, rotation and the format's append (in one launch where n_rot is 64, or 128 of 128): cache bytes as the CPU twins give them
