@@ -6,13 +6,15 @@
 //            parts in rows 8-15, B the int8 rows: both halves of the product come from one instruction.
 //   values   O^T[dim, row] += v8^T[dim, pos] . (P * vs)^T[pos, row] : the weights take each block's scale before they are
 //            split into high and low f16 parts.
-// q is first scaled by a power of two per row so that its largest value lies in [2^12, 2^13), P * vs by one per row, 32-dim
-// block and step of 16 positions so that its largest lies in [2^13, 2^14) : high + low are then within 2^-23 of that value and
+// q is first scaled by a power of two per row and 32-dim block so that its largest value lies in [2^12, 2^13) (one for the
+// whole row left a block 2^-20 below the others, against keys as much larger, scores off by 5e-6), P * vs by one per row, block
+// and step of 16 positions so that its largest lies in [2^13, 2^14) : high + low are then within 2^-23 of that value and
 // within 2^-38 of it of every smaller one (an unscaled P * vs of 1e-4 would sit among f16's subnormals).  The power is a row's
 // and a block's own, and positions a row does not see are not in it: with one for all rows and dims of a warp, a large V scale
 // anywhere took bits from everything else (a block at 2^-20 of its neighbours was off by 9e-6 of itself, now 3e-7 as with f32
 // operands), and an infinite one of a later column made NaN of earlier ones.  It takes 4 shuffles and some 30
-// instructions per pair of blocks and step: 179 us where one power took 173 (the token below), 341 where 319 (the prompt).
+// instructions per pair of blocks and step, q's 32 multiplications: 179 us where one power each took 173 (the token below), 346
+// where 319 (the prompt).
 //
 // A warp owns eight query rows (heads of the GQA group, columns) and runs an online softmax over the positions it takes,
 // P in registers from one product to the next; no barrier but the ring's.  A CTA is four warps over a ring of 64-position
@@ -22,7 +24,7 @@
 // converts for its eight rows alone), about 700 instructions per 16 positions and eight rows against 64 MMAs; at long
 // contexts of a single token HBM (1.125 bytes a value).
 // Measured with its front (pa_front.cu) against plain f32 loops, a CTA per column: ten layers of a token over 12345 rows (16 q / 2 kv
-// heads x 256, head-norm) 918 -> 179 us, two layers of a 777-token prompt (24 / 4 x 256) 4231 -> 341 us; distance from float64
+// heads x 256, head-norm) 918 -> 179 us, two layers of a 777-token prompt (24 / 4 x 256) 4231 -> 346 us; distance from float64
 // no larger: 2.3e-7 against 2.9e-7 (that token), 1.7e-7 against 2.1e-7 (that prompt), relative.
 //
 // Stands in for attn_flash_q8 of pooled (engine/wgsl/qwen35.js:946-1010 and its column-wise use in prefill).
@@ -151,7 +153,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   const uint32_t my_row = row0 + 8 * rg + r;
   const bool live_row = my_row < rows;
   uint32_t qa[2 * NB][4];
-  float q_scale;      // scores come out in log2 units
+  float q_down[NB];   // back from the blocks' powers of two; scores come out in log2 units
   {
     float x[NB][8];
     const uint32_t qc = live_row ? my_row / G : 0, qh = live_row ? my_row % G : 0;
@@ -169,24 +171,23 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
         for (int e = 0; e < 8; ++e) x[b][e] = ld_act(p.q, off + 32 * b + e, p.q_f16);
       }
     }
-    float mx = 0.f;
 #pragma unroll
-    for (int b = 0; b < NB; ++b)
+    for (int b = 0; b < NB; ++b) {
+      float mx = 0.f;
 #pragma unroll
       for (int e = 0; e < 8; ++e) mx = fmaxf(mx, fabsf(x[b][e]));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    // times 2^(139 - e) with e the largest value's exponent field (at least 20, so that the factor is finite)
-    const uint32_t e = max(__float_as_uint(mx) >> 23, 20u);
-    const float up = __uint_as_float((266u - min(e, 254u)) << 23), down = __uint_as_float((min(e, 254u) - 12u) << 23);
-    q_scale = down * p.scale_log2;
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+      // times 2^(139 - e) with e the largest value's exponent field (at least 20, so that the factor is finite)
+      const uint32_t e = min(max(__float_as_uint(mx) >> 23, 20u), 254u);
+      const float up = __uint_as_float((266u - e) << 23);
+      q_down[b] = __uint_as_float((e - 12u) << 23) * p.scale_log2;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         split_h2(x[b][4 * h] * up, x[b][4 * h + 1] * up, qa[2 * b + h][0], qa[2 * b + h][1]);
         split_h2(x[b][4 * h + 2] * up, x[b][4 * h + 3] * up, qa[2 * b + h][2], qa[2 * b + h][3]);
       }
+    }
   }
   const uint32_t lim = live_row ? row_lim(my_row) : 0u;
   const uint32_t warp_lim = row_lim(row0 + 8 * rg + 7);       // no position at or past it concerns this warp
@@ -234,8 +235,8 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
           float c[4] = {0.f, 0.f, 0.f, 0.f};
           mma_16816(c, qa[2 * b][0], qa[2 * b][1], qa[2 * b][2], qa[2 * b][3], u8_h2(w.x, 0x4140u), u8_h2(w.x, 0x4342u));
           mma_16816(c, qa[2 * b + 1][0], qa[2 * b + 1][1], qa[2 * b + 1][2], qa[2 * b + 1][3], u8_h2(w.y, 0x4140u), u8_h2(w.y, 0x4342u));
-          s[2 * n] = __fmaf_rn(k0[b], c[0] + c[2], s[2 * n]);
-          s[2 * n + 1] = __fmaf_rn(k1[b], c[1] + c[3], s[2 * n + 1]);
+          s[2 * n] = __fmaf_rn(k0[b] * q_down[b], c[0] + c[2], s[2 * n]);
+          s[2 * n + 1] = __fmaf_rn(k1[b] * q_down[b], c[1] + c[3], s[2 * n + 1]);
         }
       }
       // ---- mask, running maximum, weights ----
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const uint32_t pos = pos0 + 8 * (e >> 1) + 2 * j + (e & 1);
-        s[e] = pos < lim ? s[e] * q_scale : -INFINITY;
+        s[e] = pos < lim ? s[e] : -INFINITY;
         mx = fmaxf(mx, s[e]);
       }
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));

@@ -177,6 +177,25 @@ def test_value_blocks_of_any_magnitude_keep_f32_precision(fmt, nH, nKV, hd, rows
     assert e.max() < 2e-6, f"{e.max(axis=(0, 1))}"
 
 
+@pytest.mark.parametrize("fmt", ["q8", "f32"])
+@pytest.mark.parametrize("nH,nKV,hd,rows,n_cols", [(16, 2, 256, 3000, 1), (16, 8, 128, 700, 5), (4, 2, 64, 2000, 33)])
+@pytest.mark.parametrize("log2_q", [-16, -30])
+def test_query_blocks_of_any_magnitude_keep_f32_precision(fmt, nH, nKV, hd, rows, n_cols, log2_q):
+    # q of every other 32-dim block small, K there as much larger, so that all blocks weigh alike in the scores (bound as above)
+    eng = _engine(fmt, nH, nKV, hd, rows, max_cols=rows)
+    g = np.random.default_rng(10)
+    K, V, q = (g.standard_normal(s).astype(np.float32) for s in ((rows, nKV * hd), (rows, nKV * hd), (n_cols, nH * hd)))
+    K.reshape(rows, -1, 2, 32)[:, :, 1] *= np.float32(2.0 ** -log2_q)
+    q.reshape(n_cols, -1, 2, 32)[:, :, 1] *= np.float32(2.0 ** log2_q)
+    eng.kv_append(0, 0, 0, util.torch_dev(K), util.torch_dev(V))
+    dq, pos = util.torch_dev(q), rows - n_cols
+    out = (eng.decode(0, [(0, pos, n_cols)], dq) if n_cols <= 8 else eng.prefill(0, 0, pos, dq)).cpu().numpy()
+    eng.sync()
+    Kh, Vh, _ = _held(eng, fmt, 0, rows)
+    e = _block_errs(out, po.attn_f64_kv32(q, Kh, Vh, nH, nKV, hd, pos, n_cols, None), nH, hd)
+    assert e.max() < 2e-6, f"{e.max(axis=(0, 1))}"
+
+
 @pytest.mark.parametrize("fmt,hd,n_rot,act,n_cols", [("q8", 256, 64, "f16", 1), ("q8", 128, 128, "f32", 3), ("q8", 128, 64, "f32", 70), ("f32", 64, 64, "f16", 2), ("f32", 256, 32, "f32", 5)])
 def test_front_of_a_layer_call_with_head_norm_keeps_the_bits(fmt, hd, n_rot, act, n_cols):
     # head-norm, rotation and the format's append (in one launch where n_rot is 64, or 128 of 128): cache bytes as the CPU twins give them
