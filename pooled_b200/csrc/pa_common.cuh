@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <atomic>
+#include <cfloat>
 #include <cstdlib>
 #include <stdint.h>
 
@@ -151,18 +152,19 @@ __device__ __forceinline__ float2 cluster_ld2(uint32_t addr) {
   asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
   return v;
 }
+template <int HD> __host__ __device__ constexpr float inv_sqrt_hd() { return HD == 64 ? 0.125f : HD == 256 ? 0.0625f : 0.08838834764831845f; }
 __device__ __forceinline__ float ld_act(const void* p, uint64_t i, int f16) {
   return f16 ? __half2float(reinterpret_cast<const __half*>(p)[i]) : reinterpret_cast<const float*>(p)[i];
 }
 
 // merge of one row's four dims over the CTAs of a cluster: o4 and ml are this CTA's shared addresses of its own unnormalised
-// o and of its (m in log2 units, l); every CTA keeps its rows at the same addresses.  Sums in CTA order.
-__device__ __forceinline__ float4 cluster_merge4(uint32_t o4, uint32_t ml, uint32_t n, float& L) {
+// o and of its (m in units of q . k, l; scale_log2: log2(e) / sqrt(head_dim)); every CTA keeps its rows at the same addresses.  Sums in CTA order.
+__device__ __forceinline__ float4 cluster_merge4(uint32_t o4, uint32_t ml, uint32_t n, float scale_log2, float& L) {
   float2 v[kMaxCluster];
   float4 x[kMaxCluster], o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (uint32_t s = 0; s < kMaxCluster; ++s) {
-    v[s] = make_float2(-3.0e38f, 0.f); x[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+    v[s] = make_float2(-FLT_MAX, 0.f); x[s] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (s < n) { v[s] = cluster_ld2(cluster_map(ml, s)); x[s] = cluster_ld4(cluster_map(o4, s)); }
   }
   float M = v[0].x;
@@ -171,7 +173,7 @@ __device__ __forceinline__ float4 cluster_merge4(uint32_t o4, uint32_t ml, uint3
   L = 0.f;
 #pragma unroll
   for (uint32_t s = 0; s < kMaxCluster; ++s) {
-    const float w = s < n ? exp2f(v[s].x - M) : 0.f;
+    const float w = s < n ? exp2f((v[s].x - M) * scale_log2) : 0.f;
     L = __fmaf_rn(v[s].y, w, L);
     o.x = __fmaf_rn(x[s].x, w, o.x); o.y = __fmaf_rn(x[s].y, w, o.y); o.z = __fmaf_rn(x[s].z, w, o.z); o.w = __fmaf_rn(x[s].w, w, o.w);
   }

@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
   float4 o[G][4];
 #pragma unroll
   for (int h = 0; h < G; ++h) {
-    m[h] = -1.0e30f; l[h] = 0.f;
+    m[h] = -FLT_MAX; l[h] = 0.f;      // m in units of q . k : no finite score lies below its start
 #pragma unroll
     for (int i = 0; i < 4; ++i) o[h][i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
@@ -264,18 +264,18 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
           a = __fmaf_rn(q[h][i].w, k[u][i].w, __fmaf_rn(q[h][i].z, k[u][i].z, __fmaf_rn(q[h][i].y, k[u][i].y, __fmaf_rn(q[h][i].x, k[u][i].x, a))));
 #pragma unroll
         for (int x = LPR / 2; x > 0; x >>= 1) a += __shfl_xor_sync(0xffffffffu, a, x);
-        s[u] = b0 + u * RPI + sub < r_hi ? a * p.scale_log2 : -INFINITY;
+        s[u] = b0 + u * RPI + sub < r_hi ? a : -INFINITY;
         mx = fmaxf(mx, s[u]);
       }
 #pragma unroll
       for (int x = LPR; x < 32; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
-      const float al = exp2f(m[h] - mx);
+      const float al = exp2f((m[h] - mx) * p.scale_log2);
       m[h] = mx; l[h] *= al;
 #pragma unroll
       for (int i = 0; i < 4; ++i) { o[h][i].x *= al; o[h][i].y *= al; o[h][i].z *= al; o[h][i].w *= al; }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const float w = exp2f(s[u] - mx);
+        const float w = exp2f((s[u] - mx) * p.scale_log2);
         l[h] += w;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
     for (int w = 1; w < 8; ++w) M = fmaxf(M, sml[w * G + h]);
 #pragma unroll
     for (int w = 0; w < 8; ++w) {
-      const float e = exp2f(sml[w * G + h] - M);
+      const float e = exp2f((sml[w * G + h] - M) * p.scale_log2);
       L = __fmaf_rn(sml[8 * G + w * G + h], e, L);
       a = __fmaf_rn(sm[w * G * HD + idx], e, a);
     }
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
     }
     const uint64_t slot = (col * p.n_heads + g * G + h) * p.n_splits + split;
     p.part_o[slot * HD + d] = a;
-    if (d == 0) { p.part_ml[slot * 2] = M * 0.6931471805599453f; p.part_ml[slot * 2 + 1] = L; }
+    if (d == 0) { p.part_ml[slot * 2] = M * inv_sqrt_hd<HD>(); p.part_ml[slot * 2 + 1] = L; }
   }
   if (!p.cluster) return;
   // at most eight splits: the CTAs of a (kv head, column) are a cluster and merge without another launch
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
   for (uint32_t idx = split * 256 + tid; idx < G * (HD / 4); idx += p.n_splits * 256) {
     const uint32_t h = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
     float L;
-    const float4 o4 = cluster_merge4(mine_s + (h * HD + d) * 4, mine_s + (G * HD + 2 * h) * 4, p.n_splits, L);
+    const float4 o4 = cluster_merge4(mine_s + (h * HD + d) * 4, mine_s + (G * HD + 2 * h) * 4, p.n_splits, p.scale_log2, L);
     gate_store4(o4, L, p.gate, col * p.gate_col_stride + (uint64_t)(g * G + h) * p.gate_head_stride + d, p.out,
                 col * p.out_col_stride + (uint64_t)(g * G + h) * HD + d, p.act_f16);
   }

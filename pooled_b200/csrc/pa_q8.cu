@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   const uint32_t my_row = row0 + 8 * rg + r;
   const bool live_row = my_row < rows;
   uint32_t qa[2 * NB][4];
-  float q_down[NB];   // back from the blocks' powers of two; scores come out in log2 units
+  float q_down[NB];   // back from the blocks' powers of two
   {
     float x[NB][8];
     const uint32_t qc = live_row ? my_row / G : 0, qh = live_row ? my_row % G : 0;
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
       // times 2^(139 - e) with e the largest value's exponent field (at least 20, so that the factor is finite)
       const uint32_t e = min(max(__float_as_uint(mx) >> 23, 20u), 254u);
       const float up = __uint_as_float((266u - e) << 23);
-      q_down[b] = __uint_as_float((e - 12u) << 23) * p.scale_log2;
+      q_down[b] = __uint_as_float((e - 12u) << 23);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         split_h2(x[b][4 * h] * up, x[b][4 * h + 1] * up, qa[2 * b + h][0], qa[2 * b + h][1]);
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   const uint32_t first_lim = row_lim(row0 + 8 * rg);          // every row of the warp sees the positions below it
   const bool warp_live = row0 + 8 * rg < rows;
 
-  float m = -1.0e30f, l = 0.f;
+  float m = -FLT_MAX, l = 0.f;                                // m in units of q . k : no finite score lies below its start
   float oacc[2 * NB][4];
 #pragma unroll
   for (int i = 0; i < 2 * NB; ++i) oacc[i][0] = oacc[i][1] = oacc[i][2] = oacc[i][3] = 0.f;
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
       if (__any_sync(0xffffffffu, mx > m)) {
-        const float al = exp2f(m - mx);
+        const float al = exp2f((m - mx) * p.scale_log2);
         l *= al;
         m = mx;
         const float a0 = __shfl_sync(0xffffffffu, al, 8 * j), a1 = __shfl_sync(0xffffffffu, al, 8 * j + 4);   // rows 2 j, 2 j + 1
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
         for (int i = 0; i < 2 * NB; ++i) { oacc[i][0] *= a0; oacc[i][1] *= a1; oacc[i][2] *= a0; oacc[i][3] *= a1; }
       }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { s[e] = exp2f(s[e] - m); l += s[e]; }
+      for (int e = 0; e < 4; ++e) { s[e] = exp2f((s[e] - m) * p.scale_log2); l += s[e]; }
       // ---- weights times the V scales of positions 2 j, 2 j + 1, 2 j + 8, 2 j + 9 ----
       float pv[4][NB];
 #pragma unroll
@@ -346,11 +346,11 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
     const uint32_t lr = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
     const float* wb = reinterpret_cast<const float*>(smem) + (lr >> 3) * 8 * (HD + 2);      // the row group's first warp
     const uint32_t step = p.rgw * 8 * (HD + 2), rr = lr & 7;
-    float M = -1.0e30f, Ls = 0.f;
+    float M = -FLT_MAX, Ls = 0.f;
     for (uint32_t k = 0; k < n_pw; ++k) M = fmaxf(M, wb[k * step + 8 * HD + rr]);
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
     for (uint32_t k = 0; k < n_pw; ++k) {
-      const float w = exp2f(wb[k * step + 8 * HD + rr] - M);
+      const float w = exp2f((wb[k * step + 8 * HD + rr] - M) * p.scale_log2);
       const float4 x = *reinterpret_cast<const float4*>(wb + k * step + rr * HD + d);
       Ls = __fmaf_rn(wb[k * step + 8 * HD + 8 + rr], w, Ls);
       o.x = __fmaf_rn(x.x, w, o.x); o.y = __fmaf_rn(x.y, w, o.y); o.z = __fmaf_rn(x.z, w, o.z); o.w = __fmaf_rn(x.w, w, o.w);
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
     if (ns_live > 1) {
       const uint64_t slot = ((uint64_t)c * p.n_heads + h) * p.n_splits + split;
       *reinterpret_cast<float4*>(p.part_o + slot * HD + d) = o;
-      if (d == 0) { p.part_ml[slot * 2] = M * 0.6931471805599453f; p.part_ml[slot * 2 + 1] = Ls; }
+      if (d == 0) { p.part_ml[slot * 2] = M * inv_sqrt_hd<HD>(); p.part_ml[slot * 2 + 1] = Ls; }
       continue;
     }
     // a call of one split needs no merge: gate and store here
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   for (uint32_t idx = split * kQ8Threads + tid; idx < n_rows_here * (HD / 4); idx += ns_live * kQ8Threads) {
     const uint32_t lr = idx / (HD / 4), d = (idx % (HD / 4)) * 4, row = row0 + lr, c = row / G, h = g * G + row % G;
     float Ls;
-    const float4 o = cluster_merge4(mine_s + (lr * HD + d) * 4, mine_s + (32 * HD + 2 * lr) * 4, ns_live, Ls);
+    const float4 o = cluster_merge4(mine_s + (lr * HD + d) * 4, mine_s + (32 * HD + 2 * lr) * 4, ns_live, p.scale_log2, Ls);
     gate_store4(o, Ls, p.gate, (uint64_t)c * p.gate_col_stride + (uint64_t)h * p.gate_head_stride + d, p.out, (uint64_t)c * p.out_col_stride + (uint64_t)h * HD + d,
                 p.act_f16);
   }

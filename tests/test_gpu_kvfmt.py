@@ -196,6 +196,25 @@ def test_query_blocks_of_any_magnitude_keep_f32_precision(fmt, nH, nKV, hd, rows
     assert e.max() < 2e-6, f"{e.max(axis=(0, 1))}"
 
 
+@pytest.mark.parametrize("fmt,nH,nKV,hd", [("q8", 16, 2, 256), ("q8", 6, 2, 128), ("q8", 3, 1, 64), ("f32", 4, 2, 256), ("f32", 4, 1, 128), ("f32", 2, 2, 64), ("f32", 6, 2, 128)])
+@pytest.mark.parametrize("rows,n_cols", [(1, 1), (70, 1), (70, 20), (2900, 1), (2900, 5)])
+@pytest.mark.parametrize("top", [1e31, 3.2e38])
+def test_scores_down_to_the_lowest_f32_still_weigh(fmt, nH, nKV, hd, rows, n_cols, top):
+    # q . k between -top / 2 and -top: every row's weight goes to its least negative score (what the V of that row holds comes out)
+    eng = _engine(fmt, nH, nKV, hd, rows, max_cols=rows)
+    g = np.random.default_rng(12)
+    b = np.float32(np.sqrt(top / hd))
+    K = np.repeat(-b * g.uniform(0.5, 1.0, (rows, 1)).astype(np.float32), nKV * hd, axis=1)
+    V, q = g.standard_normal((rows, nKV * hd)).astype(np.float32), np.full((n_cols, nH * hd), b, np.float32)
+    eng.kv_append(0, 0, 0, util.torch_dev(K), util.torch_dev(V))
+    dq, pos = util.torch_dev(q), rows - n_cols
+    out = (eng.decode(0, [(0, pos, n_cols)], dq) if n_cols <= 8 else eng.prefill(0, 0, pos, dq)).cpu().numpy()
+    eng.sync()
+    Kh, Vh, _ = _held(eng, fmt, 0, rows)
+    ref = po.attn_f64_kv32(q, Kh, Vh, nH, nKV, hd, pos, n_cols, None)
+    assert np.all(np.isfinite(out)) and util.errs(out, ref)[1] < util.REF_REL
+
+
 @pytest.mark.parametrize("fmt,hd,n_rot,act,n_cols", [("q8", 256, 64, "f16", 1), ("q8", 128, 128, "f32", 3), ("q8", 128, 64, "f32", 70), ("f32", 64, 64, "f16", 2), ("f32", 256, 32, "f32", 5)])
 def test_front_of_a_layer_call_with_head_norm_keeps_the_bits(fmt, hd, n_rot, act, n_cols):
     # head-norm, rotation and the format's append (in one launch where n_rot is 64, or 128 of 128): cache bytes as the CPU twins give them
