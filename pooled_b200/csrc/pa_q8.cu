@@ -194,10 +194,29 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   const uint32_t first_lim = row_lim(row0 + 8 * rg);          // every row of the warp sees the positions below it
   const bool warp_live = row0 + 8 * rg < rows;
 
-  float m = -FLT_MAX, l = 0.f;                                // m in units of q . k : no finite score lies below its start
-  float oacc[2 * NB][4];
+  // Sums in two levels, sixteen steps and the whole: one after the other the 1200 additions of a thread over 5000 rows left
+  // 4.3e-7 of the result, where f32 loops over shorter runs leave 3.2e-7 (so 2.9e-7).  At head_dim 256 l alone: there is no room
+  // for a second o, and l was the larger part (4.4e-7, f32 loops 3.9e-7, so 3.7e-7).  2 us of the prompt above.
+  constexpr bool O2 = HD <= 128;
+  float m = -FLT_MAX, l = 0.f, lt = 0.f;                      // m in units of q . k : no finite score lies below its start
+  float oacc[2 * NB][4], ot[O2 ? 2 * NB : 1][4];
+  auto zero = [](auto& o) {
 #pragma unroll
-  for (int i = 0; i < 2 * NB; ++i) oacc[i][0] = oacc[i][1] = oacc[i][2] = oacc[i][3] = 0.f;
+    for (auto& x : o) x[0] = x[1] = x[2] = x[3] = 0.f;
+  };
+  auto flush = [&]() {
+    l += lt;
+    lt = 0.f;
+    if constexpr (O2) {
+#pragma unroll
+      for (int i = 0; i < 2 * NB; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) oacc[i][k] += ot[i][k];
+      zero(ot);
+    }
+  };
+  zero(oacc); zero(ot);
+  uint32_t steps = 0;
 
   for (uint32_t t = 0; t < n_tiles; ++t) {
     asm volatile("cp.async.wait_group %0;" ::"n"(L::STAGES - 2) : "memory");
@@ -251,14 +270,18 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
       if (__any_sync(0xffffffffu, mx > m)) {
         const float al = exp2f((m - mx) * p.scale_log2);
-        l *= al;
+        l *= al; lt *= al;
         m = mx;
         const float a0 = __shfl_sync(0xffffffffu, al, 8 * j), a1 = __shfl_sync(0xffffffffu, al, 8 * j + 4);   // rows 2 j, 2 j + 1
 #pragma unroll
-        for (int i = 0; i < 2 * NB; ++i) { oacc[i][0] *= a0; oacc[i][1] *= a1; oacc[i][2] *= a0; oacc[i][3] *= a1; }
+        for (int i = 0; i < 2 * NB; ++i) {
+          oacc[i][0] *= a0; oacc[i][1] *= a1; oacc[i][2] *= a0; oacc[i][3] *= a1;
+          if constexpr (O2) { ot[i][0] *= a0; ot[i][1] *= a1; ot[i][2] *= a0; ot[i][3] *= a1; }
+        }
       }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { s[e] = exp2f((s[e] - m) * p.scale_log2); l += s[e]; }
+      for (int e = 0; e < 4; ++e) s[e] = exp2f((s[e] - m) * p.scale_log2);
+      lt += (s[0] + s[1]) + (s[2] + s[3]);
       // ---- weights times the V scales of positions 2 j, 2 j + 1, 2 j + 8, 2 j + 9 ----
       float pv[4][NB];
 #pragma unroll
@@ -319,12 +342,17 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
             mma_16816(c, a0, a1, a2, a3, ph0, ph1);
             mma_16816(c, a0, a1, a2, a3, pl0, pl1);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) oacc[2 * b + e][k] = __fmaf_rn(c[k], k & 1 ? d1 : d0, oacc[2 * b + e][k]);
+            for (int k = 0; k < 4; ++k) {
+              float& o = O2 ? ot[O2 ? 2 * b + e : 0][k] : oacc[2 * b + e][k];
+              o = __fmaf_rn(c[k], k & 1 ? d1 : d0, o);
+            }
           }
         }
       }
+      if ((++steps & 15u) == 0) flush();
     }
   }
+  flush();
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();                                            // the ring is idle
 

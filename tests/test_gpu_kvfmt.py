@@ -215,6 +215,33 @@ def test_scores_down_to_the_lowest_f32_still_weigh(fmt, nH, nKV, hd, rows, n_col
     assert np.all(np.isfinite(out)) and util.errs(out, ref)[1] < util.REF_REL
 
 
+@pytest.mark.parametrize("hd,bound", [(64, 2.6e-7), (128, 2.6e-7), (256, 3.9e-7)])
+def test_long_sums_over_int8_rows_stay_as_close_as_f32_loops(hd, bound):
+    # 40 columns x 2 heads over 5000 rows in one split: 312 steps of a warp, one after the other.  2-norm error against float64
+    # over the exact products value * scale.  An f32 addition is off by 0.72 * 2^-23 / sqrt(12) = 2.5e-8 of the sum at random, N
+    # of them on a sum that grows like a random walk by sqrt(N / 2) times that, on one that grows steadily (the weights')
+    # by sqrt(N / 3); scores and weights themselves leave 1.5e-7.  One output sum of 312 (head_dim 256): 3.5e-7; in two levels
+    # of 16 and 20: 1.9e-7; weights in one of 1248 per thread: another 2.5e-7, 4.3e-7 in all
+    import torch
+    from pooled_b200 import AttnConfig, AttnEngine
+    nH, nKV, rows, n_cols = 2, 1, 5000, 40
+    eng = AttnEngine(AttnConfig(n_heads=nH, n_kv_heads=nKV, head_dim=hd, n_rot=64, rope_theta=1e7, max_seq=rows, rope_mode="none", act_dtype=torch.float32, max_cols=rows, splits=1,
+                                kv_format="q8"))
+    g = np.random.default_rng(14)
+    K, V, q = (g.standard_normal(s).astype(np.float32) for s in ((rows, hd), (rows, hd), (n_cols, nH * hd)))
+    eng.kv_append(0, 0, 0, util.torch_dev(K), util.torch_dev(V))
+    out = eng.prefill(0, 0, rows - n_cols, util.torch_dev(q)).cpu().numpy().astype(np.float64).reshape(n_cols, nH, hd)
+    eng.sync()
+    k, ks, v, vs = _held(eng, "q8", 0, rows)[2]
+    K, V = ((x.reshape(rows, -1, 32) * sc.astype(np.float64)[..., None]).reshape(rows, hd) for x, sc in ((k, ks), (v, vs)))
+    s = np.einsum("chd,rd->chr", q.reshape(n_cols, nH, hd).astype(np.float64), K) / np.sqrt(hd)
+    s = np.where(np.arange(rows) <= (rows - n_cols + np.arange(n_cols))[:, None, None], s, -np.inf)
+    w = np.exp(s - s.max(axis=2, keepdims=True))
+    ref = np.einsum("chr,rd->chd", w / w.sum(axis=2, keepdims=True), V)
+    err = float(np.linalg.norm(out - ref) / np.linalg.norm(ref))
+    assert err < bound, f"{err:.3e}"
+
+
 @pytest.mark.parametrize("fmt,hd,n_rot,act,n_cols", [("q8", 256, 64, "f16", 1), ("q8", 128, 128, "f32", 3), ("q8", 128, 64, "f32", 70), ("f32", 64, 64, "f16", 2), ("f32", 256, 32, "f32", 5)])
 def test_front_of_a_layer_call_with_head_norm_keeps_the_bits(fmt, hd, n_rot, act, n_cols):
     # head-norm, rotation and the format's append (in one launch where n_rot is 64, or 128 of 128): cache bytes as the CPU twins give them
