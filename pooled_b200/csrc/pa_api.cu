@@ -90,6 +90,7 @@ static int make_cache_map(pa_ctx* ctx, CUtensorMap* tm, void* base, uint64_t row
 }
 
 static uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
+constexpr uint32_t kMaxGridYZ = 65535;   // blocks along a grid's y or z
 
 // ------------------------------------------------------------------------------ host mirrors --
 
@@ -701,6 +702,17 @@ struct GatherLists { const uint32_t* lists; uint32_t stride; };
 static int decode_q8_item(pa_layer* L, const pa_item& it, const void* q, int q_dtype, uint64_t qcs, uint64_t qhs, const void* gate, uint64_t gcs,
                           uint64_t ghs, void* out, uint64_t ocs, bool early, cudaStream_t st) {
   pa_ctx* ctx = L->ctx;
+  if (const uint32_t most = kMaxGridYZ * 32u / ctx->G; it.n_cols > most) {   // the row tiles (32 rows each here) are the grid's z
+    const size_t qes = q_dtype == PA_F16 ? 2 : 4, aes = ctx->cfg.act_dtype == PA_F16 ? 2 : 4;
+    for (uint32_t c0 = 0; c0 < it.n_cols; c0 += most) {
+      const pa_item piece{it.seq, it.pos + c0, std::min(most, it.n_cols - c0), 0};
+      if (int rc = decode_q8_item(L, piece, reinterpret_cast<const uint8_t*>(q) + c0 * qcs * qes, q_dtype, qcs, qhs,
+                                  gate ? reinterpret_cast<const uint8_t*>(gate) + c0 * gcs * aes : nullptr, gcs, ghs,
+                                  reinterpret_cast<uint8_t*>(out) + c0 * ocs * aes, ocs, early && c0 == 0, st))
+        return rc;
+    }
+    return PA_OK;
+  }
   const uint32_t hd = ctx->cfg.head_dim, nH = ctx->cfg.n_heads, rows = it.n_cols * ctx->G, n_rows = it.pos + it.n_cols - L->origin;
   Q8Params p{};
   p.q = q; p.q_f16 = q_dtype == PA_F16; p.q_col_stride = qcs; p.q_head_stride = qhs;

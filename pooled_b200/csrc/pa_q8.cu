@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   const bool warp_live = row0 + 8 * rg < rows;
 
   // Sums in two levels, sixteen steps and the whole: one after the other the 1200 additions of a thread over 5000 rows left
-  // 4.3e-7 of the result, where f32 loops over shorter runs leave 3.2e-7 (so 2.9e-7).  At head_dim 256 l alone: there is no room
+  // 4.3e-7 of the result, where f32 loops over shorter runs leave 3.2e-7 (so 2.1e-7).  At head_dim 256 l alone: there is no room
   // for a second o, and l was the larger part (4.4e-7, f32 loops 3.9e-7, so 3.7e-7).  2 us of the prompt above.
   constexpr bool O2 = HD <= 128;
   float m = -FLT_MAX, l = 0.f, lt = 0.f;                      // m in units of q . k : no finite score lies below its start

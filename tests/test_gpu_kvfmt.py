@@ -298,3 +298,24 @@ def test_q8_state_round_trip_and_refusals():
     with pytest.raises(PaError) as e:
         a.decode_partial(0, [(0, pos - 1, 1)], q)
     assert e.value.code == -2
+
+
+def test_an_int8_call_wider_than_the_grid():
+    # 16 heads per kv head: 131 070 columns fill the grid's 65 535 row tiles; 131 200 into an empty cache, a column of the first
+    # and the last rows and those around the seam against the oracle (one block of 64 columns of values, repeated)
+    import torch
+    nH, nKV, hd, T = 16, 1, 64, 131200
+    eng = _engine("q8", nH, nKV, hd, T, act="f16", max_cols=T)
+    K, V, q = (util.normal_f16(60 + i, (64, d)) for i, d in enumerate((hd, hd, nH * hd)))
+    wide = lambda a: util.torch_dev(a, torch.float16).repeat(T // 64, 1)
+    eng.kv_append(0, 0, 0, wide(K), wide(V))
+    out = eng.prefill(0, 0, 0, wide(q))
+    eng.sync()
+    Kh, Vh, _ = _held(eng, "q8", 0, 64)
+    for c in (0, 1, 63, 5000, 131069, 131070, 131071, T - 1):
+        reps = c // 64
+        # every whole block weighs as one: a column sees `reps` copies of the 64 rows and the first c % 64 + 1 of another
+        s = q[c % 64].reshape(nH, hd).astype(np.float64) @ Kh.T.astype(np.float64) / np.sqrt(hd)
+        w = np.exp(s - s.max(axis=1, keepdims=True)) * (reps + (np.arange(64) <= c % 64))
+        ref = (w / w.sum(axis=1, keepdims=True)) @ Vh.astype(np.float64)
+        util.assert_close(out[c].float().cpu().numpy(), ref.reshape(-1), f"column {c}")
