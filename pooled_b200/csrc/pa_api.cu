@@ -1093,6 +1093,18 @@ static int prefill_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols
   const uint64_t qm = q_dtype == PA_F16 ? 7 : 3, om = ctx->cfg.act_dtype == PA_F16 ? 7 : 3;   // 16-byte vector accesses
   if ((qcs & qm) || (qhs & qm) || ((uintptr_t)q & 15)) return fail(ctx, PA_EINVAL, "pa_prefill: q strides must be multiples of 16 bytes and q 16-byte aligned");
   if ((ocs & om) || ((uintptr_t)out & 15)) return fail(ctx, PA_EINVAL, "pa_prefill: the out column stride must be a multiple of 16 bytes and out 16-byte aligned");
+  if (const uint32_t most = kMaxGridYZ * 128u; n_cols > most) {   // the 128-column tiles are the grid's y
+    const size_t qes = q_dtype == PA_F16 ? 2 : 4, aes = ctx->cfg.act_dtype == PA_F16 ? 2 : 4;
+    for (uint32_t c0 = 0; c0 < n_cols; c0 += most) {
+      PlainQ rest{};
+      if (plain) rest = PlainQ{reinterpret_cast<const uint8_t*>(plain->q) + c0 * plain->cs * qes, plain->cs, plain->hs};
+      if (int rc = prefill_impl(L, seq, pos + c0, std::min(most, n_cols - c0), reinterpret_cast<const uint8_t*>(q) + c0 * qcs * qes, q_dtype, qcs, qhs,
+                                gate ? reinterpret_cast<const uint8_t*>(gate) + c0 * gcs * aes : nullptr, gcs, ghs,
+                                reinterpret_cast<uint8_t*>(out) + c0 * ocs * aes, ocs, st, plain ? &rest : nullptr))
+        return rc;
+    }
+    return PA_OK;
+  }
   cudaSetDevice(ctx->device);
   PrefillParams p{};
   p.q = q; p.q_f16 = q_dtype == PA_F16; p.q_col_stride = qcs; p.q_head_stride = qhs;
