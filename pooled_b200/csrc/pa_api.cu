@@ -750,6 +750,17 @@ static int decode_q8_item(pa_layer* L, const pa_item& it, const void* q, int q_d
   return PA_OK;
 }
 
+// Splits of a call of nc columns on the chunked f32 kernel: plan_cap(tiles), or tiles / 2 (an odd number of tiles then
+// makes three of them a split) where that fits one wave of two CTAs per SM and plan_cap takes a quarter more.  Two layers of
+// three columns over 9003 rows (16 / 2 heads x 256): 426 CTAs of two tiles 260 us, 282 of three 207; but one column 88 and
+// 122, eight columns over 308 rows 55 and 123, and for 308 CTAs against 220, or 616 against 440, two tiles are 5 % the better.
+static uint32_t any_splits(const pa_ctx* ctx, uint32_t rows, uint32_t nc) {
+  const uint32_t tiles = ceil_div(rows, 64), fine = plan_splits(ctx, rows, 1, nc, 1), coarse = std::min(fine, std::max(1u, tiles / 2));
+  auto ctas = [&](uint32_t ns) { return ceil_div(tiles, ceil_div(tiles, ns)) * ctx->cfg.n_kv_heads * nc; };
+  const uint32_t wave = 2u * (uint32_t)ctx->sm_count;
+  return !ctx->cfg.splits && 4 * ctas(fine) > 5 * wave && ctas(coarse) <= wave ? coarse : fine;
+}
+
 // Decode / verify / prefill over an int8 or f32 cache: per item, blocks of columns small enough for the record buffers;
 // each block is one launch of the plain split-K kernel (a CTA per (split, kv head, column)) and one combine.
 static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, const void* q, int q_dtype, uint64_t qcs, uint64_t qhs, const void* gate,
@@ -776,7 +787,8 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
       const uint32_t nc = std::min(block, items[i].n_cols - c0);
       const uint32_t pos0 = items[i].pos + c0;
       const uint32_t rows = pos0 + nc - L->origin;                 // rows the block's last column sees
-      uint32_t ns = plan_splits(ctx, rows, 1, nc, 1), live = 0;
+      const int32_t lim0 = (int32_t)(pos0 + 1 - L->origin);
+      uint32_t ns, live;
       bool merged = false;
       if (decode_f32_direct(ctx->G)) {
         // rows in whole 16s over one CTA per SM; a short context gives every warp of a CTA its 16 rows before it takes more CTAs
@@ -795,21 +807,23 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
         f.q_vec = q_dtype == PA_F32 && !(qcs & 3) && !(qhs & 3) && !((uintptr_t)f.q & 15);
         f.k = (const float*)L->k_alt; f.v = (const float*)L->v_alt;
         f.kv_dim = ctx->kv_dim; f.n_heads = nH; f.max_seq = L->max_seq; f.n_splits = ns;
-        f.seq = items[i].seq; f.lim0 = (int32_t)(pos0 + 1 - L->origin); f.n_rows = rows; f.n_cols = nc;
+        f.seq = items[i].seq; f.lim0 = lim0; f.n_rows = rows; f.n_cols = nc;
         f.early = after_front && c0 == 0 ? 1u : 0u;   // (a later block of a wide call follows a merge, not the front)
         f.scale_log2 = (float)(1.4426950408889634 / sqrt((double)hd));
         f.part_o = ctx->part_o; f.part_ml = ctx->part_ml;
         timing_mark(ctx, st, 0);
         CU_TRY(ctx, launch_decode_f32_direct(f, hd, ctx->G, ctx->cfg.n_kv_heads, st));
         timing_mark(ctx, st, 1);
-      }
-      AnyDecodeParams a{};
-      a.q = reinterpret_cast<const uint8_t*>(q) + (col + c0) * qcs * qes; a.q_f16 = q_dtype == PA_F16; a.q_col_stride = qcs; a.q_head_stride = qhs;
-      a.k = (const float*)L->k_alt; a.v = (const float*)L->v_alt;
-      a.kv_dim = ctx->kv_dim; a.hd = hd; a.G = ctx->G; a.n_heads = nH; a.max_seq = L->max_seq; a.n_splits = ns;
-      a.seq = items[i].seq; a.lim0 = (int32_t)(pos0 + 1 - L->origin); a.n_rows = rows; a.col0 = 0;
-      a.part_o = ctx->part_o; a.part_ml = ctx->part_ml;
-      if (!live) {
+      } else {
+        ns = any_splits(ctx, rows, nc);
+        AnyDecodeParams a{};
+        a.tps = ceil_div(ceil_div(rows, 64), ns);
+        live = ceil_div(ceil_div(rows, 64), a.tps);
+        a.q = reinterpret_cast<const uint8_t*>(q) + (col + c0) * qcs * qes; a.q_f16 = q_dtype == PA_F16; a.q_col_stride = qcs; a.q_head_stride = qhs;
+        a.k = (const float*)L->k_alt; a.v = (const float*)L->v_alt;
+        a.kv_dim = ctx->kv_dim; a.hd = hd; a.G = ctx->G; a.n_heads = nH; a.max_seq = L->max_seq; a.n_splits = ns;
+        a.seq = items[i].seq; a.lim0 = lim0; a.n_rows = rows; a.col0 = 0;
+        a.part_o = ctx->part_o; a.part_ml = ctx->part_ml;
         timing_mark(ctx, st, 0);
         CU_TRY(ctx, launch_decode_f32(a, dim3(ns, ctx->cfg.n_kv_heads, nc), ctx->device, st));
         timing_mark(ctx, st, 1);
@@ -820,7 +834,7 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
       c.n_heads = nH; c.fixed_parts = live; c.n_splits = ns; c.groups = 1;
       c.gate = gate ? reinterpret_cast<const uint8_t*>(gate) + (col + c0) * gcs * aes : nullptr; c.gate_col_stride = gcs; c.gate_head_stride = ghs;
       c.out = reinterpret_cast<uint8_t*>(out) + (col + c0) * ocs * aes; c.out_col_stride = ocs; c.act_f16 = ctx->cfg.act_dtype == PA_F16;
-      c.items.seq[0] = items[i].seq; c.items.lim0[0] = a.lim0; c.items.n_rows[0] = rows; c.items.n_cols[0] = nc; c.items.col0[0] = 0; c.n_items = 1;
+      c.items.seq[0] = items[i].seq; c.items.lim0[0] = lim0; c.items.n_rows[0] = rows; c.items.n_cols[0] = nc; c.items.col0[0] = 0; c.n_items = 1;
       c.err = ctx->dev_err;
       if (!ctx->core_only && !merged) CU_TRY(ctx, launch_combine((int)hd, c, nc * nH, st));
       ctx->stats.kernel_launches += ctx->core_only || merged ? 1 : 2;

@@ -85,9 +85,7 @@ __global__ void __launch_bounds__(kAnyThreads) pa_decode_f32_any_kernel(const An
   // rows this column sees, and this split's range of them (the plan is the item's: its last column's rows)
   const uint32_t lim = (uint32_t)min(max(p.lim0 + (int32_t)c, 0), (int32_t)p.n_rows);
   const uint32_t tiles = (p.n_rows + kAnyChunk - 1) / kAnyChunk;
-  const uint32_t ns_eff = min(p.n_splits, plan_cap(tiles));
-  const uint32_t tps = (tiles + ns_eff - 1) / max(ns_eff, 1u);
-  const uint32_t t0 = split * tps * kAnyChunk, t1 = min(min(tiles, (split + 1) * tps) * kAnyChunk, lim);
+  const uint32_t tps = p.tps, t0 = split * tps * kAnyChunk, t1 = min(min(tiles, (split + 1) * tps) * kAnyChunk, lim);
   if (split * tps >= tiles) return;              // no record expected from this split
   pdl_wait();
   pdl_trigger();

@@ -128,7 +128,7 @@ struct KvStoreParams {
 struct AnyDecodeParams {
   const void* q; int q_f16; uint64_t q_col_stride, q_head_stride;
   const float* k; const float* v;
-  uint32_t kv_dim, hd, G, n_heads, max_seq, n_splits;
+  uint32_t kv_dim, hd, G, n_heads, max_seq, n_splits, tps;   // tps: 64-row tiles per split
   uint32_t seq; int32_t lim0; uint32_t n_rows;   // rows column 0 sees (before clamping), rows the last column sees
   uint64_t col0;                                 // first column of the item in q and in the record buffers
   float* part_o; float* part_ml;

@@ -319,3 +319,17 @@ def test_an_int8_call_wider_than_the_grid():
         w = np.exp(s - s.max(axis=1, keepdims=True)) * (reps + (np.arange(64) <= c % 64))
         ref = (w / w.sum(axis=1, keepdims=True)) @ Vh.astype(np.float64)
         util.assert_close(out[c].float().cpu().numpy(), ref.reshape(-1), f"column {c}")
+
+
+@pytest.mark.parametrize("nH,nKV,hd", [(16, 2, 256), (6, 2, 128), (3, 1, 64)])
+@pytest.mark.parametrize("rows,n_cols", [(64, 1), (129, 2), (1100, 3), (2900, 40), (9003, 3), (8963, 8)])
+def test_f32_plans_of_many_waves(nH, nKV, hd, rows, n_cols):
+    # head counts of the chunked f32 kernel at odd numbers of 64-row tiles, few and many columns: both split plans
+    eng = _engine("f32", nH, nKV, hd, rows, max_cols=rows)
+    g = np.random.default_rng(16)
+    K, V, q = (g.standard_normal(s).astype(np.float32) for s in ((rows, nKV * hd), (rows, nKV * hd), (n_cols, nH * hd)))
+    eng.kv_append(0, 0, 0, util.torch_dev(K), util.torch_dev(V))
+    dq, pos = util.torch_dev(q), rows - n_cols
+    out = (eng.decode(0, [(0, pos, n_cols)], dq) if n_cols <= 8 else eng.prefill(0, 0, pos, dq)).cpu().numpy()
+    eng.sync()
+    assert util.errs(out, po.attn_f64_kv32(q, K, V, nH, nKV, hd, pos, n_cols, None))[1] < util.REF_REL
