@@ -24,6 +24,7 @@ cudaError_t launch_epoch_bump(unsigned int* ctr, cudaStream_t st);
 cudaError_t launch_head_norm(const HeadNormParams& p, cudaStream_t st);
 int prefill_supported(const pa_ctx* ctx);
 bool decode_f32_direct(uint32_t G);
+uint32_t decode_f32_batch(uint32_t hd, uint32_t G);
 cudaError_t launch_decode_f32_direct(const F32DecodeParams& p, uint32_t hd, uint32_t G, uint32_t n_kv, cudaStream_t st);
 cudaError_t launch_q8(const Q8Params& p, uint32_t hd, uint32_t n_kv, int dev, cudaStream_t st);
 bool front_supported(uint32_t hd, uint32_t n_rot, bool rotates);
@@ -761,6 +762,22 @@ static uint32_t any_splits(const pa_ctx* ctx, uint32_t rows, uint32_t nc) {
   return !ctx->cfg.splits && 4 * ctas(fine) > 5 * wave && ctas(coarse) <= wave ? coarse : fine;
 }
 
+// Whether eight splits, which a cluster merges, do instead of the `ns` of one CTA per SM and a merge kernel: where they add
+// no more than three quarters of a batch of rows to what a warp takes (a batch being the least), or a whole one with few kv
+// heads and short batches (1 or 2 heads of at least 128 dims).  On the device alone the line is at a third of a batch, but
+// a call that is not replayed from a graph pays for the third launch.  Eight layers of a token, eight splits / one CTA per SM, in a
+// graph and (called, hosts of 2.6 and 3.0 us a launch): 2 / 1 heads x 128 over 1024 rows (a batch) 41 / 45 (47 / 63, 71), 2048
+// 55 / 45 (58 / 62, 71); 8 / 2 x 128, 512 rows 49 / 51 (56 / 63, 71), 1024 62 / 51 (66 / 64, 72); 4 / 1 x 256, 256 rows 51 / 51
+// (57 / 62, 71), 512 62 / 51 (66 / 61, 72), 768 72 / 51 (75 / 62, 72); 16 / 8 x 128, 1024 rows 44 / 47 (50 / 63, 71), 2048 72 /
+// 68 (72 / 68, 72).  Not above twelve clusters: sixteen of eight CTAs, one per SM, are not all resident (16 kv heads x 128,
+// 2048 rows: 119 us, 92 with nine splits).
+static uint32_t f32_split_rows(uint32_t rows, uint32_t ns) { return ceil_div(ceil_div(rows, std::max(1u, ns)), 16) * 16; }
+static bool f32_eight_do(const pa_ctx* ctx, uint32_t rows, uint32_t nc, uint32_t ns) {
+  const uint32_t hd = ctx->cfg.head_dim, clusters = ctx->cfg.n_kv_heads * nc, batch = 8 * decode_f32_batch(hd, ctx->G);   // of the CTA's eight warps
+  const uint32_t more = ctx->G <= 2 && hd >= 128 && clusters <= 4 ? batch : 3 * batch / 4;
+  return ns > (uint32_t)kMaxCluster && clusters <= 12 && f32_split_rows(rows, kMaxCluster) <= std::max(f32_split_rows(rows, ns), batch) + more;
+}
+
 // Decode / verify / prefill over an int8 or f32 cache: per item, blocks of columns small enough for the record buffers;
 // each block is one launch of the plain split-K kernel (a CTA per (split, kv head, column)) and one combine.
 static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, const void* q, int q_dtype, uint64_t qcs, uint64_t qhs, const void* gate,
@@ -794,10 +811,9 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
         // rows in whole 16s over one CTA per SM; a short context gives every warp of a CTA its 16 rows before it takes more CTAs
         ns = ctx->cfg.splits ? ctx->cfg.splits : std::max(1u, (uint32_t)ctx->sm_count / (ctx->cfg.n_kv_heads * nc));
         ns = std::min(std::min(ns, ctx->max_splits), (uint32_t)(ctx->part_slots / ((size_t)nc * nH)));
-        // up to 2048 rows eight splits do (two batches a warp): a cluster merges them, which saves the merge kernel
         F32DecodeParams f{};
-        if (rows <= 2048 && !ctx->cfg.splits) ns = std::min(ns, (uint32_t)kMaxCluster);
-        f.rows_per_split = ceil_div(ceil_div(rows, std::max(1u, ns)), 16) * 16;
+        if (!ctx->cfg.splits && f32_eight_do(ctx, rows, nc, ns)) ns = kMaxCluster;
+        f.rows_per_split = f32_split_rows(rows, ns);
         ns = live = ceil_div(rows, f.rows_per_split);
         if (ns <= (uint32_t)kMaxCluster) for (f.cluster = ns; f.cluster & (f.cluster - 1); ++f.cluster) {}
         f.gate = gate ? reinterpret_cast<const uint8_t*>(gate) + (col + c0) * gcs * aes : nullptr; f.gate_col_stride = gcs; f.gate_head_stride = ghs;

@@ -202,9 +202,10 @@ size_t any_decode_smem(uint32_t G, uint32_t hd) {
 // in flight per SM, which is what HBM's latency takes at full rate.  No barrier and no shared memory until the warps' (o, m, l) are merged at the end.  A CTA's
 // rows are one or two such batches per warp at the contexts these caches serve.  28 layers of a token over 2000 rows (16 q / 8 kv
 // heads x 128), whole calls: 644 us with the chunked kernel above, 360 us with this one (floor 69: 459 MB).
+constexpr int f32_batch(int hd, int G) { return 512 / hd * (G == 4 ? 2 : 4); }
 template <int HD, int G>
 __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodeParams p) {
-  constexpr int LPR = HD / 16, RPI = 32 / LPR, U = G == 4 ? 2 : 4, BATCH = RPI * U;   // lanes per row, rows per instruction and per batch
+  constexpr int LPR = HD / 16, RPI = 32 / LPR, BATCH = f32_batch(HD, G), U = BATCH / RPI;   // lanes per row, rows per instruction and per batch
   extern __shared__ float sm[];                                             // [8 warps][G][HD], then m[8][G], l[8][G]
   const uint32_t split = blockIdx.x, g = blockIdx.y, c = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = lane / LPR, lr = lane % LPR;
@@ -348,6 +349,7 @@ static cudaError_t launch_f32_t(const F32DecodeParams& p, dim3 grid, cudaStream_
   return launch_pdl(pa_decode_f32_kernel<HD, G>, grid, dim3(256), smem, st, p);
 }
 bool decode_f32_direct(uint32_t G) { return G == 1 || G == 2 || G == 4; }
+uint32_t decode_f32_batch(uint32_t hd, uint32_t G) { return (uint32_t)f32_batch((int)hd, (int)G); }
 cudaError_t launch_decode_f32_direct(const F32DecodeParams& p, uint32_t hd, uint32_t G, uint32_t n_kv, cudaStream_t st) {
   const dim3 grid(p.cluster ? p.cluster : p.n_splits, n_kv, p.n_cols);
 #define PA_F32_CASE(H) case H: return G == 1 ? launch_f32_t<H, 1>(p, grid, st) : G == 2 ? launch_f32_t<H, 2>(p, grid, st) : launch_f32_t<H, 4>(p, grid, st);

@@ -333,3 +333,20 @@ def test_f32_plans_of_many_waves(nH, nKV, hd, rows, n_cols):
     out = (eng.decode(0, [(0, pos, n_cols)], dq) if n_cols <= 8 else eng.prefill(0, 0, pos, dq)).cpu().numpy()
     eng.sync()
     assert util.errs(out, po.attn_f64_kv32(q, K, V, nH, nKV, hd, pos, n_cols, None))[1] < util.REF_REL
+
+
+@pytest.mark.parametrize("nH,nKV,hd", [(4, 1, 256), (8, 4, 256), (8, 2, 128), (16, 8, 128), (16, 16, 128), (2, 1, 64), (8, 2, 64)])
+def test_f32_splits_around_the_end_of_eight(nH, nKV, hd):
+    # contexts below, at and past one, two and three batches of rows per warp of eight splits, one token and three
+    batch = 512 // hd * (2 if nH // nKV == 4 else 4) * 64
+    rows = 3 * batch + 65
+    eng = _engine("f32", nH, nKV, hd, rows, max_cols=rows)
+    g = np.random.default_rng(18)
+    K, V, q = (g.standard_normal(s).astype(np.float32) for s in ((rows, nKV * hd), (rows, nKV * hd), (3, nH * hd)))
+    eng.kv_append(0, 0, 0, util.torch_dev(K), util.torch_dev(V))
+    dq = util.torch_dev(q)
+    for n in sorted({3, *(f * batch // 4 + d for f in (4, 7, 8, 12) for d in (-1, 0, 1, 64))}):
+        for nc in (1, 3):
+            out = eng.decode(0, [(0, n - nc, nc)], dq[:nc]).cpu().numpy()
+            eng.sync()
+            assert util.errs(out, po.attn_f64_kv32(q[:nc], K, V, nH, nKV, hd, n - nc, nc, None))[1] < util.REF_REL, f"{n} rows x {nc}"
