@@ -212,7 +212,7 @@ static __device__ __noinline__ uint32_t rot_h_slow(uint32_t xw, uint32_t yw, int
 // walks the heads t / (half / 8), + 64 / (half / 8), ...: 16-byte loads and stores on both sides, the angles loaded once,
 // rot_h() for the arithmetic.  (Before: a CTA per column, two dims per thread, rot_exact().  Eight layers of 2999 columns of 16 + 8
 // heads x 128, whole calls, together with the order of the prefill kernel's CTAs: 834 us then, 677 now, 96 of the difference
-// in that kernel.)  n_rot / 16 is a power of two up to 16.
+// in that kernel.)  half / 8 need not divide 64: the threads past the last whole turn then only copy.
 __global__ void __launch_bounds__(256) pa_rope_append_vec_kernel(const RopeParams p, const uint32_t n_cols) {
   __shared__ float2 s_cs[4][128];
   const uint32_t cl = threadIdx.x >> 6, t = threadIdx.x & 63, col = blockIdx.x * 4 + cl, half = p.n_rot / 2, hd = p.hd;
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(256) pa_rope_append_vec_kernel(const RopeParam
 #pragma unroll
   for (int e = 0; e < 8; ++e) cs[e] = s_cs[cl][d + e];
   // ---- rotated dims: d .. d + 7 with their partners half further on, two heads in flight ----
-  for (uint32_t h0 = t / groups; h0 < nh; h0 += 2 * step) {
+  for (uint32_t h0 = t < groups * step ? t / groups : nh; h0 < nh; h0 += 2 * step) {
     uint4 A[2], B[2];
     __half* dst[2];
 #pragma unroll
@@ -392,8 +392,7 @@ __global__ void __launch_bounds__(256) pa_sigmoid_mul_kernel(const SigmoidParams
 // whether a call goes to the vectorised kernel (the only one that knows q_rot_only)
 bool rope_vec_applies(const RopeParams& p, uint32_t n_cols) {
   auto al16 = [](const void* x) { return ((uintptr_t)x & 15) == 0; };
-  return !p.n_items && n_cols >= 16 && p.mode == PA_ROPE_F64 && p.angles && p.in_f16 && p.n_rot % 16 == 0 && p.n_rot <= 256 && !((p.n_rot / 16) & (p.n_rot / 16 - 1)) &&
-         p.hd % 8 == 0 &&
+  return !p.n_items && n_cols >= 16 && p.mode == PA_ROPE_F64 && p.angles && p.in_f16 && p.n_rot % 16 == 0 && p.n_rot <= 256 && p.hd % 8 == 0 &&
          (!p.q || (p.q_out_f16 == 1 && al16(p.q) && al16(p.q_out) && p.q_col_stride % 8 == 0 && p.q_head_stride % 8 == 0 && p.q_out_col_stride % 8 == 0)) &&
          (!p.k || (p.v && al16(p.k) && al16(p.v) && p.kv_col_stride % 8 == 0 && p.v_col_stride % 8 == 0));
 }

@@ -254,10 +254,11 @@ def test_head_norm_keeps_the_bits_of_the_in_order_sum(hd, heads, n_cols, tie):
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
 
 
-@pytest.mark.parametrize("hd,n_rot,n_cols,heads", [(256, 64, 16, 2), (128, 128, 67, 8), (256, 256, 17, 1), (64, 32, 130, 3), (128, 16, 21, 2), (256, 96, 18, 2)])
+@pytest.mark.parametrize("hd,n_rot,n_cols,heads", [(256, 64, 16, 2), (128, 128, 67, 8), (256, 256, 17, 1), (64, 32, 130, 3), (128, 16, 21, 2), (256, 96, 18, 2),
+                                                   (64, 48, 33, 25), (128, 112, 19, 9), (256, 160, 16, 12), (256, 192, 35, 7), (256, 240, 17, 5)])
 def test_prompt_rotation_of_f16_rows_keeps_the_bits(hd, n_rot, n_cols, heads):
-    # chunks of f16 activations: the short f16 rotation with its exact path behind it (n_rot 96 takes the kernel of other
-    # widths), over ordinary values, zeros of both signs, subnormals, values whose rotation overflows f16, infinities and NaN.
+    # chunks of f16 activations: the short f16 rotation with its exact path behind it, also of widths whose groups of eight
+    # do not divide 64 threads, over ordinary values, zeros of both signs, subnormals, values whose rotation overflows f16, infinities and NaN.
     # The angles of wide calls come from the device's sincos, whose last place may differ from libm's: a few halves in
     # ten thousand of them by one, as an f32 result does then (probability about 1e-8 each; two are allowed)
     import torch

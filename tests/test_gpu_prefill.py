@@ -118,6 +118,22 @@ def test_config3_shape_reduced(n_cols, act, gate):
     print(f"prefill {n_cols} {act}: max-abs {ma:.2e} max-rel {mr:.2e}")
 
 
+@pytest.mark.parametrize("hd,n_rot,n_cols", [(256, 96, 150), (256, 128, 40), (256, 192, 203), (128, 48, 77), (64, 48, 19)])
+def test_prompts_of_other_rotary_widths(hd, n_rot, n_cols):
+    # widths whose groups of eight do not divide the rotation kernel's 64 threads, with (96) and without unrotated dims copied
+    import torch
+    nH, nKV = 6, 2
+    eng = _engine(nH, nKV, hd, n_cols + 8, act="f16", max_cols=n_cols, rope_mode="f64", n_rot=n_rot)
+    q, k, v, g = _inputs(31, nH, nKV, hd, n_cols)
+    d = lambda a: util.torch_dev(a, torch.float16)
+    out = eng.encode_layer(0, 0, d(q), d(k), d(v), d(g), mode="prefill").float().cpu().numpy()
+    eng.sync()
+    ref, Kf, Vf = _oracle_layer(q, k, v, g, nH, nKV, hd, n_rot, 1e7, 0)
+    gk, gv = util.read_cache(eng, 0, 0, 0, n_cols)
+    assert np.array_equal(gk, Kf) and np.array_equal(gv, Vf), "KV append is not bit-exact"
+    util.assert_close(out, ref, f"n_rot {n_rot}")
+
+
 @pytest.mark.parametrize("nH,nKV,hd", [(24, 4, 256), (16, 8, 128)])
 def test_prefill_gives_the_same_bits_twice(nH, nKV, hd):
     # two threads issue the score products of alternate tiles and two softmax groups take alternate tiles: the order of
