@@ -10,7 +10,7 @@ import sysconfig
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libpooled_attn.so")
-CALL_OUT = os.path.join(HERE, "_pa_call.so")      # CPython module: the per-layer calls without ctypes
+CALL_OUT = os.path.join(HERE, "_pa_call" + sysconfig.get_config_var("EXT_SUFFIX"))   # CPython module: the per-layer calls without ctypes
 SOURCES = ["pa_api.cu", "pa_rope_append.cu", "pa_decode.cu", "pa_prefill.cu", "pa_kvfmt.cu", "pa_q8.cu", "pa_front.cu", "pa_noalloc.cu"]
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo", "--use_fast_math=false",
          "-Xcompiler", "-fPIC,-fvisibility=hidden", "--expt-relaxed-constexpr"]
@@ -27,10 +27,19 @@ def _deps() -> list[str]:
     return [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(HERE, "..", "include", "pooled_attn.h")]
 
 
+def _call_cmd() -> list[str] | None:
+    """The command that builds the call module; None without a C compiler or this Python's headers (ctypes makes the calls then)."""
+    cc, inc = shutil.which("gcc") or shutil.which("cc"), sysconfig.get_paths()["include"]
+    if not cc or not os.path.exists(os.path.join(inc, "Python.h")):
+        return None
+    return [cc, "-O2", "-shared", "-fPIC", "-I" + inc, os.path.join(CSRC, "pa_call.c"), "-o", CALL_OUT]
+
+
 def needs_build() -> bool:
-    if not os.path.exists(OUT) or not os.path.exists(CALL_OUT):
+    outs = [OUT, CALL_OUT] if _call_cmd() else [OUT]
+    if not all(os.path.exists(o) for o in outs):
         return True
-    t = min(os.path.getmtime(OUT), os.path.getmtime(CALL_OUT))
+    t = min(os.path.getmtime(o) for o in outs)
     return any(os.path.getmtime(d) > t for d in _deps())
 
 
@@ -56,10 +65,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
         failed |= p.returncode != 0
     if failed:
         raise RuntimeError("nvcc failed")
-    cc = shutil.which("gcc") or shutil.which("cc")
-    if not cc:
-        raise RuntimeError("a C compiler is needed for the call module")
-    subprocess.check_call([cc, "-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], os.path.join(CSRC, "pa_call.c"), "-o", CALL_OUT])
+    cmd = _call_cmd()
+    if cmd:
+        subprocess.check_call(cmd)
+    else:
+        sys.stderr.write("no C compiler or no Python headers: the per-layer calls go through ctypes, some 5 us slower each\n")
+        if os.path.exists(CALL_OUT):
+            os.remove(CALL_OUT)       # of an older source
     subprocess.check_call([nvcc(), "-shared", "-o", OUT, *objs, "-lcudart_static", "-lpthread", "-ldl", "-lrt"])
     return OUT
 

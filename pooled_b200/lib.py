@@ -5,10 +5,11 @@ import ctypes as C
 import importlib.machinery
 import importlib.util
 import os
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SO_PATH = os.path.join(HERE, "libpooled_attn.so")
-CALL_PATH = os.path.join(HERE, "_pa_call.so")
+CALL_PATH = os.path.join(HERE, "_pa_call" + sysconfig.get_config_var("EXT_SUFFIX"))   # of this interpreter's ABI only
 
 PA_F32, PA_F16 = 0, 1
 PA_ROPE_NONE, PA_ROPE_F64, PA_ROPE_TABLE = 0, 1, 2
@@ -104,6 +105,38 @@ SYMBOLS = {
 }
 
 
+def _ptr(t):
+    return None if t is None else t.data_ptr()
+
+
+def _gate(t, head_stride):
+    return (None, 0, 0) if t is None else (t.data_ptr(), t.stride(0), head_stride)
+
+
+class CtypesCalls:
+    """What csrc/pa_call.c does, by ctypes (`entry` is not needed: the functions are the library's)."""
+
+    def __init__(self, lib):
+        self.lib = lib
+
+    def attn_layer(self, entry, layer, seq, pos, mode, q, q_head_stride, k, v, gate, gate_head_stride, cs_table, out, stream):
+        return self.lib.pa_attn_layer(layer, seq, pos, q.shape[0], mode, _ptr(q), q.stride(0), q_head_stride, _ptr(k), _ptr(v), k.stride(0),
+                                      *_gate(gate, gate_head_stride), _ptr(cs_table), _ptr(out), out.stride(0), stream)
+
+    def attn_items(self, entry, layer, seqs_pos, q, q_head_stride, k, v, gate, gate_head_stride, out, exchange, stream):
+        items = (PaItem * max(1, len(seqs_pos)))(*[PaItem(s, p, 1, 0) for s, p in seqs_pos])
+        return self.lib.pa_attn_items(layer, items, len(seqs_pos), _ptr(q), q.stride(0), q_head_stride, _ptr(k), _ptr(v), k.stride(0),
+                                      *_gate(gate, gate_head_stride), _ptr(out), out.stride(0), exchange, stream)
+
+    def rope_append(self, entry, layer, seq, pos, q, q_head_stride, k, v, cs_table, q_rot, stream):
+        return self.lib.pa_rope_append(layer, seq, pos, q.shape[0], _ptr(q), q.stride(0), q_head_stride, _ptr(k), _ptr(v), k.stride(0), _ptr(cs_table),
+                                       _ptr(q_rot), stream)
+
+    def decode_gather(self, entry, layer, seq, lists, list_stride, q, q_dtype, q_head_stride, gate, gate_head_stride, out, stream):
+        return self.lib.pa_decode_gather(layer, seq, q.shape[0], _ptr(lists), list_stride, _ptr(q), q_dtype, q.stride(0), q_head_stride,
+                                         *_gate(gate, gate_head_stride), _ptr(out), out.stride(0), stream)
+
+
 class Lib:
     """The loaded shared library with typed entry points."""
 
@@ -120,13 +153,14 @@ class Lib:
         self.call = self._load_call()
 
     def _load_call(self):
-        """The CPython module with the per-layer calls (csrc/pa_call.c); `entry` holds this library's addresses for them."""
+        """The CPython module with the per-layer calls (csrc/pa_call.c), which takes their addresses in this library from
+        `entry`; the same calls through ctypes where it was not built for this interpreter."""
+        self.entry = {n: C.cast(getattr(self.dll, n), C.c_void_p).value for n in ("pa_attn_layer", "pa_attn_items", "pa_rope_append", "pa_decode_gather")}
         if not os.path.exists(CALL_PATH):
-            raise PaError(-4, f"{CALL_PATH} is missing: build it with `python -m pooled_b200.build`")
+            return CtypesCalls(self)
         loader = importlib.machinery.ExtensionFileLoader("_pa_call", CALL_PATH)
         mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_pa_call", CALL_PATH, loader=loader))
         loader.exec_module(mod)
-        self.entry = {n: C.cast(getattr(self.dll, n), C.c_void_p).value for n in ("pa_attn_layer", "pa_attn_items", "pa_rope_append", "pa_decode_gather")}
         return mod
 
     def check(self, rc: int, ctx=None):

@@ -119,3 +119,43 @@ def test_product_package_does_not_import_the_oracle():
                 src = open(os.path.join(dirpath, f)).read()
                 assert "oracle" not in src.replace("pooled's CPU reference", ""), f"{f} mentions the oracle"
     assert pooled_b200.__doc__
+
+
+def test_call_module_is_of_this_interpreter_and_calls_as_ctypes_does(pa, monkeypatch):
+    # the module's file carries the interpreter's ABI tag; without one for this interpreter the library loads all the same and
+    # makes the same calls by ctypes
+    import sysconfig
+    import torch
+    assert os.path.basename(L.CALL_PATH) == "_pa_call" + sysconfig.get_config_var("EXT_SUFFIX") and os.path.exists(L.CALL_PATH)
+    monkeypatch.setattr(L, "CALL_PATH", L.CALL_PATH + ".absent")
+    plain = L.Lib()
+    assert isinstance(plain.call, L.CtypesCalls) and plain.entry.keys() == pa.entry.keys()
+    seen = []
+
+    def fake(name):
+        res, args = L.SYMBOLS[name]
+        def record(*a):
+            if name == "pa_attn_items":
+                it = C.cast(a[1], C.POINTER(L.PaItem))
+                a = (a[0], [(it[i].seq, it[i].pos, it[i].n_cols) for i in range(a[2])], *a[2:])
+            seen.append((name, *a))
+            return len(seen)
+        return C.CFUNCTYPE(res, *args)(record)
+
+    class FakeLib:
+        pass
+    lib = FakeLib()
+    for name in pa.entry:
+        setattr(lib, name, fake(name))
+    by_ctypes = L.CtypesCalls(lib)
+    entry = {name: C.cast(getattr(lib, name), C.c_void_p).value for name in pa.entry}
+    q, k, v, g, o = (torch.zeros((3, n + 2 * i))[:, :n] for i, n in enumerate((64, 16, 16, 64, 64)))
+    t, rows = torch.zeros((3, 8)), torch.zeros((3, 9), dtype=torch.int32)
+    calls = [("attn_layer", "pa_attn_layer", (4096, 1, 77, 2, q, 32, k, v, gate, 32, cs, o, 5)) for gate in (None, g) for cs in (None, t)]
+    calls += [("attn_items", "pa_attn_items", (4096, [(0, 5), (2, 2 ** 32 - 1), (1, 0)], q, 32, k, v, gate, 64, o, ex, 5)) for gate in (None, g) for ex in (0, 1)]
+    calls += [("rope_append", "pa_rope_append", (4096, 1, 77, q, 32, k, v, cs, o, 5)) for cs in (None, t)]
+    calls += [("decode_gather", "pa_decode_gather", (4096, 1, rows, 9, q, 1, 32, gate, 64, o, 5)) for gate in (None, g)]
+    for method, name, args in calls:
+        seen.clear()
+        assert getattr(pa.call, method)(entry[name], *args) == 1 and getattr(by_ctypes, method)(entry[name], *args) == 2
+        assert seen[0] == seen[1] and seen[0][0] == name, method
