@@ -156,6 +156,12 @@ template <int HD> __host__ __device__ constexpr float inv_sqrt_hd() { return HD 
 __device__ __forceinline__ float ld_act(const void* p, uint64_t i, int f16) {
   return f16 ? __half2float(reinterpret_cast<const __half*>(p)[i]) : reinterpret_cast<const float*>(p)[i];
 }
+// f32 -> f16 round to nearest even with subnormals and overflow to inf (cvt.rn.f16.f32); NaN becomes the quiet
+// pattern sign | 0x7e00 that pooled's f16_rne produces (engine/wgsl/f16.js:22), not the hardware's 0x7fff
+__device__ __forceinline__ __half f16_rne(float x) {
+  if (x != x) return __ushort_as_half((unsigned short)(((__float_as_uint(x) >> 16) & 0x8000u) | 0x7e00u));
+  return __float2half_rn(x);
+}
 
 // merge of one row's four dims over the CTAs of a cluster: o4 and ml are this CTA's shared addresses of its own unnormalised
 // o and of its (m in units of q . k, l; scale_log2: log2(e) / sqrt(head_dim)); every CTA keeps its rows at the same addresses.  Sums in CTA order.

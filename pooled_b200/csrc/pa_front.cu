@@ -11,12 +11,6 @@
 
 namespace pa {
 
-// f32 -> f16 as pooled's f16_rne: NaN becomes sign | 0x7e00
-__device__ __forceinline__ __half front_f16(float x) {
-  if (x != x) return __ushort_as_half((unsigned short)(((__float_as_uint(x) >> 16) & 0x8000u) | 0x7e00u));
-  return __float2half_rn(x);
-}
-
 // HB: 32-value groups of half the rotary width (n_rot = 64 HB); 0: nothing is rotated
 template <int HD, int HB>
 __global__ void __launch_bounds__(128) pa_front_kernel(const FrontParams p) {
@@ -92,7 +86,7 @@ __global__ void __launch_bounds__(128) pa_front_kernel(const FrontParams p) {
   void* cache = what == 1 ? p.k_cache : p.v_cache;
   if (p.format == PA_KV_F16) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i) reinterpret_cast<__half*>(cache)[eo + 32 * i] = front_f16(x[i]);
+    for (int i = 0; i < NV; ++i) reinterpret_cast<__half*>(cache)[eo + 32 * i] = f16_rne(x[i]);
   } else if (p.format == PA_KV_F32) {
 #pragma unroll
     for (int i = 0; i < NV; ++i) reinterpret_cast<float*>(cache)[eo + 32 * i] = x[i];

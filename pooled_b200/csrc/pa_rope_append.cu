@@ -16,13 +16,6 @@
 
 namespace pa {
 
-// f32 -> f16 round to nearest even with subnormals and overflow to inf (cvt.rn.f16.f32); NaN becomes the quiet
-// pattern sign | 0x7e00 that pooled's f16_rne produces (engine/wgsl/f16.js:22), not the hardware's 0x7fff
-__device__ __forceinline__ __half f16_rne(float x) {
-  if (x != x) return __ushort_as_half((unsigned short)(((__float_as_uint(x) >> 16) & 0x8000u) | 0x7e00u));
-  return __float2half_rn(x);
-}
-
 // grid (n_cols, q heads + k heads + v heads); one thread per pair of elements of the head.  Thread t < n_rot/2
 // evaluates its own cos / sin and rotates dims (t, t + n_rot/2); the other threads pass dims n_rot + 2(t - n_rot/2),
 // +1 through.  No shared memory and no barrier: every global load of the call is in flight at once, which is what

@@ -598,3 +598,34 @@ def test_cluster_merge_gives_the_combine_kernels_bits(nH, nKV, hd, act, monkeypa
             assert torch.equal(x.view(it), y.view(it)), f"{lens}"
         ref = np.concatenate([po.attn_f64(q[i:i + 1], K, V, nH, nKV, hd, m - 1, 1) for i, m in enumerate(lens)])
         util.assert_close(x.float().cpu().numpy(), ref, f"{lens}")
+
+
+@pytest.mark.parametrize("hd,n_rot", [(256, 64), (128, 128), (64, 64), (128, 64)])
+@pytest.mark.parametrize("act", ["f16", "f32"])
+@pytest.mark.parametrize("n_cols,mode", [(2, "decode"), (5, "decode"), (160, "prefill"), (17, "prefill")])
+def test_head_norm_of_blocks_and_chunks_keeps_the_bits_of_the_separate_kernel(hd, n_rot, act, n_cols, mode):
+    # an f16 cache: norm, rotation and append in the front kernel against pa_head_norm followed by the same call on a layer
+    # without a norm -- in f16 the normed values are rounded to f16 before the rotation, and q leaves as f16, as high and low
+    # planes (blocks from 128 dims on) or as f32
+    import torch
+    from pooled_b200 import AttnConfig, AttnEngine
+    nH, nKV, pos, eps = 8, 2, 133, 1e-6
+    td = torch.float16 if act == "f16" else torch.float32
+    engs = [AttnEngine(AttnConfig(n_heads=nH, n_kv_heads=nKV, head_dim=hd, n_rot=n_rot, rope_theta=1e6, max_seq=320, act_dtype=td, max_cols=160)) for _ in range(2)]
+    rng = np.random.default_rng(21)
+    dev = lambda *s: util.torch_dev((rng.standard_normal(s) * 2).astype(np.float32), td)
+    k0, v0 = dev(pos, nKV * hd), dev(pos, nKV * hd)
+    for e in engs:
+        e.kv_append(0, 0, 0, k0, v0)
+    q, k, v = dev(n_cols, 2 * nH * hd), dev(n_cols, nKV * hd), dev(n_cols, nKV * hd)       # q and gate interleaved
+    w = [util.torch_dev((1 + 0.1 * rng.standard_normal(hd)).astype(np.float32)) for _ in range(2)]
+    engs[0].set_head_norm(0, w[0], w[1], eps)
+    nq = engs[1].head_norm(q, nH, w[0], eps, head_stride=2 * hd, out=torch.zeros_like(q))
+    nk = engs[1].head_norm(k, nKV, w[1], eps, out=torch.empty_like(k))
+    outs = [e.encode_layer(0, pos, a, b, v, q[:, hd:], mode=mode, q_head_stride=2 * hd, gate_head_stride=2 * hd) for e, a, b in ((engs[0], q, k), (engs[1], nq, nk))]
+    for e in engs:
+        e.sync()
+    it = torch.int16 if act == "f16" else torch.int32
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[0].view(it), outs[1].view(it))
+    for which in "kv":
+        assert torch.equal(engs[0].cache(0, which)[0, :pos + n_cols], engs[1].cache(0, which)[0, :pos + n_cols])
