@@ -116,8 +116,8 @@ extern "C" uint32_t pa_tile_split_len(uint32_t seq_end, uint32_t fa_split, uint3
   return m < fa_split ? m : fa_split;
 }
 
-// Splits per (item, kv head): enough CTAs to give every SM one, never more than one wave, at least two
-// 64-row tiles each.  Depends on the call's longest column and item count only.
+// Splits per (item, kv head): enough CTAs to give every SM one, never more than one wave, at most plan_cap(tiles)
+// (a 64-row tile each up to eight, then two).  Depends on the call's longest column and item count only.
 static uint32_t plan_splits(const pa_ctx* ctx, uint32_t n_rows, uint32_t n_items, uint32_t total_cols = 0, uint32_t groups = 1) {
   const uint32_t tiles = ceil_div(n_rows, 64);
   if (!total_cols) total_cols = n_items;
@@ -778,8 +778,8 @@ static bool f32_eight_do(const pa_ctx* ctx, uint32_t rows, uint32_t nc, uint32_t
   return ns > (uint32_t)kMaxCluster && clusters <= 12 && f32_split_rows(rows, kMaxCluster) <= std::max(f32_split_rows(rows, ns), batch) + more;
 }
 
-// Decode / verify / prefill over an int8 or f32 cache: per item, blocks of columns small enough for the record buffers;
-// each block is one launch of the plain split-K kernel (a CTA per (split, kv head, column)) and one combine.
+// Decode / verify / prefill over an int8 or f32 cache.  Int8: decode_q8_item per item.  F32: per item, blocks of columns small
+// enough for the record buffers, each one launch (a CTA per (split, kv head, column)), and a combine unless a cluster merges.
 static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, const void* q, int q_dtype, uint64_t qcs, uint64_t qhs, const void* gate,
                            uint64_t gcs, uint64_t ghs, void* out, uint64_t ocs, cudaStream_t st, const char* who, bool after_front = false) {
   pa_ctx* ctx = L->ctx;

@@ -201,7 +201,7 @@ size_t any_decode_smem(uint32_t G, uint32_t hd) {
 // 64: 32, 256: 8; with four heads half of that) rows together, 128 registers a thread, before it uses the first: 128 KB
 // in flight per SM, which is what HBM's latency takes at full rate.  No barrier and no shared memory until the warps' (o, m, l) are merged at the end.  A CTA's
 // rows are one or two such batches per warp at the contexts these caches serve.  28 layers of a token over 2000 rows (16 q / 8 kv
-// heads x 128), whole calls: 644 us with the chunked kernel above, 360 us with this one (floor 69: 459 MB).
+// heads x 128), whole calls with the one-launch front: 644 us with the chunked kernel above, 257 us with this one (floor 70: 459 MB).
 constexpr int f32_batch(int hd, int G) { return 512 / hd * (G == 4 ? 2 : 4); }
 template <int HD, int G>
 __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodeParams p) {

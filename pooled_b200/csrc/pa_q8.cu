@@ -7,25 +7,26 @@
 //   values   O^T[dim, row] += v8^T[dim, pos] . (P * vs)^T[pos, row] : the weights take each block's scale before they are
 //            split into high and low f16 parts.
 // q is first scaled by a power of two per row and 32-dim block so that its largest value lies in [2^12, 2^13) (one for the
-// whole row left a block 2^-20 below the others, against keys as much larger, scores off by 5e-6), P * vs by one per row, block
+// whole row left outputs off by 3e-6 where a block lay 2^-20 below the others, against keys as much larger), P * vs by one per row, block
 // and step of 16 positions so that its largest lies in [2^13, 2^14) : high + low are then within 2^-23 of that value and
 // within 2^-38 of it of every smaller one (an unscaled P * vs of 1e-4 would sit among f16's subnormals).  The power is a row's
 // and a block's own, and positions a row does not see are not in it: with one for all rows and dims of a warp, a large V scale
 // anywhere took bits from everything else (a block at 2^-20 of its neighbours was off by 9e-6 of itself, now 3e-7 as with f32
 // operands), and an infinite one of a later column made NaN of earlier ones.  It takes 4 shuffles and some 30
-// instructions per pair of blocks and step, q's 32 multiplications: 179 us where one power each took 173 (the token below), 346
+// instructions per pair of blocks and step, q's 32 multiplications: 181 us where one power each took 174 (the token below), 348
 // where 319 (the prompt).
 //
 // A warp owns eight query rows (heads of the GQA group, columns) and runs an online softmax over the positions it takes,
 // P in registers from one product to the next; no barrier but the ring's.  A CTA is four warps over a ring of 64-position
 // tiles (cp.async, three or four tiles deep): with few query rows the warps share the positions of a tile and merge their (o, m, l)
 // at the end, with many each has rows of its own and all positions.  Two CTAs fit an SM.
-// What bounds it: conversions (int8 -> f16 costs a byte permute and an f16 subtraction per two values, and a warp
-// converts for its eight rows alone), about 700 instructions per 16 positions and eight rows against 64 MMAs; at long
-// contexts of a single token HBM (1.125 bytes a value).
+// What bounds it: the latency of two warps per scheduler.  A warp executes some 1400 instructions per 16 positions and eight rows
+// (loading its share of the tiles included) against 64 MMAs, most of them conversions, which it makes for its eight rows alone (int8 ->
+// f16 costs a byte permute and an f16 subtraction per two values): issue slots 49 %, ALU 38 %, tensor pipe 18 % of the active cycles of
+// the prompt below; of a single token's, 30, 25 and 7 %, HBM 11 %.
 // Measured with its front (pa_front.cu) against plain f32 loops, a CTA per column: ten layers of a token over 12345 rows (16 q / 2 kv
-// heads x 256, head-norm) 918 -> 179 us, two layers of a 777-token prompt (24 / 4 x 256) 4231 -> 346 us; distance from float64
-// no larger: 2.3e-7 against 2.9e-7 (that token), 1.7e-7 against 2.1e-7 (that prompt), relative.
+// heads x 256, head-norm) 918 -> 181 us, two layers of a 777-token prompt (24 / 4 x 256) 4231 -> 350 us; distance from float64
+// no larger: 2.2e-7 against 3.1e-7 (a token over 20000 rows), 1.6e-7 against 2.0e-7 (that prompt), relative.
 //
 // Stands in for attn_flash_q8 of pooled (engine/wgsl/qwen35.js:946-1010 and its column-wise use in prefill).
 #include "pa_params.cuh"
