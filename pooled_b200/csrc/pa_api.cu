@@ -754,12 +754,13 @@ static int decode_q8_item(pa_layer* L, const pa_item& it, const void* q, int q_d
 // Splits of a call of nc columns on the chunked f32 kernel: plan_cap(tiles), or tiles / 2 (an odd number of tiles then
 // makes three of them a split) where that fits one wave of two CTAs per SM and plan_cap takes a quarter more.  Two layers of
 // three columns over 9003 rows (16 / 2 heads x 256): 426 CTAs of two tiles 260 us, 282 of three 207; but one column 88 and
-// 122, eight columns over 308 rows 55 and 123, and for 308 CTAs against 220, or 616 against 440, two tiles are 5 % the better.
+// 122, eight columns over 308 rows 55 and 123, and for 308 CTAs against 220, or 616 against 440, two tiles are 5 % the better, as is
+// one tile each for 440 CTAs against 176 of three (up to eight tiles plan_cap gives one each).
 static uint32_t any_splits(const pa_ctx* ctx, uint32_t rows, uint32_t nc) {
   const uint32_t tiles = ceil_div(rows, 64), fine = plan_splits(ctx, rows, 1, nc, 1), coarse = std::min(fine, std::max(1u, tiles / 2));
   auto ctas = [&](uint32_t ns) { return ceil_div(tiles, ceil_div(tiles, ns)) * ctx->cfg.n_kv_heads * nc; };
   const uint32_t wave = 2u * (uint32_t)ctx->sm_count;
-  return !ctx->cfg.splits && 4 * ctas(fine) > 5 * wave && ctas(coarse) <= wave ? coarse : fine;
+  return !ctx->cfg.splits && tiles > 8 && 4 * ctas(fine) > 5 * wave && ctas(coarse) <= wave ? coarse : fine;
 }
 
 // Whether eight splits, which a cluster merges, do instead of the `ns` of one CTA per SM and a merge kernel: where they add
