@@ -720,14 +720,17 @@ static int decode_q8_item(pa_layer* L, const pa_item& it, const void* q, int q_d
   p.q_vec = q_dtype == PA_F32 && !(qcs & 3) && !(qhs & 3) && !((uintptr_t)q & 15);
   p.k = (const int8_t*)L->k_alt; p.v = (const int8_t*)L->v_alt; p.ks = L->k_scale; p.vs = L->v_scale;
   p.kv_dim = ctx->kv_dim; p.G = ctx->G; p.n_heads = nH; p.max_seq = L->max_seq;
-  p.rgw = rows <= 8 ? 1 : rows <= 16 ? 2 : 4;
+  // more than 16 query rows: eight warps that share one conversion of a tile; 64 rows a CTA where those fill the chip, else 32, with
+  // two warps on each eight rows
+  const bool cv = rows > 16;
+  p.rgw = rows <= 8 ? 1 : rows <= 16 ? 2 : ceil_div(rows, 64) * ctx->cfg.n_kv_heads >= (uint32_t)ctx->sm_count ? 8 : 4;
   p.seq = it.seq; p.lim0 = (int32_t)(it.pos + 1 - L->origin); p.n_rows = n_rows; p.n_cols = it.n_cols;
   p.early = early ? 1u : 0u;
   p.scale_log2 = (float)(1.4426950408889634 / sqrt((double)hd));
   p.part_o = ctx->part_o; p.part_ml = ctx->part_ml;
   p.gate = gate; p.gate_col_stride = gcs; p.gate_head_stride = ghs; p.out = out; p.out_col_stride = ocs; p.act_f16 = ctx->cfg.act_dtype == PA_F16;
   const uint32_t ctas = ceil_div(rows, 8 * p.rgw) * ctx->cfg.n_kv_heads, tiles = ceil_div(n_rows, 64);
-  uint32_t ns = ctx->cfg.splits ? ctx->cfg.splits : std::max(1u, 2u * (uint32_t)ctx->sm_count / ctas);
+  uint32_t ns = ctx->cfg.splits ? ctx->cfg.splits : std::max(1u, (cv && hd >= 128 ? 1u : 2u) * (uint32_t)ctx->sm_count / ctas);   // CTAs per SM
   ns = std::min(std::min(ns, plan_cap(tiles)), ctx->max_splits);
   ns = (uint32_t)std::max<size_t>(1, std::min<size_t>(ns, ctx->pf_slots / ((size_t)it.n_cols * nH)));
   p.n_splits = ns;

@@ -14,18 +14,18 @@
 // anywhere took bits from everything else (a block at 2^-20 of its neighbours was off by 9e-6 of itself, now 3e-7 as with f32
 // operands), and an infinite one of a later column made NaN of earlier ones.  It takes 4 shuffles and some 30
 // instructions per pair of blocks and step, q's 32 multiplications: 181 us where one power each took 174 (the token below), 348
-// where 319 (the prompt).
+// where 319 (the prompt, each warp then converting for itself).
 //
 // A warp owns eight query rows (heads of the GQA group, columns) and runs an online softmax over the positions it takes,
-// P in registers from one product to the next; no barrier but the ring's.  A CTA is four warps over a ring of 64-position
-// tiles (cp.async, three or four tiles deep): with few query rows the warps share the positions of a tile and merge their (o, m, l)
-// at the end, with many each has rows of its own and all positions.  Two CTAs fit an SM.
+// P in registers from one product to the next; no barrier but the ring's.  A CTA is four or eight warps over a ring of 64-position
+// tiles (cp.async): with few query rows the warps share the positions of a tile and merge their (o, m, l)
+// at the end, with many each has rows of its own and all positions.  Eight warps fit an SM.
 // What bounds it: the latency of two warps per scheduler.  A warp executes some 1400 instructions per 16 positions and eight rows
 // (loading its share of the tiles included) against 64 MMAs, most of them conversions, which it makes for its eight rows alone (int8 ->
 // f16 costs a byte permute and an f16 subtraction per two values): issue slots 49 %, ALU 38 %, tensor pipe 18 % of the active cycles of
 // the prompt below; of a single token's, 30, 25 and 7 %, HBM 11 %.
 // Measured with its front (pa_front.cu) against plain f32 loops, a CTA per column: ten layers of a token over 12345 rows (16 q / 2 kv
-// heads x 256, head-norm) 918 -> 181 us, two layers of a 777-token prompt (24 / 4 x 256) 4231 -> 350 us; distance from float64
+// heads x 256, head-norm) 918 -> 181 us, two layers of a 777-token prompt (24 / 4 x 256) 4231 -> 322 us; distance from float64
 // no larger: 2.2e-7 against 3.1e-7 (a token over 20000 rows), 1.6e-7 against 2.0e-7 (that prompt), relative.
 //
 // Stands in for attn_flash_q8 of pooled (engine/wgsl/qwen35.js:946-1010 and its column-wise use in prefill).
@@ -33,22 +33,34 @@
 
 namespace pa {
 
-constexpr int kQ8Tile = 64, kQ8Threads = 128;
+constexpr int kQ8Tile = 64;
 
-template <int HD>
+// CV: the CTA converts a tile once, to f16 in shared memory, for all of its warps (see the kernel)
+template <int HD, bool CV>
 struct Q8Smem {
+  static constexpr int NW = CV ? 8 : 4, THREADS = 32 * NW;
   static constexpr int NB = HD / 32;                       // scale blocks per row of a kv head
   static constexpr int KB = kQ8Tile * HD, SB = kQ8Tile * NB * 4;
-  static constexpr int STAGE = 2 * KB + 2 * SB;            // K values, V values, K scales, V scales
-  static constexpr int STAGES = HD == 256 ? 3 : 4;
-  static constexpr int RING = STAGE * STAGES;
-  static constexpr int MERGE = 4 * 8 * (HD + 2) * 4;       // the warps' (o, m, l), over the idle ring
-  static constexpr int MINE = 32 * (HD + 2) * 4;           // the CTA's merged rows behind them, for the cluster's merge
+  // values: K, V (int8); scales: K, V.  CV: two stages of values (a tile is converted while the one before it is used), and
+  // four of scales, which are read until the tile's end
+  static constexpr int STAGES = CV ? 2 : HD == 256 ? 3 : 4, SC_STAGES = CV ? 4 : STAGES;
+  static constexpr int F16 = CV ? 2 * 2 * KB * 2 : 0;      // two tiles of K and V as f16, ahead of the rings
+  static constexpr int OFF_RAW = F16, OFF_SC = OFF_RAW + STAGES * 2 * KB;
+  static constexpr int RING = OFF_SC + SC_STAGES * 2 * SB;
+  static constexpr int MROWS = 8 * NW;                     // most query rows of a CTA
+  static constexpr int MERGE = MROWS * (HD + 2) * 4;       // the warps' (o, m, l), over the idle ring
+  static constexpr int MINE = MROWS * (HD + 2) * 4;        // the CTA's merged rows behind them, for the cluster's merge
   static constexpr int TOTAL = RING > MERGE + MINE ? RING : MERGE + MINE;
 };
 
 // 16-byte chunk c of row r, permuted so that the reads below hit 32 different banks: the score reads take four rows r ..
 // r + 3 at a time (8 bytes per lane), the value reads rows r, r + 2, r + 4, r + 6 (4 bytes per lane)
+// (CV: the conversion reads one chunk of eight neighbouring rows at a time)
+template <int HD> __device__ __forceinline__ uint32_t q8_cv_off(uint32_t r, uint32_t c) {
+  return HD == 64 ? r * HD + ((c ^ ((r >> 1) & 3u)) << 4) : r * HD + ((c ^ (r & 7u)) << 4);
+}
+// 16-byte chunk c (eight values) of row r of an f16 tile: eight neighbouring rows of a chunk hit different banks
+template <int HD> __device__ __forceinline__ uint32_t q8_h_off(uint32_t r, uint32_t c) { return r * (HD * 2) + ((c ^ (r & 7u)) << 4); }
 template <int HD> __device__ __forceinline__ uint32_t q8_k_off(uint32_t r, uint32_t c) {
   if (HD == 64) return r * HD + ((c ^ ((r >> 1) & 3u)) << 4);
   return r * HD + ((c ^ (((r & 3u) << 1) | ((r >> 2) & 1u))) << 4);
@@ -86,18 +98,23 @@ __device__ __forceinline__ void cp8(uint32_t dst, const void* src, bool live) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(live ? 8 : 0) : "memory");
 }
 
-// grid (splits, kv heads, row tiles).  rgw row groups per CTA (1, 2 or 4): warp w has row group w % rgw and takes the
-// 16-position steps w / rgw, w / rgw + 4 / rgw, ... of a tile.
-template <int HD>
-__global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) {
-  using L = Q8Smem<HD>;
-  constexpr int NB = L::NB;
+// grid (splits, kv heads, row tiles).  rgw row groups per CTA (of NW warps): warp w has row group w % rgw and takes the
+// 16-position steps w / rgw, w / rgw + NW / rgw, ... of a tile.
+//
+// CV, for more than 16 query rows: eight warps, and each tile is converted to f16 once for all of them instead of by every
+// warp for its own eight rows, then read with ldmatrix: two layers of the 777-token prompt below 350 -> 322 us.
+// K's values go to the places the other form's lanes take them from (a score's products meet in the same order) and V's
+// stay in theirs, so both forms give the same bits for the same split plan.
+template <int HD, bool CV>
+__global__ void __launch_bounds__((Q8Smem<HD, CV>::THREADS), CV && HD >= 128 ? 1 : 2) pa_q8_kernel(const Q8Params p) {
+  using L = Q8Smem<HD, CV>;
+  constexpr int NB = L::NB, NW = L::NW, kQ8Threads = L::THREADS;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sm0 = smem_u32(smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, j = lane & 3;
   const uint32_t split = blockIdx.x, g = blockIdx.y, G = p.G, RT = 8 * p.rgw;
   const uint32_t row0 = (gridDim.z - 1 - blockIdx.z) * RT, rows = p.n_cols * G;    // the longest rows first
-  const uint32_t rg = warp % p.rgw, pw = warp / p.rgw, n_pw = 4 / p.rgw;
+  const uint32_t rg = warp % p.rgw, pw = warp / p.rgw, n_pw = NW / p.rgw;
   // the plan is the call's (its last column's rows); a row tile stops at what its own last row sees
   const uint32_t tiles = (p.n_rows + kQ8Tile - 1) / kQ8Tile;
   const uint32_t ns_eff = min(p.n_splits, plan_cap(tiles)), tps = (tiles + ns_eff - 1) / max(ns_eff, 1u);
@@ -111,15 +128,15 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
 
   auto load_tile = [&](uint32_t t) {      // one commit group per call, empty past the range
     if (t < n_tiles) {
-      const uint32_t s = t % L::STAGES, pos0 = (t_lo + t) * kQ8Tile, base = sm0 + s * L::STAGE;
+      const uint32_t pos0 = (t_lo + t) * kQ8Tile, base = sm0 + L::OFF_RAW + (t % L::STAGES) * 2 * L::KB, sbase = sm0 + L::OFF_SC + (t % L::SC_STAGES) * 2 * L::SB;
       constexpr int CPR = HD / 16;
 #pragma unroll
       for (int it = 0; it < kQ8Tile * CPR / kQ8Threads; ++it) {
         const uint32_t idx = tid + it * kQ8Threads, rr = idx / CPR, c = idx % CPR;
         const bool live = pos0 + rr < p.n_rows;
         const uint64_t off = (seq_row0 + (live ? pos0 + rr : 0)) * kv_dim + (uint64_t)g * HD + c * 16;
-        cp16(base + q8_k_off<HD>(rr, c), p.k + off, live);
-        cp16(base + L::KB + q8_v_off<HD>(rr, c), p.v + off, live);
+        cp16(base + (CV ? q8_cv_off<HD>(rr, c) : q8_k_off<HD>(rr, c)), p.k + off, live);
+        cp16(base + L::KB + (CV ? q8_cv_off<HD>(rr, c) : q8_v_off<HD>(rr, c)), p.v + off, live);
       }
       if (HD >= 128) {
         constexpr int SC = NB >= 4 ? NB / 4 : 1;
@@ -127,14 +144,14 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
           const uint32_t rr = idx / SC, c = idx % SC;
           const bool live = pos0 + rr < p.n_rows;
           const uint64_t off = (seq_row0 + (live ? pos0 + rr : 0)) * nbk + g * NB + c * 4;
-          cp16(base + 2 * L::KB + rr * (NB * 4) + c * 16, p.ks + off, live);
-          cp16(base + 2 * L::KB + L::SB + rr * (NB * 4) + c * 16, p.vs + off, live);
+          cp16(sbase + rr * (NB * 4) + c * 16, p.ks + off, live);
+          cp16(sbase + L::SB + rr * (NB * 4) + c * 16, p.vs + off, live);
         }
       } else if (tid < kQ8Tile) {
         const bool live = pos0 + tid < p.n_rows;
         const uint64_t off = (seq_row0 + (live ? pos0 + tid : 0)) * nbk + g * NB;
-        cp8(base + 2 * L::KB + tid * 8, p.ks + off, live);
-        cp8(base + 2 * L::KB + L::SB + tid * 8, p.vs + off, live);
+        cp8(sbase + tid * 8, p.ks + off, live);
+        cp8(sbase + L::SB + tid * 8, p.vs + off, live);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -143,7 +160,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   const uint32_t old_rows = p.early ? p.n_rows - min(p.n_rows, p.n_cols) : 0u;
   bool waited = false;
 #pragma unroll
-  for (int t = 0; t < L::STAGES - 1; ++t) {
+  for (int t = 0; t < (CV ? 2 : L::STAGES - 1); ++t) {
     if (!waited && (t_lo + t + 1) * kQ8Tile > old_rows) { pdl_wait(); waited = true; }
     load_tile(t);
   }
@@ -218,16 +235,54 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   };
   zero(oacc); zero(ot);
   uint32_t steps = 0;
+  // CV: tile t to f16, a (row, block of 32) of K or V per thread and turn
+  auto convert = [&](uint32_t t) {
+    const uint8_t* raw = smem + L::OFF_RAW + (t & 1) * 2 * L::KB;
+    uint8_t* dst = smem + (t & 1) * 4 * L::KB;
+#pragma unroll
+    for (int it = 0; it < 2 * kQ8Tile * NB / kQ8Threads; ++it) {
+      const uint32_t idx = tid + it * kQ8Threads, rr = idx % kQ8Tile, b = (idx / kQ8Tile) % NB, which = idx / (kQ8Tile * NB);
+      const uint8_t* src = raw + which * L::KB;
+      const uint4 x = *reinterpret_cast<const uint4*>(src + q8_cv_off<HD>(rr, 2 * b)), y = *reinterpret_cast<const uint4*>(src + q8_cv_off<HD>(rr, 2 * b + 1));
+      const uint32_t w[8] = {x.x ^ 0x80808080u, x.y ^ 0x80808080u, x.z ^ 0x80808080u, x.w ^ 0x80808080u,
+                             y.x ^ 0x80808080u, y.y ^ 0x80808080u, y.z ^ 0x80808080u, y.w ^ 0x80808080u};
+      uint8_t* d = dst + which * 2 * L::KB;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        // K: chunk (h, half) of a block holds dims 8 j + 4 h + 2 half, + 1 of j = 0 .. 3, the pairs lane j multiplies
+        const uint32_t sel = c & 1 ? 0x4342u : 0x4140u;
+        const uint4 v = which ? make_uint4(u8_h2(w[2 * c], 0x4140u), u8_h2(w[2 * c], 0x4342u), u8_h2(w[2 * c + 1], 0x4140u), u8_h2(w[2 * c + 1], 0x4342u))
+                              : make_uint4(u8_h2(w[c >> 1], sel), u8_h2(w[2 + (c >> 1)], sel), u8_h2(w[4 + (c >> 1)], sel), u8_h2(w[6 + (c >> 1)], sel));
+        *reinterpret_cast<uint4*>(d + q8_h_off<HD>(rr, 4 * b + c)) = v;
+      }
+    }
+  };
+  if constexpr (CV) {
+    if (n_tiles) {
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncthreads();
+      convert(0);
+    }
+  }
 
   for (uint32_t t = 0; t < n_tiles; ++t) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(L::STAGES - 2) : "memory");
-    __syncthreads();                                          // tile t has landed for every thread, tile t - 1 is consumed
-    load_tile(t + L::STAGES - 1);
+    if constexpr (CV) {
+      // tile t + 1 has landed and tile t is converted for every thread; tile t - 1, whose f16 place the next one takes, is consumed
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      load_tile(t + 2);
+      if (t + 1 < n_tiles) convert(t + 1);
+    } else {
+      asm volatile("cp.async.wait_group %0;" ::"n"(L::STAGES - 2) : "memory");
+      __syncthreads();                                        // tile t has landed for every thread, tile t - 1 is consumed
+      load_tile(t + L::STAGES - 1);
+    }
     if (!warp_live) continue;
-    const uint8_t* kt = smem + (t % L::STAGES) * L::STAGE;
-    const uint8_t* vt = kt + L::KB;
-    const float* kst = reinterpret_cast<const float*>(kt + 2 * L::KB);
-    const float* vst = reinterpret_cast<const float*>(kt + 2 * L::KB + L::SB);
+    const uint8_t* kt = smem + (CV ? (t & 1) * 4 * L::KB : L::OFF_RAW + (t % L::STAGES) * 2 * L::KB);
+    const uint8_t* vt = kt + (CV ? 2 : 1) * L::KB;
+    const float* kst = reinterpret_cast<const float*>(smem + L::OFF_SC + (t % L::SC_STAGES) * 2 * L::SB);
+    const float* vst = kst + kQ8Tile * NB;
+    const uint32_t kt_s = smem_u32(kt), vt_s = smem_u32(vt);
 #pragma unroll 1
     for (uint32_t st = pw; st < kQ8Tile / 16; st += n_pw) {
       const uint32_t pos0 = (t_lo + t) * kQ8Tile + 16 * st;
@@ -250,11 +305,17 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
         }
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
-          uint2 w = *reinterpret_cast<const uint2*>(kt + q8_k_off<HD>(pr + r, 2 * b + (j >> 1)) + (j & 1) * 8);
-          w.x ^= 0x80808080u; w.y ^= 0x80808080u;
+          uint32_t k8[4];
+          if constexpr (CV) {
+            ldsm_x4(kt_s + q8_h_off<HD>(pr + (lane & 7), 4 * b + (lane >> 3)), k8[0], k8[1], k8[2], k8[3]);
+          } else {
+            uint2 w = *reinterpret_cast<const uint2*>(kt + q8_k_off<HD>(pr + r, 2 * b + (j >> 1)) + (j & 1) * 8);
+            w.x ^= 0x80808080u; w.y ^= 0x80808080u;
+            k8[0] = u8_h2(w.x, 0x4140u); k8[1] = u8_h2(w.x, 0x4342u); k8[2] = u8_h2(w.y, 0x4140u); k8[3] = u8_h2(w.y, 0x4342u);
+          }
           float c[4] = {0.f, 0.f, 0.f, 0.f};
-          mma_16816(c, qa[2 * b][0], qa[2 * b][1], qa[2 * b][2], qa[2 * b][3], u8_h2(w.x, 0x4140u), u8_h2(w.x, 0x4342u));
-          mma_16816(c, qa[2 * b + 1][0], qa[2 * b + 1][1], qa[2 * b + 1][2], qa[2 * b + 1][3], u8_h2(w.y, 0x4140u), u8_h2(w.y, 0x4342u));
+          mma_16816(c, qa[2 * b][0], qa[2 * b][1], qa[2 * b][2], qa[2 * b][3], k8[0], k8[1]);
+          mma_16816(c, qa[2 * b + 1][0], qa[2 * b + 1][1], qa[2 * b + 1][2], qa[2 * b + 1][3], k8[2], k8[3]);
           s[2 * n] = __fmaf_rn(k0[b] * q_down[b], c[0] + c[2], s[2 * n]);
           s[2 * n + 1] = __fmaf_rn(k1[b] * q_down[b], c[1] + c[3], s[2 * n + 1]);
         }
@@ -329,14 +390,19 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
           pl0 = h2_min8(pl0); pl1 = h2_min8(pl1);
           uint32_t w[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
+          for (int e = 0; !CV && e < 4; ++e) {
             const uint32_t pr = 16 * st + 8 * (e >> 1) + 2 * j + (e & 1);
             w[e] = *reinterpret_cast<const uint32_t*>(vt + q8_v_off<HD>(pr, 2 * b + (r >> 2)) + (r & 3) * 4) ^ 0x80808080u;
           }
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const uint32_t ta = prmt(w[0], w[1], e ? 0x7362u : 0x5140u), tb = prmt(w[2], w[3], e ? 0x7362u : 0x5140u);
-            const uint32_t a0 = u8_h2(ta, 0x4140u), a1 = u8_h2(ta, 0x4342u), a2 = u8_h2(tb, 0x4140u), a3 = u8_h2(tb, 0x4342u);
+            uint32_t a0, a1, a2, a3;
+            if constexpr (CV) {     // rows of the tile: dims 32 b + 16 e .. + 15
+              ldsm_x4_t(vt_s + q8_h_off<HD>(16 * st + (lane & 7) + ((lane >> 4) << 3), 4 * b + 2 * e + ((lane >> 3) & 1)), a0, a1, a2, a3);
+            } else {                // dims 32 b + 4 i + 2 e, then those + 1
+              const uint32_t ta = prmt(w[0], w[1], e ? 0x7362u : 0x5140u), tb = prmt(w[2], w[3], e ? 0x7362u : 0x5140u);
+              a0 = u8_h2(ta, 0x4140u); a1 = u8_h2(ta, 0x4342u); a2 = u8_h2(tb, 0x4140u); a3 = u8_h2(tb, 0x4342u);
+            }
             // into a fresh accumulator, added in f32: the tensor cores' own accumulation rounds towards zero, and over the
             // 250 steps of 4000 rows the result lost 4.4e-6 of itself (2.9e-7 so, as f32 loops do; a 777-token prompt takes 3 % longer)
             float c[4] = {0.f, 0.f, 0.f, 0.f};
@@ -363,9 +429,14 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   float* so = reinterpret_cast<float*>(smem) + warp * 8 * (HD + 2);   // [8][HD], then m[8], l[8]
 #pragma unroll
   for (int i = 0; i < 2 * NB; ++i) {
-    const uint32_t d = 32 * (i >> 1) + 4 * r + 2 * (i & 1);
-    *reinterpret_cast<float2*>(so + (2 * j) * HD + d) = make_float2(oacc[i][0], oacc[i][2]);
-    *reinterpret_cast<float2*>(so + (2 * j + 1) * HD + d) = make_float2(oacc[i][1], oacc[i][3]);
+    if constexpr (CV) {
+      float* a = so + (2 * j) * HD + 16 * i + r;
+      a[0] = oacc[i][0]; a[8] = oacc[i][2]; a[HD] = oacc[i][1]; a[HD + 8] = oacc[i][3];
+    } else {
+      const uint32_t d = 32 * (i >> 1) + 4 * r + 2 * (i & 1);
+      *reinterpret_cast<float2*>(so + (2 * j) * HD + d) = make_float2(oacc[i][0], oacc[i][2]);
+      *reinterpret_cast<float2*>(so + (2 * j + 1) * HD + d) = make_float2(oacc[i][1], oacc[i][3]);
+    }
   }
   if (j == 0) { so[8 * HD + r] = m; so[8 * HD + 8 + r] = l; }
   __syncthreads();
@@ -388,7 +459,7 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
     if (p.cluster) {       // this CTA's share of the row, for the cluster's merge below
       float* mine = reinterpret_cast<float*>(smem + L::MERGE);
       *reinterpret_cast<float4*>(mine + lr * HD + d) = o;
-      if (d == 0) { mine[32 * HD + 2 * lr] = M; mine[32 * HD + 2 * lr + 1] = Ls; }
+      if (d == 0) { mine[L::MROWS * HD + 2 * lr] = M; mine[L::MROWS * HD + 2 * lr + 1] = Ls; }
       continue;
     }
     if (ns_live > 1) {
@@ -409,30 +480,32 @@ __global__ void __launch_bounds__(kQ8Threads, 2) pa_q8_kernel(const Q8Params p) 
   for (uint32_t idx = split * kQ8Threads + tid; idx < n_rows_here * (HD / 4); idx += ns_live * kQ8Threads) {
     const uint32_t lr = idx / (HD / 4), d = (idx % (HD / 4)) * 4, row = row0 + lr, c = row / G, h = g * G + row % G;
     float Ls;
-    const float4 o = cluster_merge4(mine_s + (lr * HD + d) * 4, mine_s + (32 * HD + 2 * lr) * 4, ns_live, p.scale_log2, Ls);
+    const float4 o = cluster_merge4(mine_s + (lr * HD + d) * 4, mine_s + (L::MROWS * HD + 2 * lr) * 4, ns_live, p.scale_log2, Ls);
     gate_store4(o, Ls, p.gate, (uint64_t)c * p.gate_col_stride + (uint64_t)h * p.gate_head_stride + d, p.out, (uint64_t)c * p.out_col_stride + (uint64_t)h * HD + d,
                 p.act_f16);
   }
   cluster_sync();          // no CTA leaves while another reads its rows
 }
 
-template <int HD>
+template <int HD, bool CV>
 static cudaError_t launch_q8_t(const Q8Params& p, dim3 grid, int dev, cudaStream_t st) {
+  using L = Q8Smem<HD, CV>;
+  static_assert(L::TOTAL <= 227 * 1024, "shared memory of one CTA");
   static bool attr_set[64] = {};
   if (!attr_set[dev & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(pa_q8_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q8Smem<HD>::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(pa_q8_kernel<HD, CV>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
     if (e != cudaSuccess) return e;
     attr_set[dev & 63] = true;
   }
-  if (p.cluster) return launch_pdl_cluster(pa_q8_kernel<HD>, grid, dim3(kQ8Threads), (size_t)Q8Smem<HD>::TOTAL, st, p.cluster, p);
-  return launch_pdl(pa_q8_kernel<HD>, grid, dim3(kQ8Threads), (size_t)Q8Smem<HD>::TOTAL, st, p);
+  if (p.cluster) return launch_pdl_cluster(pa_q8_kernel<HD, CV>, grid, dim3(L::THREADS), (size_t)L::TOTAL, st, p.cluster, p);
+  return launch_pdl(pa_q8_kernel<HD, CV>, grid, dim3(L::THREADS), (size_t)L::TOTAL, st, p);
 }
 cudaError_t launch_q8(const Q8Params& p, uint32_t hd, uint32_t n_kv, int dev, cudaStream_t st) {
   const dim3 grid(p.cluster ? p.cluster : p.n_splits, n_kv, (p.n_cols * p.G + 8 * p.rgw - 1) / (8 * p.rgw));
   switch (hd) {
-    case 256: return launch_q8_t<256>(p, grid, dev, st);
-    case 128: return launch_q8_t<128>(p, grid, dev, st);
-    case 64: return launch_q8_t<64>(p, grid, dev, st);
+    case 256: return p.rgw >= 4 ? launch_q8_t<256, true>(p, grid, dev, st) : launch_q8_t<256, false>(p, grid, dev, st);
+    case 128: return p.rgw >= 4 ? launch_q8_t<128, true>(p, grid, dev, st) : launch_q8_t<128, false>(p, grid, dev, st);
+    case 64: return p.rgw >= 4 ? launch_q8_t<64, true>(p, grid, dev, st) : launch_q8_t<64, false>(p, grid, dev, st);
     default: return cudaErrorInvalidValue;
   }
 }

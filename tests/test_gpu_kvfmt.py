@@ -323,6 +323,22 @@ def test_an_int8_call_wider_than_the_grid():
         util.assert_close(out[c].float().cpu().numpy(), ref.reshape(-1), f"column {c}")
 
 
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("n_cols", [9, 16, 17, 288, 289, 300])
+def test_int8_row_tiles_of_32_and_64(hd, n_cols):
+    # two heads per kv head: just past 16 query rows, one whole tile of 32 and a remainder, and either side of where 64-row tiles fill the chip
+    nH, nKV, pos = 32, 16, 77
+    rows = pos + n_cols
+    eng = _engine("q8", nH, nKV, hd, rows, max_cols=rows)
+    g = np.random.default_rng(19)
+    K, V, q = (g.standard_normal(s).astype(np.float32) for s in ((rows, nKV * hd), (rows, nKV * hd), (n_cols, nH * hd)))
+    eng.kv_append(0, 0, 0, util.torch_dev(K), util.torch_dev(V))
+    out = eng.prefill(0, 0, pos, util.torch_dev(q)).cpu().numpy()
+    eng.sync()
+    Kh, Vh, _ = _held(eng, "q8", 0, rows)
+    assert util.errs(out, po.attn_f64_kv32(q, Kh, Vh, nH, nKV, hd, pos, n_cols, None))[1] < util.REF_REL
+
+
 @pytest.mark.parametrize("nH,nKV,hd", [(16, 2, 256), (6, 2, 128), (3, 1, 64)])
 @pytest.mark.parametrize("rows,n_cols", [(64, 1), (129, 2), (1100, 3), (2900, 40), (9003, 3), (8963, 8)])
 def test_f32_plans_of_many_waves(nH, nKV, hd, rows, n_cols):
