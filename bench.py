@@ -348,7 +348,7 @@ def run_decode(R: Run, w, headline: bool):
         "dtype": "f16 cache and activations, f32 accumulate",
         "data": "synthetic (seeded N(0,1) -> f16, outlier channels x20)" if w["outliers"] else "synthetic (seeded N(0,1) -> f16)",
         "config": cfg, "pct_of_8TBs_nominal_per_gpu": round(100 * value / world / 8000, 1),
-        "roofline": {"bound": "hbm", "kernel": "pa_prefill_kernel<256,2> (split-K tcgen05 verify)" if verify_tc else "pa_decode_kernel",
+        "roofline": {"bound": "hbm", "kernel": "pa_verify_kernel<256,2> (split-K tcgen05 verify)" if verify_tc else "pa_decode_kernel",
                      "achieved": round(achieved, 1) if achieved else None, "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4) if achieved else None, "peak_source": peak_src, "launches_timed": int(core_n),
                      "us_per_launch": round(core_ms / max(core_n, 1) * 1e3, 2), "algorithmic_bytes_per_launch": kernel_bytes, "traffic": traffic},
@@ -422,7 +422,7 @@ def run_prefill(R: Run, w):
            "config": {"workload": w["desc"], "heads_per_gpu": f"{nH_r}q/{nKV_r}kv", "flops": "4*nH*hd*T(T+1)/2 per layer (masked half not credited)",
                       "l2": "q, k, v and out of a layer are 235 MB, more than the 126 MB L2; each layer has its own caches"},
            "pct_of_2250TF_nominal_per_gpu": round(100 * value / world / 2250, 1),
-           "roofline": {"bound": "tensor", "kernel": "pa_prefill_kernel<256,0>", "achieved": round(ach, 1), "peak": peak, "unit": "TFLOP/s", "frac": round(ach / peak, 4),
+           "roofline": {"bound": "tensor", "kernel": "pa_prefill_kernel<256>", "achieved": round(ach, 1), "peak": peak, "unit": "TFLOP/s", "frac": round(ach / peak, 4),
                         "peak_source": src, "launches_timed": int(core_n), "us_per_launch": round(core_ms / max(core_n, 1) * 1e3, 1), "traffic": args.traffic},
            "e2e": {"value": round(flops_layer * layers * args.steps / (ems * 1e-3) / 1e12, 1), "unit": "TFLOP/s", "ms_per_step": round(ems / args.steps, 4),
                    "h2d_bytes_per_step": int(hq.numel() + hk.numel() + hv.numel()) * 2 * world, "d2h_bytes_per_step": int(hout.numel()) * 2 * world, **espread},

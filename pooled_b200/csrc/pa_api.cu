@@ -23,6 +23,7 @@ bool rope_vec_applies(const RopeParams& p, uint32_t n_cols);
 cudaError_t launch_epoch_bump(unsigned int* ctr, cudaStream_t st);
 cudaError_t launch_head_norm(const HeadNormParams& p, cudaStream_t st);
 int prefill_supported(const pa_ctx* ctx);
+uint32_t prefill_v_rows(uint32_t head_dim);
 bool decode_f32_direct(uint32_t G);
 uint32_t decode_f32_batch(uint32_t hd, uint32_t G);
 cudaError_t launch_decode_f32_direct(const F32DecodeParams& p, uint32_t hd, uint32_t G, uint32_t n_kv, cudaStream_t st);
@@ -32,7 +33,7 @@ cudaError_t launch_front(const FrontParams& p, uint32_t hd, uint32_t n_rot, cuda
 cudaError_t launch_combine_few(int head_dim, const PrefillParams& p, cudaStream_t st);
 uint32_t prefill_splits(uint32_t pos, uint32_t n_cols, uint32_t n_heads, uint32_t head_dim, uint32_t sms, size_t slots);
 cudaError_t launch_prefill(const pa_layer* L, const PrefillParams& p, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_q,
-                           const CUtensorMap& tm_o, const CUtensorMap& tm_q2, cudaStream_t st);
+                           const CUtensorMap& tm_o, const CUtensorMap& tm_q2, const CUtensorMap& tm_g, cudaStream_t st);
 cudaError_t launch_verify(const pa_layer* L, const PrefillParams& p, const CUtensorMap& tm_k, const CUtensorMap& tm_v, uint32_t n_kv, cudaStream_t st);
 cudaError_t launch_kv_store(const KvStoreParams& p, uint32_t n_cols, cudaStream_t st);
 cudaError_t launch_decode_f32(const AnyDecodeParams& p, dim3 grid, int dev, cudaStream_t st);
@@ -1109,8 +1110,12 @@ extern "C" int pa_merge(pa_ctx* ctx, const float* parts, uint32_t n_parts, uint3
 // the caller's own (unrotated) f16 q of a layer call whose RoPE kernel wrote only the rotated dims of the rotated q
 struct PlainQ { const void* q; uint64_t cs, hs; };
 
+// f16 rows a tensor map of [columns][64-dim chunks of a column] reaches: whole chunks, every head inside its column's stride
+static bool rows_tma_ok(const pa_ctx* ctx, const void* x, uint64_t cs, uint64_t hs) {
+  return !(cs & 63) && !(hs & 63) && !((uintptr_t)x & 15) && (ctx->cfg.n_heads - 1) * hs + ctx->cfg.head_dim <= cs;
+}
 static bool q_tma_ok(const pa_ctx* ctx, int q_dtype, uint64_t qcs, uint64_t qhs, const void* q) {
-  return q_dtype == PA_F16 && ctx->cfg.head_dim == 256 && !(qcs & 63) && !(qhs & 63) && !((uintptr_t)q & 15) && !ctx->tune.no_q_tma;
+  return q_dtype == PA_F16 && rows_tma_ok(ctx, q, qcs, qhs) && !ctx->tune.no_q_tma;
 }
 
 static int prefill_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, const void* q, int q_dtype, uint64_t qcs, uint64_t qhs, const void* gate,
@@ -1151,9 +1156,9 @@ static int prefill_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols
   // appended row is zero-filled by TMA instead of carrying whatever the cache holds there (0 * NaN is NaN).
   CUtensorMap tm_k, tm_v;
   const uint64_t seq_off = (uint64_t)seq * L->max_seq * ctx->kv_dim;
-  if (int rc = make_cache_map(ctx, &tm_k, L->k + seq_off, (uint64_t)p.pos + n_cols, ctx->kv_dim, ctx->cfg.head_dim, 64)) return rc;
-  if (int rc = make_cache_map(ctx, &tm_v, L->v + seq_off, (uint64_t)p.pos + n_cols, ctx->kv_dim, ctx->cfg.head_dim, 64)) return rc;
-  // f16 query rows at head_dim 256 travel by TMA: a map of q as [n_cols][q_col_stride] in 64-element chunks, the same
+  if (int rc = make_cache_map(ctx, &tm_k, L->k + seq_off, (uint64_t)p.pos + n_cols, ctx->kv_dim, 64, 128)) return rc;
+  if (int rc = make_cache_map(ctx, &tm_v, L->v + seq_off, (uint64_t)p.pos + n_cols, ctx->kv_dim, ctx->cfg.head_dim, prefill_v_rows(ctx->cfg.head_dim))) return rc;
+  // f16 query rows travel by TMA: a map of q as [n_cols][q_col_stride] in 64-element chunks, the same
   // shape of map as a cache's (rows past n_cols read as zeros)
   CUtensorMap tm_q = tm_k, tm_q2 = tm_k;
   if (plain) {
@@ -1169,14 +1174,18 @@ static int prefill_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols
   // few columns behind many keys: the keys are split and the records merged by a second kernel
   p.n_splits = ctx->core_only ? 1u : prefill_splits(p.pos, n_cols, p.n_heads, ctx->cfg.head_dim, (uint32_t)ctx->sm_count, ctx->pf_slots);
   p.part_o = ctx->part_o; p.part_ml = ctx->part_ml;
-  // ... and f16 output tiles leave by TMA (any head_dim the kernel takes; gate, if any, f16 with 16-byte aligned rows)
-  CUtensorMap tm_o = tm_k;
-  if (ctx->cfg.act_dtype == PA_F16 && !(ocs & 63) && !ctx->tune.no_out_tma && (!gate || (!(gcs & 7) && !(ghs & 7) && !((uintptr_t)gate & 15)))) {
+  // ... and f16 output tiles leave by TMA (any head_dim the kernel takes; the gate's, if any, arrive so)
+  CUtensorMap tm_o = tm_k, tm_g = tm_k;
+  if (ctx->cfg.act_dtype == PA_F16 && !(ocs & 63) && !ctx->tune.no_out_tma && (!gate || rows_tma_ok(ctx, gate, gcs, ghs))) {
+    if (gate) {
+      if (int rc = make_cache_map(ctx, &tm_g, const_cast<void*>(gate), n_cols, (uint32_t)gcs, ctx->cfg.head_dim, 128)) return rc;
+      p.gate_tma = 1;
+    }
     if (int rc = make_cache_map(ctx, &tm_o, out, n_cols, (uint32_t)ocs, ctx->cfg.head_dim, 128)) return rc;
     p.out_tma = 1;
   }
   timing_mark(ctx, st, 0);
-  CU_TRY(ctx, launch_prefill(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, st));
+  CU_TRY(ctx, launch_prefill(L, p, tm_k, tm_v, tm_q, tm_o, tm_q2, tm_g, st));
   if (p.n_splits > 1) { CU_TRY(ctx, launch_combine_few((int)ctx->cfg.head_dim, p, st)); ctx->stats.kernel_launches++; }
   timing_mark(ctx, st, 1);
   ctx->stats.kernel_launches++; ctx->stats.calls++;

@@ -167,6 +167,35 @@ def test_chunked_prefill_and_prefill_vs_decode():
     eng.sync()
 
 
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("n_cols,pos", [(1, 0), (64, 0), (65, 63), (127, 1), (128, 128), (129, 127), (300, 85)])
+@pytest.mark.parametrize("act,order", [("f16", "cols"), ("f16", "heads"), ("f16", "padded"), ("f32", "cols"), ("f32", "heads")])
+def test_prefill_at_the_edges_of_its_tiles_and_any_order_of_heads(hd, n_cols, pos, act, order):
+    # 128 columns x 128 keys a tile; q and gate as [column][head][dim] with the gate beside q (every copy by TMA), [head][column][dim]
+    # (none), or with column strides of no whole 64-dim chunks
+    import torch
+    nH, nKV = 6, 2
+    td = torch.float16 if act == "f16" else torch.float32
+    T = pos + n_cols
+    eng = _engine(nH, nKV, hd, T + 70, act=act, max_cols=512, rope_mode="none")
+    q, g = util.normal_f16(31, (n_cols, nH * hd)), util.normal_f16(32, (n_cols, nH * hd))
+    K, V = (po.np_f16_rne(po.normal(33 + i, T * nKV * hd)).reshape(T, -1) for i in range(2))
+    poison = np.full((70, nKV * hd), 0x7e00, np.uint16)      # rows past the last one hold NaN
+    util.load_cache(eng, 0, 0, np.concatenate([K, poison]), np.concatenate([V, poison]))
+    tq, tg = (util.torch_dev(x, td).view(n_cols, nH, hd) for x in (q, g))
+    if order == "cols":
+        both = torch.cat([tq, tg], 2).view(n_cols, -1)
+        out = eng.prefill(0, 0, pos, both, both[:, hd:], q_head_stride=2 * hd, gate_head_stride=2 * hd)
+    elif order == "heads":
+        q2, g2 = (x.permute(1, 0, 2).contiguous() for x in (tq, tg))
+        out = eng.prefill(0, 0, pos, q2.view(-1)[:n_cols * hd].view(n_cols, hd), g2.view(-1)[:n_cols * hd].view(n_cols, hd), q_head_stride=n_cols * hd, gate_head_stride=n_cols * hd)
+    else:
+        q2, g2 = (torch.nn.functional.pad(x.reshape(n_cols, -1), (0, 8)) for x in (tq, tg))
+        out = eng.prefill(0, 0, pos, q2, g2)
+    eng.sync()
+    util.assert_close(out.float().cpu().numpy(), po.attn_f64(q, K, V, nH, nKV, hd, pos, n_cols, g), f"{n_cols} columns at {pos}, {act} {order}")
+
+
 @pytest.mark.parametrize("nH,nKV,hd,n_cols,pos,act,gate", [
     (24, 4, 256, 203, 3001, "f32", True),     # two q tiles, the second with 75 rows
     (16, 2, 256, 48, 1500, "f16", True),      # less than one q tile
