@@ -22,7 +22,7 @@
 // products against 1024 with N = 128, measured with nothing else running.
 //
 // Measured (whole passes, power-capped; tiles of 64 keys with two groups of four softmax warps on alternate tiles and gate rows fetched
-// by the lanes before): 4 layers of 8192 columns of 24 heads x 256 3698 -> 3294 us, 8 layers of 2999 x 16 x 128 676 -> 639,
+// by the lanes before): 4 layers of 8192 columns of 24 heads x 256 3698 -> 3294 us, 8 layers of 2999 x 16 x 128 676 -> 639 (612 with the present rotation kernel),
 // 8 layers of 203 columns of 24 x 256 behind 9001 rows 602 -> 554.  A tile of head_dim 256 takes 2220 cycles for the tensor cores'
 // 2048 and the chip runs at 1.39 GHz under its power limit; at head_dim 128 it is 1970 for 1170: there the softmax warps, whose
 // exponentials alone are 1024, set the pace.

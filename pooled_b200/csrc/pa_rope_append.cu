@@ -203,18 +203,16 @@ static __device__ __noinline__ uint32_t rot_h_slow(uint32_t xw, uint32_t yw, int
 }
 // 64 threads per column, four columns per CTA.  Thread t of a column holds the cos / sin of eight neighbouring dims and
 // walks the heads t / (half / 8), + 64 / (half / 8), ...: 16-byte loads and stores on both sides, the angles loaded once,
-// rot_h() for the arithmetic.  (Before: a CTA per column, two dims per thread, rot_exact().  Eight layers of 2999 columns of 16 + 8
-// heads x 128, whole calls, together with the order of the prefill kernel's CTAs: 834 us then, 677 now, 96 of the difference
-// in that kernel.)  half / 8 need not divide 64: the threads past the last whole turn then only copy.
-__global__ void __launch_bounds__(256) pa_rope_append_vec_kernel(const RopeParams p, const uint32_t n_cols) {
+// rot_h() for the arithmetic, everything of a thread's first turn requested before anything is used.  Eight layers of 2999
+// columns of 16 + 8 heads x 128, whole calls: 639 us with one kind of load after the other, two heads at a time, 612 so.  8192
+// columns of 24 heads of which 64 dims turn take 47 us for 117 MB: 128-byte pieces of q 1 KB apart.
+// half / 8 need not divide 64: the threads past the last whole turn then only copy.
+constexpr int kRopeU = 3, kRopeC = 4;    // heads and copied vectors a thread has in flight
+__global__ void __launch_bounds__(256, 2) pa_rope_append_vec_kernel(const RopeParams p, const uint32_t n_cols) {
   __shared__ float2 s_cs[4][128];
-  const uint32_t cl = threadIdx.x >> 6, t = threadIdx.x & 63, col = blockIdx.x * 4 + cl, half = p.n_rot / 2, hd = p.hd;
-  const bool live = col < n_cols;
+  const uint32_t cl = threadIdx.x >> 6, t = threadIdx.x & 63, col = min(blockIdx.x * 4 + cl, n_cols - 1), half = p.n_rot / 2, hd = p.hd;
+  const bool live = blockIdx.x * 4 + cl < n_cols;
   if (p.trigger_early) pdl_trigger();
-  pdl_wait();
-  if (!p.trigger_early) pdl_trigger();
-  const Angle* ang = p.angles + (uint64_t)col * half;
-  if (live) for (uint32_t i = t; i < half; i += 64) s_cs[cl][i] = make_float2(ang[i].c_hi, ang[i].s_hi);
   const uint32_t kvd = p.kv_heads * hd;
   const __half* qs = reinterpret_cast<const __half*>(p.q) + (uint64_t)col * p.q_col_stride;
   const __half* ks = reinterpret_cast<const __half*>(p.k) + (uint64_t)col * p.kv_col_stride;
@@ -222,29 +220,74 @@ __global__ void __launch_bounds__(256) pa_rope_append_vec_kernel(const RopeParam
   __half* qd = reinterpret_cast<__half*>(p.q_out) + (uint64_t)col * p.q_out_col_stride;
   __half* kd = p.k_cache + (p.cache_row0 + col) * (uint64_t)kvd;
   __half* vd = p.v_cache + (p.cache_row0 + col) * (uint64_t)kvd;
-  const uint32_t nqh = p.q ? p.q_heads : 0, nh = nqh + (p.k ? p.kv_heads : 0);
+  const uint32_t nqh = p.q ? p.q_heads : 0, nh = live ? nqh + (p.k ? p.kv_heads : 0) : 0;
   const uint32_t groups = half / 8, step = 64 / groups, d = (t % groups) * 8;
-  __syncthreads();
-  if (!live) return;
-  float2 cs[8];
+  // everything but the rotated dims: 16-byte vectors of the unrotated dims of q and k, and all of v
+  const uint32_t cv = (hd - p.n_rot) / 8, vv = hd / 8;
+  const uint32_t nq = p.q_rot_only ? 0u : nqh * cv, nk = (p.k ? p.kv_heads : 0) * cv, nv = p.v ? p.kv_heads * vv : 0, total = live ? nq + nk + nv : 0;
+  uint4 A[kRopeU], B[kRopeU], C[kRopeC];
+  auto load_heads = [&](uint32_t h0) {     // dims d .. d + 7 of heads h0, h0 + step, ... with their partners half further on
 #pragma unroll
-  for (int e = 0; e < 8; ++e) cs[e] = s_cs[cl][d + e];
-  // ---- rotated dims: d .. d + 7 with their partners half further on, two heads in flight ----
-  for (uint32_t h0 = t < groups * step ? t / groups : nh; h0 < nh; h0 += 2 * step) {
-    uint4 A[2], B[2];
-    __half* dst[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < kRopeU; ++u) {
       const uint32_t h = h0 + u * step;
       if (h >= nh) continue;
       const __half* src = (h < nqh ? qs + (uint64_t)h * p.q_head_stride : ks + (uint64_t)(h - nqh) * hd) + d;
-      dst[u] = (h < nqh ? qd + (uint64_t)h * hd : kd + (uint64_t)(h - nqh) * hd) + d;
       A[u] = *reinterpret_cast<const uint4*>(src);
       B[u] = *reinterpret_cast<const uint4*>(src + half);
     }
+  };
+  auto load_copies = [&](uint32_t w0) {
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (h0 + u * step >= nh) continue;
+    for (int u = 0; u < kRopeC; ++u) {
+      const uint32_t w = w0 + u * 64;
+      if (w >= total) continue;
+      const __half* src;
+      if (w >= nq + nk) src = vs + 8 * (w - nq - nk);
+      else {
+        const bool is_q = w < nq;
+        const uint32_t ww = is_q ? w : w - nq, head = ww / cv, dd = p.n_rot + 8 * (ww % cv);
+        src = (is_q ? qs + (uint64_t)head * p.q_head_stride : ks + (uint64_t)head * hd) + dd;
+      }
+      C[u] = *reinterpret_cast<const uint4*>(src);
+    }
+  };
+  auto store_copies = [&](uint32_t w0) {
+#pragma unroll
+    for (int u = 0; u < kRopeC; ++u) {
+      const uint32_t w = w0 + u * 64;
+      if (w >= total) continue;
+      __half* dst;
+      bool cache = true;
+      if (w >= nq + nk) dst = vd + 8 * (w - nq - nk);
+      else {
+        const bool is_q = w < nq;
+        const uint32_t ww = is_q ? w : w - nq, head = ww / cv, dd = p.n_rot + 8 * (ww % cv);
+        cache = !is_q;
+        dst = (is_q ? qd + (uint64_t)head * hd : kd + (uint64_t)head * hd) + dd;
+      }
+      uint4 o = C[u];
+      o.x = fix_nan2(o.x, cache); o.y = fix_nan2(o.y, cache); o.z = fix_nan2(o.z, cache); o.w = fix_nan2(o.w, cache);
+      *reinterpret_cast<uint4*>(dst) = o;
+    }
+  };
+  const uint32_t first_h = t < groups * step ? t / groups : nh;
+  pdl_wait();
+  if (!p.trigger_early) pdl_trigger();
+  // a column's angles, rotated dims and copies are all requested before the first of them is used
+  const Angle* ang = p.angles + (uint64_t)col * half;
+  for (uint32_t i = t; i < half; i += 64) s_cs[cl][i] = make_float2(ang[i].c_hi, ang[i].s_hi);
+  load_heads(first_h);
+  load_copies(t);
+  __syncthreads();
+  float2 cs[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) cs[e] = s_cs[cl][d + e];
+  for (uint32_t h0 = first_h; h0 < nh; h0 += kRopeU * step) {
+    if (h0 != first_h) load_heads(h0);
+#pragma unroll
+    for (int u = 0; u < kRopeU; ++u) {
+      const uint32_t h = h0 + u * step;
+      if (h >= nh) continue;
       const uint32_t aw[4] = {A[u].x, A[u].y, A[u].z, A[u].w}, bw[4] = {B[u].x, B[u].y, B[u].z, B[u].w};
       uint32_t ra[8], rb[8], bad = 0;
 #pragma unroll
@@ -257,50 +300,22 @@ __global__ void __launch_bounds__(256) pa_rope_append_vec_kernel(const RopeParam
         bad |= (ok1 ? 0u : 1u << e) | (ok2 ? 0u : 256u << e);
       }
       if (bad) {
-        const bool cache = h0 + u * step >= nqh;
+        const bool cache = h >= nqh;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           if (bad & (1u << e)) ra[e] = rot_h_slow(aw[e >> 1], bw[e >> 1], 16 * (e & 1), ang + d + e, true, cache);
           if (bad & (256u << e)) rb[e] = rot_h_slow(bw[e >> 1], aw[e >> 1], 16 * (e & 1), ang + d + e, false, cache);
         }
       }
-      *reinterpret_cast<uint4*>(dst[u]) = make_uint4(ra[0] | (ra[1] << 16), ra[2] | (ra[3] << 16), ra[4] | (ra[5] << 16), ra[6] | (ra[7] << 16));
-      *reinterpret_cast<uint4*>(dst[u] + half) = make_uint4(rb[0] | (rb[1] << 16), rb[2] | (rb[3] << 16), rb[4] | (rb[5] << 16), rb[6] | (rb[7] << 16));
+      __half* dst = (h < nqh ? qd + (uint64_t)h * hd : kd + (uint64_t)(h - nqh) * hd) + d;
+      *reinterpret_cast<uint4*>(dst) = make_uint4(ra[0] | (ra[1] << 16), ra[2] | (ra[3] << 16), ra[4] | (ra[5] << 16), ra[6] | (ra[7] << 16));
+      *reinterpret_cast<uint4*>(dst + half) = make_uint4(rb[0] | (rb[1] << 16), rb[2] | (rb[3] << 16), rb[4] | (rb[5] << 16), rb[6] | (rb[7] << 16));
     }
   }
-  // ---- everything else: 16-byte vectors of the unrotated dims of q and k, and all of v ----
-  {
-    const uint32_t cv = (hd - p.n_rot) / 8, vv = hd / 8;
-    const uint32_t nq = p.q_rot_only ? 0u : nqh * cv, nk = (nh - nqh) * cv, nv = p.v ? p.kv_heads * vv : 0, total = nq + nk + nv;
-    for (uint32_t w0 = t; w0 < total; w0 += 4 * 64) {
-      uint4 A[4]; __half* dst[4]; int kind[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t w = w0 + u * 64;
-        kind[u] = -1;
-        if (w >= total) continue;
-        const __half* src;
-        if (w >= nq + nk) {
-          const uint32_t x = w - nq - nk;
-          kind[u] = 1; src = vs + 8 * x; dst[u] = vd + 8 * x;
-        } else {
-          const bool is_q = w < nq;
-          const uint32_t ww = is_q ? w : w - nq, head = ww / cv, dd = p.n_rot + 8 * (ww % cv);
-          kind[u] = is_q ? 0 : 1;
-          src = (is_q ? qs + (uint64_t)head * p.q_head_stride : ks + (uint64_t)head * hd) + dd;
-          dst[u] = (is_q ? qd + (uint64_t)head * hd : kd + (uint64_t)head * hd) + dd;
-        }
-        A[u] = *reinterpret_cast<const uint4*>(src);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (kind[u] < 0) continue;
-        const bool cache = kind[u] != 0;
-        uint4 o = A[u];
-        o.x = fix_nan2(o.x, cache); o.y = fix_nan2(o.y, cache); o.z = fix_nan2(o.z, cache); o.w = fix_nan2(o.w, cache);
-        *reinterpret_cast<uint4*>(dst[u]) = o;
-      }
-    }
+  store_copies(t);
+  for (uint32_t w0 = t + kRopeC * 64; w0 < total; w0 += kRopeC * 64) {
+    load_copies(w0);
+    store_copies(w0);
   }
 }
 
