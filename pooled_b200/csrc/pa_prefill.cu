@@ -11,7 +11,7 @@
 //                P(j) overwrote needs no wait before S(j + 2) goes into it, and the weights of a tile have the time of a score
 //                product and of a P V product to be formed in
 //   warp 2       allocates and frees tensor memory
-//   warps 4-11   softmax: warp w and warp w + 4 share the 32 query rows of TMEM lanes 32 (w % 4) ..., 64 keys of the tile each:
+//   warps 4-11   (4-19 at head_dim 128 and 64) softmax: warp w and warp w + 4 share the 32 query rows of TMEM lanes 32 (w % 4) ..., 64 keys of the tile each:
 //                tcgen05.ld of the scores, causal mask, the row's maximum through shared memory, P = 2^(s - m) as f16 pairs
 //                back over the S tile (tcgen05.st); then the epilogue (O / l, sigmoid gate, store)
 // O is rescaled only when a row's running maximum has grown by more than 2^8 since its last rescale (weights stay below
@@ -22,10 +22,9 @@
 // products against 1024 with N = 128, measured with nothing else running.
 //
 // Measured (whole passes, power-capped; tiles of 64 keys with two groups of four softmax warps on alternate tiles and gate rows fetched
-// by the lanes before): 4 layers of 8192 columns of 24 heads x 256 3698 -> 3294 us, 8 layers of 2999 x 16 x 128 676 -> 639 (612 with the present rotation kernel),
-// 8 layers of 203 columns of 24 x 256 behind 9001 rows 602 -> 554.  A tile of head_dim 256 takes 2220 cycles for the tensor cores'
-// 2048 and the chip runs at 1.39 GHz under its power limit; at head_dim 128 it is 1970 for 1170: there the softmax warps, whose
-// exponentials alone are 1024, set the pace.
+// by the lanes before): 4 layers of 8192 columns of 24 heads x 256 3698 -> 3294 us, 8 layers of 2999 x 16 x 128 676 -> 576 (36 of it
+// sixteen softmax warps instead of eight, 27 the rotation kernel's), 8 layers of 203 columns of 24 x 256 behind 9001 rows 602 -> 554.
+// A tile of head_dim 256 takes 2220 cycles for the tensor cores' 2048 and the chip runs at 1.39 GHz under its power limit.
 //
 // Stands in for attn_flash_tile + attn_combine_tile + sigmoid_mul_mc of pooled (engine/wgsl/attn_tile.js:108-193,
 // engine/wgsl/qwen35.js:877-887); there the pass is 16 columns wide and split over the sequence, here a pass takes
@@ -42,16 +41,19 @@ struct PfSmem {
   static constexpr int KC = HD / 64, K_CHUNK = kPN * 128;       // K chunks of a tile: [128 keys][64 dims]
   static constexpr int VK = 8192 / HD < kPN ? 8192 / HD : kPN;  // keys of a V chunk: [HD / 64][VK keys][64 dims]
   static constexpr int VC = kPN / VK, V_CHUNK = VK * HD * 2;
-  static constexpr int NK = HD == 256 ? 5 : 6, NV = HD == 256 ? 5 : 6;   // ring depths in chunks
-  // S / P tiles in tensor memory (128 columns each; P takes the first 64 of its S) | O (HD).  head_dim 256: 256 + 256 = 512
+  static constexpr bool ALT = HD <= 128;      // sixteen softmax warps, eight on every other tile (see there)
+  static constexpr int NGRP = ALT ? 4 : 2, SOFT = 128 * NGRP;            // groups of four softmax warps
+  static constexpr int NK = ALT ? 6 : 5, NV = 5;                         // ring depths in chunks
+  // S / P tiles in tensor memory (128 columns each; P takes the first 32 of each half of its S) | O (HD).  head_dim 256: 256 + 256 = 512
   static constexpr int SBUF = HD == 256 ? 2 : 3;
   static constexpr int T_S = 0, T_O = SBUF * kPN, TMEM_COLS = 512;
   static_assert(T_O + HD <= 512, "tensor memory columns");
-  static constexpr int THREADS = 128 + 256;
+  static constexpr int THREADS = 128 + SOFT;
   static constexpr int OFF_Q = 0, OFF_K = HD * kPM * 2, OFF_V = OFF_K + NK * K_CHUNK, OFF_BAR = OFF_V + NV * V_CHUNK;
   static constexpr int RINGS = NK * K_CHUNK + NV * V_CHUNK;
-  static constexpr int OFF_MX = OFF_BAR + 512;                  // [2 tiles][2 halves][128] row maxima; at the end [2][128] row sums
-  static constexpr int TOTAL = OFF_MX + 2 * 2 * kPM * 4;
+  // halves' row maxima of a tile, [2 tiles][ALT: tiles' parity][2 halves][128]; ALT: the rows' references after a tile, [2][128]
+  static constexpr int OFF_MX = OFF_BAR + 512, OFF_RM = OFF_MX + NGRP * 2 * kPM * 4;
+  static constexpr int TOTAL = OFF_RM + (ALT ? 2 * kPM * 4 : 0);
   static_assert(TOTAL <= 227 * 1024, "shared memory of one CTA");
 };
 
@@ -82,11 +84,11 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
                   const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ CUtensorMap tm_q2, const __grid_constant__ CUtensorMap tm_g,
                   const PrefillParams p) {
   using L = PfSmem<HD>;
-  constexpr int NK = L::NK, NV = L::NV, SB = L::SBUF;
+  constexpr int NK = L::NK, NV = L::NV, SB = L::SBUF, NGRP = L::NGRP, SOFT = L::SOFT;
   extern __shared__ __align__(1024) uint8_t base[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + L::OFF_BAR);
   enum { K_FULL = 0, K_EMPTY = NK, V_FULL = 2 * NK, V_EMPTY = 2 * NK + NV, S_FULL = 2 * NK + 2 * NV, P_FULL = S_FULL + SB, PV_DONE = P_FULL + SB, O_DONE = PV_DONE + 2,
-         Q_FULL = O_DONE + 1, G_FULL = O_DONE + 2, N_BARS = G_FULL + 1 };
+         Q_FULL = O_DONE + 1, G_FULL = O_DONE + 2, M_READY = O_DONE + 3, N_BARS = M_READY + 2 };
   static_assert(N_BARS <= 62, "barrier slots");
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(bars + 62);
   volatile uint32_t* s_err = s_tmem + 1;
@@ -117,10 +119,10 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     for (int i = 0; i < NK; ++i) { mbar_init(BAR(K_FULL, i), 1); mbar_init(BAR(K_EMPTY, i), 1); }
     for (int i = 0; i < NV; ++i) { mbar_init(BAR(V_FULL, i), 1); mbar_init(BAR(V_EMPTY, i), 1); }
     for (int i = 0; i < SB; ++i) { mbar_init(BAR(S_FULL, i), 1); mbar_init(BAR(P_FULL, i), 8); }
-    for (int i = 0; i < 2; ++i) mbar_init(BAR(PV_DONE, i), 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(BAR(PV_DONE, i), 1); mbar_init(BAR(M_READY, i), 8); }
     mbar_init(BAR(O_DONE, 0), 1);
     mbar_init(BAR(G_FULL, 0), 1);
-    mbar_init(BAR(Q_FULL, 0), q_by_tma ? 1 : 256);
+    mbar_init(BAR(Q_FULL, 0), q_by_tma ? 1 : SOFT);
     fence_barrier_init();
   }
   if (warp == 2) {
@@ -209,7 +211,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     for (uint32_t j = 0; j < n_tiles; ++j) {
       // the scores SB - 1 tiles ahead go into the tile whose weights the product just issued reads: in order on the tensor cores
       if (j + SB - 1 < n_tiles) scores(j + SB - 1);
-      const uint32_t tp = t_s0 + (j % SB) * kPN;     // P(j): packed f16 pairs in the first 64 columns of S(j)'s tile
+      const uint32_t tp = t_s0 + (j % SB) * kPN;     // P(j): packed f16 pairs in the first 32 columns of each half of S(j)'s tile
       mbar_wait(BAR(P_FULL, j % SB), (j / SB) & 1, s_err, WAIT_MMA);
 #pragma unroll
       for (int c = 0; c < L::VC; ++c) {              // O += P(j) V(j)
@@ -218,7 +220,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         const uint64_t vd = v_desc + (uint64_t)(vst * (L::V_CHUNK >> 4));
 #pragma unroll
         for (int ks = 0; ks < L::VK / 16; ++ks)
-          umma_f16_ts(leader, t_o, tp + (c * (L::VK / 16) + ks) * 8, vd + (uint64_t)((ks * 2048) >> 4), idesc_pv, (j > 0 || c > 0 || ks > 0) ? 1u : 0u);
+          umma_f16_ts(leader, t_o, tp + (c * L::VK + ks * 16) / 64 * 64 + ((c * L::VK / 16 + ks) & 3) * 8, vd + (uint64_t)((ks * 2048) >> 4), idesc_pv, (j > 0 || c > 0 || ks > 0) ? 1u : 0u);
         umma_commit_elected(leader, BAR(V_EMPTY, vst));
         if (++vst == NV) { vst = 0; vph ^= 1; }
       }
@@ -227,16 +229,16 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     umma_commit_elected(leader, BAR(O_DONE, 0));
   } else if (warp >= 4) {
     // ------------------------------------------------------------------ softmax + epilogue ----
-    const uint32_t wg = (warp - 4) >> 2;                 // half of the tile's keys
+    const uint32_t wg = (warp - 4) >> 2, half = wg & 1;  // group; half of a tile's keys
     const uint32_t qd = warp & 3, row = qd * 32 + lane;  // a warp reaches the 32 TMEM lanes of its index mod 4
     const uint32_t lane_addr = (qd * 32) << 16;
     const bool live = row < rows_valid;
     const uint32_t lim = p0 + row + 1;                   // keys [0, lim) are visible to this row
     pdl_trigger();
     if (!q_by_tma) {
-      // this thread's half of its Q row as f16 into the layout the score products read
-      constexpr int PC = HD / 16;                        // 16-byte pieces of the half row
-      const uint64_t off = (uint64_t)(c0 + (live ? row : 0)) * p.q_col_stride + (uint64_t)h * p.q_head_stride + wg * (HD / 2);
+      // this thread's share of its Q row as f16 into the layout the score products read
+      constexpr int PC = HD / 8 / NGRP;                  // 16-byte pieces
+      const uint64_t off = (uint64_t)(c0 + (live ? row : 0)) * p.q_col_stride + (uint64_t)h * p.q_head_stride + wg * (HD / NGRP);
       uint4 x[PC];
 #pragma unroll
       for (int i = 0; i < PC; ++i) {
@@ -255,80 +257,152 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       mbar_arrive(BAR(Q_FULL, 0));
     }
     // m_st: the row's reference maximum, the same in both halves' threads (the weights of a tile are 2^(s - m_st); it moves only
-    // when a tile's maximum passes it by more than 2^8).  l2: this thread's share of the row sum.  (A split that does not begin
-    // at key 0 may hold no visible key of a row, hence the finite start.)
+    // when a tile's maximum passes it by more than 2^8).  (A split that does not begin at key 0 may hold no visible key of a row, hence the finite start.)
     const bool first0 = !SPLIT || tile0 == 0;
     float m_st = first0 ? -INFINITY : -1.0e30f;
-    float2 l2 = make_float2(0.f, 0.f);
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
-    uint32_t sb = 0, sph = 0;
-    for (uint32_t j = 0; j < n_tiles; ++j) {
-      const uint32_t kv0 = (tile0 + j) * kPN + wg * 64, ts = t_s0 + sb * kPN + lane_addr;
-      mbar_wait(BAR(S_FULL, sb), sph, s_err, WAIT_MMA);
-      tc_fence_after();
-      float s[64];
-      tmem_ld32_async(ts + wg * 64, s);
-      tmem_ld32_async(ts + wg * 64 + 32, s + 32);
-      tmem_wait_ld(s);
-      // maximum of the raw scores (the scale is positive), causal mask on tiles that reach this row's diagonal
-      if (kv0 + 64 > lim) {
+    // causal mask on tiles that reach this row's diagonal
+    auto mask = [&](float* x, int n, uint32_t key0) {
+      if (key0 + n > lim) {
 #pragma unroll
-        for (int i = 0; i < 64; ++i) if (kv0 + i >= lim) s[i] = -INFINITY;
+        for (int i = 0; i < n; ++i) if (key0 + i >= lim) x[i] = -INFINITY;
       }
-      float ma = fmaxf(s[0], s[1]), mb = fmaxf(s[2], s[3]), mc = fmaxf(s[4], s[5]), md = fmaxf(s[6], s[7]);
+    };
+    auto max32 = [](const float* x, float m) {
+      float a = max3(m, x[0], x[1]), b = fmaxf(x[2], x[3]), c = fmaxf(x[4], x[5]), d = fmaxf(x[6], x[7]);
 #pragma unroll
-      for (int i = 8; i < 64; i += 8) { ma = max3(ma, s[i], s[i + 1]); mb = max3(mb, s[i + 2], s[i + 3]); mc = max3(mc, s[i + 4], s[i + 5]); md = max3(md, s[i + 6], s[i + 7]); }
-      float* mx = s_mx + (j & 1) * (2 * kPM);
-      ma = fmaxf(fmaxf(ma, mb), fmaxf(mc, md));
-      mx[wg * kPM + row] = ma;
-      tc_fence_before();
-      named_bar_sync(2 + qd, 64);        // the two warps of these rows: both have read their scores, which P overwrites
+      for (int i = 8; i < 32; i += 8) { a = max3(a, x[i], x[i + 1]); b = max3(b, x[i + 2], x[i + 3]); c = max3(c, x[i + 4], x[i + 5]); d = max3(d, x[i + 6], x[i + 7]); }
+      return fmaxf(fmaxf(a, b), fmaxf(c, d));
+    };
+    // the row's reference given the tile's maximum (scaled); how much O and the row's sum shrink if it moves
+    auto refer = [&](uint32_t j, float mt, float& alpha) {
+      alpha = 1.f;
+      if (first0 && j == 0) { m_st = mt; return false; }         // key 0 is visible to every row
+      if (!(mt > m_st + 8.f)) return false;
+      alpha = ex2_approx(m_st - mt); m_st = mt;
+      return true;
+    };
+    // O must not change under the previous P V: wait for it, then rescale this warp's 32 rows in TMEM, chunks c0, c0 + dc, ...
+    auto rescale = [&](uint32_t j, float alpha, uint32_t c0, uint32_t dc) {
+      mbar_wait(BAR(PV_DONE, (j - 1) & 1), ((j - 1) >> 1) & 1, s_err, WAIT_MMA);
       tc_fence_after();
-      const float mt = fmaxf(ma, mx[(wg ^ 1) * kPM + row]) * p.scale_log2;
-      float alpha = 1.f;
-      bool grow = false;
-      if (first0 && j == 0) m_st = mt;                 // key 0 is visible to every row
-      else if (mt > m_st + 8.f) { alpha = ex2_approx(m_st - mt); m_st = mt; grow = true; }
-      if (__any_sync(0xffffffffu, grow)) {
-        l2.x *= alpha; l2.y *= alpha;
-        if (j > 0) {
-          // O must not change under the previous P V: wait for it, then rescale this warp's 32 rows in TMEM, half of the dims per warp
-          mbar_wait(BAR(PV_DONE, (j - 1) & 1), ((j - 1) >> 1) & 1, s_err, WAIT_MMA);
-          tc_fence_after();
 #pragma unroll 1
-          for (uint32_t c = wg; c < HD / 32; c += 2) {
-            float o[32];
-            tmem_ld32(t_o + c * 32 + lane_addr, o);
+      for (uint32_t c = c0; c < HD / 32; c += dc) {
+        float o[32];
+        tmem_ld32(t_o + c * 32 + lane_addr, o);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] *= alpha;
-            tmem_st32(t_o + c * 32 + lane_addr, o);
-          }
-        }
+        for (int i = 0; i < 32; ++i) o[i] *= alpha;
+        tmem_st32(t_o + c * 32 + lane_addr, o);
       }
-      // P = 2^(s - m) as packed f16 pairs over the S tile, this half's 32 columns
-      uint32_t pw[32];
+    };
+    // P = 2^(s - m) of 32 scores as packed f16 pairs, and their sum
+    auto weigh = [&](const float* x, uint32_t* w) {
       const float2 nm = make_float2(-m_st, -m_st);
       float2 la = make_float2(0.f, 0.f), lb = la;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float2 x = fma2(make_float2(s[2 * i], s[2 * i + 1]), sc2, nm);
-        const float2 e = make_float2(ex2_approx(x.x), ex2_approx(x.y));
+      for (int i = 0; i < 16; ++i) {
+        const float2 y = fma2(make_float2(x[2 * i], x[2 * i + 1]), sc2, nm);
+        const float2 e = make_float2(ex2_approx(y.x), ex2_approx(y.y));
         if (i & 1) lb = add2(lb, e); else la = add2(la, e);
-        pw[i] = pack_h2(e.x, e.y);
+        w[i] = pack_h2(e.x, e.y);
       }
-      tmem_st32u(ts + wg * 32, pw);
-      l2 = add2(l2, add2(la, lb));
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(BAR(P_FULL, sb));
-      if (++sb == SB) { sb = 0; sph ^= 1; }
+      return add2(la, lb);
+    };
+    float l_sum;
+    if constexpr (L::ALT) {
+      // Head_dim 128 and 64: the exponentials of a tile, 1024 cycles of the four units, are as much as its products.  Eight warps on
+      // halves of every tile load, compare and exponentiate in step and the units idle in between (1970 cycles a tile of head_dim 128), as
+      // do eight on whole rows of alternate tiles (1850); so sixteen, eight on every other tile, four per scheduler.  The scores are
+      // read twice, for the maximum and for the weights (40 cycles per 64 columns): 96 registers do.  The reference travels with the tiles.
+      const uint32_t par = wg >> 1;
+      float* s_rm = reinterpret_cast<float*>(base + L::OFF_RM);
+      float m_l = m_st, l = 0.f;       // this thread's share of the row's sum, and the reference it is in
+      for (uint32_t j = par; j < n_tiles; j += 2) {
+        const uint32_t b = j % SB, kv0 = (tile0 + j) * kPN + half * 64, ts = t_s0 + b * kPN + lane_addr + half * 64;
+        mbar_wait(BAR(S_FULL, b), (j / SB) & 1, s_err, WAIT_MMA);
+        tc_fence_after();
+        float s[32], mt = -INFINITY;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          tmem_ld32(ts + c * 32, s);
+          mask(s, 32, kv0 + c * 32);
+          mt = max32(s, mt);
+        }
+        float* mx = s_mx + ((j >> 1) & 1) * (4 * kPM) + par * (2 * kPM);
+        mx[half * kPM + row] = mt;
+        named_bar_sync(2 + par * 4 + qd, 64);
+        mt = fmaxf(mt, mx[(half ^ 1) * kPM + row]);
+        if (j > 0) {
+          mbar_wait(BAR(M_READY, (j - 1) & 1), ((j - 1) >> 1) & 1, s_err, WAIT_MMA);
+          m_st = s_rm[((j - 1) & 1) * kPM + row];
+        }
+        float alpha;
+        const bool grow = refer(j, mt * p.scale_log2, alpha);
+        if (half == 0) s_rm[(j & 1) * kPM + row] = m_st;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(BAR(M_READY, j & 1));      // (both halves have read the one before: its place is free for tile j + 1)
+        if (j > 0 && __any_sync(0xffffffffu, grow)) rescale(j, alpha, half, 2);
+        if (m_st != m_l) { l *= ex2_approx(m_l - m_st); m_l = m_st; }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          tmem_ld32(ts + c * 32, s);
+          mask(s, 32, kv0 + c * 32);
+          uint32_t pw[16];
+          const float2 lt = weigh(s, pw);
+          tmem_st16u(ts + c * 16, pw);
+          l += lt.x + lt.y;
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(BAR(P_FULL, b));
+      }
+      const uint32_t last = n_tiles - 1;
+      mbar_wait(BAR(M_READY, last & 1), (last >> 1) & 1, s_err, WAIT_MMA);
+      m_st = s_rm[(last & 1) * kPM + row];
+      named_bar_sync(1, SOFT);         // the maxima are not read any more
+      s_mx[wg * kPM + row] = l * ex2_approx(m_l - m_st);
+      named_bar_sync(1, SOFT);
+      l_sum = (s_mx[row] + s_mx[kPM + row]) + (s_mx[2 * kPM + row] + s_mx[3 * kPM + row]);
+    } else {
+      float2 l2 = make_float2(0.f, 0.f);       // this thread's share of the row's sum
+      uint32_t sb = 0, sph = 0;
+      for (uint32_t j = 0; j < n_tiles; ++j) {
+        const uint32_t kv0 = (tile0 + j) * kPN + half * 64, ts = t_s0 + sb * kPN + lane_addr + half * 64;
+        mbar_wait(BAR(S_FULL, sb), sph, s_err, WAIT_MMA);
+        tc_fence_after();
+        float s[64];
+        tmem_ld32_async(ts, s);
+        tmem_ld32_async(ts + 32, s + 32);
+        tmem_wait_ld(s);
+        mask(s, 64, kv0);
+        // the two halves' maxima through shared memory
+        const float m_half = max32(s + 32, max32(s, -INFINITY));
+        float* mx = s_mx + (j & 1) * (2 * kPM);
+        mx[wg * kPM + row] = m_half;
+        named_bar_sync(2 + qd, 64);
+        float alpha;
+        if (__any_sync(0xffffffffu, refer(j, fmaxf(m_half, mx[(wg ^ 1) * kPM + row]) * p.scale_log2, alpha))) {
+          l2.x *= alpha; l2.y *= alpha;
+          if (j > 0) rescale(j, alpha, wg, 2);            // half of the dims per warp
+        }
+        uint32_t pw[32];
+        float2 lt = weigh(s, pw);
+        lt = add2(lt, weigh(s + 32, pw + 16));
+        tmem_st32u(ts, pw);
+        l2 = add2(l2, lt);
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(BAR(P_FULL, sb));
+        if (++sb == SB) { sb = 0; sph ^= 1; }
+      }
+      float* s_l = s_mx + ((n_tiles & 1) ? 2 * kPM : 0);   // the slot the last tile's maxima are not in
+      s_l[wg * kPM + row] = l2.x + l2.y;
+      named_bar_sync(1, 256);
+      l_sum = s_l[row] + s_l[kPM + row];
     }
     // ---- epilogue: O / l, gate, store ----
-    float* s_l = s_mx + ((n_tiles & 1) ? 2 * kPM : 0);   // the slot the last tile's maxima are not in
-    s_l[wg * kPM + row] = l2.x + l2.y;
-    named_bar_sync(1, 256);
-    const float l_sum = s_l[row] + s_l[kPM + row];
     mbar_wait(BAR(O_DONE, 0), 0, s_err, WAIT_MMA);
     tc_fence_after();
     const float inv_l = 1.f / l_sum;
@@ -340,14 +414,14 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       static_assert(kPM * RP * 16 <= L::RINGS, "the record tile fits the idle rings");
       float4* xs = reinterpret_cast<float4*>(base + L::OFF_K);
 #pragma unroll 1
-      for (uint32_t c = wg; c < HD / 32; c += 2) {
+      for (uint32_t c = wg; c < HD / 32; c += NGRP) {
         float o[32];
         tmem_ld32(t_o + c * 32 + lane_addr, o);
 #pragma unroll
         for (int i = 0; i < 8; ++i) xs[row * RP + c * 8 + i] = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
       }
-      named_bar_sync(1, 256);
-      for (uint32_t idx = tid - 128; idx < rows_valid * (HD / 4); idx += 256) {
+      named_bar_sync(1, SOFT);
+      for (uint32_t idx = tid - 128; idx < rows_valid * (HD / 4); idx += SOFT) {
         const uint32_t rr = idx / (HD / 4), c4 = idx % (HD / 4);
         const uint64_t slot = ((uint64_t)(c0 + rr) * p.n_heads + h) * p.n_splits + blockIdx.z;
         reinterpret_cast<float4*>(p.part_o + slot * HD)[c4] = xs[rr * RP + c4];
@@ -364,7 +438,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       uint8_t* o_s = base + L::OFF_V;
       if (p.gate) mbar_wait(BAR(G_FULL, 0), 0, s_err, WAIT_QFULL);
 #pragma unroll 1
-      for (uint32_t c = wg; c < HD / 32; c += 2) {            // the halves share the columns out
+      for (uint32_t c = wg; c < HD / 32; c += NGRP) {            // the groups share the columns out
         float o[32];
         tmem_ld32(t_o + c * 32 + lane_addr, o);
 #pragma unroll
@@ -389,7 +463,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
               make_uint4(pack_h2(o[8 * i], o[8 * i + 1]), pack_h2(o[8 * i + 2], o[8 * i + 3]), pack_h2(o[8 * i + 4], o[8 * i + 5]), pack_h2(o[8 * i + 6], o[8 * i + 7]));
       }
       fence_proxy_async();
-      named_bar_sync(1, 256);
+      named_bar_sync(1, SOFT);
       if (tid == 128) {
         tma_store_3d(&tm_o, 0, (int)c0, (int)(h * (HD / 64)), smem_u32(o_s));
         tma_store_wait_read();
@@ -397,23 +471,23 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     } else {
       // f32 activations, or strides no tensor map takes: the rows by way of shared memory, so that gate loads and output stores
       // are whole rows too
-      constexpr int RP = HD / 4 + 1, U = 8;
+      constexpr int RP = HD / 4 + 1, U = L::ALT ? 4 : 8;
       float4* xs = reinterpret_cast<float4*>(base + L::OFF_K);
 #pragma unroll 1
-      for (uint32_t c = wg; c < HD / 32; c += 2) {
+      for (uint32_t c = wg; c < HD / 32; c += NGRP) {
         float o[32];
         tmem_ld32(t_o + c * 32 + lane_addr, o);
 #pragma unroll
         for (int i = 0; i < 8; ++i) xs[row * RP + c * 8 + i] = make_float4(o[4 * i] * inv_l, o[4 * i + 1] * inv_l, o[4 * i + 2] * inv_l, o[4 * i + 3] * inv_l);
       }
-      named_bar_sync(1, 256);
+      named_bar_sync(1, SOFT);
       const bool g_vec = !p.act_f16 && !(((uintptr_t)p.gate & 15) | (p.gate_col_stride & 3) | (p.gate_head_stride & 3));
       const uint32_t n_it = rows_valid * (HD / 4);
-      for (uint32_t i0 = tid - 128; i0 < n_it; i0 += 256 * U) {
+      for (uint32_t i0 = tid - 128; i0 < n_it; i0 += SOFT * U) {
         float gv[U][4];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          const uint32_t idx = i0 + 256 * u, rr = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
+          const uint32_t idx = i0 + SOFT * u, rr = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
           if (!p.gate || idx >= n_it) continue;
           const uint64_t go = (uint64_t)(c0 + rr) * p.gate_col_stride + (uint64_t)h * p.gate_head_stride + d;
           if (g_vec) *reinterpret_cast<float4*>(gv[u]) = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.gate) + go);
@@ -424,7 +498,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          const uint32_t idx = i0 + 256 * u, rr = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
+          const uint32_t idx = i0 + SOFT * u, rr = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
           if (idx >= n_it) continue;
           float4 o = xs[rr * RP + d / 4];
           if (p.gate) {
