@@ -477,6 +477,13 @@ static int ensure_angles(pa_ctx* ctx, uint32_t pos, uint32_t n_cols, cudaStream_
 static bool front_supports(const pa_ctx* ctx, int mode) {
   return (mode == PA_ROPE_F64 || mode == PA_ROPE_NONE) && front_supported(ctx->cfg.head_dim, ctx->cfg.n_rot, mode == PA_ROPE_F64);
 }
+// the rows from pos on that the kernel just launched appends may still be in flight when the next call's kernel starts
+static void rows_in_flight(pa_layer* L, uint32_t pos) {
+  pa_ctx* ctx = L->ctx;
+  uint32_t r0 = pos - L->origin;
+  if (ctx->inflight_layer == L && ctx->inflight_row0 < r0) r0 = ctx->inflight_row0;
+  ctx->inflight_layer = L; ctx->inflight_row0 = r0;
+}
 static int front_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, const void* q, uint64_t qcs, uint64_t qhs, void* q_out, uint64_t q_out_cs,
                       const void* k, const void* v, uint64_t kcs, uint64_t vcs, int mode, int in_f16, bool norm, cudaStream_t st, int q_out_f16 = 0) {
   pa_ctx* ctx = L->ctx;
@@ -503,11 +510,7 @@ static int front_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, 
   }
   CU_TRY(ctx, launch_front(p, ctx->cfg.head_dim, half ? ctx->cfg.n_rot : 0, st));
   ctx->stats.kernel_launches++;
-  if (L->kv_format == PA_KV_F16) {   // as rope_append_impl: the rows that may still be in flight
-    uint32_t r0 = pos - L->origin;
-    if (ctx->inflight_layer == L && ctx->inflight_row0 < r0) r0 = ctx->inflight_row0;
-    ctx->inflight_layer = L; ctx->inflight_row0 = r0;
-  }
+  if (L->kv_format == PA_KV_F16) rows_in_flight(L, pos);
   return PA_OK;
 }
 
@@ -522,7 +525,7 @@ static int rope_append_impl(pa_layer* L, pa_ctx* ctx, uint32_t seq, uint32_t pos
     if (n_cols > ctx->cfg.max_cols) return fail(ctx, PA_EINVAL, "rope: %u columns exceed max_cols %u", n_cols, ctx->cfg.max_cols);
     if (k && v && front_supports(ctx, mode)) {
       if (int rc = front_impl(L, seq, pos, n_cols, q, qcs, qhs, q_out, q_out_cs, k, v, kvcs, vcs ? vcs : kvcs, mode, in_f16, false, st, q_out_f16)) return rc;
-      ctx->inflight_layer = nullptr;
+      rows_in_flight(L, pos);
       return PA_OK;
     }
     if (q)
@@ -542,7 +545,7 @@ static int rope_append_impl(pa_layer* L, pa_ctx* ctx, uint32_t seq, uint32_t pos
     }
     CU_TRY(ctx, launch_kv_store(sp, n_cols, st));
     ctx->stats.kernel_launches++;
-    ctx->inflight_layer = nullptr;
+    rows_in_flight(L, pos);
     return PA_OK;
   }
   RopeParams p{};
@@ -572,11 +575,7 @@ static int rope_append_impl(pa_layer* L, pa_ctx* ctx, uint32_t seq, uint32_t pos
   }
   CU_TRY(ctx, launch_rope_append(p, n_cols, st));
   ctx->stats.kernel_launches++;
-  if (L && k) {
-    uint32_t r0 = pos - L->origin;
-    if (ctx->inflight_layer == L && ctx->inflight_row0 < r0) r0 = ctx->inflight_row0;
-    ctx->inflight_layer = L; ctx->inflight_row0 = r0;
-  }
+  if (L && k) rows_in_flight(L, pos);
   return PA_OK;
 }
 
@@ -786,7 +785,8 @@ static bool f32_eight_do(const pa_ctx* ctx, uint32_t rows, uint32_t nc, uint32_t
 // Decode / verify / prefill over an int8 or f32 cache.  Int8: decode_q8_item per item.  F32: per item, blocks of columns small
 // enough for the record buffers, each one launch (a CTA per (split, kv head, column)), and a combine unless a cluster merges.
 static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, const void* q, int q_dtype, uint64_t qcs, uint64_t qhs, const void* gate,
-                           uint64_t gcs, uint64_t ghs, void* out, uint64_t ocs, cudaStream_t st, const char* who, bool after_front = false) {
+                           uint64_t gcs, uint64_t ghs, void* out, uint64_t ocs, cudaStream_t st, const char* who, bool after_front = false,
+                           const FusedFront* fz = nullptr) {   // fz: one token over f32 rows (decode_f32_direct) whose front is the kernel's
   pa_ctx* ctx = L->ctx;
   if (!q || !out) return fail(ctx, PA_EINVAL, "%s: null q or output", who);
   if (!items || n_items < 1) return fail(ctx, PA_EINVAL, "%s: no items", who);
@@ -830,6 +830,11 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
         f.kv_dim = ctx->kv_dim; f.n_heads = nH; f.max_seq = L->max_seq; f.n_splits = ns;
         f.seq = items[i].seq; f.lim0 = lim0; f.n_rows = rows; f.n_cols = nc;
         f.early = after_front && c0 == 0 ? 1u : 0u;   // (a later block of a wide call follows a merge, not the front)
+        if (fz) {
+          f.k_new = fz->k; f.v_new = fz->v; f.half = ctx->cfg.n_rot / 2; f.early = 1;
+          f.early_limit = ctx->inflight_layer == L ? ctx->inflight_row0 : 0xffffffffu;
+          memcpy(f.ang, host_angles(ctx, fz->pos, 1), (size_t)f.half * sizeof(Angle));
+        }
         f.scale_log2 = (float)(1.4426950408889634 / sqrt((double)hd));
         f.part_o = ctx->part_o; f.part_ml = ctx->part_ml;
         timing_mark(ctx, st, 0);
@@ -864,7 +869,8 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
     col += items[i].n_cols;
   }
   ctx->stats.calls++;
-  ctx->inflight_layer = nullptr;
+  ctx->inflight_layer = fz ? L : nullptr;      // the kernel's own row may still be in flight
+  if (fz) ctx->inflight_row0 = fz->pos - L->origin;
   return PA_OK;
 }
 
@@ -1288,6 +1294,13 @@ static int layer_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols, 
   if (L->kv_format != PA_KV_F16) {
     if (sharded) return fail(ctx, PA_EUNSUPPORTED, "pa_attn_layer_sharded: the peer exchange is for f16 caches");
     if (n_cols > ctx->cfg.max_cols) return fail(ctx, PA_EINVAL, "pa_attn_layer: %u columns exceed max_cols %u", n_cols, ctx->cfg.max_cols);
+    // one token over f32 rows: the front is the attention kernel's
+    if (L->kv_format == PA_KV_F32 && alt_front && n_cols == 1 && ctx->cfg.rope_mode == PA_ROPE_F64 && !L->qnorm_w && decode_f32_direct(ctx->G) && !ctx->core_only &&
+        !ctx->tune.no_fuse) {
+      pa_item it{seq, pos, 1, 0};
+      const FusedFront fz{k, v, 1u, pos};
+      return decode_any_impl(L, &it, 1, q, (int)ctx->cfg.act_dtype, qcs, qhs, gate, gcs, ghs, out, ocs, st, "pa_attn_layer", false, &fz);
+    }
     if (!ctx->core_only) {
       const int rc = alt_front ? front_impl(L, seq, pos, n_cols, q, qcs, qhs, ctx->q_rot, ctx->q_dim, k, v, kvcs, kvcs, ctx->cfg.rope_mode,
                                             ctx->cfg.act_dtype == PA_F16, L->qnorm_w != nullptr, st)

@@ -201,9 +201,14 @@ size_t any_decode_smem(uint32_t G, uint32_t hd) {
 // 64: 32, 256: 8; with four heads half of that) rows together, 128 registers a thread, before it uses the first: 128 KB
 // in flight per SM, which is what HBM's latency takes at full rate.  No barrier and no shared memory until the warps' (o, m, l) are merged at the end.  A CTA's
 // rows are one or two such batches per warp at the contexts these caches serve.  28 layers of a token over 2000 rows (16 q / 8 kv
-// heads x 128), whole calls with the one-launch front: 644 us with the chunked kernel above, 257 us with this one (floor 70: 459 MB).
+// heads x 128), whole calls: 644 us with the chunked kernel above and a front kernel, 257 us with this one and a front kernel, 218 us with
+// the front in this one (floor 70: 459 MB).
+//
+// FU: one token whose front the kernel makes itself, as pa_decode_kernel does: the 256 threads rotate the G query rows (rot_exact,
+// host cos / sin) into shared memory; the CTA of the sequence's last rows also rotates k, stores the row, and takes it from shared
+// memory, not from the cache, into its own sums.  As a kernel of its own ahead of this one the front was 3 us of a layer's 9.2.
 constexpr int f32_batch(int hd, int G) { return 512 / hd * (G == 4 ? 2 : 4); }
-template <int HD, int G>
+template <int HD, int G, bool FU>
 __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodeParams p) {
   constexpr int LPR = HD / 16, RPI = 32 / LPR, BATCH = f32_batch(HD, G), U = BATCH / RPI;   // lanes per row, rows per instruction and per batch
   extern __shared__ float sm[];                                             // [8 warps][G][HD], then m[8][G], l[8][G]
@@ -228,11 +233,49 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
   };
   uint32_t b0 = r_lo + warp * BATCH;
   // rows the kernel before this one does not write may be fetched while it runs
-  const bool ahead = p.early && b0 + BATCH <= p.n_rows - min(p.n_rows, p.n_cols);
+  const bool ahead = p.early && b0 + BATCH <= min(p.n_rows - min(p.n_rows, p.n_cols), FU ? p.early_limit : 0xffffffffu);
   if (ahead && b0 < r_hi) load(b0);
+  __shared__ Angle s_ang[FU ? 64 : 1];
+  __shared__ __align__(16) float s_new[FU ? G + 2 : 1][HD];     // the rotated query rows, the token's own k and v
+  if constexpr (FU) {      // (launch parameters indexed per thread are served one address at a time: staged while the predecessor runs)
+    if ((uint32_t)tid < 2 * p.half) reinterpret_cast<uint4*>(s_ang)[tid] = reinterpret_cast<const uint4*>(p.ang)[tid];
+    __syncthreads();
+  }
   pdl_wait();
   pdl_trigger();
-  if (!ahead && b0 < r_hi) load(b0);
+  const bool own = FU && r_hi == p.n_rows && r_lo < r_hi;
+  if constexpr (FU) {
+    constexpr uint32_t P = HD / 2, TURNS = ((G + 2) * P + 255) / 256;
+    const uint32_t n_it = (own ? G + 2 : G) * P;
+    float a[TURNS], b[TURNS];
+    auto dims = [&](uint32_t pr, uint32_t& d0, uint32_t& d1) { d0 = pr < p.half ? pr : 2 * pr; d1 = pr < p.half ? pr + p.half : d0 + 1; };
+#pragma unroll
+    for (uint32_t t = 0; t < TURNS; ++t) {
+      const uint32_t it = tid + 256 * t, hh = it / P;
+      if (it >= n_it) continue;
+      uint32_t d0, d1;
+      dims(it % P, d0, d1);
+      const void* src = hh < G ? p.q : hh == G ? p.k_new : p.v_new;
+      const uint64_t so = hh < G ? (uint64_t)(g * G + hh) * p.q_head_stride : (uint64_t)g * HD;
+      a[t] = ld_act(src, so + d0, p.q_f16); b[t] = ld_act(src, so + d1, p.q_f16);
+    }
+    if (!ahead && b0 < r_hi) load(b0);
+#pragma unroll
+    for (uint32_t t = 0; t < TURNS; ++t) {
+      const uint32_t it = tid + 256 * t, hh = it / P, pr = it % P;
+      if (it >= n_it) continue;
+      uint32_t d0, d1;
+      dims(pr, d0, d1);
+      float x = a[t], y = b[t];
+      if (hh <= G && pr < p.half) { x = rot_exact(a[t], b[t], s_ang[pr], true); y = rot_exact(b[t], a[t], s_ang[pr], false); }
+      s_new[hh][d0] = x; s_new[hh][d1] = y;
+      if (hh >= G) {
+        float* dst = const_cast<float*>(hh == G ? p.k : p.v) + ((uint64_t)p.seq * p.max_seq + p.n_rows - 1) * p.kv_dim + (uint64_t)g * HD;
+        dst[d0] = x; dst[d1] = y;
+      }
+    }
+    __syncthreads();
+  } else if (!ahead && b0 < r_hi) load(b0);
   const uint64_t col = c;
   float4 q[G][4];
 #pragma unroll
@@ -240,7 +283,8 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const uint64_t off = col * p.q_col_stride + (uint64_t)(g * G + h) * p.q_head_stride + i * LPR * 4 + lr * 4;
-      if (p.q_vec) q[h][i] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.q) + off);
+      if constexpr (FU) q[h][i] = *reinterpret_cast<const float4*>(&s_new[h][i * LPR * 4 + lr * 4]);
+      else if (p.q_vec) q[h][i] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.q) + off);
       else q[h][i] = make_float4(ld_act(p.q, off, p.q_f16), ld_act(p.q, off + 1, p.q_f16), ld_act(p.q, off + 2, p.q_f16), ld_act(p.q, off + 3, p.q_f16));
     }
   float m[G], l[G];
@@ -252,6 +296,17 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
     for (int i = 0; i < 4; ++i) o[h][i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   while (b0 < r_hi) {
+    if (FU && own) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (b0 + u * RPI + sub == p.n_rows - 1) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            k[u][i] = *reinterpret_cast<const float4*>(&s_new[FU ? G : 0][i * LPR * 4 + lr * 4]);
+            v[u][i] = *reinterpret_cast<const float4*>(&s_new[FU ? G + 1 : 0][i * LPR * 4 + lr * 4]);
+          }
+        }
+    }
 #pragma unroll
     for (int h = 0; h < G; ++h) {
       float s[U], mx = m[h];
@@ -342,11 +397,15 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
   cluster_sync();            // no CTA leaves while another reads its rows
 }
 
+template <int HD, int G, bool FU>
+static cudaError_t launch_f32_fu(const F32DecodeParams& p, dim3 grid, cudaStream_t st) {
+  const size_t smem = (size_t)(9 * G * (HD + 2)) * 4;       // (at most 37 KB)
+  if (p.cluster) return launch_pdl_cluster(pa_decode_f32_kernel<HD, G, FU>, grid, dim3(256), smem, st, p.cluster, p);
+  return launch_pdl(pa_decode_f32_kernel<HD, G, FU>, grid, dim3(256), smem, st, p);
+}
 template <int HD, int G>
 static cudaError_t launch_f32_t(const F32DecodeParams& p, dim3 grid, cudaStream_t st) {
-  const size_t smem = (size_t)(9 * G * (HD + 2)) * 4;       // (at most 37 KB)
-  if (p.cluster) return launch_pdl_cluster(pa_decode_f32_kernel<HD, G>, grid, dim3(256), smem, st, p.cluster, p);
-  return launch_pdl(pa_decode_f32_kernel<HD, G>, grid, dim3(256), smem, st, p);
+  return p.k_new ? launch_f32_fu<HD, G, true>(p, grid, st) : launch_f32_fu<HD, G, false>(p, grid, st);
 }
 bool decode_f32_direct(uint32_t G) { return G == 1 || G == 2 || G == 4; }
 uint32_t decode_f32_batch(uint32_t hd, uint32_t G) { return (uint32_t)f32_batch((int)hd, (int)G); }

@@ -144,6 +144,9 @@ struct F32DecodeParams {
   float* part_o; float* part_ml;
   const void* gate; uint64_t gate_col_stride, gate_head_stride;                // cluster: gate and output
   void* out; uint64_t out_col_stride; int act_f16;
+  // one token with its front in the kernel (k_new != nullptr): q unrotated, the token's own k / v row in q's type, cos / sin by value
+  const void* k_new; const void* v_new; uint32_t half; uint32_t early_limit;   // early_limit: rows the call before may still be writing
+  Angle ang[64];
 };
 
 // the front of a layer call in one launch (pa_front_kernel): head-norm, rotation, append in the cache's format
