@@ -178,7 +178,6 @@ extern "C" int pa_create(int device, const pa_config* cfg, pa_ctx** out) {
   if (const char* e = getenv("POOLED_ATTN_XCH_PREFETCH")) ctx->tune.xch_prefetch = atoi(e);
   if (const char* e = getenv("POOLED_ATTN_KV_EVICT_FIRST")) ctx->tune.kv_evict_first = atoi(e) != 0;
   if (const char* e = getenv("POOLED_ATTN_NO_Q_TMA")) ctx->tune.no_q_tma = atoi(e) != 0;
-  if (const char* e = getenv("POOLED_ATTN_OLD_TAIL")) ctx->tune.old_tail = atoi(e) != 0;
   if (const char* e = getenv("POOLED_ATTN_NO_OUT_TMA")) ctx->tune.no_out_tma = atoi(e) != 0;
   auto bail = [&](int code, const char* what, cudaError_t e) {
     std::string msg = std::string("pa_create: ") + what + ": " + cudaGetErrorString(e);
@@ -204,9 +203,9 @@ extern "C" int pa_create(int device, const pa_config* cfg, pa_ctx** out) {
   ctx->pf_slots = std::max<size_t>(ctx->part_slots, std::min<size_t>(32768, (size_t)cfg->max_cols * cfg->n_heads * kPrefillSplits));
   if ((e = cudaMalloc(&ctx->part_o, ctx->pf_slots * cfg->head_dim * 4)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(part_o)", e);
   if ((e = cudaMalloc(&ctx->part_ml, ctx->pf_slots * 2 * 4)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(part_ml)", e);
-  ctx->merge_slots = 2u * kMaxItems * cfg->n_kv_heads;
-  if ((e = cudaMalloc(&ctx->merge_ctr, ctx->merge_slots * 4)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(merge counters)", e);
-  if ((e = cudaMemset(ctx->merge_ctr, 0, ctx->merge_slots * 4)) != cudaSuccess) return bail(PA_ECUDA, "cudaMemset(merge counters)", e);
+  ctx->merge_bytes = (size_t)ctx->sm_count * 16 * (cfg->head_dim + cfg->head_dim / 32) * 4;   // one CTA per SM, at most 16 query rows each
+  if ((e = cudaMalloc(&ctx->merge_rec, ctx->merge_bytes)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(merge records)", e);
+  if ((e = cudaMemset(ctx->merge_rec, 0xff, ctx->merge_bytes)) != cudaSuccess) return bail(PA_ECUDA, "cudaMemset(merge records)", e);
   if ((e = cudaMalloc(&ctx->dev_err, 4)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(err)", e);
   if ((e = cudaMemset(ctx->dev_err, 0, 4)) != cudaSuccess) return bail(PA_ECUDA, "cudaMemset(err)", e);
   if ((e = cudaMallocHost(&ctx->host_err, 4)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMallocHost(err)", e);
@@ -218,7 +217,7 @@ extern "C" int pa_create(int device, const pa_config* cfg, pa_ctx** out) {
 extern "C" int pa_destroy(pa_ctx* ctx) {
   if (!ctx) return PA_OK;
   cudaSetDevice(ctx->device);
-  cudaFree(ctx->inv_freq); cudaFree(ctx->angles); cudaFree(ctx->norm_q); cudaFree(ctx->norm_k); cudaFree(ctx->q_rot); cudaFree(ctx->k_rot); cudaFree(ctx->part_o); cudaFree(ctx->part_ml); cudaFree(ctx->dev_err); cudaFree(ctx->merge_ctr);
+  cudaFree(ctx->inv_freq); cudaFree(ctx->angles); cudaFree(ctx->norm_q); cudaFree(ctx->norm_k); cudaFree(ctx->q_rot); cudaFree(ctx->k_rot); cudaFree(ctx->part_o); cudaFree(ctx->part_ml); cudaFree(ctx->dev_err); cudaFree(ctx->merge_rec);
   cudaFree(ctx->stage_dev);
   for (cudaEvent_t e : ctx->ev) cudaEventDestroy(e);
   if (ctx->host_err) cudaFreeHost(ctx->host_err);
@@ -337,7 +336,7 @@ extern "C" int pa_reset(pa_ctx* ctx) {
   if (!ctx) return PA_EINVAL;
   cudaGetLastError();
   if (cudaDeviceSynchronize() != cudaSuccess || cudaMemset(ctx->dev_err, 0, 4) != cudaSuccess ||
-      cudaMemset(ctx->merge_ctr, 0, ctx->merge_slots * 4) != cudaSuccess)
+      cudaMemset(ctx->merge_rec, 0xff, ctx->merge_bytes) != cudaSuccess)
     return fail(ctx, PA_ECUDA, "pa_reset: the device does not answer");
   *ctx->host_err = 0;
   ctx->failed = false;
@@ -1013,7 +1012,7 @@ static int decode_impl(pa_layer* L, const pa_item* items, uint32_t n_items, cons
                        ns <= (uint32_t)kMaxCluster;
   if (cluster) while (ns & (ns - 1)) ++ns;      // 1, 2, 4 or 8 CTAs (those without a tile leave at once); the plan is p.n_splits'
   if (merge || cluster) {
-    p.merge = cluster ? 3u : ctx->tune.old_tail ? 1u : 2u; p.merge_ctr = ctx->merge_ctr;
+    p.merge = cluster ? 3u : 2u; p.merge_rec = ctx->merge_rec;
     p.gate = gate; p.gate_col_stride = gcs; p.gate_head_stride = ghs; p.out = out; p.out_col_stride = ocs; p.act_f16 = ctx->cfg.act_dtype == PA_F16;
   }
   // an exchanging call numbers itself ahead of its combine kernel: in the decode kernel where that runs

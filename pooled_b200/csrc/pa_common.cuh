@@ -393,8 +393,8 @@ struct pa_ctx {
   uint32_t max_splits = 0;
   size_t part_slots = 0;       // (query row, split) records a decode / verify call may use
   size_t pf_slots = 0;         // records the partial buffers hold, and a split prefill may use
-  unsigned int* merge_ctr = nullptr;   // device: per (item, kv head) of a decode call, records left and CTAs done merging (zero between calls)
-  uint32_t merge_slots = 0;
+  float* merge_rec = nullptr;    // device: the records of a decode call that merges them itself, a block per CTA; all bits set between calls
+  size_t merge_bytes = 0;
   uint32_t* dev_err = nullptr;   // device error word (bounded waits)
   uint32_t* host_err = nullptr;  // pinned mirror
   void* norm_q = nullptr;        // normed q / k of the current layer call (act_dtype, [max_cols][q_dim] / [max_cols][kv_dim])
@@ -416,7 +416,6 @@ struct pa_ctx {
     int own_prefetch = 0;        // POOLED_ATTN_OWN_PREFETCH=n: L2 requests for n of a decode CTA's own later tiles at entry
     int xch_prefetch = 0;        // POOLED_ATTN_XCH_PREFETCH=n: the same for calls that end in a cross-GPU exchange
     bool no_q_tma = false;       // POOLED_ATTN_NO_Q_TMA=1: the prefill kernel's query rows through the softmax threads' registers
-    bool old_tail = false;       // POOLED_ATTN_OLD_TAIL=1: in-kernel merge with every CTA waiting for the records (unit-less ones too)
     bool no_out_tma = false;     // POOLED_ATTN_NO_OUT_TMA=1: ... and its output rows by per-thread stores
     bool kv_evict_first = true;  // POOLED_ATTN_KV_EVICT_FIRST=0: decode / verify K and V tiles enter L2 with the default policy instead of evict-first
     bool no_merge = false;       // POOLED_ATTN_NO_MERGE: always merge the split records in the combine kernel

@@ -150,32 +150,68 @@ __device__ __forceinline__ void exchange_slice(const ExchangeView& x, uint32_t p
   }
 }
 
+// Records that the CTAs of one call leave for one another say themselves when they are there: every 32-bit word of the buffer holds
+// kNoWord until its value is stored, a reader repeats its loads until no word of them does, and puts kNoWord back for the next call
+// (whose CTAs write after this call's end).  A 32-bit word lands whole, so nothing else orders the two sides: with a fence behind
+// the records, a count and a wait for it ahead of the first load, three more trips to L2 stood between a CTA's last product and its merge
+// (ten layers of a token over 32768 rows, 16 / 2 heads x 256, 200 us so and 185 now; 16 over 4099 rows, 24 / 4 x 256, host buffers, 235 and 209).  A value that has kNoWord's bits (a NaN no instruction here produces) is stored as the ordinary NaN.
+constexpr uint32_t kNoWord = 0xffffffffu;
+__device__ __forceinline__ float word_for(float x) { return __float_as_uint(x) == kNoWord ? __uint_as_float(0x7fffffffu) : x; }
+__device__ __forceinline__ uint4 ld_words4(const float* p) {
+  uint4 v;
+  asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 ld_words2(const float* p) {
+  uint2 v;
+  asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ bool all_words(const uint4& v) { return v.x != kNoWord && v.y != kNoWord && v.z != kNoWord && v.w != kNoWord; }
+__device__ __forceinline__ float4 as_float4(const uint4& v) { return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)); }
+constexpr uint32_t kMergePolls = 1u << 20;
+
 // LSE merge of the ns split records of one query row over one 64-dim slice, gate and store, by the 128 consumer threads
 // of a decode CTA: the arithmetic of pa_combine_kernel, operation for operation and in the same order (that kernel has
 // 256 threads; thread t here does the work of its threads t and t + 128), so a call gives the same bits whether its
-// records are merged here or there.  o_rec / ml_rec: record 0 of the row; records follow one another.  Scratch: 6 KB of
-// shared memory no one else uses any more.  bar: the group's named barrier.
+// records are merged here or there.  o_rec / ml_rec: the slice of record 0 of the row; records lie `stride` floats apart.  Scratch:
+// 6 KB of shared memory no one else uses any more.  bar: the group's named barrier.
 struct MergeScratch { float w[512]; float red[8]; float red2[8]; float4 acc[16][16]; };
 template <int HD>
-__device__ __forceinline__ void merge_slice_128(const float* __restrict__ o_rec, const float* __restrict__ ml_rec, uint32_t ns, uint32_t slice, int t,
-                                                MergeScratch& sc, uint32_t bar, bool gated, float gv, bool empty_is_zero, int act_f16, void* out, uint64_t oo) {
+__device__ __forceinline__ void merge_slice_128(float* o_rec, float* ml_rec, size_t stride, uint32_t ns, int t, MergeScratch& sc, uint32_t bar, bool gated,
+                                                float gv, bool empty_is_zero, int act_f16, void* out, uint64_t oo, volatile uint32_t* s_err) {
   const int wv = t >> 5, lane = t & 31, ln = t & 15, gA = t >> 4;
-  // everything is requested before the first use: one memory round trip
+  float* ob = o_rec + ln * 4;
+  const uint4 none = make_uint4(kNoWord, kNoWord, kNoWord, kNoWord);
+  // everything is requested before the first use, and whatever was not there yet once more
+  uint4 xw[16];          // records gA + 8 i of this thread's four dims
+  uint2 mw[4];
+  uint32_t want = 0;     // bits 0-15: xw, 16-19: mw
+#pragma unroll
+  for (int i = 0; i < 16; ++i) { xw[i] = make_uint4(0, 0, 0, 0); want |= (gA + 8u * i < ns ? 1u : 0u) << i; }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) { mw[k] = make_uint2(__float_as_uint(-3.0e38f), 0u); want |= (t + 128u * k < ns ? 1u : 0u) << (16 + k); }
+  const uint32_t mine = want;
+  for (uint32_t polls = 0; want && !*s_err; ++polls) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) if ((want >> (16 + k)) & 1u) mw[k] = ld_words2(ml_rec + (size_t)(t + 128 * k) * stride);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) if ((want >> i) & 1u) xw[i] = ld_words4(ob + (size_t)(gA + 8 * i) * stride);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) if (((want >> (16 + k)) & 1u) && mw[k].x != kNoWord && mw[k].y != kNoWord) want &= ~(1u << (16 + k));
+#pragma unroll
+    for (int i = 0; i < 16; ++i) if (((want >> i) & 1u) && all_words(xw[i])) want &= ~(1u << i);
+    if (polls > kMergePolls) *s_err = WAIT_MERGE;
+    if (want && polls > 16) __nanosleep(32);
+  }
   float mv[4], lv[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const uint32_t s = t + 128 * k;
-    mv[k] = -3.0e38f; lv[k] = 0.f;
-    if (s < ns) { mv[k] = __ldcg(ml_rec + 2 * s); lv[k] = __ldcg(ml_rec + 2 * s + 1); }
+    mv[k] = __uint_as_float(mw[k].x); lv[k] = __uint_as_float(mw[k].y);
+    if ((mine >> (16 + k)) & 1u) *reinterpret_cast<uint2*>(ml_rec + (size_t)(t + 128 * k) * stride) = make_uint2(kNoWord, kNoWord);
   }
-  const float* ob = o_rec + slice * 64 + ln * 4;
-  float4 xa[8], xb[8];
 #pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    const uint32_t sa = gA + 16 * u, sb = gA + 8 + 16 * u;
-    xa[u] = sa < ns ? __ldcg(reinterpret_cast<const float4*>(ob + (size_t)sa * HD)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    xb[u] = sb < ns ? __ldcg(reinterpret_cast<const float4*>(ob + (size_t)sb * HD)) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+  for (int i = 0; i < 16; ++i) if ((mine >> i) & 1u) *reinterpret_cast<uint4*>(ob + (size_t)(gA + 8 * i) * stride) = none;
   float M = fmaxf(fmaxf(mv[0], mv[1]), fmaxf(mv[2], mv[3]));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
@@ -205,23 +241,27 @@ __device__ __forceinline__ void merge_slice_128(const float* __restrict__ o_rec,
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     const uint32_t sa = gA + 16 * u, sb = gA + 8 + 16 * u;
-    fma4(accA, xa[u], sa < ns ? sc.w[sa] : 0.f);
-    fma4(accB, xb[u], sb < ns ? sc.w[sb] : 0.f);
+    fma4(accA, as_float4(xw[2 * u]), sa < ns ? sc.w[sa] : 0.f);
+    fma4(accB, as_float4(xw[2 * u + 1]), sb < ns ? sc.w[sb] : 0.f);
   }
   for (int h = 0; h < 2; ++h) {
     const uint32_t g = gA + 8 * h;
     float4& acc = h ? accB : accA;
     for (uint32_t s0 = g + 128; s0 < ns; s0 += 64) {
-      float4 x[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const uint32_t s = s0 + 16 * u;
-        x[u] = s < ns ? __ldcg(reinterpret_cast<const float4*>(ob + (size_t)s * HD)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t s = s0 + 16 * u;
-        fma4(acc, x[u], s < ns ? sc.w[s] : 0.f);
+        uint4 x = make_uint4(0, 0, 0, 0);
+        if (s < ns) {
+          for (uint32_t polls = 0; !*s_err; ++polls) {
+            x = ld_words4(ob + (size_t)s * stride);
+            if (all_words(x)) break;
+            if (polls > kMergePolls) *s_err = WAIT_MERGE;
+            if (polls > 16) __nanosleep(32);
+          }
+          *reinterpret_cast<uint4*>(ob + (size_t)s * stride) = none;
+        }
+        fma4(acc, as_float4(x), s < ns ? sc.w[s] : 0.f);
       }
     }
   }
@@ -1162,32 +1202,45 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     cluster_sync();                                // no CTA leaves while another reads its rows
     if (*s_err && tid == 0) atomicMax(p.err, *s_err);
   } else {
-  for (uint32_t idx = ltid; idx < live_rows * (HD / 4); idx += kConsumers) {
-    const uint32_t row = idx / (HD / 4), c4 = idx % (HD / 4);
-    const uint32_t c = row / G, hh = row % G;
-    const uint64_t prow = (uint64_t)(p.items.col0[item] + c) * p.n_heads + g * G + hh;
-    const uint64_t slot = prow * p.n_splits + split;
-    reinterpret_cast<float4*>(p.part_o + slot * HD)[c4] = reinterpret_cast<const float4*>(xo + row * HD)[c4];
-    if (c4 == 0) {
-      p.part_ml[slot * 2] = xml_out[row * 2] * 0.6931471805599453f;
-      p.part_ml[slot * 2 + 1] = xml_out[row * 2 + 1];
+  if (!p.merge) {
+    for (uint32_t idx = ltid; idx < live_rows * (HD / 4); idx += kConsumers) {
+      const uint32_t row = idx / (HD / 4), c4 = idx % (HD / 4);
+      const uint32_t c = row / G, hh = row % G;
+      const uint64_t prow = (uint64_t)(p.items.col0[item] + c) * p.n_heads + g * G + hh;
+      const uint64_t slot = prow * p.n_splits + split;
+      reinterpret_cast<float4*>(p.part_o + slot * HD)[c4] = reinterpret_cast<const float4*>(xo + row * HD)[c4];
+      if (c4 == 0) {
+        p.part_ml[slot * 2] = xml_out[row * 2] * 0.6931471805599453f;
+        p.part_ml[slot * 2 + 1] = xml_out[row * 2 + 1];
+      }
     }
   }
   if constexpr (NT <= 2) if (p.merge) {
-    // ---- one kernel per call: when every CTA of this (item, kv head) has left its record, the CTAs share out the
-    //      merge: (query row, 64-dim slice) units, dealt round-robin; LSE merge, gate and store as pa_combine_kernel does.
+    // ---- one kernel per call: the CTAs of this (item, kv head) leave their records for one another (see kNoWord) and share out
+    //      the merge: (query row, 64-dim slice) units, dealt round-robin; LSE merge, gate and store as pa_combine_kernel does.
     //      All CTAs of the launch are resident together (the host checks that the grid fits the GPU in one wave), so
-    //      the wait below is for CTAs that are running; it is bounded all the same. ----
+    //      the wait is for CTAs that are running; it is bounded all the same.  A CTA without a unit leaves at once. ----
     const uint32_t ns_live = (tiles + tps - 1) / tps;             // CTAs of this (item, kv head) that hold tiles
     const uint32_t n_units = live_rows * (HD / 64);
-    unsigned int* ctr = p.merge_ctr + 2 * ((size_t)item * gridDim.y + g);   // [0] records left, [1] CTAs done merging
+    // a CTA's block: o [ROWS][HD], then (m, l) once for each 64-dim slice, [ROWS][HD / 64][2]
+    constexpr size_t BLK = (size_t)ROWS * (HD + HD / 32);
+    float* const blk0 = p.merge_rec + ((size_t)item * gridDim.y + g) * p.n_splits * BLK;
+    {
+      float* mine = blk0 + split * BLK;
+      for (uint32_t idx = ltid; idx < live_rows * (HD / 4); idx += kConsumers) {
+        const uint32_t row = idx / (HD / 4), c4 = idx % (HD / 4);
+        const float4 x = reinterpret_cast<const float4*>(xo + row * HD)[c4];
+        if (c4 % 16 == 0)
+          *reinterpret_cast<float2*>(mine + ROWS * HD + (row * (HD / 64) + c4 / 16) * 2) = make_float2(word_for(xml_out[row * 2] * 0.6931471805599453f), word_for(xml_out[row * 2 + 1]));
+        reinterpret_cast<float4*>(mine + row * HD)[c4] = make_float4(word_for(x.x), word_for(x.y), word_for(x.z), word_for(x.w));
+      }
+    }
     // the gate value of this CTA's first unit is requested now and has landed by the time the records may be read
     float gv0 = 0.f;
     const bool gated = p.gate != nullptr;
-    auto unit_addr = [&](uint32_t u, uint64_t& prow, uint32_t& slice, uint64_t& go, uint64_t& oo) {
+    auto unit_addr = [&](uint32_t u, uint32_t& slice, uint64_t& go, uint64_t& oo) {
       const uint32_t row = u / (HD / 64); slice = u % (HD / 64);
       const uint32_t c = row / G, hh = row % G, col = p.items.col0[item] + c, h = g * G + hh;
-      prow = (uint64_t)col * p.n_heads + h;
       go = (uint64_t)col * p.gate_col_stride + (uint64_t)h * p.gate_head_stride + slice * 64;
       oo = (uint64_t)col * p.out_col_stride + (uint64_t)h * HD + slice * 64;
     };
@@ -1195,40 +1248,20 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       return p.act_f16 ? __half2float(reinterpret_cast<const __half*>(p.gate)[go + ltid]) : reinterpret_cast<const float*>(p.gate)[go + ltid];
     };
     if (split < n_units && gated && ltid < 64) {
-      uint64_t prow, go, oo; uint32_t slice;
-      unit_addr(split, prow, slice, go, oo);
+      uint64_t go, oo; uint32_t slice;
+      unit_addr(split, slice, go, oo);
       gv0 = gate_ld(go);
     }
-    // A CTA that holds no merge unit counts itself in and leaves at once: its SM is free for the next kernel's CTA
-    // (p.merge == 1: every CTA waits for the records, for comparison).  The fence stays in every thread: a single one
-    // in the counting thread behind the barrier measured slower.
-    const bool has_units = split < n_units || p.merge == 1;
-    __threadfence();                       // this thread's record stores, device-wide
-    named_bar_sync(gbar, kConsumers);
-    if (ltid == 0) {
-      atomicAdd(ctr, 1u);
-      if (has_units) {
-        uint32_t polls = 0;
-        while (*reinterpret_cast<volatile unsigned int*>(ctr) < ns_live && !*s_err) {
-          if (++polls > (1u << 20)) { *s_err = WAIT_MERGE; break; }
-          if (polls > 8) __nanosleep(64);
-        }
-        __threadfence();
-      }
-    }
-    if (has_units) named_bar_sync(gbar, kConsumers);
+    named_bar_sync(gbar, kConsumers);     // every thread has read its rows: the scratch takes their place
     MergeScratch& sc = *reinterpret_cast<MergeScratch*>(k_slots);   // the ring is idle: every tile has been consumed
-    if (!*s_err) {
-      for (uint32_t u = split; u < n_units; u += ns_live) {
-        uint64_t prow, go, oo; uint32_t slice;
-        unit_addr(u, prow, slice, go, oo);
-        const float gv = (u == split) ? gv0 : ((gated && ltid < 64) ? gate_ld(go) : 0.f);
-        const uint64_t rec0 = prow * p.n_splits;
-        merge_slice_128<HD>(p.part_o + rec0 * HD, p.part_ml + rec0 * 2, ns_live, slice, ltid, sc, gbar, gated, gv, p.gather != nullptr, p.act_f16, p.out, oo);
-      }
+    for (uint32_t u = split; u < n_units; u += ns_live) {
+      uint64_t go, oo; uint32_t slice;
+      unit_addr(u, slice, go, oo);
+      const float gv = (u == split) ? gv0 : ((gated && ltid < 64) ? gate_ld(go) : 0.f);
+      const uint32_t row = u / (HD / 64);
+      merge_slice_128<HD>(blk0 + (size_t)row * HD + slice * 64, blk0 + ROWS * HD + (row * (HD / 64) + slice) * 2, BLK, ns_live, ltid, sc, gbar, gated, gv,
+                          p.gather != nullptr, p.act_f16, p.out, oo, s_err);
     }
-    // the last CTA to finish clears the counters for the next call (every other CTA is past its wait by then)
-    if (ltid == 0 && atomicAdd(ctr + 1, 1u) == ns_live - 1) { ctr[0] = 0; ctr[1] = 0; }
   }
   if (*s_err && tid == 0) atomicMax(p.err, *s_err);
   }

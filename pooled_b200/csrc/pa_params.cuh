@@ -38,10 +38,9 @@ struct DecodeParams {
   // gather mode: item i is one column attending the rows listed at gather + col0[i] * gather_stride: [0] = n, then n
   // cache rows ascending (k_cache / v_cache above are the layer's caches)
   const uint32_t* gather; uint32_t gather_stride;
-  // merge != 0: no combine kernel follows; the CTAs of each (item, kv head) merge their own records, gate and store
-  // (2: CTAs without a merge unit leave as soon as their record is counted; 1: they wait like the others)
-  // (3: the CTAs of an (item, kv head) are one thread-block cluster and merge through its shared memory, no record leaves the SMs)
-  uint32_t merge; unsigned int* merge_ctr;
+  // merge != 0: no combine kernel follows; the CTAs of each (item, kv head) merge their own records, gate and store: 2 by way of
+  // merge_rec, 3 as one thread-block cluster through its shared memory
+  uint32_t merge; float* merge_rec;   // merge_rec: a block per CTA of a merging call, every word kNoWord between calls
   unsigned int* xch_ctr;   // != nullptr: the call ends in a cross-GPU exchange; the kernel's first thread advances its call counter
   const void* gate; uint64_t gate_col_stride, gate_head_stride;
   void* out; uint64_t out_col_stride; int act_f16;
