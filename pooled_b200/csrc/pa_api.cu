@@ -822,7 +822,10 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
         if (ns <= (uint32_t)kMaxCluster) for (f.cluster = ns; f.cluster & (f.cluster - 1); ++f.cluster) {}
         f.gate = gate ? reinterpret_cast<const uint8_t*>(gate) + (col + c0) * gcs * aes : nullptr; f.gate_col_stride = gcs; f.gate_head_stride = ghs;
         f.out = reinterpret_cast<uint8_t*>(out) + (col + c0) * ocs * aes; f.out_col_stride = ocs; f.act_f16 = ctx->cfg.act_dtype == PA_F16;
-        merged = f.cluster != 0;
+        // one wave of CTAs (one per SM) merges its records itself
+        if (!f.cluster && !ctx->core_only && !ctx->tune.no_merge && (uint64_t)live * ctx->cfg.n_kv_heads * nc <= (uint64_t)ctx->sm_count) f.merge_rec = ctx->merge_rec;
+        f.err = ctx->dev_err;
+        merged = f.cluster != 0 || f.merge_rec;
         f.q = reinterpret_cast<const uint8_t*>(q) + (col + c0) * qcs * qes; f.q_f16 = q_dtype == PA_F16; f.q_col_stride = qcs; f.q_head_stride = qhs;
         f.q_vec = q_dtype == PA_F32 && !(qcs & 3) && !(qhs & 3) && !((uintptr_t)f.q & 15);
         f.k = (const float*)L->k_alt; f.v = (const float*)L->v_alt;

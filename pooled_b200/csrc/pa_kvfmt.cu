@@ -8,7 +8,7 @@
 //   softmax  32 threads per head, online rescale across chunks (m starts at -3.0e38, as in the reference)
 //   values   a thread per four dims and group of positions, the groups summed in a fixed order at the end
 // A row of kv_dim values costs kv_dim * 1.125 bytes (int8) or kv_dim * 4 bytes (f32) against kv_dim * 2 for f16.
-#include "pa_params.cuh"
+#include "pa_merge.cuh"
 
 namespace pa {
 
@@ -201,8 +201,8 @@ size_t any_decode_smem(uint32_t G, uint32_t hd) {
 // 64: 32, 256: 8; with four heads half of that) rows together, 128 registers a thread, before it uses the first: 128 KB
 // in flight per SM, which is what HBM's latency takes at full rate.  No barrier and no shared memory until the warps' (o, m, l) are merged at the end.  A CTA's
 // rows are one or two such batches per warp at the contexts these caches serve.  28 layers of a token over 2000 rows (16 q / 8 kv
-// heads x 128), whole calls: 644 us with the chunked kernel above and a front kernel, 257 us with this one and a front kernel, 218 us with
-// the front in this one (floor 70: 459 MB).
+// heads x 128), whole calls: 644 us with the chunked kernel above and a front kernel, 257 us with this one, a front and a merge
+// kernel, 218 us with the front in this one, 199 us with the merge in it too (floor 70: 459 MB).
 //
 // FU: one token whose front the kernel makes itself, as pa_decode_kernel does: the 256 threads rotate the G query rows (rot_exact,
 // host cos / sin) into shared memory; the CTA of the sequence's last rows also rotates k, stores the row, and takes it from shared
@@ -362,6 +362,7 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
     if (lane == 0) { sml[warp * G + h] = m[h]; sml[8 * G + warp * G + h] = l[h]; }
   }
   __syncthreads();
+  const bool keep = p.cluster || p.merge_rec;      // behind the warps' shares
   for (uint32_t idx = tid; idx < G * HD; idx += 256) {
     const uint32_t h = idx / HD, d = idx % HD;
     float M = sml[h], L = 0.f, a = 0.f;
@@ -373,7 +374,7 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
       L = __fmaf_rn(sml[8 * G + w * G + h], e, L);
       a = __fmaf_rn(sm[w * G * HD + idx], e, a);
     }
-    if (p.cluster) {         // behind the warps' shares
+    if (keep) {
       float* mine = sm + 8 * G * (HD + 2);
       mine[idx] = a;
       if (d == 0) { mine[G * HD + 2 * h] = M; mine[G * HD + 2 * h + 1] = L; }
@@ -382,6 +383,30 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
     const uint64_t slot = (col * p.n_heads + g * G + h) * p.n_splits + split;
     p.part_o[slot * HD + d] = a;
     if (d == 0) { p.part_ml[slot * 2] = M * inv_sqrt_hd<HD>(); p.part_ml[slot * 2 + 1] = L; }
+  }
+  if (p.merge_rec) {
+    // one wave of CTAs: those of a (kv head, column) leave their records for one another (see kNoWord) and share out the merge
+    __shared__ uint32_t s_err;
+    if (tid == 0) s_err = 0;
+    __syncthreads();
+    if (warp >= 4) return;
+    constexpr size_t BLK = merge_block(HD, G);
+    const float* mine = sm + 8 * G * (HD + 2);
+    float* const blk0 = p.merge_rec + ((size_t)c * gridDim.y + g) * p.n_splits * BLK;
+    for (uint32_t idx = tid; idx < G * (HD / 4); idx += 128) {
+      const uint32_t h = idx / (HD / 4), c4 = idx % (HD / 4);
+      put_record4<HD>(blk0 + split * BLK, G, h, c4, *reinterpret_cast<const float4*>(mine + h * HD + c4 * 4), mine[G * HD + 2 * h] * inv_sqrt_hd<HD>(),
+                      mine[G * HD + 2 * h + 1]);
+    }
+    named_bar_sync(1, 128);                        // the scratch takes the place of the warps' shares, which nobody reads any more
+    for (uint32_t u = split; u < G * (HD / 64); u += p.n_splits) {
+      const uint32_t row = u / (HD / 64), slice = u % (HD / 64), h = g * G + row;
+      const float gv = p.gate && tid < 64 ? ld_act(p.gate, col * p.gate_col_stride + (uint64_t)h * p.gate_head_stride + slice * 64 + tid, p.act_f16) : 0.f;
+      merge_slice_128<HD>(blk0 + row * HD + slice * 64, blk0 + G * HD + (row * (HD / 64) + slice) * 2, BLK, p.n_splits, tid, *reinterpret_cast<MergeScratch*>(sm), 1,
+                          p.gate != nullptr, gv, false, p.act_f16, p.out, col * p.out_col_stride + (uint64_t)h * HD + slice * 64, &s_err);
+    }
+    if (tid == 0 && s_err) atomicMax(p.err, s_err);
+    return;
   }
   if (!p.cluster) return;
   // at most eight splits: the CTAs of a (kv head, column) are a cluster and merge without another launch
@@ -399,7 +424,7 @@ __global__ void __launch_bounds__(256, 1) pa_decode_f32_kernel(const F32DecodePa
 
 template <int HD, int G, bool FU>
 static cudaError_t launch_f32_fu(const F32DecodeParams& p, dim3 grid, cudaStream_t st) {
-  const size_t smem = (size_t)(9 * G * (HD + 2)) * 4;       // (at most 37 KB)
+  const size_t smem = std::max((size_t)(9 * G * (HD + 2)) * 4, sizeof(MergeScratch));       // (at most 37 KB)
   if (p.cluster) return launch_pdl_cluster(pa_decode_f32_kernel<HD, G, FU>, grid, dim3(256), smem, st, p.cluster, p);
   return launch_pdl(pa_decode_f32_kernel<HD, G, FU>, grid, dim3(256), smem, st, p);
 }

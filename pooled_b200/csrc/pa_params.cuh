@@ -141,7 +141,8 @@ struct F32DecodeParams {
   uint32_t seq; int32_t lim0; uint32_t n_rows, n_cols, early, cluster;         // as in Q8Params
   float scale_log2;
   float* part_o; float* part_ml;
-  const void* gate; uint64_t gate_col_stride, gate_head_stride;                // cluster: gate and output
+  float* merge_rec; uint32_t* err;                                             // != nullptr: no cluster, the CTAs merge by way of it
+  const void* gate; uint64_t gate_col_stride, gate_head_stride;                // cluster or merge_rec: gate and output
   void* out; uint64_t out_col_stride; int act_f16;
   // one token with its front in the kernel (k_new != nullptr): q unrotated, the token's own k / v row in q's type, cos / sin by value
   const void* k_new; const void* v_new; uint32_t half; uint32_t early_limit;   // early_limit: rows the call before may still be writing

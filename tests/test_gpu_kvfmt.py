@@ -355,7 +355,7 @@ def test_f32_plans_of_many_waves(nH, nKV, hd, rows, n_cols):
 
 @pytest.mark.parametrize("nH,nKV,hd,n_rot", [(4, 1, 256, 64), (4, 2, 256, 64), (2, 2, 256, 64), (8, 2, 128, 128), (16, 8, 128, 64), (4, 4, 128, 128), (4, 1, 64, 64), (4, 2, 64, 64), (2, 2, 64, 64)])
 @pytest.mark.parametrize("act", ["f32", "f16"])
-def test_f32_tokens_with_the_front_in_the_kernel(nH, nKV, hd, n_rot, act, monkeypatch):
+def test_f32_tokens_with_front_and_merge_in_the_kernel(nH, nKV, hd, n_rot, act, monkeypatch):
     # against the three-kernel chain bit for bit, cache rows too: tokens straight behind an append and one another, two layers, contexts
     # from none to several batches of rows per warp and either side of their edges
     import torch
@@ -365,7 +365,8 @@ def test_f32_tokens_with_the_front_in_the_kernel(nH, nKV, hd, n_rot, act, monkey
     rnd = lambda seed, *shape: torch.from_numpy(po.normal(seed, int(np.prod(shape))).astype(np.float32).reshape(shape)).cuda().to(td)
     K, V, q, k, v, g = (rnd(70 + i, T if i < 2 else 2 * n, (nH if i in (2, 5) else nKV) * hd) for i in range(6))
     for chain in (False, True):
-        monkeypatch.setenv("POOLED_ATTN_NO_FUSE", "1") if chain else monkeypatch.delenv("POOLED_ATTN_NO_FUSE", raising=False)
+        for var in ("POOLED_ATTN_NO_FUSE", "POOLED_ATTN_NO_MERGE"):
+            monkeypatch.setenv(var, "1") if chain else monkeypatch.delenv(var, raising=False)
         eng = AttnEngine(AttnConfig(n_heads=nH, n_kv_heads=nKV, head_dim=hd, n_rot=n_rot, rope_theta=1e6, max_seq=T + n, n_layers=2, act_dtype=td, max_cols=T, kv_format="f32"))
         o = []
         for ctx in (0, 1, 15, 16, 127, 128, 129, 1000, 2047, T):
@@ -375,7 +376,7 @@ def test_f32_tokens_with_the_front_in_the_kernel(nH, nKV, hd, n_rot, act, monkey
                 before = eng.stats()["kernel_launches"]
                 for t in range(n):
                     o.append(eng.encode_layer(li, ctx + t, q[li * n + t:li * n + t + 1], k[li * n + t:li * n + t + 1], v[li * n + t:li * n + t + 1], g[li * n + t:li * n + t + 1]))
-                assert chain or eng.stats()["kernel_launches"] - before <= 2 * n
+                assert chain or eng.stats()["kernel_launches"] - before == n
             o += [eng.cache(li, w)[0, :ctx + n].clone() for li in range(2) for w in "kv"]
         eng.sync()
         outs.append(o)
