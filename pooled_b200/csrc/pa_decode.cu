@@ -156,11 +156,13 @@ struct DecSmem {
   static constexpr int P_BYTES = kT * PP * (PRECISE ? 2 : 1);      // per group
   static constexpr int MISC = NG * 4 * ROWS * 4 * 2 + kMaxStages * 4 * 8 + 64 + 2048 + 1024 + 64;   // + the fused front's angles and new row, the slots' tile numbers
   static constexpr int fixed_bytes() { return Q_BYTES + NG * P_BYTES + MISC; }
-  static int stages_for(int smem_limit) {
-    int s = (smem_limit - 1024 - fixed_bytes()) / (2 * SLOT);
+  static int stages_for(int smem_limit, int extra) {
+    int s = (smem_limit - 1024 - fixed_bytes() - extra) / (2 * SLOT);
     return s > kMaxStages ? kMaxStages : s;
   }
   static int total_bytes(int stages) { return 1024 + stages * 2 * SLOT + fixed_bytes(); }
+  // a cluster's merge: what the CTAs send this one, at most 1024 vectors of four values and (m, l) of 8 rows from eight CTAs
+  static constexpr int RECV = NT == 1 ? 1024 * 16 + 64 * 8 : 0;
 };
 
 static_assert(sizeof(DecodeParams) + 4 * sizeof(CUtensorMap) <= 4096, "the decode kernel's launch parameters must fit 4 KB");
@@ -216,6 +218,8 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     }
     return;
   }
+  constexpr bool PUSH = CL && NT == 1;       // the cluster's CTAs send one another their rows (see the end)
+  if constexpr (PUSH) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");    // this CTA runs: others may write to it
   const uint32_t tile1 = min(tiles, tile0 + tps);
   const uint32_t n_tiles = tile1 - tile0;
   const uint32_t NS = p.n_stages;
@@ -518,6 +522,7 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         atomicMax(p.err, *s_err);
       }
     }
+    if constexpr (PUSH) { __syncwarp(); asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
     return;
   }
 
@@ -999,10 +1004,11 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
   }
   named_bar_sync(gbar, kConsumers);
   if constexpr (CL) {
-    // ---- at most eight splits: a cluster.  Every CTA's rows lie in its shared memory (xo, xml_out); after one cluster
-    //      barrier the CTAs share out the output, four dims per thread, and read one another's rows.  Through global
-    //      memory the same merge is a record written, a fence, a counter, a wait and a round trip: 4.3 us of a 9.6 us call over
-    //      301 rows.  The arithmetic is pa_combine_kernel's for up to eight records, operation for operation and in
+    // ---- at most eight splits: a cluster.  The CTAs share out the output, four dims per thread.  With eight query rows every CTA
+    //      sends each vector of its rows straight to the CTA that merges it: one cluster barrier, then local reads, and nobody
+    //      waits for readers before it leaves (28 layers of a token over 301 rows, 16 / 8 heads x 128: 175 us with remote reads and a second barrier, 166 so).  With sixteen, for which there is no room beside the ring, its rows stay in
+    //      its own shared memory (xo, xml_out), are read by the others after the barrier, and a second one follows.  Through global
+    //      memory the same merge is a record written, a fence, a counter, a wait and a round trip: 4.3 us of a 9.6 us call.  The arithmetic is pa_combine_kernel's for up to eight records, operation for operation and in
     //      its order, so the bits are the same whichever merges. ----
     const uint32_t ns_live = (tiles + tps - 1) / tps, n_it = live_rows * (HD / 4);
     uint32_t idx = split * kConsumers + ltid;
@@ -1019,9 +1025,27 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     };
     float gv[4] = {0.f, 0.f, 0.f, 0.f};
     if (p.gate && idx < n_it) gate4(idx, gv);      // lands while the cluster meets
+    float4* rx = nullptr;      // [turn][CTA][128] vectors, then [CTA][8 rows] (m, l)
+    float2* rml = nullptr;
+    if constexpr (PUSH) {
+      rx = reinterpret_cast<float4*>(base + NS * 2 * SLOT + L::fixed_bytes());
+      rml = reinterpret_cast<float2*>(rx + 1024);
+      const uint32_t rx_s = smem_u32(rx), rml_s = smem_u32(rml);
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");       // every CTA of the cluster has begun
+      for (uint32_t ix = ltid; ix < n_it; ix += kConsumers) {
+        const uint32_t unit = ix / kConsumers, owner = unit % ns_live, turn = unit / ns_live;
+        const float4 x = reinterpret_cast<const float4*>(xo)[ix];
+        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
+                     ::"r"(cluster_map(rx_s + ((turn * ns_live + split) * kConsumers + ltid) * 16, owner)), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w) : "memory");
+      }
+      if ((ltid & 7u) < live_rows && (ltid >> 3) < ns_live)
+        asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};"
+                     ::"r"(cluster_map(rml_s + (split * 8 + (ltid & 7)) * 8, ltid >> 3)), "f"(xml_out[(ltid & 7) * 2]), "f"(xml_out[(ltid & 7) * 2 + 1]) : "memory");
+    }
     cluster_sync();
     const uint32_t xo_s = smem_u32(xo), xml_s = smem_u32(xml_out);
-    for (bool first = true; idx < n_it; idx += ns_live * kConsumers, first = false) {
+    uint32_t turn = 0;
+    for (bool first = true; idx < n_it; idx += ns_live * kConsumers, first = false, ++turn) {
       if (p.gate && !first) gate4(idx, gv);
       const uint32_t row = idx / (HD / 4), c4 = idx % (HD / 4);
       float2 ml[kMaxCluster];
@@ -1030,8 +1054,13 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       for (uint32_t s = 0; s < kMaxCluster; ++s) {
         ml[s] = make_float2(-3.0e38f, 0.f); x[s] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (s >= ns_live) continue;
-        ml[s] = cluster_ld2(cluster_map(xml_s, s) + row * 8);
-        x[s] = cluster_ld4(cluster_map(xo_s, s) + (row * HD + c4 * 4) * 4);
+        if constexpr (PUSH) {
+          ml[s] = rml[s * 8 + row];
+          x[s] = rx[(turn * ns_live + s) * kConsumers + ltid];
+        } else {
+          ml[s] = cluster_ld2(cluster_map(xml_s, s) + row * 8);
+          x[s] = cluster_ld4(cluster_map(xo_s, s) + (row * HD + c4 * 4) * 4);
+        }
         ml[s].x *= 0.6931471805599453f;
       }
       float M = ml[0].x;
@@ -1060,7 +1089,7 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         else reinterpret_cast<float*>(p.out)[oo + k] = rv;
       }
     }
-    cluster_sync();                                // no CTA leaves while another reads its rows
+    if constexpr (!PUSH) cluster_sync();           // no CTA leaves while another reads its rows
     if (*s_err && tid == 0) atomicMax(p.err, *s_err);
   } else {
   if (!p.merge) {
@@ -1257,10 +1286,11 @@ template <int HD, int NT, bool PRECISE, bool NORM = false, bool CL = false>
 static cudaError_t launch_decode_t(const pa_layer* L, const DecodeParams& p, dim3 grid, cudaStream_t st) {
   using S = DecSmem<HD, NT, PRECISE>;
   DecodeParams pp = p;
-  int stages = S::stages_for(L->ctx->smem_optin);
+  constexpr int EXTRA = CL ? S::RECV : 0;
+  int stages = S::stages_for(L->ctx->smem_optin, EXTRA);
   if (stages < 2) return cudaErrorInvalidConfiguration;
   pp.n_stages = (uint32_t)stages;
-  const int bytes = S::total_bytes(stages);
+  const int bytes = S::total_bytes(stages) + EXTRA;
   static bool attr_set[64] = {};
   if (pp.gather && (!pp.k_cache || !pp.v_cache)) return cudaErrorInvalidValue;
   auto kern = pa_decode_kernel<HD, NT, PRECISE, NORM, CL>;
