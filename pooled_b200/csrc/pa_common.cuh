@@ -402,6 +402,8 @@ struct pa_ctx {
   void* stage_dev = nullptr;     // device staging of the host-buffer entry point
   void* stage_host = nullptr;    // pinned staging
   size_t stage_bytes = 0;
+  cudaStream_t side = nullptr;   // copies of a host step beside its layers, and their order
+  cudaEvent_t side_ev[4] = {};   // the caller's earlier work | later layers uploaded | earlier layers done | their outputs downloaded
   pa::ExchangeView xc{};         // peer exchange (pa_exchange_init); world == 0: not set up
   std::vector<cudaEvent_t> ev;   // timing: event pairs around core-kernel launches
   size_t ev_used = 0;

@@ -324,6 +324,40 @@ def test_host_buffer_entry_points_match_the_device_path():
     assert torch.equal(one, want[1])
 
 
+@pytest.mark.parametrize("layers", [5, 12, 13, 24])
+@pytest.mark.parametrize("gate", [None, "own", "in q"])
+@pytest.mark.parametrize("pinned", [True, False])
+def test_host_step_over_many_layers_with_its_copies_beside_them(layers, gate, pinned):
+    # from 512 KB on the copies of page-locked buffers run beside the layers: outputs and caches of ordinary calls, steps that follow
+    # one another without a pause, inputs that the stream's earlier work writes
+    import torch
+    from pooled_b200 import AttnConfig, AttnEngine
+    nH, nKV, hd, ctx, steps = 24, 4, 256, 300, 3      # 40 KB a layer (52 with a gate of its own): 512 KB with 13 layers (10)
+    rnd = lambda seed, *shape: torch.from_numpy(util.normal_f16(seed, shape)).to(torch.float16)
+    q2 = rnd(1, steps, layers, 1, nH * 2 * hd)
+    hk, hv, hg = (rnd(2 + i, steps, layers, 1, (nH if i == 2 else nKV) * hd) for i in range(3))
+    engs = [AttnEngine(AttnConfig(n_heads=nH, n_kv_heads=nKV, head_dim=hd, n_rot=64, rope_theta=1e7, max_seq=ctx + 8, n_layers=layers, act_dtype=torch.float16, max_cols=8)) for _ in range(2)]
+    for li in range(layers):
+        K, V = (po.np_f16_rne(po.normal(40 + 2 * li + i, ctx * nKV * hd)).reshape(ctx, -1) for i in range(2))
+        for e in engs:
+            util.load_cache(e, li, 0, K, V)
+    pin = lambda *shape: torch.zeros(shape, dtype=torch.float16, pin_memory=pinned)
+    q, k, v, g, out = pin(layers, 1, nH * 2 * hd), pin(layers, 1, nKV * hd), pin(layers, 1, nKV * hd), pin(layers, 1, nH * hd), pin(layers, 1, nH * hd)
+    for t in range(steps):
+        torch.cuda.synchronize()
+        for dst, src in ((q, q2[t]), (k, hk[t]), (v, hv[t]), (g, hg[t])):
+            dst.copy_(src.cuda(), non_blocking=pinned)
+        gt = {None: None, "own": g, "in q": q[:, :, hd:]}[gate]
+        engs[0].encode_step_host(ctx + t, q, k, v, gt, out, mode="decode", q_head_stride=2 * hd, gate_head_stride=2 * hd if gate == "in q" else hd)
+        for li in range(layers):
+            dq = q2[t, li].cuda()
+            dg = {None: None, "own": hg[t, li].cuda(), "in q": dq[:, hd:]}[gate]
+            want = engs[1].encode_layer(li, ctx + t, dq, hk[t, li].cuda(), hv[t, li].cuda(), dg, mode="decode", q_head_stride=2 * hd, gate_head_stride=2 * hd if gate == "in q" else hd)
+            assert torch.equal(out[li], want.cpu()), f"step {t} layer {li}"
+    for li in range(layers):
+        assert all(torch.equal(engs[0].cache(li, w), engs[1].cache(li, w)) for w in "kv")
+
+
 def test_exchange_merge_with_one_rank_matches_decode_over_many_calls():
     # the peer-exchange combine with world = 1 (the rank publishes to and reads from its own buffer): the call counter,
     # the two buffer parities and the flags are exercised by consecutive calls of different sizes
