@@ -45,8 +45,10 @@ struct Q8Smem {
   // four of scales, which are read until the tile's end
   static constexpr int STAGES = CV ? 2 : HD == 256 ? 3 : 4, SC_STAGES = CV ? 4 : STAGES;
   static constexpr int F16 = CV ? 2 * 2 * KB * 2 : 0;      // two tiles of K and V as f16, ahead of the rings
-  static constexpr int OFF_RAW = F16, OFF_SC = OFF_RAW + STAGES * 2 * KB;
-  static constexpr int RING = OFF_SC + SC_STAGES * 2 * SB;
+  // (a stage's scales lie behind its values, or, CV, in a ring of their own)
+  static constexpr int STAGE = CV ? 2 * KB : 2 * KB + 2 * SB, SC_STAGE = CV ? 2 * SB : STAGE;
+  static constexpr int OFF_RAW = F16, OFF_SC = CV ? OFF_RAW + STAGES * STAGE : OFF_RAW + 2 * KB;
+  static constexpr int RING = OFF_RAW + STAGES * STAGE + (CV ? SC_STAGES * SC_STAGE : 0);
   static constexpr int MROWS = 8 * NW;                     // most query rows of a CTA
   static constexpr int MERGE = MROWS * (HD + 2) * 4;       // the warps' (o, m, l), over the idle ring
   static constexpr int MINE = MROWS * (HD + 2) * 4;        // the CTA's merged rows behind them, for the cluster's merge
@@ -128,7 +130,8 @@ __global__ void __launch_bounds__((Q8Smem<HD, CV>::THREADS), CV && HD >= 128 ? 1
 
   auto load_tile = [&](uint32_t t) {      // one commit group per call, empty past the range
     if (t < n_tiles) {
-      const uint32_t pos0 = (t_lo + t) * kQ8Tile, base = sm0 + L::OFF_RAW + (t % L::STAGES) * 2 * L::KB, sbase = sm0 + L::OFF_SC + (t % L::SC_STAGES) * 2 * L::SB;
+      const uint32_t pos0 = (t_lo + t) * kQ8Tile, base = sm0 + L::OFF_RAW + (t % L::STAGES) * L::STAGE,
+                     sbase = CV ? sm0 + L::OFF_SC + (t % L::SC_STAGES) * L::SC_STAGE : base + 2 * L::KB;
       constexpr int CPR = HD / 16;
 #pragma unroll
       for (int it = 0; it < kQ8Tile * CPR / kQ8Threads; ++it) {
@@ -278,9 +281,9 @@ __global__ void __launch_bounds__((Q8Smem<HD, CV>::THREADS), CV && HD >= 128 ? 1
       load_tile(t + L::STAGES - 1);
     }
     if (!warp_live) continue;
-    const uint8_t* kt = smem + (CV ? (t & 1) * 4 * L::KB : L::OFF_RAW + (t % L::STAGES) * 2 * L::KB);
+    const uint8_t* kt = smem + (CV ? (t & 1) * 4 * L::KB : L::OFF_RAW + (t % L::STAGES) * L::STAGE);
     const uint8_t* vt = kt + (CV ? 2 : 1) * L::KB;
-    const float* kst = reinterpret_cast<const float*>(smem + L::OFF_SC + (t % L::SC_STAGES) * 2 * L::SB);
+    const float* kst = reinterpret_cast<const float*>(CV ? smem + L::OFF_SC + (t % L::SC_STAGES) * L::SC_STAGE : kt + 2 * L::KB);
     const float* vst = kst + kQ8Tile * NB;
     const uint32_t kt_s = smem_u32(kt), vt_s = smem_u32(vt);
 #pragma unroll 1

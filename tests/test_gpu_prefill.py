@@ -82,6 +82,27 @@ def test_head_dim_64_prefill_chunks_and_decode(n_cols, pos, act):
     eng.sync()
 
 
+@pytest.mark.parametrize("n_rot", [64, 128])
+@pytest.mark.parametrize("n_cols,pos", [(130, 0), (48, 300), (257, 5)])
+def test_head_dim_128_prompts_rotated_in_part_and_in_full(n_rot, n_cols, pos):
+    # rotated in part, the 64 dims no rotation touches come from the caller's q: interleaved with its gate, as the q projection delivers both
+    import torch
+    nH, nKV, hd = 6, 2, 128
+    eng = _engine(nH, nKV, hd, pos + n_cols + 8, act="f16", max_cols=512, n_rot=n_rot, rope_mode="f64")
+    q, k, v, g = _inputs(8, nH, nKV, hd, pos + n_cols)
+    d = lambda a: util.torch_dev(a, torch.float16)
+    both = torch.cat([d(q).view(-1, nH, hd), d(g).view(-1, nH, hd)], 2).view(pos + n_cols, -1)
+    run = lambda a, b: eng.encode_layer(0, a, both[a:b], d(k[a:b]), d(v[a:b]), both[a:b, hd:], mode="prefill", q_head_stride=2 * hd, gate_head_stride=2 * hd)
+    if pos:
+        run(0, pos)
+    out = run(pos, pos + n_cols).float().cpu().numpy()
+    eng.sync()
+    ref, Kf, Vf = _oracle_layer(q, k, v, g, nH, nKV, hd, n_rot, 1e7, 0)
+    gk, gv = util.read_cache(eng, 0, 0, 0, pos + n_cols)
+    assert np.array_equal(gk, Kf) and np.array_equal(gv, Vf), "KV append is not bit-exact"
+    util.assert_close(out, ref[pos:], f"{n_cols} columns at {pos}, {n_rot} rotated dims")
+
+
 def _inputs(cfg_id, nH, nKV, hd, n_cols):
     q = util.normal_f16(0xA11CE + cfg_id, (n_cols, nH * hd)); k = util.normal_f16(0xB0B + cfg_id, (n_cols, nKV * hd))
     v = util.normal_f16(0xC0DE + cfg_id, (n_cols, nKV * hd)); g = util.normal_f16(0x6A7E + cfg_id, (n_cols, nH * hd))
