@@ -1186,7 +1186,7 @@ static int prefill_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols
   }
   // few columns behind many keys: the keys are split and the records merged by a second kernel
   p.n_splits = ctx->core_only ? 1u : prefill_splits(p.pos, n_cols, p.n_heads, ctx->cfg.head_dim, (uint32_t)ctx->sm_count, ctx->pf_slots);
-  p.part_o = ctx->part_o; p.part_ml = ctx->part_ml;
+  p.part_o = ctx->part_o; p.part_ml = ctx->part_ml; p.sms = (uint32_t)ctx->sm_count;
   // ... and f16 output tiles leave by TMA (any head_dim the kernel takes; the gate's, if any, arrive so)
   CUtensorMap tm_o = tm_k, tm_g = tm_k;
   if (ctx->cfg.act_dtype == PA_F16 && !(ocs & 63) && !ctx->tune.no_out_tma && (!gate || rows_tma_ok(ctx, gate, gcs, ghs))) {

@@ -192,6 +192,7 @@ struct PrefillParams {
                                 // q_rot_chunks 64-dim chunks of a head from tm_q (the rotated q), the others from tm_q2
                                 // (the caller's own q, head stride q2_head_stride: unrotated dims are not copied anywhere)
   uint32_t q_rot_chunks; uint64_t q2_head_stride;
+  uint32_t sms;                 // prefill: SMs of the device, the CTAs that run together
   uint32_t gate_tma;            // prefill, with out_tma: the gate's rows come by TMA (tm_g)
   uint32_t out_tma;             // prefill, f16 out: the CTA's output tile leaves through shared memory by one TMA store (tm_o)
 };

@@ -22,7 +22,7 @@
 // products against 1024 with N = 128, measured with nothing else running.
 //
 // Measured (whole passes, power-capped; tiles of 64 keys with two groups of four softmax warps on alternate tiles and gate rows fetched
-// by the lanes before): 4 layers of 8192 columns of 24 heads x 256 3698 -> 3294 us, 8 layers of 2999 x 16 x 128 676 -> 576 (36 of it
+// by the lanes before): 4 layers of 8192 columns of 24 heads x 256 3698 -> 3265 us, 8 layers of 2999 x 16 x 128 676 -> 572 (36 of it
 // sixteen softmax warps instead of eight, 27 the rotation kernel's), 8 layers of 203 columns of 24 x 256 behind 9001 rows 602 -> 554.
 // A tile of head_dim 256 takes 2220 cycles for the tensor cores' 2048 and the chip runs at 1.39 GHz under its power limit.
 //
@@ -145,6 +145,18 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         tma_load_3d(q_s, &tm_q, 0, (int)c0, (int)(h * (p.q_head_stride / 64)), BAR(Q_FULL, 0));
         if (p.q_tma == 2)   // the chunks no rotation touches come straight from the caller's q
           tma_load_3d(q_s + p.q_rot_chunks * (kPM * 128), &tm_q2, 0, (int)c0, (int)(h * (p.q2_head_stride / 64) + p.q_rot_chunks), BAR(Q_FULL, 0));
+      }
+      if (!SPLIT && p.gate_tma) tma_prefetch_3d(&tm_g, 0, (int)c0, (int)(h * (p.gate_head_stride / 64)));
+      if (!SPLIT && p.q_tma) {
+        // the query rows of the CTA that takes this one's place, as far as no kernel wrote them just now, into L2: 128-byte pieces of
+        // rows 12 KB and more apart, for which it would wait for HBM at its start.  (The gate's above likewise, for the end.)  8 layers of 2999 columns of 16
+        // heads x 128 577 -> 572 us, 4 of 8192 of 24 x 256 3310 -> 3265.
+        const uint32_t next = blockIdx.y * gridDim.x + blockIdx.x + p.sms;
+        if (next < gridDim.x * gridDim.y) {
+          const uint32_t hn = next % gridDim.x, cn = (gridDim.y - 1 - next / gridDim.x) * kPM;
+          if (p.q_tma == 2) tma_prefetch_3d(&tm_q2, 0, (int)cn, (int)(hn * (p.q2_head_stride / 64) + p.q_rot_chunks));
+          else tma_prefetch_3d(&tm_q, 0, (int)cn, (int)(hn * (p.q_head_stride / 64)));
+        }
       }
       uint32_t st = 0, ph = 1;
       for (uint32_t j = 0; j < n_tiles; ++j) {
