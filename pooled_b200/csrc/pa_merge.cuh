@@ -146,11 +146,13 @@ __device__ __forceinline__ void merge_slice_128(float* o_rec, float* ml_rec, siz
   named_bar_sync(bar, 128);   // the scratch is free again
 }
 
-// A CTA's block of a record buffer: o [rows][HD], then (m, l) once for each 64-dim slice, [rows][HD / 64][2]
-__host__ __device__ constexpr size_t merge_block(int hd, int rows) { return (size_t)rows * (hd + hd / 32); }
+// A CTA's block of a record buffer: o [rows][HD], then (m, l) once for each 64-dim slice, [rows][HD / 64][2]; whole 16-byte vectors, so
+// that every block's rows are aligned for the vector accesses (one row of 64 dims alone is 264 bytes)
+__host__ __device__ constexpr size_t merge_block(int hd, int rows) { return ((size_t)rows * (hd + hd / 32) + 3) & ~(size_t)3; }
 // row `row` of a CTA's record: four of its values, and beside the first of each 64 (m in natural-log units, l)
 template <int HD>
 __device__ __forceinline__ void put_record4(float* blk, uint32_t rows, uint32_t row, uint32_t c4, float4 x, float m, float l) {
+  static_assert(HD % 4 == 0 && merge_block(HD, 1) % 4 == 0 && merge_block(HD, 2) % 4 == 0, "records are read and written 16 bytes at a time");
   if (c4 % 16 == 0) *reinterpret_cast<float2*>(blk + (size_t)rows * HD + (row * (HD / 64) + c4 / 16) * 2) = make_float2(word_for(m), word_for(l));
   reinterpret_cast<float4*>(blk + (size_t)row * HD)[c4] = make_float4(word_for(x.x), word_for(x.y), word_for(x.z), word_for(x.w));
 }

@@ -399,3 +399,23 @@ def test_f32_splits_around_the_end_of_eight(nH, nKV, hd):
             out = eng.decode(0, [(0, n - nc, nc)], dq[:nc]).cpu().numpy()
             eng.sync()
             assert util.errs(out, po.attn_f64_kv32(q[:nc], K, V, nH, nKV, hd, n - nc, nc, None))[1] < util.REF_REL, f"{n} rows x {nc}"
+
+
+@pytest.mark.parametrize("nH,nKV,n_cols,ctx", [(13, 13, 1, (128, 129, 1000)), (16, 16, 1, (129, 131, 700)), (8, 8, 2, (129, 300)), (5, 5, 3, (129, 300)), (2, 2, 1, (3585, 4000)),
+                                               (1, 1, 1, (3585, 5003)), (8, 8, 1, (3585,)), (12, 12, 1, (4736, 4737)), (24, 12, 1, (4737,)), (13, 13, 1, (2500,))])
+def test_f32_records_of_one_head_of_64_dims(nH, nKV, n_cols, ctx, monkeypatch):
+    # the CTAs of one query head x 64 dims leave 66 floats each: merged in the kernel as by the kernel behind it, bit for bit, where more
+    # than eight CTAs a (kv head, column) merge there
+    hd, outs = 64, []
+    rows = max(ctx)
+    rnd = lambda seed, *shape: util.torch_dev(po.normal(seed, int(np.prod(shape))).astype(np.float32).reshape(shape))
+    K, V, q, g = rnd(90, rows, nKV * hd), rnd(91, rows, nKV * hd), rnd(92, n_cols, nH * hd), rnd(93, n_cols, nH * hd)
+    for chain in (False, True):
+        monkeypatch.setenv("POOLED_ATTN_NO_MERGE", "1") if chain else monkeypatch.delenv("POOLED_ATTN_NO_MERGE", raising=False)
+        eng = _engine("f32", nH, nKV, hd, rows, max_cols=rows)
+        eng.kv_append(0, 0, 0, K, V)
+        o = [eng.decode(0, [(0, n - n_cols, n_cols)], q, gate) for n in ctx for gate in (None, g) for _ in range(2)]
+        eng.sync()
+        outs.append([x.cpu().numpy() for x in o])
+    assert all(np.isfinite(a).all() and np.array_equal(a, b) for a, b in zip(*outs))
+    assert util.errs(outs[0][-3], po.attn_f64_kv32(q.cpu().numpy(), K.cpu().numpy(), V.cpu().numpy(), nH, nKV, hd, ctx[-1] - n_cols, n_cols, None))[1] < util.REF_REL
