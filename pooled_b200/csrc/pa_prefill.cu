@@ -57,6 +57,9 @@ struct PfSmem {
   static_assert(TOTAL <= 227 * 1024, "shared memory of one CTA");
 };
 
+// keys of each of ns splits of `keys` keys, in whole 64s
+__device__ __forceinline__ uint32_t split_keys(uint32_t keys, uint32_t ns) { return ((keys + 63) / 64 + ns - 1) / ns * 64; }
+
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -104,14 +107,15 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
   const uint32_t h = blockIdx.x, g = h / p.G, c0 = q_tile * kPM;
   const uint32_t rows_valid = min((uint32_t)kPM, p.n_cols - c0);
   const uint32_t p0 = p.pos + c0;                       // cache row of column c0's own token
-  uint32_t tile0 = 0, n_tiles = (p0 + rows_valid + kPN - 1) / kPN;
+  uint32_t key0 = 0, key_end = p0 + rows_valid;         // this CTA's keys
   if constexpr (SPLIT) {
     // a short prompt behind a long context: the keys of a q tile are split over blockIdx.z (see prefill_splits)
-    const uint32_t tps = (n_tiles + p.n_splits - 1) / p.n_splits;
-    tile0 = blockIdx.z * tps;
-    if (tile0 >= n_tiles) return;                       // uniform for the CTA; the merge derives the same count
-    n_tiles = min(n_tiles, tile0 + tps) - tile0;
+    const uint32_t per = split_keys(key_end, p.n_splits);
+    key0 = blockIdx.z * per;
+    if (key0 >= key_end) return;                        // uniform for the CTA; the merge derives the same count
+    key_end = min(key_end, key0 + per);
   }
+  const uint32_t n_tiles = (key_end - key0 + kPN - 1) / kPN;
   // f16 q: the 128 query rows land in shared memory, in the layout the score products read, by one TMA copy
   const bool q_by_tma = p.q_tma != 0;
   if (warp == 1 && lane == 0) {
@@ -163,7 +167,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         for (int c = 0; c < L::KC; ++c) {
           mbar_wait(BAR(K_EMPTY, st), ph, s_err, WAIT_EMPTY);
           mbar_expect_tx(BAR(K_FULL, st), L::K_CHUNK);
-          tma_load_3d(k_s + st * L::K_CHUNK, &tm_k, 0, (int)((tile0 + j) * kPN), (int)(g * L::KC + c), BAR(K_FULL, st));
+          tma_load_3d(k_s + st * L::K_CHUNK, &tm_k, 0, (int)(key0 + j * kPN), (int)(g * L::KC + c), BAR(K_FULL, st));
           if (++st == NK) { st = 0; ph ^= 1; }
         }
       }
@@ -189,7 +193,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         for (int c = 0; c < L::VC; ++c) {
           mbar_wait(BAR(V_EMPTY, st), ph, s_err, WAIT_EMPTY);
           mbar_expect_tx(BAR(V_FULL, st), L::V_CHUNK);
-          tma_load_3d(v_s + st * L::V_CHUNK, &tm_v, 0, (int)((tile0 + j) * kPN + c * L::VK), (int)(g * L::KC), BAR(V_FULL, st));
+          tma_load_3d(v_s + st * L::V_CHUNK, &tm_v, 0, (int)(key0 + j * kPN + c * L::VK), (int)(g * L::KC), BAR(V_FULL, st));
           if (++st == NV) { st = 0; ph ^= 1; }
         }
       }
@@ -245,7 +249,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     const uint32_t qd = warp & 3, row = qd * 32 + lane;  // a warp reaches the 32 TMEM lanes of its index mod 4
     const uint32_t lane_addr = (qd * 32) << 16;
     const bool live = row < rows_valid;
-    const uint32_t lim = p0 + row + 1;                   // keys [0, lim) are visible to this row
+    const uint32_t lim = min(p0 + row + 1, key_end);     // of the CTA's keys those below lim are visible to this row
     pdl_trigger();
     if (!q_by_tma) {
       // this thread's share of its Q row as f16 into the layout the score products read
@@ -269,8 +273,8 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       mbar_arrive(BAR(Q_FULL, 0));
     }
     // m_st: the row's reference maximum, the same in both halves' threads (the weights of a tile are 2^(s - m_st); it moves only
-    // when a tile's maximum passes it by more than 2^8).  (A split that does not begin at key 0 may hold no visible key of a row, hence the finite start.)
-    const bool first0 = !SPLIT || tile0 == 0;
+    // when the maximum of a tile's half passes it by more than 2^8).  (A split that does not begin at key 0 may hold no visible key of a row, hence the finite start.)
+    const bool first0 = !SPLIT || key0 == 0;
     float m_st = first0 ? -INFINITY : -1.0e30f;
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
     // causal mask on tiles that reach this row's diagonal
@@ -286,12 +290,17 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       for (int i = 8; i < 32; i += 8) { a = max3(a, x[i], x[i + 1]); b = max3(b, x[i + 2], x[i + 3]); c = max3(c, x[i + 4], x[i + 5]); d = max3(d, x[i + 6], x[i + 7]); }
       return fmaxf(fmaxf(a, b), fmaxf(c, d));
     };
-    // the row's reference given the tile's maximum (scaled); how much O and the row's sum shrink if it moves
-    auto refer = [&](uint32_t j, float mt, float& alpha) {
+    // the row's reference given the maxima (scaled) of the tile's halves; how much O and the row's sum shrink if it moves.  It is the
+    // running reference of 64 keys after 64, whatever the tile: the f16 roundings of the weights depend on it, and with one
+    // maximum for the tile a result moved by 2e-4 of itself, as much as all of those roundings.
+    auto refer = [&](uint32_t j, float mt0, float mt1, float& alpha) {
+      const bool start = first0 && j == 0;                       // key 0 is visible to every row
+      const float was = m_st;
+      if (start || mt0 > m_st + 8.f) m_st = mt0;
+      if (mt1 > m_st + 8.f) m_st = mt1;
       alpha = 1.f;
-      if (first0 && j == 0) { m_st = mt; return false; }         // key 0 is visible to every row
-      if (!(mt > m_st + 8.f)) return false;
-      alpha = ex2_approx(m_st - mt); m_st = mt;
+      if (start || m_st == was) return false;
+      alpha = ex2_approx(was - m_st);
       return true;
     };
     // O must not change under the previous P V: wait for it, then rescale this warp's 32 rows in TMEM, chunks c0, c0 + dc, ...
@@ -330,7 +339,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       float* s_rm = reinterpret_cast<float*>(base + L::OFF_RM);
       float m_l = m_st, l = 0.f;       // this thread's share of the row's sum, and the reference it is in
       for (uint32_t j = par; j < n_tiles; j += 2) {
-        const uint32_t b = j % SB, kv0 = (tile0 + j) * kPN + half * 64, ts = t_s0 + b * kPN + lane_addr + half * 64;
+        const uint32_t b = j % SB, kv0 = key0 + j * kPN + half * 64, ts = t_s0 + b * kPN + lane_addr + half * 64;
         mbar_wait(BAR(S_FULL, b), (j / SB) & 1, s_err, WAIT_MMA);
         tc_fence_after();
         float s[32], mt = -INFINITY;
@@ -343,13 +352,13 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         float* mx = s_mx + ((j >> 1) & 1) * (4 * kPM) + par * (2 * kPM);
         mx[half * kPM + row] = mt;
         named_bar_sync(2 + par * 4 + qd, 64);
-        mt = fmaxf(mt, mx[(half ^ 1) * kPM + row]);
+        const float mo = mx[(half ^ 1) * kPM + row];
         if (j > 0) {
           mbar_wait(BAR(M_READY, (j - 1) & 1), ((j - 1) >> 1) & 1, s_err, WAIT_MMA);
           m_st = s_rm[((j - 1) & 1) * kPM + row];
         }
         float alpha;
-        const bool grow = refer(j, mt * p.scale_log2, alpha);
+        const bool grow = refer(j, (half ? mo : mt) * p.scale_log2, (half ? mt : mo) * p.scale_log2, alpha);
         if (half == 0) s_rm[(j & 1) * kPM + row] = m_st;
         __syncwarp();
         if (lane == 0) mbar_arrive(BAR(M_READY, j & 1));      // (both halves have read the one before: its place is free for tile j + 1)
@@ -380,7 +389,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       float2 l2 = make_float2(0.f, 0.f);       // this thread's share of the row's sum
       uint32_t sb = 0, sph = 0;
       for (uint32_t j = 0; j < n_tiles; ++j) {
-        const uint32_t kv0 = (tile0 + j) * kPN + half * 64, ts = t_s0 + sb * kPN + lane_addr + half * 64;
+        const uint32_t kv0 = key0 + j * kPN + half * 64, ts = t_s0 + sb * kPN + lane_addr + half * 64;
         mbar_wait(BAR(S_FULL, sb), sph, s_err, WAIT_MMA);
         tc_fence_after();
         float s[64];
@@ -393,8 +402,9 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         float* mx = s_mx + (j & 1) * (2 * kPM);
         mx[wg * kPM + row] = m_half;
         named_bar_sync(2 + qd, 64);
+        const float mo = mx[(wg ^ 1) * kPM + row];
         float alpha;
-        if (__any_sync(0xffffffffu, refer(j, fmaxf(m_half, mx[(wg ^ 1) * kPM + row]) * p.scale_log2, alpha))) {
+        if (__any_sync(0xffffffffu, refer(j, (wg ? mo : m_half) * p.scale_log2, (wg ? m_half : mo) * p.scale_log2, alpha))) {
           l2.x *= alpha; l2.y *= alpha;
           if (j > 0) rescale(j, alpha, wg, 2);            // half of the dims per warp
         }
@@ -545,9 +555,8 @@ __global__ void __launch_bounds__(256) pa_combine_few_kernel(const PrefillParams
   pdl_trigger();
   if (prow >= p.n_cols * p.n_heads) return;
   const uint32_t col = prow / p.n_heads, h = prow % p.n_heads, c0 = col / kPM * kPM;
-  const uint32_t n_tiles = (p.pos + c0 + min((uint32_t)kPM, p.n_cols - c0) + kPN - 1) / kPN;
-  const uint32_t tps = (n_tiles + p.n_splits - 1) / p.n_splits;
-  const uint32_t ns = (n_tiles + tps - 1) / tps;   // live splits of this q tile
+  const uint32_t keys = p.pos + c0 + min((uint32_t)kPM, p.n_cols - c0), per = split_keys(keys, p.n_splits);
+  const uint32_t ns = (keys + per - 1) / per;      // live splits of this q tile
   const float* ml = p.part_ml + (uint64_t)prow * p.n_splits * 2;
   const float* ob = p.part_o + (uint64_t)prow * p.n_splits * HD + lane * W;
   float m[kPrefillSplits], l[kPrefillSplits], x[kPrefillSplits][NV * W];
@@ -614,23 +623,23 @@ cudaError_t launch_combine_few(int head_dim, const PrefillParams& p, cudaStream_
 
 // Key splits of a prefill call.  One CTA per (128 columns, head) leaves most of the chip idle when a short prompt follows
 // a long context (203 columns of 24 heads behind 9001: 48 CTAs of 73 tiles on 148 SMs, a third of the rate of three ways
-// split).  The count is the one with the least estimated makespan, in units of a tile's time (1.2 us): a CTA costs its tiles and
-// about 5 more for its start and end, equal CTAs run in whole waves, CTAs of a causal triangle (heavy ones first) pack;
-// a split call adds the merge launch (3) and its records' way through L2 (1 KB each, about 3 TB/s both ways).
+// split).  The count is the one with the least estimated makespan, in units of 64 keys' time (0.6 us): a CTA costs its keys and
+// about 8 more for its start and end, equal CTAs run in whole waves, CTAs of a causal triangle (heavy ones first) pack;
+// a split call adds the merge launch (6) and its records' way through L2 (1 KB each, about 3 TB/s both ways).
 uint32_t prefill_splits(uint32_t pos, uint32_t n_cols, uint32_t n_heads, uint32_t head_dim, uint32_t sms, size_t slots) {
   const uint32_t q_tiles = (n_cols + kPM - 1) / kPM;
-  const double longest = (double)((pos + n_cols + kPN - 1) / kPN), avg = (double)((pos + n_cols / 2 + kPN - 1) / kPN);
+  const double longest = (double)((pos + n_cols + 63) / 64), avg = (double)((pos + n_cols / 2 + 63) / 64);
   const uint64_t rows = (uint64_t)n_cols * n_heads, ctas = (uint64_t)q_tiles * n_heads;
   uint32_t best = 1;
   double best_t = 0;
   for (uint32_t ns = 1; ns <= (uint32_t)kPrefillSplits; ++ns) {
-    if (ns > 1 && (rows * ns > slots || longest / ns < 2.0)) break;
+    if (ns > 1 && (rows * ns > slots || longest / ns < 4.0)) break;
     const double waves = (double)(ctas * ns) / sms;
     double t;
-    if (waves <= 1.0) t = longest / ns + 5.0;
-    else if (avg >= 0.8 * longest) t = ceil(waves) * (longest / ns + 5.0);
-    else t = waves * (avg / ns + 5.0) + 0.5 * longest / ns;
-    if (ns > 1) t += 3.0 + (double)(rows * ns) * (head_dim * 8.0) / 3.0e6 / 1.2;
+    if (waves <= 1.0) t = longest / ns + 8.0;
+    else if (avg >= 0.8 * longest) t = ceil(waves) * (longest / ns + 8.0);
+    else t = waves * (avg / ns + 8.0) + 0.5 * longest / ns;
+    if (ns > 1) t += 6.0 + (double)(rows * ns) * (head_dim * 8.0) / 3.0e6 / 0.8;
     if (ns == 1 || t < 0.95 * best_t) { best = ns; best_t = t; }
   }
   return best;

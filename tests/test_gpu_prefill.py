@@ -265,3 +265,69 @@ def test_config3_full_size_properties():
     vmax = np.maximum.accumulate(po.h2f(Vf).reshape(T, nKV, hd), axis=0)[::512]
     o = out[::512].reshape(-1, nKV, nH // nKV, hd)
     assert np.all(o <= vmax[:, :, None, :] + 2e-3)
+
+
+def _prefill_splits(pos, n_cols, n_heads, hd, sms, slots):
+    longest, avg = (pos + n_cols + 63) // 64, (pos + n_cols // 2 + 63) // 64
+    rows, ctas, best, best_t = n_cols * n_heads, -(-n_cols // 128) * n_heads, 1, 0.0
+    for ns in range(1, 9):
+        if ns > 1 and (rows * ns > slots or longest / ns < 4):
+            break
+        waves = ctas * ns / sms
+        t = longest / ns + 8 if waves <= 1 else np.ceil(waves) * (longest / ns + 8) if avg >= 0.8 * longest else waves * (avg / ns + 8) + 0.5 * longest / ns
+        if ns > 1:
+            t += 6 + rows * ns * (hd * 8.0) / 3.0e6 / 0.8
+        if ns == 1 or t < 0.95 * best_t:
+            best, best_t = ns, t
+    return best
+
+
+def _rounded_weights(q, K, V, nH, nKV, hd, pos, ns):
+    """Attention whose softmax weights are f16 values in the running reference maximum of 64 keys after 64 (moved when it grows by more
+    than 2^8), the rest in float64: the keys of each 128 columns in ns splits of whole 64s, each with a reference of its own."""
+    n, G, out = q.shape[0], nH // nKV, np.zeros((q.shape[0], nH * hd))
+    q, K, V = q.astype(np.float64), po.np_h2f(K).astype(np.float64), po.np_h2f(V).astype(np.float64)
+    for c0 in range(0, n, 128):
+        cols = np.arange(c0, min(n, c0 + 128))
+        keys = pos + cols[-1] + 1
+        per = -(-(-(-keys // 64)) // ns) * 64
+        for h in range(nH):
+            sl, kl = slice(h * hd, (h + 1) * hd), slice(h // G * hd, (h // G + 1) * hd)
+            x = q[cols, sl] @ K[:keys, kl].T * (1.4426950408889634 / np.sqrt(hd))
+            x[np.arange(keys)[None] > (pos + cols)[:, None]] = -np.inf
+            parts = []
+            for z in range(0, keys, per):
+                m, l, o = np.full(len(cols), -1e30), np.zeros(len(cols)), np.zeros((len(cols), hd))
+                for b in range(z, min(keys, z + per), 64):
+                    e = min(keys, z + per, b + 64)
+                    top = x[:, b:e].max(1)
+                    new = np.where((b == 0) | (top > m + 8), np.maximum(top, -1e30), m)
+                    w = np.exp2(x[:, b:e] - new[:, None])
+                    a = np.exp2(np.maximum(m - new, -2000.0))
+                    l, o, m = l * a + w.sum(1), o * a[:, None] + w.astype(np.float16).astype(np.float64) @ V[b:e, kl], new
+                parts.append((m, l, o))
+            M = np.max([p[0] for p in parts], 0)
+            L = sum(l * np.exp2(m - M) for m, l, o in parts)
+            out[cols, sl] = sum(o * np.exp2(m - M)[:, None] for m, l, o in parts) / L[:, None]
+    return out
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("nH,nKV,pos,n_cols", [(4, 2, 0, 300), (4, 1, 0, 500), (4, 2, 3000, 40), (6, 2, 4031, 130), (6, 1, 1100, 200)])
+def test_weights_round_in_the_running_reference_of_64_keys(hd, nH, nKV, pos, n_cols):
+    # a result carries the f16 roundings of its weights (2e-4 of itself): they are those of this reference and of these splits, which is
+    # what keeps a prompt's f32 outputs the same whatever the kernel's tiles.  What is left are weights that an error of some 3e-6 in 2^y, the
+    # sum of a score's products, takes across a rounding's edge: one in 300, 3e-5 of the result
+    import torch
+    rows = pos + n_cols
+    eng = _engine(nH, nKV, hd, rows, max_cols=512)
+    K = po.np_f16_rne(po.normal(41, rows * nKV * hd)).reshape(rows, nKV * hd); V = po.np_f16_rne(po.normal(42, rows * nKV * hd)).reshape(rows, nKV * hd)
+    util.load_cache(eng, 0, 0, K, V)
+    q = util.normal_f16(43, (n_cols, nH * hd))
+    out = eng.prefill(0, 0, pos, util.torch_dev(q)).cpu().numpy().astype(np.float64)
+    eng.sync()
+    slots = max(16384, min(32768, 512 * nH * 8))
+    ns = _prefill_splits(pos, n_cols, nH, hd, torch.cuda.get_device_properties(0).multi_processor_count, slots)
+    assert (ns > 1) == (pos > 1000)
+    ref = _rounded_weights(q, K, V, nH, nKV, hd, pos, ns)
+    assert np.linalg.norm(out - ref) / np.linalg.norm(ref) < 8e-5
