@@ -7,13 +7,18 @@
 //
 //   warps 0, 3   TMA producers: K in chunks of 128 keys x 64 dims, V in chunks of 16 KB of keys x all dims, a ring each
 //                (whole 64 KB tiles of head_dim 256 would leave room for one of each beside Q)
-//   warp 1       issues every MMA, in the order S(j + 1), P V(j), S(j + 2), ...: one in-order stream, so the S tile that
-//                P(j) overwrote needs no wait before S(j + 2) goes into it, and the weights of a tile have the time of a score
-//                product and of a P V product to be formed in
+//   warp 1       issues every MMA, in the order S(j + 1), P V(j), S(j + 2), ... (head_dim 128 and 64: S one tile further ahead), so that the
+//                weights of a tile have the time of a score product and of a P V product to be formed in
 //   warp 2       allocates and frees tensor memory
 //   warps 4-11   (4-19 at head_dim 128 and 64) softmax: warp w and warp w + 4 share the 32 query rows of TMEM lanes 32 (w % 4) ..., 64 keys of the tile each:
 //                tcgen05.ld of the scores, causal mask, the row's maximum through shared memory, P = 2^(s - m) as f16 pairs
-//                back over the S tile (tcgen05.st); then the epilogue (O / l, sigmoid gate, store)
+//                into tensor memory (tcgen05.st); then the epilogue (O / l, sigmoid gate, store)
+// What a product overwrites has been read: the order of the issue is promised for products of one accumulator and shape only,
+// which scores and P V are not.  At head_dim 256 the next scores take the place of scores that the softmax warps have taken into registers, and P
+// has two tiles of its own: no wait in the stream (4 layers of 8192 columns of 24 heads 3270 us, as with two S tiles that P overwrites and
+// nothing but that order).  At 128 and 64, where a thread has no room for its scores, P lies over S, and S(j + 2) waits for the P V(j - 1)
+// that reads it: 318 -> 338 us (8192 columns of 16 heads x 128; 8 layers of 2999 571 -> 596; scores in registers all the same, with spills, 332), 266 both at 64.
+//
 // O is rescaled only when a row's running maximum has grown by more than 2^8 since its last rescale (weights stay below
 // 2^8, exact in f32 sums and safe in f16); the rescale waits for the previous P V to retire and rewrites the row in TMEM.
 //
@@ -44,9 +49,10 @@ struct PfSmem {
   static constexpr bool ALT = HD <= 128;      // sixteen softmax warps, eight on every other tile (see there)
   static constexpr int NGRP = ALT ? 4 : 2, SOFT = 128 * NGRP;            // groups of four softmax warps
   static constexpr int NK = ALT ? 6 : 5, NV = 5;                         // ring depths in chunks
-  // S / P tiles in tensor memory (128 columns each; P takes the first 32 of each half of its S) | O (HD).  head_dim 256: 256 + 256 = 512
-  static constexpr int SBUF = HD == 256 ? 2 : 3;
-  static constexpr int T_S = 0, T_O = SBUF * kPN, TMEM_COLS = 512;
+  // tensor memory.  ALT: three S tiles (128 columns each; P takes the first 32 of each half of its S) | O (HD).  head_dim 256, whose O
+  // leaves 256 columns: one S tile, which the softmax warps take into registers at once | two P tiles of 64 columns | O
+  static constexpr int SBUF = ALT ? 3 : 1, PBUF = ALT ? SBUF : 2;
+  static constexpr int T_S = 0, T_P = ALT ? 0 : kPN, P_COLS = ALT ? kPN : kPN / 2, P_HALF = P_COLS / 2, T_O = T_P + PBUF * P_COLS, TMEM_COLS = 512;
   static_assert(T_O + HD <= 512, "tensor memory columns");
   static constexpr int THREADS = 128 + SOFT;
   static constexpr int OFF_Q = 0, OFF_K = HD * kPM * 2, OFF_V = OFF_K + NK * K_CHUNK, OFF_BAR = OFF_V + NV * V_CHUNK;
@@ -87,11 +93,11 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
                   const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ CUtensorMap tm_q2, const __grid_constant__ CUtensorMap tm_g,
                   const PrefillParams p) {
   using L = PfSmem<HD>;
-  constexpr int NK = L::NK, NV = L::NV, SB = L::SBUF, NGRP = L::NGRP, SOFT = L::SOFT;
+  constexpr int NK = L::NK, NV = L::NV, SB = L::SBUF, PB = L::PBUF, NGRP = L::NGRP, SOFT = L::SOFT;
   extern __shared__ __align__(1024) uint8_t base[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + L::OFF_BAR);
-  enum { K_FULL = 0, K_EMPTY = NK, V_FULL = 2 * NK, V_EMPTY = 2 * NK + NV, S_FULL = 2 * NK + 2 * NV, P_FULL = S_FULL + SB, PV_DONE = P_FULL + SB, O_DONE = PV_DONE + 2,
-         Q_FULL = O_DONE + 1, G_FULL = O_DONE + 2, M_READY = O_DONE + 3, N_BARS = M_READY + 2 };
+  enum { K_FULL = 0, K_EMPTY = NK, V_FULL = 2 * NK, V_EMPTY = 2 * NK + NV, S_FULL = 2 * NK + 2 * NV, P_FULL = S_FULL + SB, PV_DONE = P_FULL + PB, O_DONE = PV_DONE + 2,
+         Q_FULL = O_DONE + 1, G_FULL = O_DONE + 2, M_READY = O_DONE + 3, S_READ = M_READY + 2, N_BARS = S_READ + 1 };
   static_assert(N_BARS <= 62, "barrier slots");
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(bars + 62);
   volatile uint32_t* s_err = s_tmem + 1;
@@ -122,7 +128,9 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     *s_err = 0;
     for (int i = 0; i < NK; ++i) { mbar_init(BAR(K_FULL, i), 1); mbar_init(BAR(K_EMPTY, i), 1); }
     for (int i = 0; i < NV; ++i) { mbar_init(BAR(V_FULL, i), 1); mbar_init(BAR(V_EMPTY, i), 1); }
-    for (int i = 0; i < SB; ++i) { mbar_init(BAR(S_FULL, i), 1); mbar_init(BAR(P_FULL, i), 8); }
+    for (int i = 0; i < SB; ++i) mbar_init(BAR(S_FULL, i), 1);
+    for (int i = 0; i < PB; ++i) mbar_init(BAR(P_FULL, i), 8);
+    mbar_init(BAR(S_READ, 0), 8);
     for (int i = 0; i < 2; ++i) { mbar_init(BAR(PV_DONE, i), 1); mbar_init(BAR(M_READY, i), 8); }
     mbar_init(BAR(O_DONE, 0), 1);
     mbar_init(BAR(G_FULL, 0), 1);
@@ -138,7 +146,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
-  const uint32_t t_s0 = tmem + L::T_S, t_o = tmem + L::T_O;
+  const uint32_t t_s0 = tmem + L::T_S, t_p0 = tmem + L::T_P, t_o = tmem + L::T_O;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer, Q and K ----
@@ -221,14 +229,21 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     };
     mbar_wait(BAR(Q_FULL, 0), 0, s_err, WAIT_QFULL);
     tc_fence_after();
+    // Nothing rests on the order in which products of different accumulators run: what a product overwrites has been read.
+    constexpr uint32_t AHEAD = L::ALT ? SB - 1 : 1;
 #pragma unroll 1
-    for (uint32_t j = 0; j < (uint32_t)(SB - 1) && j < n_tiles; ++j) scores(j);
+    for (uint32_t j = 0; j < AHEAD && j < n_tiles; ++j) scores(j);
 #pragma unroll 1
     for (uint32_t j = 0; j < n_tiles; ++j) {
-      // the scores SB - 1 tiles ahead go into the tile whose weights the product just issued reads: in order on the tensor cores
-      if (j + SB - 1 < n_tiles) scores(j + SB - 1);
-      const uint32_t tp = t_s0 + (j % SB) * kPN;     // P(j): packed f16 pairs in the first 32 columns of each half of S(j)'s tile
-      mbar_wait(BAR(P_FULL, j % SB), (j / SB) & 1, s_err, WAIT_MMA);
+      if (j + AHEAD < n_tiles) {
+        // ALT: the scores two tiles ahead take the place of the weights P(j - 1), once the product that reads them has retired.  Otherwise
+        // the next tile's take the place of S(j), which the softmax warps hold in registers while P V(j - 1) runs
+        if (!L::ALT) mbar_wait(BAR(S_READ, 0), j & 1, s_err, WAIT_MMA);
+        else if (j > 0) mbar_wait(BAR(PV_DONE, (j - 1) & 1), ((j - 1) >> 1) & 1, s_err, WAIT_MMA);
+        scores(j + AHEAD);
+      }
+      const uint32_t tp = t_p0 + (j % PB) * L::P_COLS;     // P(j): packed f16 pairs in the first 32 columns of each half
+      mbar_wait(BAR(P_FULL, j % PB), (j / PB) & 1, s_err, WAIT_MMA);
 #pragma unroll
       for (int c = 0; c < L::VC; ++c) {              // O += P(j) V(j)
         mbar_wait(BAR(V_FULL, vst), vph, s_err, WAIT_VFULL);
@@ -236,7 +251,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         const uint64_t vd = v_desc + (uint64_t)(vst * (L::V_CHUNK >> 4));
 #pragma unroll
         for (int ks = 0; ks < L::VK / 16; ++ks)
-          umma_f16_ts(leader, t_o, tp + (c * L::VK + ks * 16) / 64 * 64 + ((c * L::VK / 16 + ks) & 3) * 8, vd + (uint64_t)((ks * 2048) >> 4), idesc_pv, (j > 0 || c > 0 || ks > 0) ? 1u : 0u);
+          umma_f16_ts(leader, t_o, tp + (c * L::VK + ks * 16) / 64 * L::P_HALF + ((c * L::VK / 16 + ks) & 3) * 8, vd + (uint64_t)((ks * 2048) >> 4), idesc_pv, (j > 0 || c > 0 || ks > 0) ? 1u : 0u);
         umma_commit_elected(leader, BAR(V_EMPTY, vst));
         if (++vst == NV) { vst = 0; vph ^= 1; }
       }
@@ -387,15 +402,18 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       l_sum = (s_mx[row] + s_mx[kPM + row]) + (s_mx[2 * kPM + row] + s_mx[3 * kPM + row]);
     } else {
       float2 l2 = make_float2(0.f, 0.f);       // this thread's share of the row's sum
-      uint32_t sb = 0, sph = 0;
+      const uint32_t ts = t_s0 + lane_addr + half * 64;
       for (uint32_t j = 0; j < n_tiles; ++j) {
-        const uint32_t kv0 = key0 + j * kPN + half * 64, ts = t_s0 + sb * kPN + lane_addr + half * 64;
-        mbar_wait(BAR(S_FULL, sb), sph, s_err, WAIT_MMA);
+        const uint32_t kv0 = key0 + j * kPN + half * 64;
+        mbar_wait(BAR(S_FULL, 0), j & 1, s_err, WAIT_MMA);
         tc_fence_after();
         float s[64];
         tmem_ld32_async(ts, s);
         tmem_ld32_async(ts + 32, s + 32);
         tmem_wait_ld(s);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(BAR(S_READ, 0));
         mask(s, 64, kv0);
         // the two halves' maxima through shared memory
         const float m_half = max32(s + 32, max32(s, -INFINITY));
@@ -411,13 +429,16 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         uint32_t pw[32];
         float2 lt = weigh(s, pw);
         lt = add2(lt, weigh(s + 32, pw + 16));
-        tmem_st32u(ts, pw);
+        if (j >= 2) {      // P(j - 2), in the same place, has been read
+          mbar_wait(BAR(PV_DONE, j & 1), ((j >> 1) - 1) & 1, s_err, WAIT_MMA);
+          tc_fence_after();
+        }
+        tmem_st32u(t_p0 + (j & 1) * L::P_COLS + lane_addr + half * L::P_HALF, pw);
         l2 = add2(l2, lt);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(BAR(P_FULL, sb));
-        if (++sb == SB) { sb = 0; sph ^= 1; }
+        if (lane == 0) mbar_arrive(BAR(P_FULL, j & 1));
       }
       float* s_l = s_mx + ((n_tiles & 1) ? 2 * kPM : 0);   // the slot the last tile's maxima are not in
       s_l[wg * kPM + row] = l2.x + l2.y;

@@ -331,3 +331,22 @@ def test_weights_round_in_the_running_reference_of_64_keys(hd, nH, nKV, pos, n_c
     assert (ns > 1) == (pos > 1000)
     ref = _rounded_weights(q, K, V, nH, nKV, hd, pos, ns)
     assert np.linalg.norm(out - ref) / np.linalg.norm(ref) < 8e-5
+
+
+@pytest.mark.parametrize("hd,nH,nKV,pos,n_cols", [(64, 8, 4, 0, 3000), (128, 8, 4, 0, 3000), (256, 8, 4, 0, 3000), (64, 4, 1, 20000, 70), (128, 4, 1, 20000, 70), (256, 4, 1, 20000, 70)])
+def test_many_tiles_repeat_bit_for_bit(hd, nH, nKV, pos, n_cols):
+    # scores and weights of up to 160 tiles take turns in the same tensor-memory columns
+    import torch
+    eng = _engine(nH, nKV, hd, pos + n_cols, act="f32", max_cols=n_cols)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for w in "kv":
+        c = eng.cache(0, w)
+        c.copy_(torch.randn(c.shape, device="cuda", generator=g).half().view(torch.int16))
+    q = torch.randn((n_cols, nH * hd), device="cuda", generator=g).half().float()
+    outs = [eng.prefill(0, 0, pos, q) for _ in range(12)]
+    eng.sync()
+    assert torch.isfinite(outs[0]).all() and all(torch.equal(outs[0], o) for o in outs[1:])
+    K, V = (eng.cache(0, w)[0].cpu().numpy().view(np.uint16) for w in "kv")
+    last = [n_cols - 1]
+    ref = po.attn_f64(q[last].cpu().numpy(), K, V, nH, nKV, hd, pos + n_cols - 1, 1)
+    util.assert_close(outs[0][last].cpu().numpy(), ref, "last column")
