@@ -17,7 +17,7 @@
 // which scores and P V are not.  At head_dim 256 the next scores take the place of scores that the softmax warps have taken into registers, and P
 // has two tiles of its own: no wait in the stream (4 layers of 8192 columns of 24 heads 3270 us, as with two S tiles that P overwrites and
 // nothing but that order).  At 128 and 64, where a thread has no room for its scores, P lies over S, and S(j + 2) waits for the P V(j - 1)
-// that reads it: 318 -> 338 us (8192 columns of 16 heads x 128; 8 layers of 2999 571 -> 596; scores in registers all the same, with spills, 332), 266 both at 64.
+// that reads it: 318 -> 338 us (8192 columns of 16 heads x 128; 8 layers of 2999 571 -> 592; scores in registers all the same, with spills, 332), 266 both at 64.
 //
 // O is rescaled only when a row's running maximum has grown by more than 2^8 since its last rescale (weights stay below
 // 2^8, exact in f32 sums and safe in f16); the rescale waits for the previous P V to retire and rewrites the row in TMEM.
@@ -198,7 +198,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       prefetch_tmap(&tm_v);
       uint32_t st = 0, ph = 1;
       for (uint32_t j = 0; j < n_tiles; ++j) {
-        for (int c = 0; c < L::VC; ++c) {
+        for (int c = 0; c < L::VC && key0 + j * kPN + c * L::VK < key_end; ++c) {      // (every chunk is waited for: the epilogue uses the ring)
           mbar_wait(BAR(V_EMPTY, st), ph, s_err, WAIT_EMPTY);
           mbar_expect_tx(BAR(V_FULL, st), L::V_CHUNK);
           tma_load_3d(v_s + st * L::V_CHUNK, &tm_v, 0, (int)(key0 + j * kPN + c * L::VK), (int)(g * L::KC), BAR(V_FULL, st));
@@ -233,16 +233,23 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     constexpr uint32_t AHEAD = L::ALT ? SB - 1 : 1;
 #pragma unroll 1
     for (uint32_t j = 0; j < AHEAD && j < n_tiles; ++j) scores(j);
+    auto ahead = [&](uint32_t j) {
+      if (j + AHEAD >= n_tiles) return;
+      // ALT: the scores two tiles ahead take the place of the weights P(j - 1), once the product that reads them has retired.  Otherwise
+      // the next tile's take the place of S(j), which the softmax warps hold in registers while P V(j - 1) runs
+      if (!L::ALT) mbar_wait(BAR(S_READ, 0), j & 1, s_err, WAIT_MMA);
+      else if (j > 0) mbar_wait(BAR(PV_DONE, (j - 1) & 1), ((j - 1) >> 1) & 1, s_err, WAIT_MMA);
+      scores(j + AHEAD);
+    };
+    // P(j): packed f16 pairs in the first 32 columns of each half; 16 keys of them
+    auto p_at = [&](uint32_t j, int k16) { return t_p0 + (j % PB) * L::P_COLS + (k16 >> 2) * L::P_HALF + (k16 & 3) * 8; };
+    // The last tile's product goes no further than the 16 keys that hold the CTA's last: a weight of zero times an infinite value of
+    // a later row is NaN.  In a loop of its own, since the others' issue bears no test between products (2999 columns of 16
+    // heads x 128, 8 layers: 592 us; 612 with a branch per product, 654 with the test in the product's predicate).
+    const uint32_t whole = (key_end - key0 + 15) / kPN;
 #pragma unroll 1
-    for (uint32_t j = 0; j < n_tiles; ++j) {
-      if (j + AHEAD < n_tiles) {
-        // ALT: the scores two tiles ahead take the place of the weights P(j - 1), once the product that reads them has retired.  Otherwise
-        // the next tile's take the place of S(j), which the softmax warps hold in registers while P V(j - 1) runs
-        if (!L::ALT) mbar_wait(BAR(S_READ, 0), j & 1, s_err, WAIT_MMA);
-        else if (j > 0) mbar_wait(BAR(PV_DONE, (j - 1) & 1), ((j - 1) >> 1) & 1, s_err, WAIT_MMA);
-        scores(j + AHEAD);
-      }
-      const uint32_t tp = t_p0 + (j % PB) * L::P_COLS;     // P(j): packed f16 pairs in the first 32 columns of each half
+    for (uint32_t j = 0; j < whole; ++j) {
+      ahead(j);
       mbar_wait(BAR(P_FULL, j % PB), (j / PB) & 1, s_err, WAIT_MMA);
 #pragma unroll
       for (int c = 0; c < L::VC; ++c) {              // O += P(j) V(j)
@@ -251,11 +258,25 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         const uint64_t vd = v_desc + (uint64_t)(vst * (L::V_CHUNK >> 4));
 #pragma unroll
         for (int ks = 0; ks < L::VK / 16; ++ks)
-          umma_f16_ts(leader, t_o, tp + (c * L::VK + ks * 16) / 64 * L::P_HALF + ((c * L::VK / 16 + ks) & 3) * 8, vd + (uint64_t)((ks * 2048) >> 4), idesc_pv, (j > 0 || c > 0 || ks > 0) ? 1u : 0u);
+          umma_f16_ts(leader, t_o, p_at(j, c * L::VK / 16 + ks), vd + (uint64_t)((ks * 2048) >> 4), idesc_pv, (j > 0 || c > 0 || ks > 0) ? 1u : 0u);
         umma_commit_elected(leader, BAR(V_EMPTY, vst));
         if (++vst == NV) { vst = 0; vph ^= 1; }
       }
       umma_commit_elected(leader, BAR(PV_DONE, j & 1));
+    }
+    if (whole < n_tiles) {
+      const uint32_t j = whole, steps = (key_end - key0 - j * kPN + 15) / 16;
+      mbar_wait(BAR(P_FULL, j % PB), (j / PB) & 1, s_err, WAIT_MMA);
+#pragma unroll 1
+      for (int k16 = 0; k16 < (int)steps; ++k16) {
+        if (k16 % (L::VK / 16) == 0) {
+          if (k16 > 0 && ++vst == NV) { vst = 0; vph ^= 1; }
+          mbar_wait(BAR(V_FULL, vst), vph, s_err, WAIT_VFULL);
+          tc_fence_after();
+        }
+        umma_f16_ts(leader, t_o, p_at(j, k16), v_desc + (uint64_t)(vst * (L::V_CHUNK >> 4)) + (uint64_t)((k16 % (L::VK / 16) * 2048) >> 4), idesc_pv,
+                    (j > 0 || k16 > 0) ? 1u : 0u);
+      }
     }
     umma_commit_elected(leader, BAR(O_DONE, 0));
   } else if (warp >= 4) {

@@ -350,3 +350,25 @@ def test_many_tiles_repeat_bit_for_bit(hd, nH, nKV, pos, n_cols):
     last = [n_cols - 1]
     ref = po.attn_f64(q[last].cpu().numpy(), K, V, nH, nKV, hd, pos + n_cols - 1, 1)
     util.assert_close(outs[0][last].cpu().numpy(), ref, "last column")
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("pos,n_cols,bad", [(1, 256, 144), (1, 300, 200), (0, 300, 130), (70, 250, 208), (3000, 260, 3136)])
+def test_infinite_values_of_later_rows_stay_out_of_earlier_tiles(hd, pos, n_cols, bad):
+    # the columns of the first 128 do not see row `bad`, nor do the 16 rows that hold the last that one of them sees: an infinity there leaves
+    # them as they are, bit for bit
+    import torch
+    nH, nKV = 4, 2
+    assert bad >= (pos + 128 + 15) // 16 * 16
+    eng = _engine(nH, nKV, hd, pos + n_cols, act="f32", max_cols=512)
+    g = torch.Generator(device="cuda").manual_seed(6)
+    for w in "kv":
+        c = eng.cache(0, w)
+        c.copy_(torch.randn(c.shape, device="cuda", generator=g).half().view(torch.int16))
+    q = torch.randn((n_cols, nH * hd), device="cuda", generator=g).half().float()
+    want = eng.prefill(0, 0, pos, q)
+    eng.cache(0, "v")[0, bad:bad + 8] = 0x7c00
+    got = eng.prefill(0, 0, pos, q)
+    eng.sync()
+    assert torch.isfinite(want).all() and torch.equal(got[:128], want[:128])
+    assert not torch.isfinite(got[bad - pos:]).all()
