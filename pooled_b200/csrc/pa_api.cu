@@ -1187,13 +1187,13 @@ static int prefill_impl(pa_layer* L, uint32_t seq, uint32_t pos, uint32_t n_cols
   // few columns behind many keys: the keys are split and the records merged by a second kernel
   p.n_splits = ctx->core_only ? 1u : prefill_splits(p.pos, n_cols, p.n_heads, ctx->cfg.head_dim, (uint32_t)ctx->sm_count, ctx->pf_slots);
   p.part_o = ctx->part_o; p.part_ml = ctx->part_ml; p.sms = (uint32_t)ctx->sm_count;
-  // ... and f16 output tiles leave by TMA (any head_dim the kernel takes; the gate's, if any, arrive so)
+  // ... and f16 output tiles leave by TMA and gate tiles arrive so (any head_dim the kernel takes), each where a map takes its strides
   CUtensorMap tm_o = tm_k, tm_g = tm_k;
-  if (ctx->cfg.act_dtype == PA_F16 && !(ocs & 63) && !ctx->tune.no_out_tma && (!gate || rows_tma_ok(ctx, gate, gcs, ghs))) {
-    if (gate) {
-      if (int rc = make_cache_map(ctx, &tm_g, const_cast<void*>(gate), n_cols, (uint32_t)gcs, ctx->cfg.head_dim, 128)) return rc;
-      p.gate_tma = 1;
-    }
+  if (ctx->cfg.act_dtype == PA_F16 && gate && rows_tma_ok(ctx, gate, gcs, ghs) && !ctx->tune.no_out_tma) {
+    if (int rc = make_cache_map(ctx, &tm_g, const_cast<void*>(gate), n_cols, (uint32_t)gcs, ctx->cfg.head_dim, 128)) return rc;
+    p.gate_tma = 1;
+  }
+  if (ctx->cfg.act_dtype == PA_F16 && !(ocs & 63) && !ctx->tune.no_out_tma) {
     if (int rc = make_cache_map(ctx, &tm_o, out, n_cols, (uint32_t)ocs, ctx->cfg.head_dim, 128)) return rc;
     p.out_tma = 1;
   }

@@ -193,7 +193,7 @@ struct PrefillParams {
                                 // (the caller's own q, head stride q2_head_stride: unrotated dims are not copied anywhere)
   uint32_t q_rot_chunks; uint64_t q2_head_stride;
   uint32_t sms;                 // prefill: SMs of the device, the CTAs that run together
-  uint32_t gate_tma;            // prefill, with out_tma: the gate's rows come by TMA (tm_g)
+  uint32_t gate_tma;            // prefill, f16 gate: its 128 rows come by TMA (tm_g)
   uint32_t out_tma;             // prefill, f16 out: the CTA's output tile leaves through shared memory by one TMA store (tm_o)
 };
 

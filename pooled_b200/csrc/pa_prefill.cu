@@ -287,6 +287,10 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     const bool live = row < rows_valid;
     const uint32_t lim = min(p0 + row + 1, key_end);     // of the CTA's keys those below lim are visible to this row
     pdl_trigger();
+    const __half* gate_row = reinterpret_cast<const __half*>(p.gate) + (uint64_t)(c0 + row) * p.gate_col_stride + (uint64_t)h * p.gate_head_stride;
+    const bool by_pieces = p.act_f16 && (!p.gate || p.gate_tma || !(((uintptr_t)p.gate & 15) | (p.gate_col_stride & 7) | (p.gate_head_stride & 7)));
+    if (!SPLIT && by_pieces && p.gate && !p.gate_tma && live)      // a lane's own row of the gate, for the end
+      for (uint32_t d = wg * 64; d < HD; d += NGRP * 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(gate_row + d));
     if (!q_by_tma) {
       // this thread's share of its Q row as f16 into the layout the score products read
       constexpr int PC = HD / 8 / NGRP;                  // 16-byte pieces
@@ -494,25 +498,31 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         const uint64_t slot = ((uint64_t)col * p.n_heads + h) * p.n_splits + blockIdx.z;
         p.part_ml[slot * 2] = m_st * 0.6931471805599453f; p.part_ml[slot * 2 + 1] = l_sum;
       }
-    } else if (p.out_tma) {
-      // The output tile leaves as the query tile came: through shared memory in the TMA layout ([64-dim chunk][row][128 B],
+    } else if (by_pieces) {
+      // f16: the output tile leaves as the query tile came: through shared memory in the TMA layout ([64-dim chunk][row][128 B],
       // 16-byte pieces XOR-swizzled by the row), one bulk tensor store for the CTA, from the V ring (every product
       // has retired).  Rows past the prompt's end are not written: the map ends at n_cols.
-      // (A lane storing its own row issues 16-byte stores 12 KB apart.)
+      // (A lane storing its own row issues 16-byte stores 12 KB apart.)  Where no map takes the output's stride, the threads store whole rows.
       uint8_t* o_s = base + L::OFF_V;
-      if (p.gate) mbar_wait(BAR(G_FULL, 0), 0, s_err, WAIT_QFULL);
+      const uint4* gp = reinterpret_cast<const uint4*>(gate_row);
+      if (p.gate_tma) mbar_wait(BAR(G_FULL, 0), 0, s_err, WAIT_QFULL);
 #pragma unroll 1
       for (uint32_t c = wg; c < HD / 32; c += NGRP) {            // the groups share the columns out
+        const uint32_t at = (c >> 1) * (kPM * 128) + row * 128;
+        uint4 gq[4];      // (a gate no tensor map takes: each lane its own row)
+        if (p.gate) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            gq[i] = p.gate_tma ? *reinterpret_cast<const uint4*>(base + L::OFF_K + at + ((((c & 1) * 4 + i) ^ (row & 7)) << 4)) : live ? gp[c * 4 + i] : make_uint4(0, 0, 0, 0);
+        }
         float o[32];
         tmem_ld32(t_o + c * 32 + lane_addr, o);
 #pragma unroll
         for (int i = 0; i < 32; ++i) o[i] *= inv_l;
-        const uint32_t at = (c >> 1) * (kPM * 128) + row * 128;
         if (p.gate) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const uint4 gq = *reinterpret_cast<const uint4*>(base + L::OFF_K + at + ((((c & 1) * 4 + i) ^ (row & 7)) << 4));
-            const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
+            const uint32_t gw[4] = {gq[i].x, gq[i].y, gq[i].z, gq[i].w};
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               const float2 gv = __half22float2(*reinterpret_cast<const __half2*>(&gw[k]));
@@ -526,15 +536,21 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
           *reinterpret_cast<uint4*>(o_s + at + ((((c & 1) * 4 + i) ^ (row & 7)) << 4)) =
               make_uint4(pack_h2(o[8 * i], o[8 * i + 1]), pack_h2(o[8 * i + 2], o[8 * i + 3]), pack_h2(o[8 * i + 4], o[8 * i + 5]), pack_h2(o[8 * i + 6], o[8 * i + 7]));
       }
-      fence_proxy_async();
+      if (p.out_tma) fence_proxy_async();
       named_bar_sync(1, SOFT);
-      if (tid == 128) {
+      if (!p.out_tma) {
+        for (uint32_t idx = tid - 128; idx < rows_valid * (HD / 8); idx += SOFT) {
+          const uint32_t rr = idx / (HD / 8), pc = idx % (HD / 8);
+          *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(p.out) + (uint64_t)(c0 + rr) * p.out_col_stride + (uint64_t)h * HD + pc * 8) =
+              *reinterpret_cast<const uint4*>(o_s + (pc >> 3) * (kPM * 128) + rr * 128 + (((pc & 7) ^ (rr & 7)) << 4));
+        }
+      } else if (tid == 128) {
         tma_store_3d(&tm_o, 0, (int)c0, (int)(h * (HD / 64)), smem_u32(o_s));
         tma_store_wait_read();
       }
     } else {
-      // f32 activations, or strides no tensor map takes: the rows by way of shared memory, so that gate loads and output stores
-      // are whole rows too
+      // f32 activations, or a gate that is not read 16 bytes at a time: the rows by way of shared memory, so that gate loads and output
+      // stores are whole rows too
       constexpr int RP = HD / 4 + 1, U = L::ALT ? 4 : 8;
       float4* xs = reinterpret_cast<float4*>(base + L::OFF_K);
 #pragma unroll 1

@@ -372,3 +372,34 @@ def test_infinite_values_of_later_rows_stay_out_of_earlier_tiles(hd, pos, n_cols
     eng.sync()
     assert torch.isfinite(want).all() and torch.equal(got[:128], want[:128])
     assert not torch.isfinite(got[bad - pos:]).all()
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("act", ["f16", "f32"])
+@pytest.mark.parametrize("n_cols", [100, 300])
+def test_prompts_of_any_stride_carry_the_same_bits(hd, act, n_cols):
+    # tiles of q, gate and output travel by tensor map, by lanes and by rows, each as its stride and alignment allow
+    import torch
+    nH, nKV, pos = 4, 2, 37
+    td = torch.float16 if act == "f16" else torch.float32
+    eng = _engine(nH, nKV, hd, pos + n_cols, act=act, max_cols=512)
+    g = torch.Generator(device="cuda").manual_seed(8)
+    for w in "kv":
+        c = eng.cache(0, w)
+        c.copy_(torch.randn(c.shape, device="cuda", generator=g).half().view(torch.int16))
+    q, gate = (torch.randn((n_cols, nH * hd), device="cuda", generator=g).to(td) for _ in range(2))
+    def at(x, pad, skip=0):      # the same values, rows `pad` values further apart, `skip` past an aligned address
+        buf = torch.full((n_cols * (nH * hd + pad) + 64,), float("nan"), device="cuda", dtype=td)
+        v = buf[skip:skip + n_cols * (nH * hd + pad)].view(n_cols, -1)[:, :nH * hd]
+        return v.copy_(x), buf
+    for gt in (None, gate):
+        want = eng.prefill(0, 0, pos, q, gt).clone()
+        ref = po.attn_f64(q.float().cpu().numpy(), *(eng.cache(0, w)[0].cpu().numpy().view(np.uint16) for w in "kv"), nH, nKV, hd, pos, n_cols, None if gt is None else gt.float().cpu().numpy())
+        util.assert_close(want.float().cpu().numpy(), ref, f"{act} {hd}")
+        for qp, op in ((0, 8), (8, 0), (64, 72)):
+            for gp, skip in ((0, 0), (8, 0), (8, 8), (4, 0), (0, 2), (5, 1)) if gt is not None else ((0, 0),):
+                out, buf = at(torch.zeros_like(want), op)
+                got = eng.prefill(0, 0, pos, at(q, qp)[0], None if gt is None else at(gt, gp, skip)[0], out=out)
+                eng.sync()
+                assert torch.equal(got, want), (qp, op, gp, skip)
+                assert torch.isnan(buf).sum() == buf.numel() - want.numel()      # nothing written between the rows
