@@ -14,12 +14,12 @@ __device__ __forceinline__ void fma4(float4& acc, const float4& x, float w) {
 
 // Records that the CTAs of one call leave for one another say themselves when they are there: every 32-bit word of the buffer holds
 // kNoWord until its value is stored, a reader repeats its loads until no word of them does, and puts kNoWord back for the next call
-// (whose CTAs write after this call's end).  A 32-bit word lands whole, so nothing else orders the two sides: with a fence behind
+// (whose CTAs write after this call's end).  Both sides use relaxed accesses of whole 32-bit words, which land whole, and nothing else orders them: with a fence behind
 // the records, a count and a wait for it ahead of the first load, three more trips to L2 stood between a CTA's last product and its merge
 // (ten layers of a token over 32768 rows, 16 / 2 heads x 256: 200 us with them, 185 without; 16 over 4099 rows, 24 / 4 x 256, host
 // buffers: 235 and 209).  A value that has kNoWord's bits (a NaN no instruction here produces) is stored as the ordinary NaN.
 constexpr uint32_t kNoWord = 0xffffffffu;
-__device__ __forceinline__ float word_for(float x) { return __float_as_uint(x) == kNoWord ? __uint_as_float(0x7fffffffu) : x; }
+__device__ __forceinline__ uint32_t word_for(float x) { return __float_as_uint(x) == kNoWord ? 0x7fffffffu : __float_as_uint(x); }
 __device__ __forceinline__ uint4 ld_words4(const float* p) {
   uint4 v;
   asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
@@ -29,6 +29,12 @@ __device__ __forceinline__ uint2 ld_words2(const float* p) {
   uint2 v;
   asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
   return v;
+}
+__device__ __forceinline__ void st_words4(float* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void st_words2(float* p, uint32_t a, uint32_t b) {
+  asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(a), "r"(b) : "memory");
 }
 __device__ __forceinline__ bool all_words(const uint4& v) { return v.x != kNoWord && v.y != kNoWord && v.z != kNoWord && v.w != kNoWord; }
 __device__ __forceinline__ float4 as_float4(const uint4& v) { return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)); }
@@ -45,7 +51,6 @@ __device__ __forceinline__ void merge_slice_128(float* o_rec, float* ml_rec, siz
                                                 float gv, bool empty_is_zero, int act_f16, void* out, uint64_t oo, volatile uint32_t* s_err) {
   const int wv = t >> 5, lane = t & 31, ln = t & 15, gA = t >> 4;
   float* ob = o_rec + ln * 4;
-  const uint4 none = make_uint4(kNoWord, kNoWord, kNoWord, kNoWord);
   // everything is requested before the first use, and whatever was not there yet once more
   uint4 xw[16];          // records gA + 8 i of this thread's four dims
   uint2 mw[4];
@@ -71,10 +76,10 @@ __device__ __forceinline__ void merge_slice_128(float* o_rec, float* ml_rec, siz
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     mv[k] = __uint_as_float(mw[k].x); lv[k] = __uint_as_float(mw[k].y);
-    if ((mine >> (16 + k)) & 1u) *reinterpret_cast<uint2*>(ml_rec + (size_t)(t + 128 * k) * stride) = make_uint2(kNoWord, kNoWord);
+    if ((mine >> (16 + k)) & 1u) st_words2(ml_rec + (size_t)(t + 128 * k) * stride, kNoWord, kNoWord);
   }
 #pragma unroll
-  for (int i = 0; i < 16; ++i) if ((mine >> i) & 1u) *reinterpret_cast<uint4*>(ob + (size_t)(gA + 8 * i) * stride) = none;
+  for (int i = 0; i < 16; ++i) if ((mine >> i) & 1u) st_words4(ob + (size_t)(gA + 8 * i) * stride, kNoWord, kNoWord, kNoWord, kNoWord);
   float M = fmaxf(fmaxf(mv[0], mv[1]), fmaxf(mv[2], mv[3]));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
@@ -122,7 +127,7 @@ __device__ __forceinline__ void merge_slice_128(float* o_rec, float* ml_rec, siz
             if (polls > kMergePolls) *s_err = WAIT_MERGE;
             if (polls > 16) __nanosleep(32);
           }
-          *reinterpret_cast<uint4*>(ob + (size_t)s * stride) = none;
+          st_words4(ob + (size_t)s * stride, kNoWord, kNoWord, kNoWord, kNoWord);
         }
         fma4(acc, as_float4(x), s < ns ? sc.w[s] : 0.f);
       }
@@ -153,8 +158,8 @@ __host__ __device__ constexpr size_t merge_block(int hd, int rows) { return ((si
 template <int HD>
 __device__ __forceinline__ void put_record4(float* blk, uint32_t rows, uint32_t row, uint32_t c4, float4 x, float m, float l) {
   static_assert(HD % 4 == 0 && merge_block(HD, 1) % 4 == 0 && merge_block(HD, 2) % 4 == 0, "records are read and written 16 bytes at a time");
-  if (c4 % 16 == 0) *reinterpret_cast<float2*>(blk + (size_t)rows * HD + (row * (HD / 64) + c4 / 16) * 2) = make_float2(word_for(m), word_for(l));
-  reinterpret_cast<float4*>(blk + (size_t)row * HD)[c4] = make_float4(word_for(x.x), word_for(x.y), word_for(x.z), word_for(x.w));
+  if (c4 % 16 == 0) st_words2(blk + (size_t)rows * HD + (row * (HD / 64) + c4 / 16) * 2, word_for(m), word_for(l));
+  st_words4(blk + (size_t)row * HD + c4 * 4, word_for(x.x), word_for(x.y), word_for(x.z), word_for(x.w));
 }
 
 }  // namespace pa

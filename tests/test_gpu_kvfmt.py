@@ -419,3 +419,20 @@ def test_f32_records_of_one_head_of_64_dims(nH, nKV, n_cols, ctx, monkeypatch):
         outs.append([x.cpu().numpy() for x in o])
     assert all(np.isfinite(a).all() and np.array_equal(a, b) for a, b in zip(*outs))
     assert util.errs(outs[0][-3], po.attn_f64_kv32(q.cpu().numpy(), K.cpu().numpy(), V.cpu().numpy(), nH, nKV, hd, ctx[-1] - n_cols, n_cols, None))[1] < util.REF_REL
+
+
+@pytest.mark.parametrize("fmt", ["f16", "f32"])
+def test_merged_records_of_many_calls_keep_their_bits(fmt):
+    # calls of different plans, one straight behind the other, through the one buffer of records that say themselves when they are there
+    import torch
+    nH, nKV, hd, ctx = 4, 2, 128, (9000, 3001, 12000, 7777)
+    eng = _engine(fmt, nH, nKV, hd, max(ctx))
+    g = torch.Generator(device="cuda").manual_seed(9)
+    for w in "kv":
+        c = eng.cache(0, w)
+        x = torch.randn(c.shape, device="cuda", generator=g)
+        c.copy_(x.half().view(torch.int16) if fmt == "f16" else x)
+    q = torch.randn((1, nH * hd), device="cuda", generator=g)
+    outs = [eng.decode(0, [(0, n - 1, 1)], q) for _ in range(60) for n in ctx]
+    eng.sync()
+    assert torch.isfinite(torch.stack(outs)).all() and all(torch.equal(o, outs[i % len(ctx)]) for i, o in enumerate(outs))
