@@ -275,7 +275,11 @@ PA_API int pa_shared_close(pa_ctx* ctx, void* dev_ptr);
 PA_API int pa_exchange_init(pa_ctx* ctx, uint32_t rank, uint32_t world, void* const* bufs, uint32_t max_rows);
 /* Limit of the polling loop in which an exchanging call waits for the other ranks' records (sweeps over the missing
  * entries; 0 restores the built-in 2^20, about a second).  When it runs out the kernel records status 7, finishes with
- * what it has, and pa_sync reports PA_ETIMEOUT: a peer that died between steps costs one bounded wait, not a hang. */
+ * what it has, and pa_sync reports PA_ETIMEOUT: a peer that died between steps costs one bounded wait, not a hang.
+ * The same limit (0: 2^20 looks, about a second) bounds the wait of a single-token call over an f16 cache for the records of its own
+ * CTAs, which need an SM each at the same time: beside a longer kernel of another stream that leaves them none it
+ * ends with status 8 and PA_ETIMEOUT.  Calls over f32 caches wait no more than 2^12 looks, or this limit if that is less, and
+ * then leave their share to the CTA that finishes last: they need no SM of their own and only take longer. */
 PA_API int pa_set_wait_limit(pa_ctx* ctx, uint32_t sweeps);
 /* pa_decode over this rank's shard with the cross-GPU merge inside the combine kernel: each CTA stores its merged
  * (o, m, l) slice into every rank's exchange buffer over NVLink, each value as one 8-byte {value, call tag} store,

@@ -521,7 +521,7 @@ class AttnEngine:
         self._xc_keep = None
 
     def set_wait_limit(self, sweeps: int):
-        """Polling limit of the cross-GPU exchange wait (0: the built-in limit, about a second)."""
+        """Polling limit of the waits for other GPUs' and a call's own CTAs' records (0: the built-in limits, about a second)."""
         self._ck(self.L.pa_set_wait_limit(self.ctx, sweeps))
 
     def decode_exchange(self, li: int, items, q: torch.Tensor, gate: torch.Tensor | None = None, out: torch.Tensor | None = None,

@@ -206,12 +206,15 @@ extern "C" int pa_create(int device, const pa_config* cfg, pa_ctx** out) {
   ctx->merge_bytes = (size_t)ctx->sm_count * 16 * (cfg->head_dim + cfg->head_dim / 32) * 4;   // one CTA per SM, at most 16 query rows each
   if ((e = cudaMalloc(&ctx->merge_rec, ctx->merge_bytes)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(merge records)", e);
   if ((e = cudaMemset(ctx->merge_rec, 0xff, ctx->merge_bytes)) != cudaSuccess) return bail(PA_ECUDA, "cudaMemset(merge records)", e);
+  if ((e = cudaMalloc(&ctx->merge_ctr, ctx->sm_count * 8)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(merge counters)", e);
+  if ((e = cudaMemset(ctx->merge_ctr, 0, ctx->sm_count * 8)) != cudaSuccess) return bail(PA_ECUDA, "cudaMemset(merge counters)", e);
   if ((e = cudaMalloc(&ctx->dev_err, 4)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMalloc(err)", e);
   if ((e = cudaMemset(ctx->dev_err, 0, 4)) != cudaSuccess) return bail(PA_ECUDA, "cudaMemset(err)", e);
   if ((e = cudaMallocHost(&ctx->host_err, 4)) != cudaSuccess) return bail(PA_ENOMEM, "cudaMallocHost(err)", e);
   if ((e = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking)) != cudaSuccess) return bail(PA_ECUDA, "cudaStreamCreate", e);
   for (cudaEvent_t& v : ctx->side_ev)
     if ((e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming)) != cudaSuccess) return bail(PA_ECUDA, "cudaEventCreate", e);
+  if ((e = cudaStreamSynchronize(nullptr)) != cudaSuccess) return bail(PA_ECUDA, "cudaStreamSynchronize", e);   // the buffers above are set before any stream uses them
   *ctx->host_err = 0;
   *out = ctx;
   return PA_OK;
@@ -220,7 +223,7 @@ extern "C" int pa_create(int device, const pa_config* cfg, pa_ctx** out) {
 extern "C" int pa_destroy(pa_ctx* ctx) {
   if (!ctx) return PA_OK;
   cudaSetDevice(ctx->device);
-  cudaFree(ctx->inv_freq); cudaFree(ctx->angles); cudaFree(ctx->norm_q); cudaFree(ctx->norm_k); cudaFree(ctx->q_rot); cudaFree(ctx->k_rot); cudaFree(ctx->part_o); cudaFree(ctx->part_ml); cudaFree(ctx->dev_err); cudaFree(ctx->merge_rec);
+  cudaFree(ctx->inv_freq); cudaFree(ctx->angles); cudaFree(ctx->norm_q); cudaFree(ctx->norm_k); cudaFree(ctx->q_rot); cudaFree(ctx->k_rot); cudaFree(ctx->part_o); cudaFree(ctx->part_ml); cudaFree(ctx->dev_err); cudaFree(ctx->merge_rec); cudaFree(ctx->merge_ctr);
   cudaFree(ctx->stage_dev);
   for (cudaEvent_t e : ctx->side_ev) if (e) cudaEventDestroy(e);
   if (ctx->side) cudaStreamDestroy(ctx->side);
@@ -341,7 +344,8 @@ extern "C" int pa_reset(pa_ctx* ctx) {
   if (!ctx) return PA_EINVAL;
   cudaGetLastError();
   if (cudaDeviceSynchronize() != cudaSuccess || cudaMemset(ctx->dev_err, 0, 4) != cudaSuccess ||
-      cudaMemset(ctx->merge_rec, 0xff, ctx->merge_bytes) != cudaSuccess)
+      cudaMemset(ctx->merge_rec, 0xff, ctx->merge_bytes) != cudaSuccess || cudaMemset(ctx->merge_ctr, 0, ctx->sm_count * 8) != cudaSuccess ||
+      cudaDeviceSynchronize() != cudaSuccess)
     return fail(ctx, PA_ECUDA, "pa_reset: the device does not answer");
   *ctx->host_err = 0;
   ctx->failed = false;
@@ -829,6 +833,7 @@ static int decode_any_impl(pa_layer* L, const pa_item* items, uint32_t n_items, 
         f.out = reinterpret_cast<uint8_t*>(out) + (col + c0) * ocs * aes; f.out_col_stride = ocs; f.act_f16 = ctx->cfg.act_dtype == PA_F16;
         // one wave of CTAs (one per SM) merges its records itself
         if (!f.cluster && !ctx->core_only && !ctx->tune.no_merge && (uint64_t)live * ctx->cfg.n_kv_heads * nc <= (uint64_t)ctx->sm_count) f.merge_rec = ctx->merge_rec;
+        f.merge_ctr = ctx->merge_ctr; f.merge_polls = ctx->tune.wait_polls ? std::min(ctx->tune.wait_polls, kMergeLeave) : kMergeLeave;
         f.err = ctx->dev_err;
         merged = f.cluster != 0 || f.merge_rec;
         f.q = reinterpret_cast<const uint8_t*>(q) + (col + c0) * qcs * qes; f.q_f16 = q_dtype == PA_F16; f.q_col_stride = qcs; f.q_head_stride = qhs;
@@ -1020,7 +1025,7 @@ static int decode_impl(pa_layer* L, const pa_item* items, uint32_t n_items, cons
                        ns <= (uint32_t)kMaxCluster;
   if (cluster) while (ns & (ns - 1)) ++ns;      // 1, 2, 4 or 8 CTAs (those without a tile leave at once); the plan is p.n_splits'
   if (merge || cluster) {
-    p.merge = cluster ? 3u : 2u; p.merge_rec = ctx->merge_rec;
+    p.merge = cluster ? 3u : 2u; p.merge_rec = ctx->merge_rec; p.merge_polls = ctx->tune.wait_polls ? ctx->tune.wait_polls : kMergePolls;
     p.gate = gate; p.gate_col_stride = gcs; p.gate_head_stride = ghs; p.out = out; p.out_col_stride = ocs; p.act_f16 = ctx->cfg.act_dtype == PA_F16;
   }
   // an exchanging call numbers itself ahead of its combine kernel: in the decode kernel where that runs

@@ -20,6 +20,8 @@ namespace pa {
 // error word and carries on as if the wait had succeeded, so control flow stays uniform, every thread
 // reaches the end of the kernel and the host reports PA_ETIMEOUT instead of a hung GPU.
 constexpr uint32_t kWaitPolls = 1u << 24;  // with 32..64 ns back-off: well under a second
+constexpr uint32_t kMergePolls = 1u << 20; // looks for another CTA's record: about a second
+constexpr uint32_t kMergeLeave = 1u << 12; // ... before a unit is left to the CTA that comes last (f32 tokens): some milliseconds
 
 enum : uint32_t { WAIT_KFULL = 1, WAIT_VFULL = 2, WAIT_EMPTY = 3, WAIT_MMA = 4, WAIT_TMEM = 5, WAIT_QFULL = 6, WAIT_PEER = 7, WAIT_MERGE = 8 };
 
@@ -395,6 +397,7 @@ struct pa_ctx {
   size_t pf_slots = 0;         // records the partial buffers hold, and a split prefill may use
   float* merge_rec = nullptr;    // device: the records of a decode call that merges them itself, a block per CTA; all bits set between calls
   size_t merge_bytes = 0;
+  unsigned int* merge_ctr = nullptr;   // device: two words for each SM (see pa_decode_f32_kernel), zero between calls
   uint32_t* dev_err = nullptr;   // device error word (bounded waits)
   uint32_t* host_err = nullptr;  // pinned mirror
   void* norm_q = nullptr;        // normed q / k of the current layer call (act_dtype, [max_cols][q_dim] / [max_cols][kv_dim])
@@ -421,7 +424,7 @@ struct pa_ctx {
     bool no_out_tma = false;     // POOLED_ATTN_NO_OUT_TMA=1: ... and its output rows by per-thread stores
     bool kv_evict_first = true;  // POOLED_ATTN_KV_EVICT_FIRST=0: decode / verify K and V tiles enter L2 with the default policy instead of evict-first
     bool no_merge = false;       // POOLED_ATTN_NO_MERGE: always merge the split records in the combine kernel
-    uint32_t wait_polls = 0;     // pa_set_wait_limit: limit of the cross-GPU exchange wait (0: the built-in limit)
+    uint32_t wait_polls = 0;     // pa_set_wait_limit: limit of the waits for other CTAs' and other GPUs' records (0: the built-in limits)
   } tune;
   bool failed = false;
   std::string err;

@@ -1145,8 +1145,8 @@ pa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       unit_addr(u, slice, go, oo);
       const float gv = (u == split) ? gv0 : ((gated && ltid < 64) ? gate_ld(go) : 0.f);
       const uint32_t row = u / (HD / 64);
-      merge_slice_128<HD>(blk0 + (size_t)row * HD + slice * 64, blk0 + ROWS * HD + (row * (HD / 64) + slice) * 2, BLK, ns_live, ltid, sc, gbar, gated, gv,
-                          p.gather != nullptr, p.act_f16, p.out, oo, s_err);
+      merge_slice_128<HD, false>(blk0 + (size_t)row * HD + slice * 64, blk0 + ROWS * HD + (row * (HD / 64) + slice) * 2, BLK, ns_live, ltid, sc, gbar, gated, gv,
+                                 p.gather != nullptr, p.act_f16, p.out, oo, p.merge_polls, s_err);
     }
   }
   if (*s_err && tid == 0) atomicMax(p.err, *s_err);

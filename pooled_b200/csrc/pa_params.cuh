@@ -41,6 +41,7 @@ struct DecodeParams {
   // merge != 0: no combine kernel follows; the CTAs of each (item, kv head) merge their own records, gate and store: 2 by way of
   // merge_rec, 3 as one thread-block cluster through its shared memory
   uint32_t merge; float* merge_rec;   // merge_rec: a block per CTA of a merging call, every word kNoWord between calls
+  uint32_t merge_polls;               // looks for a record before the wait has run out
   unsigned int* xch_ctr;   // != nullptr: the call ends in a cross-GPU exchange; the kernel's first thread advances its call counter
   const void* gate; uint64_t gate_col_stride, gate_head_stride;
   void* out; uint64_t out_col_stride; int act_f16;
@@ -142,6 +143,7 @@ struct F32DecodeParams {
   float scale_log2;
   float* part_o; float* part_ml;
   float* merge_rec; uint32_t* err;                                             // != nullptr: no cluster, the CTAs merge by way of it
+  unsigned int* merge_ctr; uint32_t merge_polls;                               // per (column, kv head): CTAs with their record out, units left; looks before a unit is left
   const void* gate; uint64_t gate_col_stride, gate_head_stride;                // cluster or merge_rec: gate and output
   void* out; uint64_t out_col_stride; int act_f16;
   // one token with its front in the kernel (k_new != nullptr): q unrotated, the token's own k / v row in q's type, cos / sin by value
