@@ -706,6 +706,44 @@ struct FusedFront {
 // a gathered call: the columns' row lists on the device, one list of `stride` words per column
 struct GatherLists { const uint32_t* lists; uint32_t stride; };
 
+// The plan of a call over int8 rows.  Up to 16 query rows: four warps, whose positions they share.  More: 32 rows a CTA, either by four
+// warps that convert for themselves (two CTAs an SM), or by eight that share one conversion of a tile (head_dim 64: two CTAs an SM, otherwise
+// one), or 64 rows by eight where those fill the chip.
+struct Q8Plan { uint32_t rgw, ns, live, cluster; bool cv; double time; };
+static Q8Plan q8_plan_of(const pa_ctx* ctx, uint32_t rows, uint32_t n_rows, uint32_t n_cols, uint32_t rgw, bool cv) {
+  const uint32_t hd = ctx->cfg.head_dim, sms = (uint32_t)ctx->sm_count, per_sm = cv && hd >= 128 ? 1u : 2u;
+  const uint32_t ctas = ceil_div(rows, 8 * rgw) * ctx->cfg.n_kv_heads, tiles = ceil_div(n_rows, 64);
+  Q8Plan p{rgw, 0, 0, 0, cv, 0.0};
+  p.ns = ctx->cfg.splits ? ctx->cfg.splits : std::max(1u, per_sm * sms / ctas);
+  p.ns = std::min(std::min(p.ns, plan_cap(tiles)), ctx->max_splits);
+  p.ns = (uint32_t)std::max<size_t>(1, std::min<size_t>(p.ns, ctx->pf_slots / ((size_t)n_cols * ctx->cfg.n_heads)));
+  const uint32_t tps = ceil_div(tiles, p.ns);
+  p.live = ceil_div(tiles, tps);
+  if (p.live > 1 && p.ns <= (uint32_t)kMaxCluster) for (p.cluster = p.ns; p.cluster & (p.cluster - 1); ++p.cluster) {}
+  // Its time, in units of a tile for a pair of four-warp CTAs (8.1 us at head_dim 256): waves x tiles a CTA.  Clusters don't fill the chip (one
+  // CTA per SM: 12 of eight, 32 of four, 70 of two are resident; CTAs of a cluster without a tile leave at once); what is left of a wave
+  // for the SMs' first places takes `part` of one; rows of a prompt into an empty cache are half as long on average and pack.
+  const double resident = per_sm * (p.cluster == 8 ? sms / 12 * 8.0 / p.live : p.cluster == 4 ? sms * 2 / 9 : p.cluster == 2 ? sms * 10 / 21 : sms);
+  const double waves = (p.cluster ? ctas : (double)ctas * p.live) / resident, whole = floor(waves), mean = 1.0 - 0.5 * n_cols / n_rows;
+  const double tile = !cv ? 1.0 : hd >= 128 ? (rgw == 8 ? 0.955 : 0.55) : (rgw == 8 ? 1.7 : 0.78);
+  const double lone = !cv ? 0.65 : hd >= 128 ? 1.0 : 0.7, part = !cv ? 0.65 : hd >= 128 ? 1.0 : 1.5;
+  const double turns = waves <= 0.5 ? lone : waves <= 1.0 ? 1.0
+                     : p.ns > 1 || mean >= 0.9 ? whole + (waves == whole ? 0.0 : waves - whole <= 0.5 ? part : 1.0) : waves * mean + (cv ? 0.5 : 0.44);
+  // (in one wave the eight warps begin a tile's time earlier than the four)
+  p.time = turns * tile * tps + (cv && waves <= 1.0 ? 0.0 : 1.0);
+  return p;
+}
+// Which form: the one with the lesser estimate.  Against either form alone, 496 calls of 17 to 8192 query rows over 0 to 40000 older rows (16 / 2
+// and 24 / 4 heads x 256, 16 / 8 x 128 and 64): none more than 2 % slower than four warps, and 14 more than 5 % slower than
+// eight.  Eight warps alone had taken 937 us where four take 460 (32 columns of 24 / 4 x 256 behind 40000 rows: 24 clusters that do not fit at once), four
+// alone 69 for 44 (150 columns of 16 / 2 x 256 behind 300) and 350 for 322 (two layers of 777 of 24 / 4 x 256 into an empty cache).
+static Q8Plan q8_plan(const pa_ctx* ctx, uint32_t rows, uint32_t n_rows, uint32_t n_cols) {
+  if (rows <= 16) return q8_plan_of(ctx, rows, n_rows, n_cols, rows <= 8 ? 1 : 2, false);
+  const uint32_t rgw = ceil_div(rows, 64) * ctx->cfg.n_kv_heads >= (uint32_t)ctx->sm_count ? 8 : 4;
+  const Q8Plan four = q8_plan_of(ctx, rows, n_rows, n_cols, 4, false), eight = q8_plan_of(ctx, rows, n_rows, n_cols, rgw, true);
+  return eight.time <= four.time ? eight : four;
+}
+
 // Decode / blocks / prompts over an int8 cache, one launch per item.  Splits fill two CTAs per SM; a call whose rows alone
 // do that is not split, and then writes its outputs itself.  early: the kernel before this one is the call's own front.
 static int decode_q8_item(pa_layer* L, const pa_item& it, const void* q, int q_dtype, uint64_t qcs, uint64_t qhs, const void* gate, uint64_t gcs,
@@ -728,23 +766,16 @@ static int decode_q8_item(pa_layer* L, const pa_item& it, const void* q, int q_d
   p.q_vec = q_dtype == PA_F32 && !(qcs & 3) && !(qhs & 3) && !((uintptr_t)q & 15);
   p.k = (const int8_t*)L->k_alt; p.v = (const int8_t*)L->v_alt; p.ks = L->k_scale; p.vs = L->v_scale;
   p.kv_dim = ctx->kv_dim; p.G = ctx->G; p.n_heads = nH; p.max_seq = L->max_seq;
-  // more than 16 query rows: eight warps that share one conversion of a tile; 64 rows a CTA where those fill the chip, else 32, with
-  // two warps on each eight rows
-  const bool cv = rows > 16;
-  p.rgw = rows <= 8 ? 1 : rows <= 16 ? 2 : ceil_div(rows, 64) * ctx->cfg.n_kv_heads >= (uint32_t)ctx->sm_count ? 8 : 4;
+  const Q8Plan pl = q8_plan(ctx, rows, n_rows, it.n_cols);
+  p.rgw = pl.rgw; p.cv = pl.cv ? 1u : 0u;
   p.seq = it.seq; p.lim0 = (int32_t)(it.pos + 1 - L->origin); p.n_rows = n_rows; p.n_cols = it.n_cols;
   p.early = early ? 1u : 0u;
   p.scale_log2 = (float)(1.4426950408889634 / sqrt((double)hd));
   p.part_o = ctx->part_o; p.part_ml = ctx->part_ml;
   p.gate = gate; p.gate_col_stride = gcs; p.gate_head_stride = ghs; p.out = out; p.out_col_stride = ocs; p.act_f16 = ctx->cfg.act_dtype == PA_F16;
-  const uint32_t ctas = ceil_div(rows, 8 * p.rgw) * ctx->cfg.n_kv_heads, tiles = ceil_div(n_rows, 64);
-  uint32_t ns = ctx->cfg.splits ? ctx->cfg.splits : std::max(1u, (cv && hd >= 128 ? 1u : 2u) * (uint32_t)ctx->sm_count / ctas);   // CTAs per SM
-  ns = std::min(std::min(ns, plan_cap(tiles)), ctx->max_splits);
-  ns = (uint32_t)std::max<size_t>(1, std::min<size_t>(ns, ctx->pf_slots / ((size_t)it.n_cols * nH)));
-  p.n_splits = ns;
-  const uint32_t live = ceil_div(tiles, ceil_div(tiles, ns));
   // two to eight splits: a cluster merges them itself (with core_only too: there is no second kernel to leave out)
-  if (live > 1 && ns <= (uint32_t)kMaxCluster) for (p.cluster = ns; p.cluster & (p.cluster - 1); ++p.cluster) {}
+  const uint32_t ns = pl.ns, live = pl.live;
+  p.n_splits = ns; p.cluster = pl.cluster;
   timing_mark(ctx, st, 0);
   CU_TRY(ctx, launch_q8(p, hd, ctx->cfg.n_kv_heads, ctx->device, st));
   timing_mark(ctx, st, 1);

@@ -168,6 +168,7 @@ struct Q8Params {
   const int8_t* k; const int8_t* v; const float* ks; const float* vs;
   uint32_t kv_dim, G, n_heads, max_seq, n_splits, rgw;                      // rgw: 8-row groups per CTA
   uint32_t cluster;                                                         // CTAs of a cluster that merges a row tile's splits (0: records)
+  uint32_t cv;                                                              // eight warps that share one conversion of a tile
   uint32_t seq; int32_t lim0; uint32_t n_rows, n_cols;                      // rows column 0 sees (before clamping), rows the last column sees
   uint32_t early;                                                           // 1: rows older than the call's own may be fetched before the predecessor ends
   float scale_log2;

@@ -506,9 +506,9 @@ static cudaError_t launch_q8_t(const Q8Params& p, dim3 grid, int dev, cudaStream
 cudaError_t launch_q8(const Q8Params& p, uint32_t hd, uint32_t n_kv, int dev, cudaStream_t st) {
   const dim3 grid(p.cluster ? p.cluster : p.n_splits, n_kv, (p.n_cols * p.G + 8 * p.rgw - 1) / (8 * p.rgw));
   switch (hd) {
-    case 256: return p.rgw >= 4 ? launch_q8_t<256, true>(p, grid, dev, st) : launch_q8_t<256, false>(p, grid, dev, st);
-    case 128: return p.rgw >= 4 ? launch_q8_t<128, true>(p, grid, dev, st) : launch_q8_t<128, false>(p, grid, dev, st);
-    case 64: return p.rgw >= 4 ? launch_q8_t<64, true>(p, grid, dev, st) : launch_q8_t<64, false>(p, grid, dev, st);
+    case 256: return p.cv ? launch_q8_t<256, true>(p, grid, dev, st) : launch_q8_t<256, false>(p, grid, dev, st);
+    case 128: return p.cv ? launch_q8_t<128, true>(p, grid, dev, st) : launch_q8_t<128, false>(p, grid, dev, st);
+    case 64: return p.cv ? launch_q8_t<64, true>(p, grid, dev, st) : launch_q8_t<64, false>(p, grid, dev, st);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -436,3 +436,20 @@ def test_merged_records_of_many_calls_keep_their_bits(fmt):
     outs = [eng.decode(0, [(0, n - 1, 1)], q) for _ in range(60) for n in ctx]
     eng.sync()
     assert torch.isfinite(torch.stack(outs)).all() and all(torch.equal(o, outs[i % len(ctx)]) for i, o in enumerate(outs))
+
+
+@pytest.mark.parametrize("nH,nKV,hd,pos,n_cols", [(24, 4, 256, 1000, 24), (24, 4, 256, 1000, 8), (24, 4, 256, 4096, 48), (16, 2, 256, 300, 48), (16, 2, 256, 300, 150), (16, 2, 256, 9000, 17),
+                                                 (16, 8, 128, 2048, 48), (16, 8, 128, 1000, 64), (16, 8, 128, 4096, 200), (16, 8, 64, 300, 150), (16, 8, 64, 300, 200), (24, 4, 256, 0, 400)])
+def test_int8_blocks_in_either_form(nH, nKV, hd, pos, n_cols):
+    # more than 16 query rows: by four warps that convert for themselves and by eight that share a conversion, split in clusters, by records and not at all
+    rows = pos + n_cols
+    eng = _engine("q8", nH, nKV, hd, rows, max_cols=rows)
+    g = np.random.default_rng(23)
+    K, V, q = (g.standard_normal(s).astype(np.float32) for s in ((rows, nKV * hd), (rows, nKV * hd), (n_cols, nH * hd)))
+    eng.kv_append(0, 0, 0, util.torch_dev(K), util.torch_dev(V))
+    dq = util.torch_dev(q)
+    outs = [eng.prefill(0, 0, pos, dq).cpu().numpy() for _ in range(2)]
+    eng.sync()
+    Kh, Vh, _ = _held(eng, "q8", 0, rows)
+    assert np.array_equal(*outs)
+    assert util.errs(outs[0], po.attn_f64_kv32(q, Kh, Vh, nH, nKV, hd, pos, n_cols, None))[1] < util.REF_REL
