@@ -37,14 +37,13 @@ struct VfSmem {
   static constexpr int KV_BYTES = HD * 128;         // [HD/64][64 rows][128 B]
   // tensor memory columns: the first TQC 64-dim chunks of Q (32 columns of f16 pairs each) | S tiles (64 each; P
   // overwrites the first 32 of its S) | O (HD).  HD 256: 64 + 192 + 256 = 512.
-  static constexpr int TQC = HD == 64 ? 1 : HD / 128;
-  static constexpr int QS_BYTES = (HD / 64 - TQC > 0 ? HD / 64 - TQC : 1) * 128 * 128;   // the chunks of Q not in tensor memory: [chunk][128 rows][128 B]
-  static constexpr int X_BYTES = 0;
+  static constexpr int TQC = HD / 128;
+  static constexpr int QS_BYTES = (HD / 64 - TQC) * 128 * 128;   // the chunks of Q not in tensor memory: [chunk][128 rows][128 B]
   // softmax warpgroups, on alternate KV tiles: with one group the softmax of a tile, not the arrival of the tile from HBM, set
   // the pace of the seven-tile loop
   static constexpr int NGRP = 2;
   static constexpr int THREADS = 128 + 128 * NGRP;
-  static constexpr int OFF_K = 0, OFF_V = NK * KV_BYTES, OFF_Q = (NK + NV) * KV_BYTES, OFF_X = OFF_Q + QS_BYTES, OFF_BAR = OFF_X + X_BYTES;
+  static constexpr int OFF_K = 0, OFF_V = NK * KV_BYTES, OFF_Q = (NK + NV) * KV_BYTES, OFF_BAR = OFF_Q + QS_BYTES;
   static constexpr int OFF_ROW = OFF_BAR + 256;      // per-row hand-over between the softmax groups: the reference maximum, m[128]
   static constexpr int TOTAL = 1024 + OFF_ROW + 128 * 4;
   static_assert(TOTAL <= 227 * 1024, "shared memory of one CTA");
