@@ -1525,7 +1525,7 @@ extern "C" int pa_attn_step_host(pa_layer* const* layers, uint32_t n_layers, uin
   // (a gate inside q has to come with its own layer's q)
   const bool by_layer = !gate_in_q || (gate_layer_stride == q_layer_stride && (uint64_t)(gh - qh) < q_layer_stride * es);
   // Dividing the copies costs eight more calls and two kernel boundaries: 166 -> 169 us for 260 KB in all (10 layers, 16 / 2 heads x 256, f16),
-  // 219 -> 217 for 640 KB, 209 -> 196 for 1.7 MB.
+  // 219 -> 217 for 640 KB, 209 -> 196 for 1.3 MB.
   cudaStream_t side = n_layers >= 6 && by_layer && need >= (512u << 10) ? side_stream(ctx, {q, k, v, gate, out}) : nullptr;
   const uint32_t head = side ? std::max(2u, n_layers / 5) : n_layers, tail = side ? 2u : n_layers;
   auto upload = [&](uint8_t* dst, const void* src, uint64_t layer_stride, uint32_t l0, uint32_t l1, cudaStream_t on) {

@@ -16,8 +16,8 @@ __device__ __forceinline__ void fma4(float4& acc, const float4& x, float w) {
 // kNoWord until its value is stored, a reader repeats its loads until no word of them does, and puts kNoWord back for the next call
 // (whose CTAs write after this call's end).  Both sides use relaxed accesses of whole 32-bit words, which land whole, and nothing else orders them: with a fence behind
 // the records, a count and a wait for it ahead of the first load, three more trips to L2 stood between a CTA's last product and its merge
-// (ten layers of a token over 32768 rows, 16 / 2 heads x 256: 200 us with them, 185 without; 16 over 4099 rows, 24 / 4 x 256, host
-// buffers: 235 and 209).  A value that has kNoWord's bits (a NaN no instruction here produces) is stored as the ordinary NaN.
+// (ten layers of a token over 32768 rows, 16 / 2 heads x 256, head-norm: 193.5 us with them, 185 without; 16 over 4099 rows, 24 / 4 x 256, host
+// buffers: 238 and 209).  A value that has kNoWord's bits (a NaN no instruction here produces) is stored as the ordinary NaN.
 constexpr uint32_t kNoWord = 0xffffffffu;
 __device__ __forceinline__ uint32_t word_for(float x) { return __float_as_uint(x) == kNoWord ? 0x7fffffffu : __float_as_uint(x); }
 __device__ __forceinline__ uint4 ld_words4(const float* p) {

@@ -22,14 +22,14 @@
 // O is rescaled only when a row's running maximum has grown by more than 2^8 since its last rescale (weights stay below
 // 2^8, exact in f32 sums and safe in f16); the rescale waits for the previous P V to retire and rewrites the row in TMEM.
 //
-// What bounds it: the tensor cores' issue.  An instruction of 128 x N x 16 takes no less than 67 cycles, so scores in
-// tiles of 64 keys (N = 64, 32 cycles of work) ran at under half of the rate: 1394 cycles per 64 keys of head_dim 256 for both
-// products against 1024 with N = 128, measured with nothing else running.
+// What bounds it: at head_dim 256 the chip's power, under whose limit it runs at 1.39 GHz, and the tensor cores, whose 2048 cycles a tile
+// takes 2220 for; at 128 the exponentials (1024 cycles a tile of the four units) and the wait above.  Why tiles of 128 keys: an instruction of
+// 128 x N x 16 takes no less than 67 cycles, so scores in tiles of 64 keys (N = 64, 32 cycles of work) ran at under half of the
+// rate: 1394 cycles per 64 keys of head_dim 256 for both products against 1024 with N = 128, measured with nothing else running.
 //
 // Measured (whole passes, power-capped; tiles of 64 keys with two groups of four softmax warps on alternate tiles and gate rows fetched
-// by the lanes before): 4 layers of 8192 columns of 24 heads x 256 3698 -> 3265 us, 8 layers of 2999 x 16 x 128 676 -> 572 (36 of it
-// sixteen softmax warps instead of eight, 27 the rotation kernel's), 8 layers of 203 columns of 24 x 256 behind 9001 rows 602 -> 554.
-// A tile of head_dim 256 takes 2220 cycles for the tensor cores' 2048 and the chip runs at 1.39 GHz under its power limit.
+// by the lanes before): 4 layers of 8192 columns of 24 heads x 256 3675 -> 3317 us, 8 layers of 2999 x 16 x 128 676 -> 594 (36 of it
+// sixteen softmax warps instead of eight, 27 the rotation kernel's), 8 layers of 203 columns of 24 x 256 behind 9001 rows 595 -> 549.
 //
 // Stands in for attn_flash_tile + attn_combine_tile + sigmoid_mul_mc of pooled (engine/wgsl/attn_tile.js:108-193,
 // engine/wgsl/qwen35.js:877-887); there the pass is 16 columns wide and split over the sequence, here a pass takes
@@ -160,7 +160,7 @@ pa_prefill_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       }
       if (!SPLIT && p.gate_tma) tma_prefetch_3d(&tm_g, 0, (int)c0, (int)(h * (p.gate_head_stride / 64)));
       if (!SPLIT && p.q_tma) {
-        // the query rows of the CTA that takes this one's place, as far as no kernel wrote them just now, into L2: 128-byte pieces of
+        // the query rows of the CTA that takes this one's place, into L2 (those a kernel wrote just now are there): 128-byte pieces of
         // rows 12 KB and more apart, for which it would wait for HBM at its start.  (The gate's above likewise, for the end.)  8 layers of 2999 columns of 16
         // heads x 128 577 -> 572 us, 4 of 8192 of 24 x 256 3310 -> 3265.
         const uint32_t next = blockIdx.y * gridDim.x + blockIdx.x + p.sms;

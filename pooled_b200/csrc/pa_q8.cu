@@ -20,10 +20,11 @@
 // P in registers from one product to the next; no barrier but the ring's.  A CTA is four or eight warps over a ring of 64-position
 // tiles (cp.async): with few query rows the warps share the positions of a tile and merge their (o, m, l)
 // at the end, with many each has rows of its own and all positions.  Eight warps fit an SM.
-// What bounds it: the latency of two warps per scheduler.  A warp executes some 1400 instructions per 16 positions and eight rows
+// What bounds it: the latency of two warps per scheduler.  Four warps: each executes some 1400 instructions per 16 positions and eight rows
 // (loading its share of the tiles included) against 64 MMAs, most of them conversions, which it makes for its eight rows alone (int8 ->
-// f16 costs a byte permute and an f16 subtraction per two values): issue slots 49 %, ALU 38 %, tensor pipe 18 % of the active cycles of
-// the prompt below; of a single token's, 30, 25 and 7 %, HBM 11 %.
+// f16 costs a byte permute and an f16 subtraction per two values): issue slots 30 %, ALU 25 %, tensor pipe 7 %, HBM 11 % of the active cycles
+// of the token below.  Eight warps that share a conversion: some 1000 instructions; issue slots 37 %, ALU 23 %, tensor pipe 19 %, shared
+// memory 48 % of those of the prompt below.
 // Measured with its front (pa_front.cu) against plain f32 loops, a CTA per column: ten layers of a token over 12345 rows (16 q / 2 kv
 // heads x 256, head-norm) 918 -> 181 us, two layers of a 777-token prompt (24 / 4 x 256) 4231 -> 322 us; distance from float64
 // no larger: 2.2e-7 against 3.1e-7 (a token over 20000 rows), 1.6e-7 against 2.0e-7 (that prompt), relative.
@@ -103,7 +104,7 @@ __device__ __forceinline__ void cp8(uint32_t dst, const void* src, bool live) {
 // grid (splits, kv heads, row tiles).  rgw row groups per CTA (of NW warps): warp w has row group w % rgw and takes the
 // 16-position steps w / rgw, w / rgw + NW / rgw, ... of a tile.
 //
-// CV, for more than 16 query rows: eight warps, and each tile is converted to f16 once for all of them instead of by every
+// CV, for more than 16 query rows where it is the faster form (q8_plan): eight warps, and each tile is converted to f16 once for all of them instead of by every
 // warp for its own eight rows, then read with ldmatrix: two layers of the 777-token prompt below 350 -> 322 us.
 // K's values go to the places the other form's lanes take them from (a score's products meet in the same order) and V's
 // stay in theirs, so both forms give the same bits for the same split plan.
