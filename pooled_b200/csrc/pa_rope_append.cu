@@ -207,7 +207,13 @@ static __device__ __noinline__ uint32_t rot_h_slow(uint32_t xw, uint32_t yw, int
 // columns of 16 + 8 heads x 128, whole calls: 639 us with one kind of load after the other, two heads at a time, 612 so.  8192
 // columns of 24 heads of which 64 dims turn take 47 us for 117 MB: 128-byte pieces of q 1 KB apart.
 // half / 8 need not divide 64: the threads past the last whole turn then only copy.
-constexpr int kRopeU = 3, kRopeC = 4;    // heads and copied vectors a thread has in flight
+// kRopeU heads and kRopeC copied vectors a thread has in flight: three and four, or, up to kRopeFew columns (one wave of two CTAs an SM),
+// one and two.  There a CTA's time is the fetch of its instructions, which the kernels between two of its launches have put out
+// of the SM's caches, and three heads' arithmetic is three times as long.  A layer call of 48 columns of 16 / 8 heads x 128: 13.5 us
+// with three and four, 12.5 with one and two (two heads one after the other's loads, as before both: 12.9); 300 columns 15.9 and 15.0, 1100 25.7
+// and 24.8, 2999 73.8 and 75.2.
+constexpr uint32_t kRopeFew = 1184;
+template <int kRopeU, int kRopeC>
 __global__ void __launch_bounds__(256, 2) pa_rope_append_vec_kernel(const RopeParams p, const uint32_t n_cols) {
   __shared__ float2 s_cs[4][128];
   const uint32_t cl = threadIdx.x >> 6, t = threadIdx.x & 63, col = min(blockIdx.x * 4 + cl, n_cols - 1), half = p.n_rot / 2, hd = p.hd;
@@ -406,7 +412,11 @@ bool rope_vec_applies(const RopeParams& p, uint32_t n_cols) {
 }
 
 cudaError_t launch_rope_append(const RopeParams& p, uint32_t n_cols, cudaStream_t st) {
-  if (rope_vec_applies(p, n_cols)) return launch_pdl(pa_rope_append_vec_kernel, dim3((n_cols + 3) / 4), dim3(256), 0, st, p, n_cols);
+  if (rope_vec_applies(p, n_cols)) {
+    const dim3 grid((n_cols + 3) / 4);
+    return n_cols <= kRopeFew ? launch_pdl(pa_rope_append_vec_kernel<1, 2>, grid, dim3(256), 0, st, p, n_cols)
+                              : launch_pdl(pa_rope_append_vec_kernel<3, 4>, grid, dim3(256), 0, st, p, n_cols);
+  }
   if (n_cols >= 16 && !p.n_items) return launch_pdl(pa_rope_append_cols_kernel, dim3(n_cols), dim3(256), 0, st, p);
   const uint32_t slots = (p.q ? p.q_heads : 0) + (p.k ? p.kv_heads : 0) + (p.v ? p.kv_heads : 0);
   return launch_pdl(pa_rope_append_kernel, dim3(n_cols, slots), dim3(128), 0, st, p);

@@ -311,3 +311,21 @@ def test_rope_append_items_equals_per_sequence_calls():
             assert np.array_equal(after[s, p - 100].cpu().numpy().view(np.uint16), util.read_cache(a, 0, s, p, 1)[0][0])
     touched = (after != before).any(dim=2).sum().item()
     assert touched <= sum(1 for _, p in seqs_pos if p >= 100)
+
+
+@pytest.mark.parametrize("nH,nKV,hd,n_rot", [(16, 8, 128, 128), (24, 4, 256, 64), (5, 1, 64, 64), (6, 3, 128, 96), (16, 2, 256, 48)])
+@pytest.mark.parametrize("n_cols", [1184, 1185, 1301])
+def test_long_chunks_rotate_as_their_pieces_do(nH, nKV, hd, n_rot, n_cols):
+    # either side of where a thread takes three heads and four vectors at a time instead of one and two: the same bits, q and cache rows
+    import torch
+    from pooled_b200 import AttnConfig, AttnEngine
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q = torch.randn((n_cols, 2 * nH * hd), device="cuda", generator=g).half(); k, v = (torch.randn((n_cols, nKV * hd), device="cuda", generator=g).half() for _ in range(2))
+    outs = []
+    for piece in (n_cols, 400):
+        eng = AttnEngine(AttnConfig(n_heads=nH, n_kv_heads=nKV, head_dim=hd, n_rot=n_rot, rope_theta=1e6, max_seq=n_cols, act_dtype=torch.float16, max_cols=n_cols))
+        o = [eng.encode_layer(0, c, q[c:c + piece], k[c:c + piece], v[c:c + piece], mode="prefill", q_head_stride=2 * hd) for c in range(0, n_cols, piece)]
+        eng.sync()
+        outs.append([eng.cache(0, w)[0].clone() for w in "kv"] + [torch.cat(o).float()])
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    assert torch.isfinite(outs[0][2]).all() and (outs[0][2] - outs[1][2]).abs().max() < 4e-3      # (chunks split their keys in other places)
